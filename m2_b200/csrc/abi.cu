@@ -12,6 +12,18 @@ int m2_set_error(int code, const char* fmt, ...) {
   return code;
 }
 
+int m2_sm_count() {
+  static std::atomic<int> cached[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev > 63) return 148;
+  int n = cached[dev].load(std::memory_order_relaxed);
+  if (n == 0) {
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) { cudaGetLastError(); return 148; }
+    cached[dev].store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
+
 extern "C" int m2_version(void) { return M2_B200_ABI_VERSION; }
 
 extern "C" const char* m2_last_error(void) { return g_err; }

@@ -7,6 +7,7 @@
 #include <stdio.h>
 #include <stdarg.h>
 #include <string.h>
+#include <atomic>
 #include "../../include/m2_b200.h"
 
 // ---- host side error plumbing -------------------------------------------------------
@@ -22,6 +23,20 @@ int m2_set_error(int code, const char* fmt, ...);   // stores a thread-local mes
 #define M2_LAUNCH_CHECK(name) \
   do { cudaError_t e_ = cudaGetLastError(); \
        if (e_ != cudaSuccess) return m2_set_error(M2_ERR_CUDA, "launch of %s failed: %s", name, cudaGetErrorString(e_)); } while (0)
+
+// Multiprocessors of the current device (asked for once per device).
+int m2_sm_count();
+
+// Allows `kern` `bytes` of dynamic shared memory, once per call site and device (the runtime call costs about as much
+// as a launch).  The byte count of one call site is a constant.
+#define M2_SMEM_ONCE(kern, bytes) \
+  do { static std::atomic<unsigned long long> done_{0}; \
+       int dev_ = 0; \
+       M2_CUDA(cudaGetDevice(&dev_)); \
+       const unsigned long long bit_ = 1ull << (dev_ & 63); \
+       if (!(done_.load(std::memory_order_relaxed) & bit_) || dev_ > 63) { \
+         M2_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(bytes))); \
+         done_.fetch_or(bit_, std::memory_order_relaxed); } } while (0)
 
 static inline bool m2_is_pow2(long long v) { return v > 0 && (v & (v - 1)) == 0; }
 static inline int m2_ilog2(long long v) { int l = 0; while ((1LL << l) < v) ++l; return l; }

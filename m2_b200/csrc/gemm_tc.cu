@@ -139,7 +139,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   uint64_t* tempty = tfull + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = tc::uniform_warp_id(), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::NSTAGES; ++s) { tc::mbar_init(full + s, 1); tc::mbar_init(empty + s, C::NACC); }
@@ -160,7 +160,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
   if (warp == 0) {
     // ------------------------------- TMA producer -------------------------------
-    if (lane == 0) {
+    if (tc::elect_one()) {
       int stage = 0; uint32_t phase = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < P.total_tiles && ok; tile += gridDim.x) {
@@ -182,17 +182,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     }
   } else if (warp >= 1 && warp <= C::NACC) {
     // ------------------------------- MMA issuers --------------------------------
-    // The issuing thread spends 100-270 cycles per K step on the barrier test and the commit besides the
-    // MMAs themselves (measured stand-alone: 4 MMAs of N = 128 per K step take 523 cycles with a satisfied
-    // mbarrier wait in the loop, 256 without; the tensor pipe alone runs them at 64 cycles each).  The
-    // two accumulators of the gated product therefore have one issuing thread each: warp 1 the gate
-    // block, warp 2 the linear block.  Both wait for the same stage and both commit to its `empty`
-    // barrier and to the accumulator buffer's `tfull` (count NACC).
-    if (lane == 0) {
+    // The two accumulators of the gated product have one issuing thread each: warp 1 the gate block, warp 2 the
+    // linear block.  Both wait for the same stage and both commit to its `empty` barrier and to the accumulator
+    // buffer's `tfull` (count NACC).
+    if (tc::elect_one()) {
       constexpr uint32_t idesc = tc::make_idesc(BM, BN, 1);
       const int chain = warp - 1;
       const uint64_t dA0 = tc::smem_desc_k_sw128(tc::smem_u32(smem + chain * (A_BYTES + C::B_BYTES)));
-      const uint64_t dB0 = dA0 + (uint64_t)(A_BYTES >> 4);
+      const uint64_t dB0 = tc::desc_advance(dA0, A_BYTES >> 4);
       int stage = 0; uint32_t phase = 0;
       int buf = 0; uint32_t bphase = 0;
       bool ok = true;
@@ -203,12 +200,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         for (int ks = 0; ks < P.ksteps; ++ks) {
           if (!tc::mbar_wait(full + stage, phase, abort_flag, tc::ST_TIMEOUT_TMA)) { ok = false; break; }
           tc::tc_fence_after();
-          const uint64_t off = (uint64_t)(stage * (C::STAGE_BYTES >> 4));
-          const uint64_t dA = dA0 + off, dB = dB0 + off;
+          const uint32_t off = (uint32_t)(stage * (C::STAGE_BYTES >> 4));
+          const uint64_t dA = tc::desc_advance(dA0, off), dB = tc::desc_advance(dB0, off);
 #pragma unroll
           for (int kk = 0; kk < BK / 16; ++kk) {
             // 16 bf16 along K = 32 bytes = 2 units of the descriptor's 16-byte address field
-            tc::mma_ss(acc, dA + 2 * kk, dB + 2 * kk, idesc, (ks | kk) ? 1u : 0u);
+            tc::mma_ss(acc, tc::desc_advance(dA, 2 * kk), tc::desc_advance(dB, 2 * kk), idesc, (ks | kk) ? 1u : 0u);
           }
           tc::mma_commit(empty + stage);        // stage reusable once these MMAs have read it
           if (++stage == C::NSTAGES) { stage = 0; phase ^= 1; }
@@ -334,7 +331,7 @@ glu_res_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   uint64_t* tempty = tfull + 2;              // [2]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + NBARS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = tc::uniform_warp_id(), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < NSTB; ++s) { tc::mbar_init(b_full + s, 1); tc::mbar_init(b_empty + s, 2); }
@@ -367,7 +364,7 @@ glu_res_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
   if (warp == 0) {
     // ------------------------------- TMA producer -------------------------------
-    if (lane == 0) {
+    if (tc::elect_one()) {
       int stage = 0; uint32_t phase = 0;
       int epoch = -1, prev_pair = -1;
       bool ok = true;
@@ -400,7 +397,7 @@ glu_res_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     // ------------------------------- MMA issuers: warp 1 gate, warp 2 linear ----------------------
     // Each thread issues every tile's MMAs of its accumulator in order, so its commit to `a_empty` after
     // the last tile that reads the old x covers all of its earlier MMAs as well.
-    if (lane == 0) {
+    if (tc::elect_one()) {
       constexpr uint32_t idesc = tc::make_idesc(BM, BN, 1);
       const int chain = warp - 1;
       const uint64_t dA0 = tc::smem_desc_k_sw128(tc::smem_u32(smem + chain * MAX_KS * A_BYTES));
@@ -420,9 +417,9 @@ glu_res_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           for (int ks = 0; ks < P.ksteps; ++ks) {
             if (!tc::mbar_wait(b_full + stage, phase, abort_flag, tc::ST_TIMEOUT_TMA)) { ok = false; break; }
             tc::tc_fence_after();
-            const uint64_t dA = dA0 + (uint64_t)(ks * (A_BYTES >> 4)), dB = dB0 + (uint64_t)(stage * (B_STAGE >> 4));
+            const uint64_t dA = tc::desc_advance(dA0, ks * (A_BYTES >> 4)), dB = tc::desc_advance(dB0, stage * (B_STAGE >> 4));
 #pragma unroll
-            for (int kk = 0; kk < BK / 16; ++kk) tc::mma_ss(acc, dA + 2 * kk, dB + 2 * kk, idesc, (ks | kk) ? 1u : 0u);
+            for (int kk = 0; kk < BK / 16; ++kk) tc::mma_ss(acc, tc::desc_advance(dA, 2 * kk), tc::desc_advance(dB, 2 * kk), idesc, (ks | kk) ? 1u : 0u);
             tc::mma_commit(b_empty + stage);
             if (release_x) tc::mma_commit(a_empty + ks);
             if (++stage == NSTB) { stage = 0; phase ^= 1; }
@@ -470,21 +467,12 @@ glu_res_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 }
 
 
-static int sm_count() {
-  static int cached[64] = {0};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) dev = 0;
-  if (!cached[dev]) cudaDeviceGetAttribute(&cached[dev], cudaDevAttrMultiProcessorCount, dev);
-  return cached[dev] > 0 ? cached[dev] : 148;
-}
-
 template <int BN, bool GLU>
 static int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const Params& P, cudaStream_t st) {
   using C = Cfg<BN, GLU>;
   auto kern = gemm_tc_kernel<BN, GLU>;
-  M2_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
-  int grid = P.total_tiles < sm_count() ? P.total_tiles : sm_count();
+  M2_SMEM_ONCE(kern, C::SMEM);
+  int grid = P.total_tiles < m2_sm_count() ? P.total_tiles : m2_sm_count();
   kern<<<grid, THREADS, C::SMEM, st>>>(tmA, tmB, P);
   M2_LAUNCH_CHECK("gemm_tc_kernel");
   return M2_OK;
@@ -555,12 +543,12 @@ int glu_tc_launch(const m2_glu_args* a, cudaStream_t st) {
     // column tiles per unit: about 6 units per SM, so that the contiguous ranges balance
     const long long pairs = (long long)P.ntm * R.nb_half;
     int gs = R.ntn;
-    while (gs > 1 && pairs * ((R.ntn + gs - 1) / gs) < 6LL * sm_count()) gs = (gs + 1) / 2;
+    while (gs > 1 && pairs * ((R.ntn + gs - 1) / gs) < 6LL * m2_sm_count()) gs = (gs + 1) / 2;
     R.gs = gs; R.ngroups = (R.ntn + gs - 1) / gs;
     R.total_units = (int)(pairs * R.ngroups);
     R.wide_out = P.wide_out; R.out = a->h; R.ldo = a->ldh;
-    M2_CUDA(cudaFuncSetAttribute(glu_res_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, res::SMEM));
-    const int grid = R.total_units < sm_count() ? R.total_units : sm_count();
+    M2_SMEM_ONCE(glu_res_kernel, res::SMEM);
+    const int grid = R.total_units < m2_sm_count() ? R.total_units : m2_sm_count();
     glu_res_kernel<<<grid, THREADS, res::SMEM, st>>>(tmA, tmB, R);
     M2_LAUNCH_CHECK("glu_res_kernel");
     return M2_OK;

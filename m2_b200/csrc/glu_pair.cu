@@ -58,7 +58,7 @@ glu_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   uint64_t* tempty = tfull + 2;              // [2] leader's: both CTAs' epilogues have drained the buffer
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + NBARS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = tc::uniform_warp_id(), lane = threadIdx.x & 31;
   const uint32_t rank = tc::cluster_ctarank();
   const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
 
@@ -94,7 +94,7 @@ glu_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 
   if (warp == 0) {
     // ------------------------------- TMA producer (both CTAs) -------------------------------
-    if (lane == 0) {
+    if (tc::elect_one()) {
       int stage = 0; uint32_t phase = 0;
       int epoch = -1, prev_xp = -1;
       bool ok = true;
@@ -129,7 +129,7 @@ glu_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     // ------------------------------- MMA issuers (leader CTA): warp 1 gate, warp 2 linear -------------------------------
     // Each thread issues every tile's MMAs of its accumulator in order, so its commit to `a_empty` after the last
     // tile that reads the old x covers all of its earlier MMAs as well.
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && tc::elect_one()) {
       constexpr uint32_t idesc = tc::make_idesc(2 * BM, BN, 1);
       const int chain = warp - 1;
       const uint64_t dA0 = tc::smem_desc_k_sw128(tc::smem_u32(smem + chain * MAX_KS * A_BYTES));
@@ -149,9 +149,9 @@ glu_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
           for (int ks = 0; ks < P.ksteps; ++ks) {
             if (!tc::mbar_wait(b_full + stage, phase, abort_flag, tc::ST_TIMEOUT_TMA)) { ok = false; break; }
             tc::tc_fence_after();
-            const uint64_t dA = dA0 + (uint64_t)(ks * (A_BYTES >> 4)), dB = dB0 + (uint64_t)(stage * (B_STAGE >> 4));
+            const uint64_t dA = tc::desc_advance(dA0, ks * (A_BYTES >> 4)), dB = tc::desc_advance(dB0, stage * (B_STAGE >> 4));
 #pragma unroll
-            for (int kk = 0; kk < BK / 16; ++kk) tc::mma_ss2(acc, dA + 2 * kk, dB + 2 * kk, idesc, (ks | kk) ? 1u : 0u);
+            for (int kk = 0; kk < BK / 16; ++kk) tc::mma_ss2(acc, tc::desc_advance(dA, 2 * kk), tc::desc_advance(dB, 2 * kk), idesc, (ks | kk) ? 1u : 0u);
             tc::mma_commit2_mc(b_empty + stage, 3);
             if (release_x) tc::mma_commit2_mc(a_empty + ks, 3);
             if (++stage == NSTB) { stage = 0; phase ^= 1; }

@@ -79,7 +79,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   uint64_t* tempty = tfull + 2;           // [2]   leader's: both CTAs' epilogues have drained the accumulator
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + NBARS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = tc::uniform_warp_id(), lane = threadIdx.x & 31;
   const uint32_t rank = tc::cluster_ctarank();          // 0 = leader of the pair
   const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
 
@@ -115,7 +115,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
 
   if (warp == 0) {
     // ------------------------------- TMA producer (both CTAs) -------------------------------
-    if (lane == 0) {
+    if (tc::elect_one()) {
       int stage = 0; uint32_t phase = 0;
       bool ok = true;
       for (int tile = pair; tile < P.total_tiles && ok; tile += npairs) {
@@ -147,13 +147,13 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     }
   } else if (warp == 1) {
     // ------------------------------- MMA issue (leader CTA only) -------------------------------
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && tc::elect_one()) {
       const uint32_t idesc = P.idesc;
       // M-side operand: K-major rows of 128 bytes, or (TIMEIN) MN-major: 64-token chunks 8 KB apart, 8-K groups 1 KB apart
       const uint64_t dA0 = MODE == TIMEIN ? tc::smem_desc_sw128(tc::smem_u32(smem), A_BYTES / 2, 1024)
                                           : tc::smem_desc_k_sw128(tc::smem_u32(smem));
       const uint64_t dB0 = tc::smem_desc_k_sw128(tc::smem_u32(smem + A_BYTES));
-      constexpr uint64_t a_step = MODE == TIMEIN ? (16 * 128) >> 4 : 2;      // 16 K rows of 128 bytes, or 32 bytes along a row
+      constexpr uint32_t a_step = MODE == TIMEIN ? (16 * 128) >> 4 : 2;      // 16 K rows of 128 bytes, or 32 bytes along a row
       int stage = 0; uint32_t phase = 0;
       int buf = 0; uint32_t bphase = 0;
       bool ok = true;
@@ -164,10 +164,10 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         for (int ks = 0; ks < P.ksteps; ++ks) {
           if (!tc::mbar_wait(full + stage, phase, abort_flag, tc::ST_TIMEOUT_TMA)) { ok = false; break; }
           tc::tc_fence_after();
-          const uint64_t off = (uint64_t)(stage * (STAGE >> 4));
+          const uint32_t off = (uint32_t)(stage * (STAGE >> 4));
 #pragma unroll
           for (int kk = 0; kk < BK / 16; ++kk)
-            tc::mma_ss2(acc, dA0 + off + a_step * kk, dB0 + off + 2 * kk, idesc, (ks | kk) ? 1u : 0u);
+            tc::mma_ss2(acc, tc::desc_advance(dA0, off + a_step * kk), tc::desc_advance(dB0, off + 2 * kk), idesc, (ks | kk) ? 1u : 0u);
           tc::mma_commit2_mc(empty + stage, 3);        // both CTAs' stage is free once these MMAs have read it
           if (++stage == NST) { stage = 0; phase ^= 1; }
         }
@@ -372,8 +372,7 @@ static int max_pairs(const void* kern) {
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) dev = 0;
   if (!cached[dev]) {
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int sms = m2_sm_count();
     int n = 0;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * (sms / 2));
@@ -392,7 +391,7 @@ static int max_pairs(const void* kern) {
 template <int MODE>
 static int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const Params& P, cudaStream_t st) {
   auto kern = linear_pair_kernel<MODE>;
-  M2_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
+  M2_SMEM_ONCE(kern, SMEM);
   const int mp = max_pairs(reinterpret_cast<const void*>(kern));
   const int pairs = P.total_tiles < mp ? P.total_tiles : mp;
   kern<<<2 * pairs, THREADS, SMEM, st>>>(tmA, tmB, P);
