@@ -26,7 +26,7 @@
 extern "C" {
 #endif
 
-#define M2_B200_ABI_VERSION 2
+#define M2_B200_ABI_VERSION 3
 
 typedef enum { M2_F32 = 0, M2_BF16 = 1, M2_F16 = 2 /* only where an entry point says so */ } m2_dtype;
 
@@ -101,19 +101,24 @@ int m2_hyena_filter(const m2_filter_args* args, void* stream);
  * m2_longconv_kind() names the kernel family used for (seq_len, act_dtype, d_model): 0 = float32
  * arithmetic on CUDA cores (any shape), 1 = tcgen05 tensor cores (bf16, 64 < seq_len <= 128,
  * d_model a multiple of 128, channel-contiguous tensors), 2 = tcgen05 tensor cores for long rows
- * (bf16, 128 < seq_len <= 32768, a multiple of 4, transform length 4096 / 16384 / 65536 for
+ * (bf16, 128 < seq_len <= 32768, transform length 4096 / 16384 / 65536 for
  * seq_len up to 2048 / 8192 / 32768; needs time-contiguous tensors, i.e. xin_st == u_st ==
- * out_st == 1; when seq_len is a multiple of 8, u is a 2-byte type and every row of xin, u and out
- * starts on a 16-byte boundary, the kernel copies its rows into shared memory asynchronously, ahead
- * of their use -- same results bit for bit, 15-35 % less time);
+ * out_st == 1; when u is a 2-byte type and every row of xin, u and out starts on a 16-byte boundary,
+ * the kernel copies its rows into shared memory asynchronously, ahead of their use -- same results bit
+ * for bit, 15-35 % less time);
  * 3 = tcgen05 Toeplitz GEMMs with the batch as the M dimension (bf16, 16 <= seq_len <= 128, a
  * multiple of 8, batch >= 64; time-contiguous tensors, the residual input as fp16 from
- * m2_time_major_f16).  m2_longconv_kind() never returns 3; m2_longconv_kind_batch() does when
- * the batch is large enough to fill the 128-row tiles.
+ * m2_time_major_f16); 4 = tcgen05 block-Toeplitz GEMMs (bf16, seq_len <= 2048, any batch; time-contiguous
+ * tensors, u as fp16 or bf16).  m2_longconv_kind() never returns 3; m2_longconv_kind_batch() does when
+ * the batch is large enough to fill the 128-row tiles.  Both answer for tensors whose rows are seq_len steps
+ * apart: kind 2 for multiples of 4 only, never 4.  m2_longconv_pick() is the choice for a caller that lays
+ * its time-contiguous rows out itself, every row on a 16-byte boundary and readable up to the next multiple of
+ * 8 steps (what lies there is never used; kinds 2 and 4 write nothing at or beyond seq_len): the fastest family
+ * at (batch, seq_len), whatever the length.
  * m2_filter_spectrum_floats() is the number of float32 the spectrum of one filter takes.
  * m2_filter_spectrum_bias() is m2_filter_spectrum() with the convolution's bias term (the
  * `+ u * bias` of fftconv_ref, bert/src/mm/hyena_utils.py:35-36; float32 (d_model), device, or
- * NULL) folded into the table: required for kind 3, whose m2_longconv_fwd call then takes
+ * NULL) folded into the table: required for kinds 3 and 4, whose m2_longconv_fwd call then takes
  * bias = NULL; rejected for the other kinds, which take the bias in m2_longconv_fwd.
  * k (device, float32): (d_model, m2_filter_row_len(seq_len)) as written by m2_hyena_filter.
  * ------------------------------------------------------------------------------------- */
@@ -122,6 +127,7 @@ size_t m2_filter_spectrum_floats(int kind, int d_model, int seq_len);
 int    m2_filter_spectrum(int kind, int d_model, int seq_len, const float* k, float* spec_out,
                           void* stream);
 int    m2_longconv_kind_batch(int batch, int seq_len, m2_dtype act_dtype, int d_model);
+int    m2_longconv_pick(int batch, int seq_len, m2_dtype act_dtype, int d_model);
 int    m2_filter_spectrum_bias(int kind, int d_model, int seq_len, const float* k, const float* bias,
                                float* spec_out, void* stream);
 
@@ -175,7 +181,7 @@ typedef struct {
   int plain;                /* != 0: HyenaFilter.forward alone -- out = conv(xin, filter 0) + bias*xin
                                with xin (b, t, c) of d_model channels: no short conv, no gates,
                                n_filters must be 1 */
-  int kind;                 /* from m2_longconv_kind() */
+  int kind;                 /* from m2_longconv_kind(), _kind_batch() or _pick() */
   m2_dtype act_dtype;       /* dtype of xin and out */
   m2_dtype u_dtype;         /* dtype of u */
   int bf16_rounding;
@@ -185,8 +191,8 @@ typedef struct {
   const float* short_w;     /* device (3*d_model, 3): short_filter.weight */
   const float* short_b;     /* device (3*d_model):    short_filter.bias */
   const float* spec[2];     /* device, from m2_filter_spectrum (filter_fn, filter_fn2) */
-  const float* bias[2];     /* device (d_model): filter_fn.bias, filter_fn2.bias (NULL for kind 3) */
-  int yu_bf16;              /* with an fp16 u (kind 3 always, kind 2 optionally): != 0 rounds the residual
+  const float* bias[2];     /* device (d_model): filter_fn.bias, filter_fn2.bias (NULL for kinds 3 and 4) */
+  int yu_bf16;              /* with an fp16 u (kind 3 always, kinds 2 and 4 optionally): != 0 rounds the residual
                                convolution to bf16 before the final add, as the reference does when the
                                layer input is bf16 (with a float32 / bf16 u this follows from u_dtype) */
 } m2_longconv_args;
@@ -285,6 +291,8 @@ typedef struct {
   int bf16_pad_cols;   /* > 0: also write columns n .. n+bf16_pad_cols of each out_bf16 row as
                           [1, 0, 0, ...] -- the constant column through which a following GEMM adds
                           its bias (a multiple of 8, at most 256) */
+  int valid_len;       /* 0, or the steps of each seq_len-row sequence that are not padding: `out` then has
+                          batch * valid_len rows, packed (a, b and the copies keep seq_len rows per sequence) */
 } m2_add_layernorm_args;
 
 int m2_add_layernorm_fwd(const m2_add_layernorm_args* args, void* stream);
@@ -312,9 +320,75 @@ typedef struct {
   void* out_bf16; long long ld_bf16; int bf16_pad_cols;
   void* out_tm_f16; long long tm_sb, tm_sc; int seq_len;
   long long vocab_rows, type_rows, pos_rows;
+  int valid_len;      /* as in m2_add_layernorm_args; input_ids, token_type_ids and position_ids are packed too */
 } m2_embed_layernorm_args;
 
 int m2_embed_layernorm_fwd(const m2_embed_layernorm_args* args, void* stream);
+
+/* ---------------------------------------------------------------------------------------
+ * Whole modules in one call (bf16): the launches of the entry points above with the buffers between them.
+ *
+ * m2_mixer_fwd: MonarchMixerSequenceMixing.forward under bf16 autocast
+ *   (bert/src/mm/monarch_mixer_sequence_mixer.py:100-154) -- in_linear, convolution, out_linear.
+ *   Activations are token rows, `pitch` (a multiple of 8, >= seq_len) rows per sequence; what the rows at and beyond
+ *   seq_len hold is never used.
+ *   x    : bf16 (batch * pitch, d_model), packed rows.
+ *   u    : fp16 (d_model, batch, pitch), channels u_stride elements apart (a multiple of 8); n_filters == 2 only.
+ *   xin, conv : workspace, bf16 (3 d_model, stride) and (d_model, stride), stride a multiple of 16 >= batch * pitch.
+ *   out  : bf16, packed rows, out_pitch = pitch or seq_len of them per sequence.
+ *   kind : 2, 3 or 4, from m2_longconv_pick(); spec and bias as m2_longconv_fwd takes them for that kind.
+ * ------------------------------------------------------------------------------------- */
+typedef struct {
+  int batch, seq_len, pitch, out_pitch, d_model, kind, n_filters, yu_bf16;
+  const void* x;
+  const void* u; long long u_stride;
+  const void* w_in; const float* b_in;       /* bf16 (3 d_model, d_model), float32 (3 d_model) */
+  const float* short_w; const float* short_b;
+  const float* spec[2]; const float* bias[2];
+  const void* w_out; const float* b_out;     /* bf16 (d_model, d_model), float32 (d_model) */
+  void* xin; void* conv; long long stride;
+  void* out;
+} m2_mixer_args;
+
+int m2_mixer_fwd(const m2_mixer_args* args, void* stream);
+
+/* BertGatedLinearUnitMLP.forward under bf16 autocast (bert/src/bert_layers.py:482-508): GLU GEMM, wo GEMM, add + LayerNorm.
+ * x bf16 (m, d_model); h, o workspace bf16 (m, inter), (m, d_model); outputs as in m2_add_layernorm_fwd: `out` float32 or
+ * NULL, out_bf16 (m, d_model) and out_tm_f16 (d_model, m / seq_len, seq_len) with channels tm_stride apart, or NULL. */
+typedef struct {
+  int m, d_model, inter, nblocks;
+  const void* x;
+  const void* wg; const void* wo; const float* wo_bias;
+  const float* ln_w; const float* ln_b; float eps;
+  void* h; void* o;
+  float* out; void* out_bf16; void* out_tm_f16; long long tm_stride;
+  int seq_len, valid_len;
+} m2_mlp_args;
+
+int m2_mlp_fwd(const m2_mlp_args* args, void* stream);
+
+/* The encoder (bert/src/bert_layers.py:186-252 embeddings, :552-813 layers) from token ids to the last layer's float32
+ * output (batch, seq_len, d_model): 1 + 6 n_layers launches.
+ *   embed : tables, ids, LayerNorm of the embeddings as m2_embed_layernorm_fwd takes them (ids packed, batch * seq_len);
+ *           its outputs and sizes are filled in here.
+ *   workspace : m2_encoder_workspace() bytes on a 256-byte boundary, pitch = seq_len rounded up to a multiple of 8. */
+typedef struct {
+  const void* w_in; const float* b_in; const float* short_w; const float* short_b;
+  const float* spec[2]; const float* bias[2];
+  const void* w_out; const float* b_out;
+  const void* wg; const void* wo; const float* wo_bias; const float* ln_w; const float* ln_b; float eps;
+} m2_encoder_layer;
+
+typedef struct {
+  int batch, seq_len, d_model, inter, nblocks, n_layers, kind, n_filters;
+  m2_embed_layernorm_args embed;
+  const m2_encoder_layer* layers;            /* host memory */
+  void* workspace;
+  float* out;
+} m2_encoder_args;
+
+long long m2_encoder_workspace(int batch, int pitch, int d_model, int inter);
+int m2_encoder_fwd(const m2_encoder_args* args, void* stream);
 
 #ifdef __cplusplus
 }

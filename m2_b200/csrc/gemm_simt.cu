@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(512)
 add_layernorm_warp_kernel(const TI* a, long long lda, const TI* b, long long ldb, const LnGather gt,
                           const float* __restrict__ w, const float* __restrict__ bias, float eps, TO* out,
                           long long ldo, __nv_bfloat16* out2, long long ld2, int m,
-                          __half* out_tm, long long tm_sb, long long tm_sc, int seq_len, int rpw, int pad2) {
+                          __half* out_tm, long long tm_sb, long long tm_sc, int seq_len, int valid, int rpw, int pad2) {
   extern __shared__ __half ln_tile[];   // [rows of the block][n] fp16, only with out_tm
   const int wib = threadIdx.x >> 5, nw = blockDim.x >> 5, lane = threadIdx.x & 31;
   constexpr int n = VI * 256;
@@ -180,6 +180,15 @@ add_layernorm_warp_kernel(const TI* a, long long lda, const TI* b, long long ldb
   const int trow = ri * nw + wib;                                   // row within the block
   const long long warp = (long long)blockIdx.x * nw * rpw + trow;   // row of the tensor
   if (warp >= m) break;
+  // rows of a sequence beyond its `valid` steps are padding: ids and `out` are packed without them, so a padding row
+  // reads the last step's ids and writes no `out`
+  long long crow = warp;
+  bool live = true;
+  if (valid < seq_len) {
+    const int b = (int)(warp / seq_len), t = (int)(warp - (long long)b * seq_len);
+    live = t < valid;
+    crow = (long long)b * valid + (live ? t : valid - 1);
+  }
   float v[VI][8];
   float sum = 0.f;
   if constexpr (sizeof(TI) == 2) {
@@ -199,9 +208,9 @@ add_layernorm_warp_kernel(const TI* a, long long lda, const TI* b, long long ldb
     }
   } else {
     bool bad = false;
-    const long long ra = gt.ids_a ? clamp_row(gt.ids_a[warp], gt.rows_a, bad) : warp;
-    const long long rb = gt.ids_b ? clamp_row(gt.ids_b[warp], gt.rows_b, bad) : (gt.b_mod > 0 ? warp % gt.b_mod : warp);
-    const long long rc = gt.ids_c ? clamp_row(gt.ids_c[warp], gt.rows_c, bad) : 0;
+    const long long ra = gt.ids_a ? clamp_row(gt.ids_a[crow], gt.rows_a, bad) : warp;
+    const long long rb = gt.ids_b ? clamp_row(gt.ids_b[crow], gt.rows_b, bad) : (gt.b_mod > 0 ? crow % gt.b_mod : warp);
+    const long long rc = gt.ids_c ? clamp_row(gt.ids_c[crow], gt.rows_c, bad) : 0;
     if (bad && lane == 0) atomicOr(&m2_dev_status_word, ST_BAD_INDEX);
     const float4* pa = reinterpret_cast<const float4*>(a + ra * lda);
     const float4* pb = b ? reinterpret_cast<const float4*>(b + rb * ldb) : nullptr;
@@ -249,14 +258,14 @@ add_layernorm_warp_kernel(const TI* a, long long lda, const TI* b, long long ldb
       __nv_bfloat162 h = __floats2bfloat162_rn(y[2 * j], y[2 * j + 1]);
       pk[j] = *reinterpret_cast<uint32_t*>(&h);
     }
-    if (out == nullptr) {
+    if (out == nullptr || !live) {
       // only the copies are wanted
     } else if (sizeof(TO) == 4) {
-      float4* po = reinterpret_cast<float4*>(reinterpret_cast<float*>(out) + (long long)warp * ldo + c0);
+      float4* po = reinterpret_cast<float4*>(reinterpret_cast<float*>(out) + crow * ldo + c0);
       po[0] = make_float4(y[0], y[1], y[2], y[3]);
       po[1] = make_float4(y[4], y[5], y[6], y[7]);
     } else {
-      *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(out) + (long long)warp * ldo + c0) =
+      *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(out) + crow * ldo + c0) =
           make_uint4(pk[0], pk[1], pk[2], pk[3]);
     }
     if (out2) *reinterpret_cast<uint4*>(out2 + (long long)warp * ld2 + c0) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
@@ -404,8 +413,9 @@ extern "C" int m2_embed_layernorm_fwd(const m2_embed_layernorm_args* e, void* st
              "m2_embed_layernorm_fwd: position table without position_ids needs seq_len");
   M2_REQUIRE(e->vocab_rows > 0 && e->type_rows > 0 && (!e->pos_table || e->pos_rows > 0), M2_ERR_ARG,
              "m2_embed_layernorm_fwd: table row counts must be positive");
-  M2_REQUIRE(!e->pos_table || e->position_ids || e->seq_len <= e->pos_rows, M2_ERR_ARG,
-             "m2_embed_layernorm_fwd: seq_len %d exceeds the position table's %lld rows", e->seq_len, e->pos_rows);
+  const int steps = e->valid_len > 0 ? e->valid_len : e->seq_len;
+  M2_REQUIRE(!e->pos_table || e->position_ids || steps <= e->pos_rows, M2_ERR_ARG,
+             "m2_embed_layernorm_fwd: seq_len %d exceeds the position table's %lld rows", steps, e->pos_rows);
   M2_REQUIRE(e->n % 256 == 0 && e->n <= 2048 && m2_aligned(e->word_table, 16) && m2_aligned(e->type_table, 16) &&
              m2_aligned(e->pos_table, 16), M2_ERR_UNSUPPORTED,
              "m2_embed_layernorm_fwd: needs hidden size a multiple of 256 up to 2048 and 16-byte aligned tables");
@@ -415,8 +425,8 @@ extern "C" int m2_embed_layernorm_fwd(const m2_embed_layernorm_args* e, void* st
   a.a = e->word_table; a.lda = e->n; a.b = e->pos_table; a.ldb = e->n;
   a.weight = e->weight; a.bias = e->bias; a.eps = e->eps;
   a.out = e->out; a.ldo = e->ldo; a.out_bf16 = e->out_bf16; a.ld_bf16 = e->ld_bf16; a.bf16_pad_cols = e->bf16_pad_cols;
-  a.out_tm_f16 = e->out_tm_f16; a.tm_sb = e->tm_sb; a.tm_sc = e->tm_sc; a.seq_len = e->seq_len;
-  const m2::LnGather g = {e->input_ids, e->pos_table ? e->position_ids : nullptr, e->pos_table && !e->position_ids ? e->seq_len : 0,
+  a.out_tm_f16 = e->out_tm_f16; a.tm_sb = e->tm_sb; a.tm_sc = e->tm_sc; a.seq_len = e->seq_len; a.valid_len = e->valid_len;
+  const m2::LnGather g = {e->input_ids, e->pos_table ? e->position_ids : nullptr, e->pos_table && !e->position_ids ? steps : 0,
                           e->type_table, e->n, e->token_type_ids, e->vocab_rows, e->pos_rows, e->type_rows};
   return add_layernorm_core(&a, g, stream);
 }
@@ -448,12 +458,17 @@ static int add_layernorm_core(const m2_add_layernorm_args* a, const m2::LnGather
     M2_REQUIRE(m2_aligned(a->out_tm_f16, 16) && a->tm_sb % 8 == 0 && a->tm_sc % 8 == 0, M2_ERR_ALIGN,
                "m2_add_layernorm_fwd: the time-major copy needs 16-byte aligned rows");
   }
+  M2_REQUIRE(a->valid_len >= 0 && (a->valid_len == 0 || (a->seq_len > 0 && a->valid_len <= a->seq_len && a->m % a->seq_len == 0)),
+             M2_ERR_ARG, "m2_add_layernorm_fwd: valid_len needs m = batch * seq_len rows and valid_len <= seq_len");
+  M2_REQUIRE(vec || a->valid_len == 0, M2_ERR_UNSUPPORTED, "m2_add_layernorm_fwd: valid_len needs n a multiple of 256 (<= 2048) and 16-byte aligned rows");
   if (vec) {
-    // with the time-major copy a block covers 16 (or 8) consecutive steps of one sequence, so a
-    // channel's run of them is one 32-byte sector
+    // with the time-major copy a block covers 8, 16 or 32 consecutive steps of one sequence: 16 steps make a channel's
+    // run of them one 32-byte sector, 32 steps two.  Few rows take short blocks all the same: 128 rows are four blocks
+    // of 32 (11 us) or 16 of 8; from two blocks per SM on the runs decide.
     int rows = 8, threads = 256, rpw = 1;
     if (a->out_tm_f16) {
-      rows = a->seq_len % 32 == 0 && a->n <= 768 ? 32 : a->seq_len % 16 == 0 ? 16 : 8;   // 32 rows: 64-byte runs per channel
+      const int sms = m2_sm_count();
+      rows = a->seq_len % 32 == 0 && a->n <= 768 && a->m >= 64 * sms ? 32 : a->seq_len % 16 == 0 && a->m >= 32 * sms ? 16 : 8;
       threads = rows >= 16 ? 512 : 256;
       rpw = rows / (threads / 32);
     }
@@ -461,11 +476,11 @@ static int add_layernorm_core(const m2_add_layernorm_args* a, const m2::LnGather
     const size_t tile = a->out_tm_f16 ? (size_t)rows * a->n * 2 : 0;
 #define M2_LNW(TO, VI) do { if (a->in_dtype == M2_F32) M2_LNW2(float, float, VI); else M2_LNW2(__nv_bfloat16, TO, VI); } while (0)
 #define M2_LNW2(TI, TO, VI) do { \
-      if (tile > 48 * 1024) M2_CUDA(cudaFuncSetAttribute(add_layernorm_warp_kernel<TI, TO, VI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile)); \
+      if (tile > 48 * 1024) M2_SMEM_ONCE((add_layernorm_warp_kernel<TI, TO, VI>), 64 * 1024); /* at most 16 x 2048 x 2 bytes */ \
       add_layernorm_warp_kernel<TI, TO, VI><<<blocks, threads, tile, st>>>( \
       (const TI*)a->a, a->lda, (const TI*)a->b, a->ldb, gather, a->weight, a->bias, a->eps, \
       (TO*)a->out, a->ldo, (__nv_bfloat16*)a->out_bf16, a->ld_bf16, a->m, \
-      (__half*)a->out_tm_f16, a->tm_sb, a->tm_sc, a->seq_len, rpw, a->bf16_pad_cols); } while (0)
+      (__half*)a->out_tm_f16, a->tm_sb, a->tm_sc, a->seq_len, a->valid_len > 0 ? a->valid_len : a->seq_len, rpw, a->bf16_pad_cols); } while (0)
 #define M2_LNW_VI(TO) switch (a->n / 256) { case 1: M2_LNW(TO, 1); break; case 2: M2_LNW(TO, 2); break; \
       case 3: M2_LNW(TO, 3); break; case 4: M2_LNW(TO, 4); break; case 5: M2_LNW(TO, 5); break; \
       case 6: M2_LNW(TO, 6); break; case 7: M2_LNW(TO, 7); break; default: M2_LNW(TO, 8); break; }

@@ -17,12 +17,17 @@ int longconv_tz_supported(int batch, int seq_len, m2_dtype act_dtype);
 size_t spectrum_kind3_floats(int D, int L);
 int spectrum_kind3_launch(int D, int L, const float* k, const float* bias, float* spec, cudaStream_t st);
 int longconv_tz_launch(const m2_longconv_args* a, cudaStream_t st);
+int longconv_bt_supported(int seq_len, m2_dtype act_dtype);
+bool longconv_bt_preferred(int batch, int seq_len, int d_model);
+size_t spectrum_kind4_floats(int D, int L);
+int spectrum_kind4_launch(int D, int L, const float* k, const float* bias, float* spec, cudaStream_t st);
+int longconv_bt_launch(const m2_longconv_args* a, cudaStream_t st);
 int time_major_f16_launch(const m2_time_major_args* a, cudaStream_t st);
 }  // namespace m2
 
 extern "C" int m2_longconv_kind(int seq_len, m2_dtype act_dtype, int d_model) {
   if (m2::longconv_tc_supported(seq_len, act_dtype, d_model)) return 1;
-  if (m2::longconv_tcl_supported(seq_len, act_dtype)) return 2;
+  if (m2::longconv_tcl_supported(seq_len, act_dtype) && seq_len % 4 == 0) return 2;
   return 0;
 }
 
@@ -31,9 +36,19 @@ extern "C" int m2_longconv_kind_batch(int batch, int seq_len, m2_dtype act_dtype
   return m2_longconv_kind(seq_len, act_dtype, d_model);
 }
 
+extern "C" int m2_longconv_pick(int batch, int seq_len, m2_dtype act_dtype, int d_model) {
+  if (act_dtype != M2_BF16 || batch <= 0 || d_model <= 0 || seq_len <= 0 || seq_len > 32768) return 0;
+  // up to 128 steps both families multiply by the same Toeplitz matrix; kind 3 walks tiles of 128 sequences whatever the
+  // batch (34 us at D = 768, L = 128, B = 8 .. 64), kind 4 tiles as narrow as the batch (20 us at 8, 27 at 32, 51 at 64)
+  if (seq_len <= 128) return batch >= 48 ? 3 : 4;
+  if (m2::longconv_bt_supported(seq_len, act_dtype) && m2::longconv_bt_preferred(batch, seq_len, d_model)) return 4;
+  return 2;
+}
+
 extern "C" size_t m2_filter_spectrum_floats(int kind, int d_model, int seq_len) {
   if (d_model <= 0 || seq_len <= 0) return 0;
   if (kind == 3) return m2::spectrum_kind3_floats(d_model, seq_len);
+  if (kind == 4) return m2::spectrum_kind4_floats(d_model, seq_len);
   if (kind == 1) return m2::spectrum_kind1_floats(d_model, seq_len);
   if (kind == 2) return m2::spectrum_kind2_floats(d_model, seq_len);
   const size_t M = (size_t)m2_filter_row_len(seq_len) / 2;
@@ -42,15 +57,17 @@ extern "C" size_t m2_filter_spectrum_floats(int kind, int d_model, int seq_len) 
 
 extern "C" int m2_filter_spectrum_bias(int kind, int d_model, int seq_len, const float* k, const float* bias,
                                        float* spec_out, void* stream) {
-  if (kind != 3) {
+  if (kind != 3 && kind != 4) {
     M2_REQUIRE(bias == nullptr, M2_ERR_ARG,
-               "m2_filter_spectrum_bias: only kind 3 folds the bias into the table; kind %d takes it in m2_longconv_fwd", kind);
+               "m2_filter_spectrum_bias: only kinds 3 and 4 fold the bias into the table; kind %d takes it in m2_longconv_fwd", kind);
     return m2_filter_spectrum(kind, d_model, seq_len, k, spec_out, stream);
   }
   M2_REQUIRE(d_model > 0 && seq_len > 0, M2_ERR_ARG, "m2_filter_spectrum_bias: sizes must be positive");
   M2_REQUIRE(k && spec_out, M2_ERR_ARG, "m2_filter_spectrum_bias: NULL pointer");
   M2_REQUIRE(m2_aligned(spec_out, 16), M2_ERR_ALIGN, "m2_filter_spectrum_bias: spec_out must be 16-byte aligned");
-  return m2::spectrum_kind3_launch(d_model, seq_len, k, bias, spec_out, static_cast<cudaStream_t>(stream));
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  return kind == 4 ? m2::spectrum_kind4_launch(d_model, seq_len, k, bias, spec_out, st)
+                   : m2::spectrum_kind3_launch(d_model, seq_len, k, bias, spec_out, st);
 }
 
 extern "C" int m2_time_major_f16(const m2_time_major_args* a, void* stream) {
@@ -72,6 +89,7 @@ extern "C" int m2_filter_spectrum(int kind, int d_model, int seq_len, const floa
              "m2_filter_spectrum: k must be 8-byte and spec_out 16-byte aligned");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (kind == 3) return m2::spectrum_kind3_launch(d_model, seq_len, k, nullptr, spec_out, st);
+  if (kind == 4) return m2::spectrum_kind4_launch(d_model, seq_len, k, nullptr, spec_out, st);
   if (kind == 0) return m2::spectrum_kind0_launch(d_model, seq_len, k, spec_out, st);
   if (kind == 1) return m2::spectrum_kind1_launch(d_model, seq_len, k, spec_out, st);
   if (kind == 2) return m2::spectrum_kind2_launch(d_model, seq_len, k, spec_out, st);
@@ -85,7 +103,7 @@ extern "C" int m2_longconv_fwd(const m2_longconv_args* a, void* stream) {
   M2_REQUIRE(a->n_filters == 1 || a->n_filters == 2, M2_ERR_ARG, "m2_longconv_fwd: n_filters must be 1 or 2");
   M2_REQUIRE(!a->plain || a->n_filters == 1, M2_ERR_ARG, "m2_longconv_fwd: plain mode takes one filter");
   if (a->batch == 0) return M2_OK;
-  const bool folded = a->kind == 3 && !a->plain;       // kind 3 has the bias inside its spectrum
+  const bool folded = (a->kind == 3 || a->kind == 4) && !a->plain;   // these have the bias inside their spectrum
   M2_REQUIRE(a->xin && a->out && (a->plain || (a->short_w && a->short_b)) && a->spec[0] && (folded || a->bias[0]), M2_ERR_ARG,
              "m2_longconv_fwd: NULL tensor pointer");
   M2_REQUIRE(a->n_filters == 1 || (a->u && a->spec[1] && (folded || a->bias[1])), M2_ERR_ARG,
@@ -100,5 +118,6 @@ extern "C" int m2_longconv_fwd(const m2_longconv_args* a, void* stream) {
   if (a->kind == 1) return m2::longconv_tc_launch(a, st);
   if (a->kind == 2) return m2::longconv_tcl_launch(a, st);
   if (a->kind == 3) return m2::longconv_tz_launch(a, st);
+  if (a->kind == 4) return m2::longconv_bt_launch(a, st);
   return m2_set_error(M2_ERR_ARG, "m2_longconv_fwd: unknown kind %d", a->kind);
 }

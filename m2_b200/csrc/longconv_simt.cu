@@ -17,6 +17,8 @@
 
 namespace m2 {
 
+constexpr size_t SIMT_SMEM_MAX = 200 * 1024;
+
 struct ConvParams {
   int B, L, D, M, lgM, CT, nf, plain;
   const void* xin; long long xsb, xst, xsc;
@@ -205,8 +207,7 @@ longconv_simt_kernel(ConvParams p) {
 template <typename TA, typename TU, bool ROUND>
 static int launch_simt(const ConvParams& p, size_t smem, cudaStream_t st) {
   auto kern = longconv_simt_kernel<TA, TU, ROUND>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return m2_set_error(M2_ERR_CUDA, "cudaFuncSetAttribute(longconv_simt): %s", cudaGetErrorString(e));
+  M2_SMEM_ONCE(kern, SIMT_SMEM_MAX);
   dim3 grid((p.D + p.CT - 1) / p.CT, p.B);
   kern<<<grid, 256, smem, st>>>(p);
   M2_LAUNCH_CHECK("longconv_simt_kernel");
@@ -308,7 +309,7 @@ longconv_simt_cluster2_kernel(ConvParams p) {
 template <typename TA, typename TU, bool ROUND>
 static int launch_cluster2(const ConvParams& p, size_t smem, cudaStream_t st) {
   auto kern = longconv_simt_cluster2_kernel<TA, TU, ROUND>;
-  M2_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  M2_SMEM_ONCE(kern, SIMT_SMEM_MAX);
   dim3 grid(2 * p.D, p.B);
   kern<<<grid, 512, smem, st>>>(p);
   M2_LAUNCH_CHECK("longconv_simt_cluster2_kernel");
@@ -317,7 +318,6 @@ static int launch_cluster2(const ConvParams& p, size_t smem, cudaStream_t st) {
 
 static int next_pow2(int v) { int r = 2; while (r < v) r <<= 1; return r; }
 
-constexpr size_t SIMT_SMEM_MAX = 200 * 1024;
 
 int longconv_simt_launch(const m2_longconv_args* a, cudaStream_t st) {
   ConvParams p;

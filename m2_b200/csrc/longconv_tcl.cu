@@ -521,7 +521,7 @@ __device__ __forceinline__ Taps load_taps(const float* sw, const float* sb, int 
   return T;
 }
 // raw words of x[t0-2 .. t0+NV-1] of a time-contiguous bf16 row (w[0] = the two steps before t0; t0 % 8 == 0 for
-// NV = 8, % 4 for NV = 4); positions outside [0, L) read as 0.  L % 4 == 0, rows 8-byte aligned (16-byte when al16).
+// NV = 8, % 4 for NV = 4); positions outside [0, L) read as 0 up to the granularity of the loads (four steps).  Rows 8-byte aligned (16-byte when al16).
 // Split from the unpacking so that a caller can issue the loads of several chunks before using any of them.
 template <int NV>
 __device__ __forceinline__ void load_raw(const __nv_bfloat16* row, int t0, int L, bool al16, uint32_t (&w)[NV / 2 + 1]) {
@@ -573,6 +573,38 @@ __device__ __forceinline__ void conv_packed(const Taps2& T, const uint32_t (&w)[
 }
 // bf16x2 -> fp16x2 (exact for values inside fp16's range)
 __device__ __forceinline__ uint32_t bf2_to_h2(uint32_t v) { return pack_h2(bf_lo(v), bf_hi(v)); }
+
+// steps of an 8-step chunk at t0 that lie below L keep their bits, the others become zero
+__device__ __forceinline__ void mask_tail(uint32_t (&h)[4], int t0, int L) {
+  if (t0 + 8 > L) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (t0 + 2 * j >= L) h[j] = 0u;
+      else if (t0 + 2 * j + 1 >= L) h[j] &= 0xffffu;
+    }
+  }
+}
+// 8 (or 4) consecutive steps of a row at t0 < L: one store, or the steps below L one by one
+__device__ __forceinline__ void store_chunk8(__nv_bfloat16* row, int t0, int L, uint4 v) {
+  if (t0 + 8 <= L) {
+    *reinterpret_cast<uint4*>(row + t0) = v;
+  } else {
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+      if (t0 + e < L) reinterpret_cast<unsigned short*>(row)[t0 + e] = (unsigned short)(w[e >> 1] >> (16 * (e & 1)));
+  }
+}
+__device__ __forceinline__ void store_chunk4(__nv_bfloat16* row, int t0, int L, uint2 v) {
+  if (t0 + 4 <= L) {
+    *reinterpret_cast<uint2*>(row + t0) = v;
+  } else {
+    const uint32_t w[2] = {v.x, v.y};
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (t0 + e < L) reinterpret_cast<unsigned short*>(row)[t0 + e] = (unsigned short)(w[e >> 1] >> (16 * (e & 1)));
+  }
+}
 
 // MMAs of one stage: 0 F1, 1 DFT_N2, 2 DFT_N3, 3 DFT_N3 on conjugated data (= inverse), 4 DFT_N2 (inverse), 5 I1.
 // A operands: MN-major (row groups `sbo` apart, K core matrices 128 bytes apart) except stage 3 (K-major rows).
@@ -638,7 +670,7 @@ __device__ __forceinline__ void issue_stage(int stage, uint32_t tm, uint32_t dat
   }
 }
 
-// ASYNC (geometries with room for it; 2-byte u, 16-byte aligned rows, L % 8 == 0):
+// ASYNC (geometries with room for it; 2-byte u, 16-byte aligned rows):
 // no thread ever waits for a global load it has just issued.  Every row this slot reads is copied into the slot's
 // shared memory with cp.async one phase ahead -- x2 while the first filter's transform runs, u during the first
 // epilogue, the next sequence's x1 / v during and after the second epilogue -- the output buffer holds bf16, and the
@@ -666,8 +698,8 @@ longconv_tcl_kernel(const Params P) {
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3 * G::SLOTS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const int slot = tid / TPS;
+  const int tid = threadIdx.x, warp = tc::uniform_warp_id();
+  const int slot = tid / TPS, slot_warp = warp % (TPS / 32);
   const int sl = tid % TPS;                      // thread index inside the slot
   const int l = sl & 127;                        // TMEM lane = row within every 128-row tile
   const int ts = sl >> 7;                        // which share of the row tiles this thread handles
@@ -713,14 +745,14 @@ longconv_tcl_kernel(const Params P) {
 #define LCL_STAGE(stage_)                                                                             \
   tc::fence_proxy_async_smem();                                                                       \
   tc::mbar_arrive(bar_ops);                                                                           \
-  if (sl == 0) {                                                                                      \
+  if (slot_warp == 0 && tc::elect_one()) {                                                            \
     if (tc::mbar_wait(bar_ops, ph_ops, abort_flag, tc::ST_TIMEOUT_MMA)) {                             \
       tc::tc_fence_after();                                                                           \
       issue_stage<G>(stage_, tm, data, hdr);                                                          \
       tc::mma_commit(bar_mma);                                                                        \
     }                                                                                                 \
-    ph_ops ^= 1;                                                                                      \
   }                                                                                                   \
+  ph_ops ^= 1;                                                                                        \
   if (!__all_sync(0xffffffffu, tc::mbar_wait(bar_mma, ph_mma, abort_flag, tc::ST_TIMEOUT_EPI))) { ok = false; break; } \
   ph_mma ^= 1;                                                                                        \
   tc::tc_fence_after();
@@ -842,6 +874,7 @@ longconv_tcl_kernel(const Params P) {
             conv_packed<8>(Tv, wv, cv);
 #pragma unroll
             for (int j = 0; j < 4; ++j) h[j] = in ? bf2_to_h2(bf2_mul(cv[j], cx[j])) : 0u;
+            mask_tail(h, t0, P.L);
             sts128(data + rg * G::SBO1 + n1 * 16, h[0], h[1], h[2], h[3]);
           }
           if (half == 0) { LCL_BARRIER() }                 // every thread is done with this half before the next lands
@@ -859,10 +892,13 @@ longconv_tcl_kernel(const Params P) {
           const int t0 = R * n1 + 8 * rg, c = t0 >> 3;
           uint4 w = make_uint4(0u, 0u, 0u, 0u);
           if (t0 < P.L) w = lds128(LR + 16 * (c ^ (n1 & 7)));
+          uint32_t h[4] = {w.x, w.y, w.z, w.w};
           if (!P.u_f16) {
-            w.x = bf2_to_h2(w.x); w.y = bf2_to_h2(w.y); w.z = bf2_to_h2(w.z); w.w = bf2_to_h2(w.w);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) h[j] = bf2_to_h2(h[j]);
           }
-          sts128(data + rg * G::SBO1 + n1 * 16, w.x, w.y, w.z, w.w);
+          mask_tail(h, t0, P.L);
+          sts128(data + rg * G::SBO1 + n1 * 16, h[0], h[1], h[2], h[3]);
         }
       } else if (ASYNC && f == 0) {
         const Taps2 Tx = taps_of(0), Tv = taps_of(2);
@@ -893,6 +929,7 @@ longconv_tcl_kernel(const Params P) {
           conv_packed<8>(Tv, wv, cv);
 #pragma unroll
           for (int j = 0; j < 4; ++j) h[j] = in ? bf2_to_h2(bf2_mul(cv[j], cx[j])) : 0u;   // steps from L on are zero padding
+          mask_tail(h, t0, P.L);
           sts128(data + rg * G::SBO1 + n1 * 16, h[0], h[1], h[2], h[3]);
         }
       } else if (ASYNC) {
@@ -903,10 +940,13 @@ longconv_tcl_kernel(const Params P) {
           const int t0 = R * n1 + 8 * rg, c = t0 >> 3;
           uint4 w = make_uint4(0u, 0u, 0u, 0u);
           if (t0 < P.L) w = lds128(RA + 16 * (c ^ (n1 & 7)));
+          uint32_t h[4] = {w.x, w.y, w.z, w.w};
           if (!P.u_f16) {
-            w.x = bf2_to_h2(w.x); w.y = bf2_to_h2(w.y); w.z = bf2_to_h2(w.z); w.w = bf2_to_h2(w.w);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) h[j] = bf2_to_h2(h[j]);
           }
-          sts128(data + rg * G::SBO1 + n1 * 16, w.x, w.y, w.z, w.w);
+          mask_tail(h, t0, P.L);
+          sts128(data + rg * G::SBO1 + n1 * 16, h[0], h[1], h[2], h[3]);
         }
       } else if (f == 0) {
         const Taps2 Tx = load_taps2(P.sw, P.sb, ch), Tv = load_taps2(P.sw, P.sb, 2 * P.D + ch);
@@ -930,13 +970,7 @@ longconv_tcl_kernel(const Params P) {
             conv_packed<8>(Tv, vr[i], cv);
 #pragma unroll
             for (int j = 0; j < 4; ++j) h[j] = bf2_to_h2(bf2_mul(cv[j], cx[j]));     // v * x1: the exact product, rounded to bf16
-            if (t0 + 8 > P.L) {                                                     // steps at and beyond L are zero padding
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                if (t0 + 2 * j >= P.L) h[j] = 0u;
-                else if (t0 + 2 * j + 1 >= P.L) h[j] &= 0xffffu;
-              }
-            }
+            mask_tail(h, t0, P.L);                                                  // steps at and beyond L are zero padding
             sts128(data + rg * G::SBO1 + n1 * 16, h[0], h[1], h[2], h[3]);
           }
         }
@@ -980,6 +1014,7 @@ longconv_tcl_kernel(const Params P) {
               if (sizeof(TU) == 4) h[j] = pack_h2(__uint_as_float(w[i][2 * j]), __uint_as_float(w[i][2 * j + 1]));
               else h[j] = P.u_f16 ? w[i][j] : pack_h2(bf_lo(w[i][j]), bf_hi(w[i][j]));
             }
+            mask_tail(h, R * n1 + 8 * rg, P.L);
             sts128(data + rg * G::SBO1 + n1 * 16, h[0], h[1], h[2], h[3]);
           }
         }
@@ -1196,7 +1231,7 @@ longconv_tcl_kernel(const Params P) {
               conv_packed<8>(T2, wx, c2);
               const uint4 y = lds128(data + 16 * c + 16 * (c >> 3));
               const uint4 o = make_uint4(bf2_mul(y.x, c2[0]), bf2_mul(y.y, c2[1]), bf2_mul(y.z, c2[2]), bf2_mul(y.w, c2[3]));
-              if (last || BIG) *reinterpret_cast<uint4*>(orow + t0) = o;
+              if (last || BIG) store_chunk8(orow, t0, P.L, o);
               else sts128(sbc, o.x, o.y, o.z, o.w);
             }
           }
@@ -1205,7 +1240,7 @@ longconv_tcl_kernel(const Params P) {
 #pragma unroll
           for (int it = 0; it < LIT; ++it) {
             const int c = it * TPS + sl, t0 = 8 * c;
-            if (t0 < P.L) *reinterpret_cast<uint4*>(orow + t0) = lds128(data + 16 * c + 16 * (c >> 3));
+            if (t0 < P.L) store_chunk8(orow, t0, P.L, lds128(data + 16 * c + 16 * (c >> 3)));
           }
         }
         if (XP && !last) cp_async_wait<0>();       // u has had the whole epilogue to arrive
@@ -1250,7 +1285,7 @@ longconv_tcl_kernel(const Params P) {
               f2_unpack(f2_mul(f2_pack(y.z, y.w), gain2), a2, a3);
               o[0] = bf2_mul(pack_bf2(a0, a1), c2[0]);                  // (conv + bias term) cast to bf16, then the gate
               o[1] = bf2_mul(pack_bf2(a2, a3), c2[1]);
-              *reinterpret_cast<uint2*>(orow + t0) = make_uint2(o[0], o[1]);
+              store_chunk4(orow, t0, P.L, make_uint2(o[0], o[1]));
             }
           }
         }
@@ -1275,9 +1310,9 @@ longconv_tcl_kernel(const Params P) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j) yv[j] = bf16r(yv[j]);
               }
-              *reinterpret_cast<uint2*>(orow + t0) =
-                  make_uint2(pack_bf2(bf_lo(prev[i].x) + yv[0], bf_hi(prev[i].x) + yv[1]),
-                             pack_bf2(bf_lo(prev[i].y) + yv[2], bf_hi(prev[i].y) + yv[3]));
+              store_chunk4(orow, t0, P.L,
+                           make_uint2(pack_bf2(bf_lo(prev[i].x) + yv[0], bf_hi(prev[i].x) + yv[1]),
+                                      pack_bf2(bf_lo(prev[i].y) + yv[2], bf_hi(prev[i].y) + yv[3])));
             }
           }
         }
@@ -1322,10 +1357,8 @@ template <typename G, typename TU, bool ASYNC = false>
 static int launch_conv(const Params& P, cudaStream_t st) {
   auto kern = longconv_tcl_kernel<G, TU, ASYNC>;
   constexpr int SMEM = !ASYNC ? G::SMEM : G::CAN_ASYNC ? G::SMEM_A : G::SMEM_B;
-  M2_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  M2_SMEM_ONCE(kern, SMEM);
+  const int sms = m2_sm_count();
   const int need = (P.rows + G::SLOTS - 1) / G::SLOTS;
   const int grid = need < sms ? need : sms;
   kern<<<grid, G::THREADS, SMEM, st>>>(P);
@@ -1338,7 +1371,7 @@ static int launch_conv(const Params& P, cudaStream_t st) {
 // 2 when the long-row tensor-core family covers (seq_len, dtype); the caller must then
 // supply time-contiguous tensors
 int longconv_tcl_supported(int seq_len, m2_dtype act_dtype) {
-  if (act_dtype != M2_BF16 || seq_len % 4 != 0) return 0;
+  if (act_dtype != M2_BF16) return 0;
   // transform length 4096 up to 2048, 16384 up to 8192, else 65536; lengths from 129 on run the 4096-point
   // transform with more zero padding (still several times faster than the float32 CUDA-core family)
   return seq_len > 128 && seq_len <= 32768;
@@ -1353,7 +1386,7 @@ size_t spectrum_kind2_floats(int D, int L) {
 
 int spectrum_kind2_launch(int D, int L, const float* k, float* spec, cudaStream_t st) {
   M2_REQUIRE(longconv_tcl_supported(L, M2_BF16), M2_ERR_UNSUPPORTED,
-             "m2_filter_spectrum: kind 2 covers 128 < seq_len <= 32768, multiples of 4");
+             "m2_filter_spectrum: kind 2 covers 128 < seq_len <= 32768");
   const int R = m2_filter_row_len(L);
   if (L <= 2048) return lcl::launch_spectrum<lcl::Geo4k>(D, R, k, spec, st);
   if (L <= 8192) return lcl::launch_spectrum<lcl::Geo16k>(D, R, k, spec, st);
@@ -1363,7 +1396,7 @@ int spectrum_kind2_launch(int D, int L, const float* k, float* spec, cudaStream_
 int longconv_tcl_launch(const m2_longconv_args* a, cudaStream_t st) {
   using namespace lcl;
   M2_REQUIRE(longconv_tcl_supported(a->seq_len, a->act_dtype), M2_ERR_UNSUPPORTED,
-             "m2_longconv_fwd: kind 2 needs bf16 activations and 128 < seq_len <= 32768, a multiple of 4");
+             "m2_longconv_fwd: kind 2 needs bf16 activations and 128 < seq_len <= 32768");
   M2_REQUIRE(a->xin_st == 1 && a->out_st == 1 && (a->n_filters == 1 || a->u_st == 1), M2_ERR_UNSUPPORTED,
              "m2_longconv_fwd: kind 2 needs time-contiguous tensors ((batch, channel, time) layout)");
   M2_REQUIRE(a->xin_sc % 4 == 0 && a->xin_sb % 4 == 0 && a->out_sc % 4 == 0 && a->out_sb % 4 == 0 &&
@@ -1390,7 +1423,7 @@ int longconv_tcl_launch(const m2_longconv_args* a, cudaStream_t st) {
                "m2_longconv_fwd: kind 2 needs rows of u aligned to four elements");
   }
   // rows staged through shared memory ahead of their use: 16-byte pieces of every row, bf16 output buffer
-  const bool staged = P.al16 && a->seq_len % 8 == 0 && a->out_sc % 8 == 0 && a->out_sb % 8 == 0 && m2_aligned(a->out, 16) &&
+  const bool staged = P.al16 && a->out_sc % 8 == 0 && a->out_sb % 8 == 0 && m2_aligned(a->out, 16) &&
                       (a->n_filters == 1 || ubf);
   if (a->seq_len <= 2048) {
     if (staged) return launch_conv<Geo4k, __nv_bfloat16, true>(P, st);

@@ -1,5 +1,5 @@
 // Fused gated long convolution as Toeplitz GEMMs on tcgen05 tensor cores, sequence lengths
-// L <= 128 (a multiple of 8), bf16 activations, time-contiguous tensors (kernel family 3).
+// L <= 128, bf16 activations, time-contiguous tensors (kernel family 3).
 //
 // For a short sequence the bidirectional long convolution of one channel is a product with an
 // L x L Toeplitz matrix, y[b, t] = sum_s a[b, s] T_c[t, s],  T_c[t, s] = k_c[(t - s) mod R]
@@ -190,7 +190,7 @@ longconv_tz_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
   uint64_t* tmem_empty = tmem_full + 2;        // 8 epilogue warps
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + NBARS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = tc::uniform_warp_id(), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < NST; ++s) { tc::mbar_init(full_main + s, 1); tc::mbar_init(empty_main + s, P_WARPS); }
@@ -221,7 +221,7 @@ longconv_tz_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
 
   if (warp == 0) {
     // ------------------------- TMA: strips, raw x1 / v, residual operand -------------------------
-    if (lane == 0) {
+    if (tc::elect_one()) {
       int it = 0, epoch = -1, prev_c = -1;
       bool ok = true;
       for (int unit = u_first; unit < u_last && ok; ++unit) {
@@ -247,7 +247,7 @@ longconv_tz_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     }
   } else if (warp == 2) {
     // ------------------------- TMA: raw x2 rows for the epilogue -------------------------
-    if (lane == 0) {
+    if (tc::elect_one()) {
       bool ok = true;
       int ui = 0, it = 0;
       for (int unit = u_first; unit < u_last && ok; ++unit, ++ui) {
@@ -272,7 +272,7 @@ longconv_tz_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     }
   } else if (warp == 1) {
     // ------------------------- MMA issuer -------------------------
-    if (lane == 0) {
+    if (tc::elect_one()) {
       // both operands fp16: kind::f16 with a bf16 A and an fp16 B is an illegal instruction on
       // sm_100a, so v*x1 (bf16 by the reference's arithmetic) is converted, exactly, to fp16
       constexpr uint32_t idesc = tc::make_idesc(TB, 128, 0);
@@ -288,25 +288,24 @@ longconv_tz_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
         if (!tc::mbar_wait(tmem_empty + acc, ((ui >> 1) & 1) ^ 1, abort_flag, tc::ST_TIMEOUT_MMA)) break;
         tc::tc_fence_after();
         const uint32_t tacc = tmem_base + acc * 256;
-        const uint32_t strip0 = tc::smem_u32(smem + OFF_STRIP + (2 * p) * STRIP_BYTES);
+        const uint64_t strip0 = tc::smem_desc_k_nosw(tc::smem_u32(smem + OFF_STRIP + (2 * p) * STRIP_BYTES), STRIP_LBO, STRIP_SBO);
         for (int j = 0; j < P.nsub; ++j, ++it) {
           const int s = it % NST, a = it % NA1;
           if (P.nf == 2 && (j & 1) == 0 &&
               !tc::mbar_wait(u_full + ut % NU, (ut / NU) & 1, abort_flag, tc::ST_TIMEOUT_TMA)) { ok = false; break; }
           if (!tc::mbar_wait(a1_full + a, (it / NA1) & 1, abort_flag, tc::ST_TIMEOUT_MMA)) { ok = false; break; }
           tc::tc_fence_after();
-          const uint32_t a1 = tc::smem_u32(smem + OFF_A1 + a * OP_BYTES);
+          const uint64_t a1 = tc::smem_desc_k_nosw(tc::smem_u32(smem + OFF_A1 + a * OP_BYTES), OP_LBO, OP_SBO);
           // 64-step tile of the residual operand: K step q of it starts 32 q bytes into the swizzled rows
-          const uint64_t udesc = tc::smem_desc_k_sw128(tc::smem_u32(smem + OFF_U + (ut % NU) * U_BYTES)) + 4 * (j & 1);
+          const uint64_t udesc = tc::smem_desc_k_sw128(tc::smem_u32(smem + OFF_U + (ut % NU) * U_BYTES + 64 * (j & 1)));
 #pragma unroll
           for (int ks = 0; ks < TW / 16; ++ks) {
             const int kk = (TW / 16) * j + ks;
-            const uint32_t boff = (uint32_t)(14 - 2 * kk) * STRIP_SBO;       // strip rows 112 - 16 kk ..
-            tc::mma_ss(tacc, tc::smem_desc_k_nosw(a1 + ks * 2 * OP_LBO, OP_LBO, OP_SBO),
-                       tc::smem_desc_k_nosw(strip0 + boff, STRIP_LBO, STRIP_SBO), idesc, kk ? 1u : 0u);
+            const uint32_t boff = (uint32_t)(14 - 2 * kk) * (STRIP_SBO >> 4);       // strip rows 112 - 16 kk ..
+            tc::mma_ss(tacc, tc::desc_advance(a1, ks * (2 * OP_LBO >> 4)), tc::desc_advance(strip0, boff), idesc, kk ? 1u : 0u);
             if (P.nf == 2)
-              tc::mma_ss(tacc + 128, udesc + 2 * ks,
-                         tc::smem_desc_k_nosw(strip0 + STRIP_BYTES + boff, STRIP_LBO, STRIP_SBO), idesc, kk ? 1u : 0u);
+              tc::mma_ss(tacc + 128, tc::desc_advance(udesc, 2 * ks), tc::desc_advance(strip0, (STRIP_BYTES >> 4) + boff), idesc,
+                         kk ? 1u : 0u);
           }
           if (P.nf == 2 && ((j & 1) || j == P.nsub - 1)) { tc::mma_commit(u_empty + ut % NU); ++ut; }
           tc::mma_commit(a1_empty + a);
@@ -380,8 +379,9 @@ longconv_tz_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
               dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
               dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
             }
-          } else {                                        // L is a multiple of 8: one full half remains
-            *reinterpret_cast<uint4*>(orow + t0) = make_uint4(o[0], o[1], o[2], o[3]);
+          } else {
+            lcl::store_chunk8(orow, t0, P.L, make_uint4(o[0], o[1], o[2], o[3]));
+            if (t0 + 8 < P.L) lcl::store_chunk8(orow, t0 + 8, P.L, make_uint4(o[4], o[5], o[6], o[7]));
           }
         }
         if (k & 1) {
@@ -508,8 +508,8 @@ static int tz_encode(CUtensorMap* map, CUtensorMapDataType dt, int rank, const v
 
 int longconv_tz_launch(const m2_longconv_args* a, cudaStream_t st) {
   using namespace tz;
-  M2_REQUIRE(a->act_dtype == M2_BF16 && a->seq_len >= 16 && a->seq_len <= 128 && a->seq_len % 8 == 0, M2_ERR_UNSUPPORTED,
-             "m2_longconv_fwd: kind 3 needs bf16 activations and 16 <= seq_len <= 128, a multiple of 8");
+  M2_REQUIRE(a->act_dtype == M2_BF16 && a->seq_len >= 1 && a->seq_len <= 128, M2_ERR_UNSUPPORTED,
+             "m2_longconv_fwd: kind 3 needs bf16 activations and seq_len <= 128");
   M2_REQUIRE(a->xin_st == 1 && a->out_st == 1 && (a->n_filters == 1 || a->u_st == 1), M2_ERR_UNSUPPORTED,
              "m2_longconv_fwd: kind 3 needs time-contiguous tensors");
   M2_REQUIRE(a->n_filters == 1 || a->u_dtype == M2_F16, M2_ERR_UNSUPPORTED,
@@ -551,12 +551,10 @@ int longconv_tz_launch(const m2_longconv_args* a, cudaStream_t st) {
   } else {
     tmU = tmX;
   }
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = m2_sm_count();
   const int grid = P.units < sms ? P.units : sms;
   auto kern = longconv_tz_kernel;
-  M2_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES));
+  M2_SMEM_ONCE(kern, SMEM_BYTES);
   kern<<<grid, THREADS, SMEM_BYTES, st>>>(tmX, tmU, P);
   M2_LAUNCH_CHECK("longconv_tz_kernel");
   return M2_OK;
