@@ -10,7 +10,7 @@ import os
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libm2b200.so")
-ABI_VERSION = 2
+ABI_VERSION = 3
 
 M2_F32, M2_BF16, M2_F16 = 0, 1, 2
 
@@ -88,7 +88,7 @@ class AddLayernormArgs(C.Structure):
         ("out", C.c_void_p), ("ldo", C.c_longlong),
         ("out_bf16", C.c_void_p), ("ld_bf16", C.c_longlong),
         ("out_tm_f16", C.c_void_p), ("tm_sb", C.c_longlong), ("tm_sc", C.c_longlong), ("seq_len", C.c_int),
-        ("bf16_pad_cols", C.c_int),
+        ("bf16_pad_cols", C.c_int), ("valid_len", C.c_int),
     ]
 
 
@@ -103,6 +103,46 @@ class EmbedLayernormArgs(C.Structure):
         ("out_bf16", C.c_void_p), ("ld_bf16", C.c_longlong), ("bf16_pad_cols", C.c_int),
         ("out_tm_f16", C.c_void_p), ("tm_sb", C.c_longlong), ("tm_sc", C.c_longlong), ("seq_len", C.c_int),
         ("vocab_rows", C.c_longlong), ("type_rows", C.c_longlong), ("pos_rows", C.c_longlong),
+        ("valid_len", C.c_int),
+    ]
+
+
+class MixerArgs(C.Structure):
+    _fields_ = [
+        ("batch", C.c_int), ("seq_len", C.c_int), ("pitch", C.c_int), ("out_pitch", C.c_int), ("d_model", C.c_int),
+        ("kind", C.c_int), ("n_filters", C.c_int), ("yu_bf16", C.c_int),
+        ("x", C.c_void_p), ("u", C.c_void_p), ("u_stride", C.c_longlong),
+        ("w_in", C.c_void_p), ("b_in", C.c_void_p), ("short_w", C.c_void_p), ("short_b", C.c_void_p),
+        ("spec", C.c_void_p * 2), ("bias", C.c_void_p * 2), ("w_out", C.c_void_p), ("b_out", C.c_void_p),
+        ("xin", C.c_void_p), ("conv", C.c_void_p), ("stride", C.c_longlong), ("out", C.c_void_p),
+    ]
+
+
+class MlpArgs(C.Structure):
+    _fields_ = [
+        ("m", C.c_int), ("d_model", C.c_int), ("inter", C.c_int), ("nblocks", C.c_int),
+        ("x", C.c_void_p), ("wg", C.c_void_p), ("wo", C.c_void_p), ("wo_bias", C.c_void_p),
+        ("ln_w", C.c_void_p), ("ln_b", C.c_void_p), ("eps", C.c_float),
+        ("h", C.c_void_p), ("o", C.c_void_p),
+        ("out", C.c_void_p), ("out_bf16", C.c_void_p), ("out_tm_f16", C.c_void_p), ("tm_stride", C.c_longlong),
+        ("seq_len", C.c_int), ("valid_len", C.c_int),
+    ]
+
+
+class EncoderLayer(C.Structure):
+    _fields_ = [
+        ("w_in", C.c_void_p), ("b_in", C.c_void_p), ("short_w", C.c_void_p), ("short_b", C.c_void_p),
+        ("spec", C.c_void_p * 2), ("bias", C.c_void_p * 2), ("w_out", C.c_void_p), ("b_out", C.c_void_p),
+        ("wg", C.c_void_p), ("wo", C.c_void_p), ("wo_bias", C.c_void_p),
+        ("ln_w", C.c_void_p), ("ln_b", C.c_void_p), ("eps", C.c_float),
+    ]
+
+
+class EncoderArgs(C.Structure):
+    _fields_ = [
+        ("batch", C.c_int), ("seq_len", C.c_int), ("d_model", C.c_int), ("inter", C.c_int), ("nblocks", C.c_int),
+        ("n_layers", C.c_int), ("kind", C.c_int), ("n_filters", C.c_int),
+        ("embed", EmbedLayernormArgs), ("layers", C.POINTER(EncoderLayer)), ("workspace", C.c_void_p), ("out", C.c_void_p),
     ]
 
 
@@ -118,6 +158,7 @@ SYMBOLS = {
     "m2_filter_spectrum_floats": (C.c_size_t, [C.c_int, C.c_int, C.c_int]),
     "m2_filter_spectrum": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p]),
     "m2_longconv_kind_batch": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_int]),
+    "m2_longconv_pick": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_int]),
     "m2_filter_spectrum_bias": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
     "m2_linear_fwd": (C.c_int, [C.POINTER(LinearArgs), C.c_void_p]),
     "m2_longconv_fwd": (C.c_int, [C.POINTER(LongconvArgs), C.c_void_p]),
@@ -126,6 +167,10 @@ SYMBOLS = {
     "m2_blockdiag_glu_fwd": (C.c_int, [C.POINTER(GluArgs), C.c_void_p]),
     "m2_add_layernorm_fwd": (C.c_int, [C.POINTER(AddLayernormArgs), C.c_void_p]),
     "m2_embed_layernorm_fwd": (C.c_int, [C.POINTER(EmbedLayernormArgs), C.c_void_p]),
+    "m2_mixer_fwd": (C.c_int, [C.POINTER(MixerArgs), C.c_void_p]),
+    "m2_mlp_fwd": (C.c_int, [C.POINTER(MlpArgs), C.c_void_p]),
+    "m2_encoder_workspace": (C.c_longlong, [C.c_int, C.c_int, C.c_int, C.c_int]),
+    "m2_encoder_fwd": (C.c_int, [C.POINTER(EncoderArgs), C.c_void_p]),
 }
 
 _lib = None

@@ -1,0 +1,83 @@
+"""What the modules lay out once per shape and keep for the next call: kernel arguments with the pointers of weights and
+filter tables filled in.  A plan is used again only while every parameter, buffer and submodule it was made from is the
+same object with the same storage and version counter; activations, workspaces and outputs are never kept.
+"""
+from __future__ import annotations
+
+from collections import OrderedDict
+from operator import attrgetter, is_
+
+import torch
+
+_version = attrgetter("_version")
+_ptr = torch.Tensor.data_ptr
+_training = attrgetter("training")
+
+
+class Watch:
+    """The parameters, buffers and submodules below `root` as they are now; `same()` says whether they still are."""
+
+    def __init__(self, root):
+        mods = list(root.modules())
+        slots = [(d, k, t) for m in mods for d in (m._parameters, m._buffers) for k, t in d.items() if t is not None]
+        kids = [(m._modules, k, c) for m in mods for k, c in m._modules.items()]
+        self.dicts, self.keys, self.values = zip(*(slots + kids))
+        self.tensors = [t for _, _, t in slots]
+        self.versions = list(map(_version, self.tensors))      # RuntimeError for tensors made under inference_mode
+        self.ptrs = list(map(_ptr, self.tensors))
+        self.norms = [m for m in mods if isinstance(m, torch.nn.LayerNorm)]
+        self.eps = [m.eps for m in self.norms]
+
+    def same(self):
+        try:
+            return (all(map(is_, map(dict.__getitem__, self.dicts, self.keys), self.values))
+                    and list(map(_version, self.tensors)) == self.versions and list(map(_ptr, self.tensors)) == self.ptrs
+                    and [m.eps for m in self.norms] == self.eps)
+        except KeyError:
+            return False
+
+
+class PlanCache:
+    """At most `most` plans of one module, the longest unused dropped first."""
+
+    def __init__(self, most=16):
+        self.most, self.watch, self.plans = most, None, OrderedDict()
+
+    def get(self, root, key, make):
+        """The plan of `key`, made by make() when there is none; None when the module's tensors cannot be watched."""
+        if self.watch is None or not self.watch.same():
+            self.plans = OrderedDict()
+            try:
+                self.watch = Watch(root)
+            except RuntimeError:
+                self.watch = None
+                return None
+        plans = self.plans
+        plan = plans.get(key)
+        if plan is None:
+            plan = make()
+            plans[key] = plan
+            while len(plans) > self.most:
+                try:
+                    plans.popitem(last=False)
+                except KeyError:             # another thread emptied it
+                    break
+        return plan
+
+    def __deepcopy__(self, memo):
+        return PlanCache(self.most)          # a copied module has other tensors
+
+    def __reduce__(self):
+        return PlanCache, (self.most,)
+
+
+def any_hooks(modules):
+    """Whether a hook would see (or change) what goes through one of `modules`."""
+    g = torch.nn.modules.module
+    if g._global_forward_hooks or g._global_forward_pre_hooks:
+        return True
+    return any(m._forward_hooks or m._forward_pre_hooks for m in modules)
+
+
+def any_training(modules):
+    return any(map(_training, modules))

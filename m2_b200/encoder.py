@@ -12,11 +12,14 @@ on the final output.
 """
 from __future__ import annotations
 
+import ctypes as C
 from dataclasses import dataclass
 
 import torch
 import torch.nn as nn
 
+from . import _lib, ops
+from ._plan import PlanCache, any_hooks, any_training
 from ._tags import attach
 from .glu_mlp import BertGatedLinearUnitMLP
 from .hyena_filter import _autocast_bf16
@@ -100,12 +103,11 @@ class M2BertEmbeddings(nn.Module):
         return self.dropout(self.LayerNorm(e))
 
     def _fused_embeddings(self, input_ids, token_type_ids, position_ids):
-        from . import ops
         B, L = input_ids.shape
         D = self.word_embeddings.weight.shape[1]
         aug = torch.empty((B * L, D), dtype=torch.bfloat16, device=input_ids.device)
         tm = None
-        if L % 8 == 0 and ops.longconv_kind_batch(B, L, torch.bfloat16, D) in (2, 3):
+        if L % 8 == 0:
             tm = torch.empty((D, B, L), dtype=torch.float16, device=input_ids.device)
         pos = self.position_embeddings.weight if self.use_positional_encodings else None
         if pos is not None and position_ids is None and L > pos.shape[0]:
@@ -117,11 +119,10 @@ class M2BertEmbeddings(nn.Module):
         return attach(y, bf16=aug, tm=tm)
 
     def _layernorm_with_copies(self, e):
-        from . import ops
         B, L, D = e.shape
         aug = torch.empty((B * L, D), dtype=torch.bfloat16, device=e.device)
         tm = None
-        if L % 8 == 0 and ops.longconv_kind_batch(B, L, torch.bfloat16, D) in (2, 3):
+        if L % 8 == 0:
             tm = torch.empty((D, B, L), dtype=torch.float16, device=e.device)
         y = ops.add_layernorm_fwd(e.reshape(B * L, D), None, self.LayerNorm.weight, self.LayerNorm.bias,
                                   self.LayerNorm.eps, torch.float32, bf16_copy=aug, tm_copy=tm, fill_pad=False)
@@ -227,11 +228,91 @@ class M2BertModel(nn.Module):
         self.encoder = M2BertEncoder(config)
         self.pooler = M2BertPooler(config) if add_pooling_layer else None
         self.check_finite = check_finite
+        self._plans = PlanCache()
+
+    def _called_modules(self):
+        """Every module whose forward() runs in the layer-by-layer path."""
+        ms = [self.embeddings, self.encoder]
+        for layer in self.encoder.layer:
+            ms += [layer, layer.attention, layer.mlp]
+        return ms
+
+    def _make_plan(self, B, L, dev):
+        """Arguments of one m2_encoder_fwd for (B, L), or None where the modules are not what that call computes."""
+        emb, layers = self.embeddings, list(self.encoder.layer)
+        D = emb.word_embeddings.weight.shape[1]
+        called = self._called_modules()
+        plain = (type(emb) is M2BertEmbeddings and type(self.encoder) is M2BertEncoder and layers and D % 256 == 0 and D <= 2048
+                 and all(type(y) is M2BertLayer and type(y.attention) is MonarchMixerSequenceMixing
+                         and type(y.mlp) is BertGatedLinearUnitMLP and not y.attention.hyena_training_additions for y in layers)
+                 and all(t.device == dev and t.dtype == torch.float32 for t in self.parameters()))
+        if not plain:
+            return None
+        cfg = layers[0].mlp.config
+        dims = {(y.attention.d_model, y.mlp.config.hidden_size, y.mlp.config.intermediate_size, y.mlp.config.monarch_mlp_nblocks,
+                 y.attention.residual_long_conv) for y in layers}
+        if dims != {(D, D, cfg.intermediate_size, cfg.monarch_mlp_nblocks, layers[0].attention.residual_long_conv)}:
+            return None
+        kind = ops.longconv_pick(B, L, torch.bfloat16, D)
+        if kind < 2:
+            return None
+        args = (_lib.EncoderLayer * len(layers))()
+        keep = []
+        for a, y in zip(args, layers):
+            keep.append((y.attention.fill_args(a, L, kind), y.mlp.fill_args(a)))
+        e = _lib.EncoderArgs()
+        e.batch, e.seq_len, e.d_model, e.inter, e.nblocks = B, L, D, cfg.intermediate_size, cfg.monarch_mlp_nblocks
+        e.n_layers, e.kind, e.n_filters = len(layers), kind, 2 if layers[0].attention.residual_long_conv else 1
+        tables = [emb.word_embeddings.weight, emb.token_type_embeddings.weight]
+        if emb.use_positional_encodings:
+            tables.append(emb.position_embeddings.weight)
+        tables = [ops._f32c(t) for t in tables + [emb.LayerNorm.weight, emb.LayerNorm.bias]]
+        e.embed.word_table, e.embed.type_table = tables[0].data_ptr(), tables[1].data_ptr()
+        e.embed.vocab_rows, e.embed.type_rows = tables[0].shape[0], tables[1].shape[0]
+        if emb.use_positional_encodings:
+            e.embed.pos_table, e.embed.pos_rows = tables[2].data_ptr(), tables[2].shape[0]
+        e.embed.weight, e.embed.bias, e.embed.eps = tables[-2].data_ptr(), tables[-1].data_ptr(), float(emb.LayerNorm.eps)
+        e.layers = C.cast(args, C.POINTER(_lib.EncoderLayer))
+        work = _lib.lib().m2_encoder_workspace(B, (L + 7) // 8 * 8, D, cfg.intermediate_size)
+        return dict(args=e, keep=(args, keep, tables), work=work, out=(B, L, D), called=called,
+                    dropping=[m for m in called if getattr(getattr(m, "dropout", None), "p", 0) > 0])
+
+    def _encode_whole(self, input_ids, token_type_ids, position_ids):
+        """Embeddings and all layers as one native call: bf16 autocast, no gradients, no hooks on the way.  None where the
+        layer-by-layer path has to do it."""
+        if not (input_ids.is_cuda and input_ids.dim() == 2 and not torch.is_grad_enabled() and _autocast_bf16()
+                and input_ids.shape[0] > 0 and input_ids.shape[1] > 0) or ops.observed():
+            return None
+        B, L = input_ids.shape
+        dev = input_ids.device
+        plan = self._plans.get(self, (B, L, dev.index), lambda: self._make_plan(B, L, dev))
+        if plan is None or any_hooks(plan["called"]) or any_training(plan["dropping"]):
+            return None
+
+        def ids64(t):
+            return t.expand(B, L).to(torch.long).contiguous() if t is not None else None
+        ids = [ids64(input_ids), ids64(token_type_ids), ids64(position_ids)]
+        out = torch.empty(plan["out"], dtype=torch.float32, device=dev)
+        work = torch.empty(plan["work"], dtype=torch.uint8, device=dev)
+        a = _lib.EncoderArgs.from_buffer_copy(plan["args"])
+        a.embed.input_ids = ids[0].data_ptr()
+        if ids[1] is not None:
+            a.embed.token_type_ids = ids[1].data_ptr()
+        if ids[2] is not None and a.embed.pos_table:
+            a.embed.position_ids = ids[2].data_ptr()
+        a.workspace, a.out = work.data_ptr(), out.data_ptr()
+        ops._launch("m2_encoder_fwd", out, _lib.lib().m2_encoder_fwd, C.byref(a), launches=1 + 6 * a.n_layers)
+        return out
 
     def forward(self, input_ids, token_type_ids=None, attention_mask=None, position_ids=None,
                 output_all_encoded_layers=False):
+        whole = None if output_all_encoded_layers else self._encode_whole(input_ids, token_type_ids, position_ids)
+        if whole is not None:
+            return self._finish([whole], attention_mask, False)
         h = self.embeddings(input_ids, token_type_ids, position_ids)
-        outs = self.encoder(h, attention_mask, output_all_encoded_layers)
+        return self._finish(self.encoder(h, attention_mask, output_all_encoded_layers), attention_mask, output_all_encoded_layers)
+
+    def _finish(self, outs, attention_mask, output_all_encoded_layers):
         if self.check_finite and not torch.isfinite(outs[-1]).all():
             raise ValueError("non-finite values in the encoder output")
         pooled = None

@@ -4,10 +4,13 @@ bert/src/bert_layers.py:457-508): gated_layers, wo, layernorm.
 """
 from __future__ import annotations
 
+import ctypes as C
+
 import torch
 import torch.nn as nn
 
-from . import ops
+from . import _lib, ops
+from ._plan import PlanCache
 from ._tags import attach, forward_only
 from .blockdiag_linear import BlockdiagLinear, _compute_dtype
 
@@ -35,6 +38,48 @@ class BertGatedLinearUnitMLP(nn.Module):
         self.dropout = nn.Dropout(config.hidden_dropout_prob)
         self.layernorm = nn.LayerNorm(config.hidden_size, eps=config.layer_norm_eps)
 
+    def fill_args(self, a):
+        """Writes the pointers of this module's weights into a (_lib.MlpArgs or _lib.EncoderLayer); returns the tensors
+        that keep them alive."""
+        keep = [self.gated_layers._weight_as(torch.bfloat16), self.wo._weight_as(torch.bfloat16)]
+        keep += [ops._f32c(t) for t in (self.wo.bias, self.layernorm.weight, self.layernorm.bias)]
+        a.wg, a.wo, a.wo_bias, a.ln_w, a.ln_b = (t.data_ptr() for t in keep)
+        a.eps = float(self.layernorm.eps)
+        return keep
+
+    def _plan(self):
+        if not hasattr(self, "_plans"):
+            self._plans = PlanCache()
+
+        def make():
+            a = _lib.MlpArgs()
+            a.d_model, a.inter, a.nblocks = self.config.hidden_size, self.config.intermediate_size, self.config.monarch_mlp_nblocks
+            return a, self.fill_args(a)
+        return self._plans.get(self, self.wo.bias.device.index, make)
+
+    def _forward_bf16(self, x, x2, plan, copies_only):
+        """The three launches as one call; outputs as in forward()."""
+        B, L, D = x.shape
+        m = B * L
+        dev = x.device
+        if not x2.is_contiguous():
+            x2 = x2.contiguous()
+        work = torch.empty((m, self.config.intermediate_size + D), dtype=torch.bfloat16, device=dev)
+        aug = torch.empty((m, D), dtype=torch.bfloat16, device=dev)
+        tm = torch.empty((D, B, L), dtype=torch.float16, device=dev) if L % 8 == 0 else None
+        y = aug.view(B, L, D) if copies_only and tm is not None else torch.empty((B, L, D), dtype=torch.float32, device=dev)
+        a = _lib.MlpArgs.from_buffer_copy(plan[0])
+        a.m, a.seq_len = m, L
+        a.x, a.h = x2.data_ptr(), work.data_ptr()
+        a.o = a.h + 2 * m * self.config.intermediate_size
+        a.out_bf16 = aug.data_ptr()
+        if y.dtype == torch.float32:
+            a.out = y.data_ptr()
+        if tm is not None:
+            a.out_tm_f16, a.tm_stride = tm.data_ptr(), m
+        ops._launch("m2_mlp_fwd", aug, _lib.lib().m2_mlp_fwd, C.byref(a), launches=3)
+        return attach(y, bf16=aug, tm=tm, src_dtype=torch.float32)
+
     @forward_only
     def forward(self, hidden_states: torch.Tensor, copies_only: bool = False) -> torch.Tensor:
         """copies_only (used by M2BertEncoder between layers): when the next mixer of this shape
@@ -49,6 +94,10 @@ class BertGatedLinearUnitMLP(nn.Module):
         x2 = x.reshape(-1, x.shape[-1])
         if x2.dtype != dt:
             x2 = x2.to(dt)
+        if dt == torch.bfloat16 and x.dim() == 3 and x2.shape[0] and x.shape[-1] % 256 == 0 and x.shape[-1] <= 2048 and not ops.observed():
+            plan = self._plan()
+            if plan is not None:
+                return self._forward_bf16(x, x2, plan, copies_only)
         h = ops.blockdiag_glu_fwd(x2, self.gated_layers._weight_as(dt), cfg.intermediate_size)
         o = ops.blockdiag_fwd(h, self.wo._weight_as(dt), self.wo.bias, cfg.intermediate_size,
                               cfg.hidden_size)
@@ -60,8 +109,7 @@ class BertGatedLinearUnitMLP(nn.Module):
             # instead of leaving it to a separate cast pass
             aug = torch.empty((x2.shape[0], x.shape[-1]), dtype=torch.bfloat16, device=x.device)
         tm = None
-        if (aug is not None and x.shape[1] % 8 == 0
-                and ops.longconv_kind_batch(x.shape[0], x.shape[1], torch.bfloat16, x.shape[2]) in (2, 3)):
+        if aug is not None and x.shape[1] % 8 == 0:
             # a following mixer of this shape runs a time-contiguous convolution kernel, which reads the
             # layer input as a time-major fp16 tensor: written here too
             tm = torch.empty((x.shape[2], x.shape[0], x.shape[1]), dtype=torch.float16, device=x.device)

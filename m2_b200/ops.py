@@ -35,25 +35,34 @@ class LaunchProfile:
         return sum(s.elapsed_time(e) for s, e in ev) / len(ev)
 
 
-def _launch(name, tensor, fn, *args):
+def _launch(name, tensor, fn, *args, launches=1):
     """Call one launching C-ABI entry point on torch's current stream of tensor's device."""
     global LAUNCHES
-    with torch.cuda.device(tensor.device):
-        st = torch.cuda.current_stream(tensor.device)
-        prof = PROFILE
-        if prof is not None:
-            s, e = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-            s.record(st)
-        if NVTX:
-            torch.cuda.nvtx.range_push(name)
-        rc = fn(*args, C.c_void_p(st.cuda_stream))
-        if NVTX:
-            torch.cuda.nvtx.range_pop()
-        if prof is not None:
-            e.record(st)
-            prof.events.setdefault(name, []).append((s, e))
-    _lib.check(rc, name)
-    LAUNCHES += 1
+    index = tensor.device.index
+    if index != torch.cuda.current_device():
+        with torch.cuda.device(index):
+            return _launch(name, tensor, fn, *args, launches=launches)
+    st = torch.cuda.current_stream(index)
+    prof = PROFILE
+    if prof is not None:
+        s, e = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        s.record(st)
+    if NVTX:
+        torch.cuda.nvtx.range_push(name)
+    rc = fn(*args, st.cuda_stream)
+    if NVTX:
+        torch.cuda.nvtx.range_pop()
+    if prof is not None:
+        e.record(st)
+        prof.events.setdefault(name, []).append((s, e))
+    if rc:
+        _lib.check(rc, name)
+    LAUNCHES += launches
+
+
+def observed():
+    """Whether single launches are being watched (timed or named): the modules then make them one by one."""
+    return PROFILE is not None or NVTX
 
 
 def _dt(t: torch.Tensor) -> int:
@@ -64,10 +73,6 @@ def _dt(t: torch.Tensor) -> int:
     if t.dtype == torch.float16:
         return M2_F16
     raise TypeError(f"m2_b200 supports float32 and bfloat16 tensors, got {t.dtype}")
-
-
-def _stream(t: torch.Tensor):
-    return C.c_void_p(torch.cuda.current_stream(t.device).cuda_stream)
 
 
 def _need_cuda(*ts):
@@ -139,20 +144,26 @@ def longconv_kind_batch(batch: int, seq_len: int, act_dtype: torch.dtype, d_mode
                                              M2_BF16 if act_dtype == torch.bfloat16 else M2_F32, int(d_model))
 
 
+def longconv_pick(batch: int, seq_len: int, act_dtype: torch.dtype, d_model: int) -> int:
+    """The kernel family for a caller that lays out time-contiguous rows itself (16-byte aligned, padded)."""
+    return _lib.lib().m2_longconv_pick(int(batch), int(seq_len), M2_BF16 if act_dtype == torch.bfloat16 else M2_F32,
+                                       int(d_model))
+
+
 def filter_spectrum(k: torch.Tensor, seq_len: int, kind: int, bias=None) -> torch.Tensor:
     """Spectrum table of one filter for kernel family `kind` (float32, opaque layout).
-    Kind 3 folds the convolution's bias term into the table: pass it here."""
+    Kinds 3 and 4 fold the convolution's bias term into the table: pass it here."""
     _need_cuda(k)
     assert k.dtype == torch.float32 and k.is_contiguous()
     d_model = k.shape[0]
     n = _lib.lib().m2_filter_spectrum_floats(kind, d_model, int(seq_len))
     spec = torch.empty(n, dtype=torch.float32, device=k.device)
-    if kind == 3:
+    if kind in (3, 4):
         b = _f32c(bias) if bias is not None else None
         _launch("m2_filter_spectrum", k, _lib.lib().m2_filter_spectrum_bias, kind, d_model, int(seq_len),
                 k.data_ptr(), b.data_ptr() if b is not None else None, spec.data_ptr())
     else:
-        assert bias is None, "only kind 3 folds the bias into the spectrum"
+        assert bias is None, "only kinds 3 and 4 fold the bias into the spectrum"
         _launch("m2_filter_spectrum", k, _lib.lib().m2_filter_spectrum, kind, d_model, int(seq_len),
                 k.data_ptr(), spec.data_ptr())
     return spec
@@ -177,8 +188,8 @@ def longconv_fwd(xin, u, short_w, short_b, specs, biases, *, kind, bf16_rounding
     """Fused short conv + gates + long convolution(s).
 
     xin (B, L, 3D) in_linear output (any strides with a unit stride along L or channels),
-    u (B, L, D) raw layer input or None, specs/biases: one entry per filter (kind 3: biases
-    None, they are inside its spectra, and u an fp16 view from time_major_f16).  Returns
+    u (B, L, D) raw layer input or None, specs/biases: one entry per filter (kinds 3 and 4: biases
+    None, they are inside their spectra; kind 3: u an fp16 view from time_major_f16).  Returns
     (B, L, D) in xin's dtype.
     """
     _need_cuda(xin)

@@ -4,10 +4,13 @@ between in_linear and out_linear is one fused CUDA kernel.
 """
 from __future__ import annotations
 
+import ctypes as C
+
 import torch
 import torch.nn as nn
 
-from . import ops
+from . import _lib, ops
+from ._plan import PlanCache
 from ._tags import copies_of, forward_only, src_dtype_of
 from .hyena_filter import HyenaFilter, _autocast_bf16
 
@@ -88,55 +91,98 @@ class MonarchMixerSequenceMixing(nn.Module):
         self.short_filter = nn.Conv1d(width, width, kernel_size=3, groups=width, padding=2)
 
     def _weights(self):
+        """bf16 copies of in_linear's and out_linear's weights."""
         if not hasattr(self, "_w_in"):
             self._w_in, self._w_out = _Bf16Linear(), _Bf16Linear()
         return self._w_in.get(self.in_linear), self._w_out.get(self.out_linear)
 
-    def _forward_long_rows(self, u, ures, specs, biases):
-        """bf16 path for long sequences: the convolution kernel works on time-contiguous rows, so in_linear
-        writes (B, 3D, L) and out_linear reads (B, D, L) -- both through the operand arrangements of
-        m2_linear_fwd, no transposed copy of an activation.  Rows are padded to a multiple of 16 steps so
-        that every row start is 32-byte aligned."""
-        B, L, D = u.shape
-        w_in, w_out = self._weights()
-        Lp = _round_up(L, 16)
-        # allocated per call: inside a CUDA-graph capture the buffers then belong to the graph's own pool
-        xin_t = torch.empty((B, 3 * D, Lp), dtype=torch.bfloat16, device=u.device)[:, :, :L]
-        ops.linear_fwd(bf16_input(u), w_in, self.in_linear.bias, out=xin_t.permute(0, 2, 1))
-        u_view, yu_bf16 = None, False
-        if ures is not None:
-            rec = copies_of(ures)
-            tm = rec.tm if rec is not None else None                         # (D, B, L) fp16 from the LayerNorm
-            if tm is not None and tm.shape == (D, B, L) and tm.device == u.device:
-                u_view = tm.permute(1, 2, 0)                                 # (B, L, D) view, time-contiguous
-                yu_bf16 = src_dtype_of(ures) == torch.bfloat16
-            else:
-                u_view = ures.transpose(1, 2).contiguous().transpose(1, 2)
-        y_t = torch.empty((B, D, Lp), dtype=torch.bfloat16, device=u.device)[:, :, :L]
-        ops.longconv_fwd(xin_t.permute(0, 2, 1), u_view, self.short_filter.weight, self.short_filter.bias, specs,
-                         biases, kind=2, bf16_rounding=True, out=y_t.permute(0, 2, 1), yu_bf16=yu_bf16)
-        return ops.linear_fwd(y_t.permute(0, 2, 1), w_out, self.out_linear.bias)                      # (B, L, D)
+    def filters(self):
+        return [self.filter_fn, self.filter_fn2] if self.residual_long_conv else [self.filter_fn]
 
-    def _forward_toeplitz(self, u, ures, specs):
-        """bf16 path for short sequences and large batches: the convolution kernel runs one Toeplitz GEMM
-        per channel with the batch as its M dimension, on channel-major time-contiguous tensors -- in_linear
-        writes (3D, B*L) and out_linear reads (D, B*L), each one launch of m2_linear_fwd."""
-        B, L, D = u.shape
+    def fill_args(self, a, L, kind):
+        """Writes the pointers of this module's weights and filter tables into a (_lib.MixerArgs or _lib.EncoderLayer);
+        returns the tensors that keep them alive."""
         w_in, w_out = self._weights()
-        xin_t = torch.empty((3 * D, B, L), dtype=torch.bfloat16, device=u.device)
-        ops.linear_fwd(bf16_input(u), w_in, self.in_linear.bias, out=xin_t.permute(1, 2, 0))
+        f32 = [ops._f32c(t) for t in (self.in_linear.bias, self.short_filter.weight, self.short_filter.bias, self.out_linear.bias)]
+        a.w_in, a.w_out = w_in.data_ptr(), w_out.data_ptr()
+        a.b_in, a.short_w, a.short_b, a.b_out = (t.data_ptr() for t in f32)
+        keep = [w_in, w_out] + f32
+        for i, f in enumerate(self.filters()):
+            spec = f.spectrum(L, True, kind)
+            a.spec[i] = spec.data_ptr()
+            keep.append(spec)
+            if kind == 2:
+                b = ops._f32c(f.conv_bias())
+                a.bias[i] = b.data_ptr()
+                keep.append(b)
+        return keep
+
+    def _make_plan(self, B, L, kind):
+        a = _lib.MixerArgs()
+        Lp = _round_up(L, 8)
+        a.batch, a.seq_len, a.pitch, a.out_pitch, a.d_model = B, L, Lp, L, self.d_model
+        a.kind, a.n_filters = kind, 2 if self.residual_long_conv else 1
+        a.stride, a.u_stride = _round_up(B * Lp, 16), B * Lp
+        return a, self.fill_args(a, L, kind)
+
+    def _forward_bf16(self, u, ures, kind):
+        """bf16 path: the convolution kernels work on channel-major, time-contiguous rows -- in_linear writes (3D, B, L)
+        and out_linear reads (D, B, L) through the operand arrangements of m2_linear_fwd, no transposed copy of an
+        activation.  Rows are padded to a multiple of 8 steps so that every one starts on a 16-byte boundary."""
+        B, L, D = u.shape
+        Lp = _round_up(L, 8)
+        dev = u.device
+        rec = copies_of(u)
+        x = rec.bf16 if rec is not None else None                                # (B*L, D) from the LayerNorm
+        if x is None or L != Lp or x.shape != (B * L, D) or x.device != dev or not x.is_contiguous():
+            if L == Lp:
+                x = u.to(torch.bfloat16).contiguous()
+            else:
+                x = torch.empty((B, Lp, D), dtype=torch.bfloat16, device=dev)
+                x[:, :L].copy_(u)
         u_t = None
         if ures is not None:
             rec = copies_of(ures)
-            u_t = rec.tm if rec is not None else None
-            if u_t is None or u_t.shape != (D, B, L) or u_t.device != u.device:
-                u_t = ops.time_major_f16(ures)
-        buf = torch.empty((D, B, L), dtype=torch.bfloat16, device=u.device)
-        ops.longconv_fwd(xin_t.permute(1, 2, 0), u_t.permute(1, 2, 0) if u_t is not None else None,
-                         self.short_filter.weight, self.short_filter.bias, specs, None,
-                         kind=3, bf16_rounding=True, out=buf.permute(1, 2, 0),
-                         yu_bf16=ures is not None and src_dtype_of(ures) == torch.bfloat16)
-        return ops.linear_fwd(buf.permute(1, 2, 0), w_out, self.out_linear.bias)                     # (B, L, D)
+            u_t = rec.tm if rec is not None else None                            # (D, B, L) fp16 from the LayerNorm
+            if u_t is None or u_t.shape != (D, B, Lp) or L != Lp or u_t.device != dev or not u_t.is_contiguous():
+                u_t = torch.empty((D, B, Lp), dtype=torch.float16, device=dev)
+                ops.time_major_f16(ures if ures.dtype in (torch.float32, torch.bfloat16) else ures.float(), out=u_t[:, :, :L])
+        yu_bf16 = ures is not None and src_dtype_of(ures) == torch.bfloat16
+        if not hasattr(self, "_plans"):
+            self._plans = PlanCache()
+        plan = self._plans.get(self, (B, L, kind, dev.index), lambda: self._make_plan(B, L, kind))
+        stride = _round_up(B * Lp, 16)
+        # allocated per call: inside a CUDA-graph capture the buffers then belong to the graph's own pool
+        work = torch.empty((4 * D, stride), dtype=torch.bfloat16, device=dev)
+        y = torch.empty((B, L, D), dtype=torch.bfloat16, device=dev)
+        if plan is None or ops.observed():
+            return self._launch_singly(x, u_t, work, y, kind, yu_bf16)
+        a = _lib.MixerArgs.from_buffer_copy(plan[0])
+        a.x, a.u = x.data_ptr(), u_t.data_ptr() if u_t is not None else None
+        a.yu_bf16 = yu_bf16
+        a.xin = work.data_ptr()
+        a.conv, a.out = a.xin + 2 * 3 * D * stride, y.data_ptr()
+        ops._launch("m2_mixer_fwd", y, _lib.lib().m2_mixer_fwd, C.byref(a), launches=3)
+        return y
+
+    def _launch_singly(self, x, u_t, work, y, kind, yu_bf16):
+        """The three launches of m2_mixer_fwd one by one."""
+        B, L, D = y.shape
+        Lp = _round_up(L, 8)
+        n = B * Lp
+        w_in, w_out = self._weights()
+        ops.linear_fwd(x.view(1, n, D), w_in, self.in_linear.bias, out=work[:3 * D, :n].t().unsqueeze(0))
+
+        def rows(t):                                                             # (B, L, C) view of channel-major rows
+            return t[:, :n].unflatten(1, (B, Lp))[:, :, :L].permute(1, 2, 0)
+        fs = self.filters()
+        ops.longconv_fwd(rows(work[:3 * D]), u_t[:, :, :L].permute(1, 2, 0) if u_t is not None else None,
+                         self.short_filter.weight, self.short_filter.bias, [f.spectrum(L, True, kind) for f in fs],
+                         [f.conv_bias() for f in fs] if kind == 2 else None, kind=kind, bf16_rounding=True,
+                         out=rows(work[3 * D:]), yu_bf16=yu_bf16)
+        if L == Lp:
+            return ops.linear_fwd(work[3 * D:, :n].t().unsqueeze(0), w_out, self.out_linear.bias, out=y.view(1, n, D)).view(B, L, D)
+        return ops.linear_fwd(rows(work[3 * D:]), w_out, self.out_linear.bias, out=y)
 
     @forward_only
     def forward_channels(self, u, lo, hi):
@@ -210,16 +256,15 @@ class MonarchMixerSequenceMixing(nn.Module):
         if u.dim() == 2:
             u = u.unsqueeze(0)
         u_orig = u
-        filters = [self.filter_fn] + ([self.filter_fn2] if self.residual_long_conv else [])
-        biases = [f.conv_bias() for f in filters]
-        act_dtype = torch.bfloat16 if bf16 else u.dtype
-        kind = ops.longconv_kind_batch(u.size(0), L, act_dtype, self.d_model)
-        specs = [f.spectrum(L, bf16, kind) for f in filters]
         ures = u_orig if self.residual_long_conv else None
-        if kind == 3:
-            return self._forward_toeplitz(u, ures, specs), None
-        if kind == 2:
-            return self._forward_long_rows(u, ures, specs, biases), None
+        if bf16:
+            kind = ops.longconv_pick(u.size(0), L, torch.bfloat16, self.d_model)
+            if kind and u.size(0):
+                return self._forward_bf16(u, ures, kind), None
+        kind = 0
+        filters = self.filters()
+        biases = [f.conv_bias() for f in filters]
+        specs = [f.spectrum(L, bf16, kind) for f in filters]
         if bf16:
             w_in, w_out = self._weights()
             xin = ops.linear_fwd(bf16_input(u), w_in, self.in_linear.bias)
