@@ -38,6 +38,31 @@ int m2_sm_count();
          M2_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(bytes))); \
          done_.fetch_or(bit_, std::memory_order_relaxed); } } while (0)
 
+// Launch that may begin while the kernel before it in the stream is still running (programmatic stream serialization): its
+// blocks take the SMs that kernel does not need and set up their barriers and tensor memory; pdl_wait() in the kernel,
+// before its first access to global memory, waits until everything before it is complete and visible.  `elements` is the
+// size of the kernel's d_model-wide activation: up to 2^24 (16 k tokens at d_model 768) kernels last 4 to 50 us and the
+// overlap is worth 1 to 2 us each (one query 812 -> 640 us, 8 x 128 889 -> 651 us); larger ones are launched plainly, as they
+// lose 2 to 3 % of a forward to it (64 x 2048 at 1536: 144.8 -> 149.5 ms).
+constexpr long long M2_OVERLAP_ELEMENTS = 1LL << 24;
+template <typename... KArgs, typename... Args>
+static int m2_launch(const char* name, long long elements, void (*kern)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t st,
+                     Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = elements <= M2_OVERLAP_ELEMENTS ? 1 : 0;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
+  if (e != cudaSuccess) return m2_set_error(M2_ERR_CUDA, "launch of %s failed: %s", name, cudaGetErrorString(e));
+  return M2_OK;
+}
+
 static inline bool m2_is_pow2(long long v) { return v > 0 && (v & (v - 1)) == 0; }
 static inline int m2_ilog2(long long v) { int l = 0; while ((1LL << l) < v) ++l; return l; }
 static inline bool m2_aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }
@@ -47,6 +72,15 @@ static inline bool m2_aligned(const void* p, size_t a) { return (reinterpret_cas
 __device__ int m2_dev_status_word = 0;
 
 // ---- device helpers -----------------------------------------------------------------
+// The next kernel of the stream may be launched; then wait for the kernels before this one.  Every thread of a kernel
+// started by m2_launch calls it before it reads or writes global memory.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait_only() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() {
+  pdl_trigger();
+  pdl_wait_only();
+}
+
 // Round a float to the nearest bf16 value (ties to even) and return it as a float.
 __device__ __forceinline__ float bf16r(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 

@@ -173,6 +173,7 @@ add_layernorm_warp_kernel(const TI* a, long long lda, const TI* b, long long ldb
                           long long ldo, __nv_bfloat16* out2, long long ld2, int m,
                           __half* out_tm, long long tm_sb, long long tm_sc, int seq_len, int valid, int rpw, int pad2) {
   extern __shared__ __half ln_tile[];   // [rows of the block][n] fp16, only with out_tm
+  pdl_wait_only();
   const int wib = threadIdx.x >> 5, nw = blockDim.x >> 5, lane = threadIdx.x & 31;
   constexpr int n = VI * 256;
   // a warp normalises rpw rows (rpw > 1 only with out_tm, where m is a multiple of the block's rows)
@@ -280,6 +281,7 @@ add_layernorm_warp_kernel(const TI* a, long long lda, const TI* b, long long ldb
     }
   }
   }
+  pdl_trigger();                        // this late: blocks of the next kernel would take issue slots from many short ones here
   if (out_tm) {
     // rows of the block are consecutive time steps of one sequence: write each channel's run
     // of them (16 to 128 contiguous bytes) into the time-major copy, two channels per thread
@@ -464,11 +466,11 @@ static int add_layernorm_core(const m2_add_layernorm_args* a, const m2::LnGather
   if (vec) {
     // with the time-major copy a block covers 8, 16 or 32 consecutive steps of one sequence: 16 steps make a channel's
     // run of them one 32-byte sector, 32 steps two.  Few rows take short blocks all the same: 128 rows are four blocks
-    // of 32 (11 us) or 16 of 8; from two blocks per SM on the runs decide.
+    // of 32 (11 us) or 16 of 8; from one and a half blocks per SM on the runs decide.
     int rows = 8, threads = 256, rpw = 1;
     if (a->out_tm_f16) {
       const int sms = m2_sm_count();
-      rows = a->seq_len % 32 == 0 && a->n <= 768 && a->m >= 64 * sms ? 32 : a->seq_len % 16 == 0 && a->m >= 32 * sms ? 16 : 8;
+      rows = a->seq_len % 32 == 0 && a->n <= 768 && a->m >= 48 * sms ? 32 : a->seq_len % 16 == 0 && a->m >= 24 * sms ? 16 : 8;
       threads = rows >= 16 ? 512 : 256;
       rpw = rows / (threads / 32);
     }
@@ -477,7 +479,7 @@ static int add_layernorm_core(const m2_add_layernorm_args* a, const m2::LnGather
 #define M2_LNW(TO, VI) do { if (a->in_dtype == M2_F32) M2_LNW2(float, float, VI); else M2_LNW2(__nv_bfloat16, TO, VI); } while (0)
 #define M2_LNW2(TI, TO, VI) do { \
       if (tile > 48 * 1024) M2_SMEM_ONCE((add_layernorm_warp_kernel<TI, TO, VI>), 64 * 1024); /* at most 16 x 2048 x 2 bytes */ \
-      add_layernorm_warp_kernel<TI, TO, VI><<<blocks, threads, tile, st>>>( \
+      return m2_launch("add_layernorm_warp_kernel", (long long)a->m * a->n, add_layernorm_warp_kernel<TI, TO, VI>, blocks, threads, tile, st, \
       (const TI*)a->a, a->lda, (const TI*)a->b, a->ldb, gather, a->weight, a->bias, a->eps, \
       (TO*)a->out, a->ldo, (__nv_bfloat16*)a->out_bf16, a->ld_bf16, a->m, \
       (__half*)a->out_tm_f16, a->tm_sb, a->tm_sc, a->seq_len, a->valid_len > 0 ? a->valid_len : a->seq_len, rpw, a->bf16_pad_cols); } while (0)
@@ -488,8 +490,6 @@ static int add_layernorm_core(const m2_add_layernorm_args* a, const m2::LnGather
 #undef M2_LNW_VI
 #undef M2_LNW
 #undef M2_LNW2
-    M2_LAUNCH_CHECK("add_layernorm_warp_kernel");
-    return M2_OK;
   }
   M2_REQUIRE(!gather.ids_a && !gather.c, M2_ERR_UNSUPPORTED, "m2_embed_layernorm_fwd: shape not covered by the vectorised kernel");
   M2_REQUIRE(a->out != nullptr && a->out_bf16 == nullptr && a->out_tm_f16 == nullptr, M2_ERR_UNSUPPORTED,

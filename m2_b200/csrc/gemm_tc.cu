@@ -157,6 +157,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   __syncthreads();
   tc::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
 
   if (warp == 0) {
     // ------------------------------- TMA producer -------------------------------
@@ -350,6 +351,7 @@ glu_res_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   __syncthreads();
   tc::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
 
   // this CTA's contiguous range of units; unit = (pair = row tile x block pair, group of column tiles)
   const int u0 = (int)((long long)blockIdx.x * P.total_units / gridDim.x);
@@ -473,21 +475,29 @@ static int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const Params& 
   auto kern = gemm_tc_kernel<BN, GLU>;
   M2_SMEM_ONCE(kern, C::SMEM);
   int grid = P.total_tiles < m2_sm_count() ? P.total_tiles : m2_sm_count();
-  kern<<<grid, THREADS, C::SMEM, st>>>(tmA, tmB, P);
-  M2_LAUNCH_CHECK("gemm_tc_kernel");
-  return M2_OK;
+  return m2_launch("gemm_tc_kernel", (long long)P.M * P.out_cols, kern, grid, THREADS, C::SMEM, st, tmA, tmB, P);
 }
 
-static int pick_bn(int q) {
-  const int cand[] = {256, 192, 128, 64};
-  for (int c : cand) if (q % c == 0) return c;
-  return 0;
+// Column tile of a block-diagonal GEMM with q columns per block: the widest that divides q is the most efficient; with
+// few row tiles narrower ones put more SMs to work (wo at 1024 rows: 32 tiles of 192 columns, or 96 of 64).  A K step
+// brings 128 rows of A and n of B at about 50 bytes per clock and multiplies for 2 n clocks, a tile costs some 2500 more.
+static int pick_bn(int q, long long row_tiles, int ksteps) {
+  int best = 0;
+  double least = 0;
+  for (int n : {256, 192, 128, 64}) {
+    if (q % n) continue;
+    const long long tiles = row_tiles * (q / n), waves = (tiles + m2_sm_count() - 1) / m2_sm_count();
+    const double load = (BM + n) * BK * 2 / 50.0, mma = 2.0 * n;
+    const double cost = waves * (ksteps * (load > mma ? load : mma) + 2500.0);
+    if (best == 0 || cost < 0.97 * least) { least = cost; best = n; }
+  }
+  return best;
 }
 
 }  // namespace gemm
 
 bool blockdiag_tc_supported(const m2_blockdiag_args* a) {
-  return a->dtype == M2_BF16 && a->p % 64 == 0 && gemm::pick_bn(a->q) != 0 &&
+  return a->dtype == M2_BF16 && a->p % 64 == 0 && a->q % 64 == 0 &&
          a->in_features == a->nblocks * a->p && a->out_features == a->nblocks * a->q &&
          a->ldx % 8 == 0 && a->ldo % 8 == 0 && m2_aligned(a->x, 16) && m2_aligned(a->w, 16) &&
          m2_aligned(a->out, 16) && a->m >= 1;
@@ -501,7 +511,7 @@ bool glu_tc_supported(const m2_glu_args* a) {
 
 int blockdiag_tc_launch(const m2_blockdiag_args* a, cudaStream_t st) {
   using namespace gemm;
-  const int bn = pick_bn(a->q);
+  const int bn = pick_bn(a->q, (long long)((a->m + BM - 1) / BM) * a->nblocks, a->p / BK);
   CUtensorMap tmA, tmB;
   int rc = m2_make_tmap_bf16_2d(&tmA, a->x, a->m, a->in_features, a->ldx, BM);
   if (rc) return rc;
@@ -549,9 +559,7 @@ int glu_tc_launch(const m2_glu_args* a, cudaStream_t st) {
     R.wide_out = P.wide_out; R.out = a->h; R.ldo = a->ldh;
     M2_SMEM_ONCE(glu_res_kernel, res::SMEM);
     const int grid = R.total_units < m2_sm_count() ? R.total_units : m2_sm_count();
-    glu_res_kernel<<<grid, THREADS, res::SMEM, st>>>(tmA, tmB, R);
-    M2_LAUNCH_CHECK("glu_res_kernel");
-    return M2_OK;
+    return m2_launch("glu_res_kernel", (long long)a->m * a->d_model, glu_res_kernel, grid, THREADS, res::SMEM, st, tmA, tmB, R);
   }
   return launch<128, true>(tmA, tmB, P, st);
 }

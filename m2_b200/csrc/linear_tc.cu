@@ -95,6 +95,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     tc::tmem_alloc2(tmem_slot, 512);
     tc::tmem_relinquish2();
   }
+  pdl_wait();
   float* sbias = reinterpret_cast<float*>(smem + OFF_BIAS);
   const bool bias_smem = MODE != CHANNELS && P.bias != nullptr && P.n_rows <= BIAS_MAX;
   if (bias_smem)
@@ -388,15 +389,30 @@ static int max_pairs(const void* kern) {
   return cached[dev];
 }
 
+// Width of the N side of a pair's tile.  A K step brings 128 rows of A and n / 2 of B to each SM at about 50 bytes per
+// clock and multiplies for 2 n clocks; a tile costs some 2500 clocks besides (first loads, last epilogue).  256 is
+// the most efficient and the choice wherever the tiles fill the pairs; with few tiles narrower ones put more SMs to work
+// (768 -> 2304 at 1024 tokens: 36 tiles of 256 on 74 pairs, or 72 of 128).
+static int pick_n_tile(int m_pairs, int n_rows, int ksteps) {
+  const int pairs = m2_sm_count() / 2;
+  int best = 2 * BNH;
+  double least = 0;
+  for (int n : {2 * BNH, 192, 128, 64, 32}) {
+    const long long tiles = (long long)m_pairs * ((n_rows + n - 1) / n), waves = (tiles + pairs - 1) / pairs;
+    const double load = (A_BYTES + n * BK) / 50.0, mma = 2.0 * n;        // bytes of BK bf16 columns: 128 rows, n / 2 rows
+    const double cost = waves * (ksteps * (load > mma ? load : mma) + 2500.0);
+    if (n == 2 * BNH || cost < 0.97 * least) { least = cost; best = n; }
+  }
+  return best;
+}
+
 template <int MODE>
-static int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const Params& P, cudaStream_t st) {
+static int launch(const CUtensorMap& tmA, const CUtensorMap& tmB, const Params& P, long long elements, cudaStream_t st) {
   auto kern = linear_pair_kernel<MODE>;
   M2_SMEM_ONCE(kern, SMEM);
   const int mp = max_pairs(reinterpret_cast<const void*>(kern));
   const int pairs = P.total_tiles < mp ? P.total_tiles : mp;
-  kern<<<2 * pairs, THREADS, SMEM, st>>>(tmA, tmB, P);
-  M2_LAUNCH_CHECK("linear_pair_kernel");
-  return M2_OK;
+  return m2_launch("linear_pair_kernel", elements, kern, 2 * pairs, THREADS, SMEM, st, tmA, tmB, P);
 }
 
 }  // namespace lin
@@ -458,37 +474,45 @@ extern "C" int m2_linear_fwd(const m2_linear_args* a, void* stream) {
   memset(&P, 0, sizeof(P));
   P.L = L; P.batch = a->batch; P.ksteps = (K + BK - 1) / BK;
   P.out = (__nv_bfloat16*)a->out; P.osb = a->out_sb; P.ost = a->out_st; P.osc = a->out_sc; P.bias = a->bias;
-  CUtensorMap tmA, tmB;
-  int rc;
-  if (x_rows && o_time) {                                     // CHANNELS: weight rows on the M side
+  const bool channels = x_rows && o_time;
+  if (channels) {                                             // CHANNELS: weight rows on the M side
     P.m_rows = N; P.n_rows = (int)tokens;
-    if ((rc = m2_make_tmap_bf16_2d(&tmA, a->w, (uint64_t)N, (uint64_t)K, (uint64_t)K, BM))) return rc;
-    if ((rc = m2_make_tmap_bf16_2d(&tmB, a->x, (uint64_t)tokens, (uint64_t)K, (uint64_t)a->x_st, BNH))) return rc;
     P.flat = a->batch == 1 || a->out_sb == L;
     P.vec = m2_aligned(a->out, 32) && a->out_sc % 16 == 0 && (P.flat || (L % 16 == 0 && a->out_sb % 16 == 0));
   } else {
     P.n_rows = N;
-    if ((rc = m2_make_tmap_bf16_2d(&tmB, a->w, (uint64_t)N, (uint64_t)K, (uint64_t)K, BNH))) return rc;
-    if (x_rows) {                                             // ROWS
-      P.m_rows = (int)tokens;
-      if ((rc = m2_make_tmap_bf16_2d(&tmA, a->x, (uint64_t)tokens, (uint64_t)K, (uint64_t)a->x_st, BM))) return rc;
-    } else {                                                  // TIMEIN
+    P.m_rows = (int)tokens;                                   // ROWS
+    if (x_time) {                                             // TIMEIN
       P.tiles_per_batch = (L + BM - 1) / BM;
       P.m_tiles = P.tiles_per_batch * a->batch;
       P.m_rows = P.m_tiles * BM;
-      if ((rc = make_tmap_bf16_3d(&tmA, a->x, (uint64_t)L, (uint64_t)K, (uint64_t)a->batch, (uint64_t)a->x_sc,
-                                  (uint64_t)(a->batch == 1 ? a->x_sc * (long long)K : a->x_sb)))) return rc;
     }
     P.vec = m2_aligned(a->out, 32) && a->out_st % 16 == 0 && a->out_sb % 16 == 0;
   }
-  P.nb = 1; P.p = K; P.q = P.n_rows; P.n_tile = 2 * BNH; P.bh = BNH; P.round_first = 0;
-  P.idesc = tc::make_idesc_major(2 * BM, P.n_tile, 1, x_time ? 1 : 0, 0);
   P.m_pairs = (P.m_rows + 2 * BM - 1) / (2 * BM);
+  P.n_tile = pick_n_tile(P.m_pairs, P.n_rows, P.ksteps);
+  P.bh = P.n_tile / 2;
+  CUtensorMap tmA, tmB;
+  int rc;
+  if (channels) {
+    if ((rc = m2_make_tmap_bf16_2d(&tmA, a->w, (uint64_t)N, (uint64_t)K, (uint64_t)K, BM))) return rc;
+    if ((rc = m2_make_tmap_bf16_2d(&tmB, a->x, (uint64_t)tokens, (uint64_t)K, (uint64_t)a->x_st, (uint32_t)P.bh))) return rc;
+  } else {
+    if ((rc = m2_make_tmap_bf16_2d(&tmB, a->w, (uint64_t)N, (uint64_t)K, (uint64_t)K, (uint32_t)P.bh))) return rc;
+    if (x_rows)
+      rc = m2_make_tmap_bf16_2d(&tmA, a->x, (uint64_t)tokens, (uint64_t)K, (uint64_t)a->x_st, BM);
+    else
+      rc = make_tmap_bf16_3d(&tmA, a->x, (uint64_t)L, (uint64_t)K, (uint64_t)a->batch, (uint64_t)a->x_sc,
+                             (uint64_t)(a->batch == 1 ? a->x_sc * (long long)K : a->x_sb));
+    if (rc) return rc;
+  }
+  P.nb = 1; P.p = K; P.q = P.n_rows; P.round_first = 0;
+  P.idesc = tc::make_idesc_major(2 * BM, P.n_tile, 1, x_time ? 1 : 0, 0);
   P.n_tiles = (P.n_rows + P.n_tile - 1) / P.n_tile;
   P.total_tiles = P.m_pairs * P.n_tiles;
-  if (x_rows && o_time) return launch<CHANNELS>(tmA, tmB, P, st);
-  if (x_rows) return launch<ROWS>(tmA, tmB, P, st);
-  return launch<TIMEIN>(tmA, tmB, P, st);
+  if (channels) return launch<CHANNELS>(tmA, tmB, P, tokens * K, st);
+  if (x_rows) return launch<ROWS>(tmA, tmB, P, tokens * K, st);
+  return launch<TIMEIN>(tmA, tmB, P, tokens * K, st);
 }
 
 namespace m2 {
@@ -520,6 +544,6 @@ int blockdiag_pair_launch(const m2_blockdiag_args* a, cudaStream_t st) {
   P.m_pairs = (P.m_rows + 2 * BM - 1) / (2 * BM);
   P.n_tiles = (a->q + P.n_tile - 1) / P.n_tile;
   P.total_tiles = P.m_pairs * P.nb * P.n_tiles;
-  return launch<ROWS>(tmA, tmB, P, st);
+  return launch<ROWS>(tmA, tmB, P, (long long)a->m * a->out_features, st);
 }
 }  // namespace m2

@@ -180,6 +180,7 @@ longconv_bt_kernel(const Params P) {
   __syncthreads();
   tc::tc_fence_after();
   const uint32_t tm = *tmem_slot;
+  pdl_wait();
 
   bool ok = true;
   uint32_t commits = 0;                              // groups of MMAs committed so far; group i signals bars[i & 1]
@@ -568,9 +569,7 @@ int longconv_bt_launch(const m2_longconv_args* a, cudaStream_t st) {
   // every CTA takes one contiguous range of units, so a channel's taps are fetched once per CTA
   const int grid = P.units < most ? P.units : most;
   M2_SMEM_ONCE(longconv_bt_kernel, SMEM_MAX);
-  longconv_bt_kernel<<<grid, THREADS, smem, st>>>(P);
-  M2_LAUNCH_CHECK("longconv_bt_kernel");
-  return M2_OK;
+  return m2_launch("longconv_bt_kernel", (long long)P.B * P.L * P.D, longconv_bt_kernel, grid, THREADS, smem, st, P);
 }
 
 }  // namespace m2

@@ -712,6 +712,7 @@ longconv_tcl_kernel(const Params P) {
     *abort_flag = 0;
     tc::mbar_fence_init();
   }
+  pdl_wait();
   {
     const uint4* src = reinterpret_cast<const uint4*>(P.spec[0]);
     uint4* dst = reinterpret_cast<uint4*>(hdrb);
@@ -1361,9 +1362,7 @@ static int launch_conv(const Params& P, cudaStream_t st) {
   const int sms = m2_sm_count();
   const int need = (P.rows + G::SLOTS - 1) / G::SLOTS;
   const int grid = need < sms ? need : sms;
-  kern<<<grid, G::THREADS, SMEM, st>>>(P);
-  M2_LAUNCH_CHECK("longconv_tcl_kernel");
-  return M2_OK;
+  return m2_launch("longconv_tcl_kernel", (long long)P.B * P.L * P.D, kern, grid, G::THREADS, SMEM, st, P);
 }
 
 }  // namespace lcl

@@ -214,6 +214,7 @@ longconv_tz_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
   __syncthreads();
   tc::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
 
   // contiguous range of units: consecutive units share the channel, so its strips stay put
   const int u_first = (int)(((long long)blockIdx.x * P.units) / gridDim.x);
@@ -555,9 +556,7 @@ int longconv_tz_launch(const m2_longconv_args* a, cudaStream_t st) {
   const int grid = P.units < sms ? P.units : sms;
   auto kern = longconv_tz_kernel;
   M2_SMEM_ONCE(kern, SMEM_BYTES);
-  kern<<<grid, THREADS, SMEM_BYTES, st>>>(tmX, tmU, P);
-  M2_LAUNCH_CHECK("longconv_tz_kernel");
-  return M2_OK;
+  return m2_launch("longconv_tz_kernel", (long long)P.B * P.L * P.D, kern, grid, THREADS, SMEM_BYTES, st, tmX, tmU, P);
 }
 
 int time_major_f16_launch(const m2_time_major_args* a, cudaStream_t st) {
