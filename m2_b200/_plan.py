@@ -11,7 +11,6 @@ import torch
 
 _version = attrgetter("_version")
 _ptr = torch.Tensor.data_ptr
-_training = attrgetter("training")
 
 
 class Watch:
@@ -72,12 +71,13 @@ class PlanCache:
 
 
 def any_hooks(modules):
-    """Whether a hook would see (or change) what goes through one of `modules`."""
+    """Whether a hook, or a forward() set on an instance, would see (or change) what goes through one of `modules`."""
     g = torch.nn.modules.module
     if g._global_forward_hooks or g._global_forward_pre_hooks:
         return True
-    return any(m._forward_hooks or m._forward_pre_hooks for m in modules)
+    return any(m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__ for m in modules)
 
 
-def any_training(modules):
-    return any(map(_training, modules))
+def any_dropping(modules):
+    """Whether a dropout of one of `modules` is on."""
+    return any(m.training and m.dropout.p > 0 for m in modules)

@@ -19,7 +19,7 @@ import torch
 import torch.nn as nn
 
 from . import _lib, ops
-from ._plan import PlanCache, any_hooks, any_training
+from ._plan import PlanCache, any_dropping, any_hooks
 from ._tags import attach
 from .glu_mlp import BertGatedLinearUnitMLP
 from .hyena_filter import _autocast_bf16
@@ -275,7 +275,7 @@ class M2BertModel(nn.Module):
         e.layers = C.cast(args, C.POINTER(_lib.EncoderLayer))
         work = _lib.lib().m2_encoder_workspace(B, (L + 7) // 8 * 8, D, cfg.intermediate_size)
         return dict(args=e, keep=(args, keep, tables), work=work, out=(B, L, D), called=called,
-                    dropping=[m for m in called if getattr(getattr(m, "dropout", None), "p", 0) > 0])
+                    dropping=[m for m in called if hasattr(m, "dropout")])
 
     def _encode_whole(self, input_ids, token_type_ids, position_ids):
         """Embeddings and all layers as one native call: bf16 autocast, no gradients, no hooks on the way.  None where the
@@ -286,7 +286,7 @@ class M2BertModel(nn.Module):
         B, L = input_ids.shape
         dev = input_ids.device
         plan = self._plans.get(self, (B, L, dev.index), lambda: self._make_plan(B, L, dev))
-        if plan is None or any_hooks(plan["called"]) or any_training(plan["dropping"]):
+        if plan is None or any_hooks(plan["called"]) or any_dropping(plan["dropping"]):
             return None
 
         def ids64(t):
