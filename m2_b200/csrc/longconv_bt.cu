@@ -102,8 +102,9 @@ __host__ __device__ constexpr int window_rows(int nb) { return nb == 1 ? 240 : W
 __host__ inline int smem_of(const Shape& s, int g, int nf) {
   return 2 * operand_bytes(g * s.cols) + 2 * g * window_rows(s.nb) * 32 + nf * g * tap_count(s.nb) * 2 + 48 * g + 16 * MAXCOLS + 64;
 }
-// channels per unit
+// channels per unit; one where an MMA takes eight rows beside its channel's data, which must be the zero rows around it
 __host__ inline int group_of(const Shape& s, int B, int D, int nf) {
+  if (s.bt % 16) return 1;
   const long long seqs = (long long)((B + s.bt - 1) / s.bt) * D;
   int g = 1;
   while (g < 4 && (g + 1) * s.cols <= MAXCOLS && smem_of(s, g + 1, nf) <= SMEM_MAX && seqs > 2LL * g * m2_sm_count()) ++g;
