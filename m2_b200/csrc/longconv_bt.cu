@@ -505,15 +505,22 @@ int longconv_bt_supported(int seq_len, m2_dtype act_dtype) {
   return act_dtype == M2_BF16 && seq_len >= 1 && seq_len <= bt::MAX_L;
 }
 
-// Whether this family beats the FFT family at 128 < L <= 1024.  Both run in waves of resident units; measured at D = 768,
-// L = 256 .. 1024, B = 1 .. 64: a wave of 8 sequences per SM takes the FFT family 19 us whatever the length, a wave of two
-// units per SM this one 0.25 us per column and 2 us per block.
-bool longconv_bt_preferred(int batch, int seq_len, int d_model) {
+// Time of the block-Toeplitz kernel in us.  It runs in waves of two units per SM; measured at D = 768, L = 256 .. 1024,
+// B = 1 .. 64, a wave takes 0.25 us per column and 2 us per block, and in the stream of a forward 0.8 of that (D = 768, one
+// sequence to eight: 12 us at 128 steps, 18 at 256, 40 at 384; D = 1536: 28, 34, 58).
+static double bt_us(int batch, int seq_len, int d_model, int nf) {
   const bt::Shape s = bt::shape_of(seq_len, batch);
-  const int g = bt::group_of(s, batch, d_model, 2), sms = m2_sm_count();
+  const int g = bt::group_of(s, batch, d_model, nf), sms = m2_sm_count();
   const long long units = (long long)((batch + s.bt - 1) / s.bt) * ((d_model + g - 1) / g);
-  const long long w4 = (units + 2 * sms - 1) / (2 * sms), w2 = ((long long)batch * d_model + 8 * sms - 1) / (8 * sms);
-  return 19.0 * w2 > (0.25 * g * s.cols + 2.0 * s.nb) * w4;
+  return 0.8 * (0.25 * g * s.cols + 2.0 * s.nb) * ((units + 2 * sms - 1) / (2 * sms));
+}
+
+// Whether this family beats the FFT family at 128 < L <= 1024, whose waves of 8 sequences per SM take 19 us whatever the
+// length (0.8 of it in the stream of a forward).
+bool longconv_bt_preferred(int batch, int seq_len, int d_model) {
+  const long long waves = ((long long)batch * d_model + 8 * m2_sm_count() - 1) / (8 * m2_sm_count());
+  const double bt = bt_us(batch, seq_len, d_model, 2), direct = longconv_direct_us(batch, seq_len, d_model, 2);
+  return 0.8 * 19.0 * waves > (bt < direct ? bt : direct);
 }
 
 size_t spectrum_kind4_floats(int D, int L) {
@@ -542,7 +549,10 @@ int longconv_bt_launch(const m2_longconv_args* a, cudaStream_t st) {
              "m2_longconv_fwd: kind 4 needs 16-byte aligned rows of xin and out");
   M2_REQUIRE(a->n_filters == 1 || (m2_aligned(a->u, 16) && a->u_sb % 8 == 0 && a->u_sc % 8 == 0),
              M2_ERR_ALIGN, "m2_longconv_fwd: kind 4 needs 16-byte aligned rows of u");
+  const int u_f16 = a->n_filters == 2 && a->u_dtype == M2_F16, yu_bf16 = a->n_filters == 2 && (a->u_dtype == M2_BF16 || a->yu_bf16);
   const Shape sh = shape_of(a->seq_len, a->batch);
+  if (longconv_direct_us(a->batch, a->seq_len, a->d_model, a->n_filters) < bt_us(a->batch, a->seq_len, a->d_model, a->n_filters))
+    return longconv_direct_launch(a, tap_count(sh.nb), 128 * sh.nb, u_f16, yu_bf16, st);
   Params P;
   P.B = a->batch; P.L = a->seq_len; P.D = a->d_model; P.nf = a->n_filters;
   P.NB = sh.nb; P.Bt = sh.bt;
@@ -559,8 +569,7 @@ int longconv_bt_launch(const m2_longconv_args* a, cudaStream_t st) {
   P.ksteps = P.NB == 1 ? (P.L + 15) / 16 : 8;
   P.tcols = 32;
   while (P.tcols < P.nf * P.cols) P.tcols *= 2;
-  P.u_f16 = a->n_filters == 2 && a->u_dtype == M2_F16;
-  P.yu_bf16 = a->n_filters == 2 && (a->u_dtype == M2_BF16 || a->yu_bf16);
+  P.u_f16 = u_f16; P.yu_bf16 = yu_bf16;
   P.xin = (const __nv_bfloat16*)a->xin; P.xsb = a->xin_sb; P.xsc = a->xin_sc;
   P.u = a->u; P.usb = a->u_sb; P.usc = a->u_sc;
   P.out = (__nv_bfloat16*)a->out; P.osb = a->out_sb; P.osc = a->out_sc;

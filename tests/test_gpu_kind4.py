@@ -1,5 +1,5 @@
-"""Kind 4 at the edges of its tiles and with several channels to a unit
-against the float32 CUDA-core family, as in test_gpu_ragged.py."""
+"""Kind 4 on both of its kernels (direct sums for little work, block-Toeplitz GEMMs beyond) at sizes around the line
+between them, against the float32 CUDA-core family, as in test_gpu_ragged.py."""
 import pytest
 import torch
 
