@@ -1,6 +1,6 @@
 // Block-diagonal linear layers and the GLU epilogue on CUDA cores with float32
-// accumulation (the float32-activation path; bf16 activations use the tensor-core
-// kernels), plus the residual-add + LayerNorm that closes the MLP.
+// accumulation, for what gemm_f32.cu (aligned float32) and the tensor-core kernels (bf16) do
+// not take, plus the residual-add + LayerNorm that closes the MLP.
 //
 // Computation replaced: bert/src/mm/blockdiag_multiply.py:49-60,
 // bert/src/mm/structured_linear.py:52-70, bert/src/bert_layers.py:492-506.
@@ -354,6 +354,7 @@ extern "C" int m2_blockdiag_fwd(const m2_blockdiag_args* a, void* stream) {
   if (blockdiag_pair_supported(a)) return blockdiag_pair_launch(a, st);
   dim3 grid((a->q + GT - 1) / GT, (a->m + GT - 1) / GT, a->nblocks);
   M2_REQUIRE(grid.y <= 65535 && grid.z <= 65535, M2_ERR_UNSUPPORTED, "m2_blockdiag_fwd: too many row tiles");
+  if (blockdiag_f32_supported(a)) return blockdiag_f32_launch(a, st);
   if (a->dtype == M2_BF16)
     blockdiag_simt_kernel<__nv_bfloat16, true><<<grid, 256, 0, st>>>(
         (const __nv_bfloat16*)a->x, a->ldx, (const __nv_bfloat16*)a->w, a->bias, (__nv_bfloat16*)a->out,
@@ -387,6 +388,7 @@ extern "C" int m2_blockdiag_glu_fwd(const m2_glu_args* a, void* stream) {
   const int p = a->d_model / a->nblocks, q = 2 * a->inter / a->nblocks;
   dim3 grid((q + GT - 1) / GT, (a->m + GT - 1) / GT, a->nblocks / 2);
   M2_REQUIRE(grid.y <= 65535, M2_ERR_UNSUPPORTED, "m2_blockdiag_glu_fwd: too many row tiles");
+  if (glu_f32_supported(a)) return glu_f32_launch(a, st);
   if (a->dtype == M2_BF16)
     blockdiag_glu_simt_kernel<__nv_bfloat16, true><<<grid, 256, 0, st>>>(
         (const __nv_bfloat16*)a->x, a->ldx, (const __nv_bfloat16*)a->wg, (__nv_bfloat16*)a->h, a->ldh,

@@ -307,8 +307,8 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
 }
 
 // ---------------------------------------------------------------------------------------
-// CUDA-core fallback with float32 accumulation: float32 tensors (the 1e-4 mode) and bf16 shapes the TMA
-// path does not take (strides that are not multiples of 8 elements).  Arbitrary element strides.
+// CUDA-core fallback with float32 accumulation: float32 tensors that gemm_f32.cu does not take (rows that are not
+// 16-byte aligned, time-contiguous input) and bf16 shapes the TMA path does not take (strides that are not multiples of 8 elements).  Arbitrary element strides.
 // ---------------------------------------------------------------------------------------
 template <typename T, bool ROUND>
 __global__ void __launch_bounds__(256)
@@ -458,6 +458,7 @@ extern "C" int m2_linear_fwd(const m2_linear_args* a, void* stream) {
   if (!tc_ok) {
     dim3 grid((N + 63) / 64, (unsigned)((tokens + 63) / 64));
     M2_REQUIRE(grid.y <= 65535, M2_ERR_UNSUPPORTED, "m2_linear_fwd: too many tokens for the CUDA-core kernel");
+    if (linear_f32_supported(a)) return linear_f32_launch(a, st);
     if (a->dtype == M2_BF16)
       lin::linear_simt_kernel<__nv_bfloat16, true><<<grid, 256, 0, st>>>(
           (const __nv_bfloat16*)a->x, a->x_sb, a->x_st, a->x_sc, (const __nv_bfloat16*)a->w, a->bias, (__nv_bfloat16*)a->out,
