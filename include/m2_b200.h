@@ -26,7 +26,7 @@
 extern "C" {
 #endif
 
-#define M2_B200_ABI_VERSION 3
+#define M2_B200_ABI_VERSION 4
 
 typedef enum { M2_F32 = 0, M2_BF16 = 1, M2_F16 = 2 /* only where an entry point says so */ } m2_dtype;
 
@@ -204,13 +204,15 @@ int m2_longconv_fwd(const m2_longconv_args* args, void* stream);
  * layer input that kind 3 of m2_longconv_fwd loads as a tensor-core operand.  Part of the
  * `u.transpose(-1, -2)` layout change of bert/src/mm/monarch_mixer_sequence_mixer.py:109.
  *   src (batch, seq_len, d_model) of src_dtype (M2_F32 or M2_BF16) with strides in elements;
- *   dst fp16, element (c, b, t) at dst[c*dst_sc + b*dst_sb + t].
+ *   dst fp16, element (c, b, t) at dst[c*dst_sc + b*dst_sb + t];
+ *   rows_bf16 NULL or a bf16 copy with contiguous channels, written in the same pass.
  * ------------------------------------------------------------------------------------- */
 typedef struct {
   int batch, seq_len, d_model;
   m2_dtype src_dtype;
   const void* src; long long src_sb, src_st, src_sc;
   void* dst;       long long dst_sb, dst_sc;
+  void* rows_bf16; long long rows_sb, rows_st;  /* optional: the same values as bf16 rows, (b, t, c) at b*rows_sb + t*rows_st + c */
 } m2_time_major_args;
 
 int m2_time_major_f16(const m2_time_major_args* args, void* stream);

@@ -10,7 +10,7 @@ import os
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libm2b200.so")
-ABI_VERSION = 3
+ABI_VERSION = 4
 
 M2_F32, M2_BF16, M2_F16 = 0, 1, 2
 
@@ -48,6 +48,7 @@ class TimeMajorArgs(C.Structure):
         ("batch", C.c_int), ("seq_len", C.c_int), ("d_model", C.c_int), ("src_dtype", C.c_int),
         ("src", C.c_void_p), ("src_sb", C.c_longlong), ("src_st", C.c_longlong), ("src_sc", C.c_longlong),
         ("dst", C.c_void_p), ("dst_sb", C.c_longlong), ("dst_sc", C.c_longlong),
+        ("rows_bf16", C.c_void_p), ("rows_sb", C.c_longlong), ("rows_st", C.c_longlong),
     ]
 
 

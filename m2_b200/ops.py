@@ -169,8 +169,9 @@ def filter_spectrum(k: torch.Tensor, seq_len: int, kind: int, bias=None) -> torc
     return spec
 
 
-def time_major_f16(u: torch.Tensor, out=None) -> torch.Tensor:
-    """fp16 copy of u (B, L, D) laid out (D, B, L): the residual-filter operand of kind 3."""
+def time_major_f16(u: torch.Tensor, out=None, rows=None) -> torch.Tensor:
+    """fp16 copy of u (B, L, D) laid out (D, B, L): the residual-filter operand of kind 3.  rows: optional (B, L, D) bf16
+    tensor with contiguous channels that receives u rounded to bf16 in the same pass."""
     _need_cuda(u)
     B, L, D = u.shape
     if out is None:
@@ -180,6 +181,9 @@ def time_major_f16(u: torch.Tensor, out=None) -> torch.Tensor:
     a.batch, a.seq_len, a.d_model, a.src_dtype = B, L, D, _dt(u)
     a.src, (a.src_sb, a.src_st, a.src_sc) = u.data_ptr(), u.stride()
     a.dst, a.dst_sc, a.dst_sb = out.data_ptr(), out.stride(0), out.stride(1)
+    if rows is not None:
+        assert rows.dtype == torch.bfloat16 and rows.shape == (B, L, D) and rows.stride(2) == 1
+        a.rows_bf16, a.rows_sb, a.rows_st = rows.data_ptr(), rows.stride(0), rows.stride(1)
     _launch("m2_time_major_f16", u, _lib.lib().m2_time_major_f16, C.byref(a))
     return out
 

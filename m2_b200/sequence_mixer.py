@@ -134,8 +134,12 @@ class MonarchMixerSequenceMixing(nn.Module):
         dev = u.device
         rec = copies_of(u)
         x = rec.bf16 if rec is not None else None                                # (B*L, D) from the LayerNorm
+        rows = None                              # bf16 rows to be written together with the time-major copy below
         if x is None or L != Lp or x.shape != (B * L, D) or x.device != dev or not x.is_contiguous():
-            if L == Lp:
+            if ures is u and u.dtype == torch.float32 and (rec is None or rec.tm is None or L != Lp):
+                x = torch.empty((B, Lp, D), dtype=torch.bfloat16, device=dev)
+                rows = x[:, :L]
+            elif L == Lp:
                 x = u.to(torch.bfloat16).contiguous()
             else:
                 x = torch.empty((B, Lp, D), dtype=torch.bfloat16, device=dev)
@@ -144,9 +148,9 @@ class MonarchMixerSequenceMixing(nn.Module):
         if ures is not None:
             rec = copies_of(ures)
             u_t = rec.tm if rec is not None else None                            # (D, B, L) fp16 from the LayerNorm
-            if u_t is None or u_t.shape != (D, B, Lp) or L != Lp or u_t.device != dev or not u_t.is_contiguous():
+            if rows is not None or u_t is None or u_t.shape != (D, B, Lp) or L != Lp or u_t.device != dev or not u_t.is_contiguous():
                 u_t = torch.empty((D, B, Lp), dtype=torch.float16, device=dev)
-                ops.time_major_f16(ures if ures.dtype in (torch.float32, torch.bfloat16) else ures.float(), out=u_t[:, :, :L])
+                ops.time_major_f16(ures if ures.dtype in (torch.float32, torch.bfloat16) else ures.float(), out=u_t[:, :, :L], rows=rows)
         yu_bf16 = ures is not None and src_dtype_of(ures) == torch.bfloat16
         if not hasattr(self, "_plans"):
             self._plans = PlanCache()

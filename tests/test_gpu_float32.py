@@ -74,3 +74,18 @@ def test_long_convolution(B, L, D, residual):
     y, ref = run(xin, u), run(along_time(xin), along_time(u))
     # 2 lg(2L) + 6 float32 roundings on each side, each below 2^-24 of the values' norm
     assert (y - ref).norm() / ref.norm() < 2 ** -24 * 2 * (2 * max(1, L).bit_length() + 8), (y - ref).norm() / ref.norm()
+
+
+@pytest.mark.parametrize("B,L,D", [(1, 1, 4), (2, 8, 8), (3, 65, 100), (2, 130, 768), (1, 63, 68), (2, 9, 7)])
+@pytest.mark.parametrize("channels_contiguous", [True, False])
+def test_row_copies(B, L, D, channels_contiguous):
+    u = rand(B, L, D, scale=300.0)
+    u[0, 0, 0] = 1e6                                     # saturates in fp16
+    if not channels_contiguous:
+        u = u.transpose(1, 2).contiguous().transpose(1, 2)
+    Lp = (L + 7) // 8 * 8
+    tm = torch.full((D, B, Lp), float("nan"), dtype=torch.float16, device=DEV)
+    rows = torch.full((B, Lp, D), float("nan"), dtype=torch.bfloat16, device=DEV)
+    ops.time_major_f16(u, out=tm[:, :, :L], rows=rows[:, :L])
+    assert torch.equal(tm[:, :, :L], u.clamp(-65504, 65504).half().permute(2, 0, 1)) and torch.isnan(tm[:, :, L:]).all()
+    assert torch.equal(rows[:, :L], u.bfloat16()) and torch.isnan(rows[:, L:]).all()
