@@ -9,8 +9,9 @@
 // bank groups.  Three stages in flight are what a tile alone on its SM needs: with one (held in registers, transposed
 // on the way) a K step of 16 took 2300 clocks at 64 tokens, 512 of them multiplications.
 // Measured (us, L2 flushed; the one-element kernels first) for 768 -> 2304 / 768 -> 768 / GLU 768 -> 3072 / wo 3072 -> 768:
-// 64 tokens 74 / 70 / 37 / 80 -> 37 / 37 / 25 / 37; 1024: 159 / 92 / 121 / 98 -> 92 / 56 / 86 / 55; 8192: 1168 / 420 / 780 /
-// 410 -> 684 / 262 / 552 / 260, 58 % of the pipe.  There a third of the stalls are register-file conflicts at dispatch and as
+// 64 tokens 74 / 70 / 37 / 80 -> 37 / 37 / 25 / 37; 1024: 159 / 92 / 121 / 98 -> 92 / 57 / 86 / 55; 2048: 303 / 127 / 213 /
+// 129 -> 178 / 86 / 158 / 86 (113 for the 768-column ones with two small tiles on an SM instead of three); 8192: 1168 / 420 /
+// 780 / 410 -> 684 / 261 / 551 / 260, 58 % of the pipe.  There a third of the stalls are register-file conflicts at dispatch and as
 // many shared loads.  Packed f32x2 FMAs over pairs of k need twice the accumulators, so 8 x 4 outputs are all a thread holds
 // and shared memory (69 % busy) binds: 745 us at 8192 tokens.
 //
@@ -40,7 +41,7 @@ __device__ __forceinline__ void copy16(uint32_t dst, const float* src, const flo
 }
 
 template <int RM, bool GLU>
-__global__ void __launch_bounds__(THREADS, 2)
+__global__ void __launch_bounds__(THREADS, RM == 1 && !GLU ? 3 : 2)
 gemm_f32_kernel(const Params P) {
   constexpr int BM = 64 * RM, BN = 64, STAGE = (BM + BN) * PITCH;
   extern __shared__ __align__(16) unsigned char smem_raw[];
