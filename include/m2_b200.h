@@ -108,8 +108,8 @@ int m2_hyena_filter(const m2_filter_args* args, void* stream);
  * for bit, 15-35 % less time);
  * 3 = tcgen05 Toeplitz GEMMs with the batch as the M dimension (bf16, 16 <= seq_len <= 128, a
  * multiple of 8, batch >= 64; time-contiguous tensors, the residual input as fp16 from
- * m2_time_major_f16); 4 = tcgen05 block-Toeplitz GEMMs (bf16, seq_len <= 2048, any batch; time-contiguous
- * tensors, u as fp16 or bf16).  m2_longconv_kind() never returns 3; m2_longconv_kind_batch() does when
+ * m2_time_major_f16); 4 = tcgen05 block-Toeplitz GEMMs, direct float32 sums for a few short rows (bf16, seq_len <= 1024, any
+ * batch; time-contiguous tensors, u as fp16 or bf16).  m2_longconv_kind() never returns 3; m2_longconv_kind_batch() does when
  * the batch is large enough to fill the 128-row tiles.  Both answer for tensors whose rows are seq_len steps
  * apart: kind 2 for multiples of 4 only, never 4.  m2_longconv_pick() is the choice for a caller that lays
  * its time-contiguous rows out itself, every row on a 16-byte boundary and readable up to the next multiple of
