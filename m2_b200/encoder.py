@@ -228,7 +228,6 @@ class M2BertModel(nn.Module):
         self.encoder = M2BertEncoder(config)
         self.pooler = M2BertPooler(config) if add_pooling_layer else None
         self.check_finite = check_finite
-        self._plans = PlanCache()
 
     def _called_modules(self):
         """Every module whose forward() runs in the layer-by-layer path."""
@@ -285,6 +284,8 @@ class M2BertModel(nn.Module):
             return None
         B, L = input_ids.shape
         dev = input_ids.device
+        if not hasattr(self, "_plans"):          # absent from models pickled whole by earlier versions, too
+            self._plans = PlanCache()
         plan = self._plans.get(self, (B, L, dev.index), lambda: self._make_plan(B, L, dev))
         if plan is None or any_hooks(plan["called"]) or any_dropping(plan["dropping"]):
             return None

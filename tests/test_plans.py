@@ -101,6 +101,8 @@ def test_encoder_plan_follows_the_modules():
         return y
     first = out()
     assert torch.equal(first, out())
+    del model._plans                              # as in a model pickled whole before there were plans
+    assert torch.equal(first, out())
     layer = model.encoder.layer[1]
     for change in (lambda: layer.mlp.wo.bias.add_(1.0), lambda: layer.attention.filter_fn.bias.add_(1.0),
                    lambda: layer.attention.in_linear.weight.mul_(1.5), lambda: model.embeddings.word_embeddings.weight.mul_(-1.0)):
