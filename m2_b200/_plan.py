@@ -70,6 +70,15 @@ class PlanCache:
         return PlanCache, (self.most,)
 
 
+def expect(dev, *tensors):
+    """Raises unless every (tensor, shape) has that shape (None: any size) and lies on `dev`, a CUDA device."""
+    for t, shape in tensors:
+        if len(t.shape) != len(shape) or any(n is not None and n != m for m, n in zip(t.shape, shape)):
+            raise AssertionError(f"weight of shape {tuple(t.shape)} where {shape} is expected")
+        if t.device != dev:
+            raise RuntimeError(f"m2_b200 kernels need weights on the input's device: {t.device} and {dev}")
+
+
 def any_hooks(modules):
     """Whether a hook, or a forward() set on an instance, would see (or change) what goes through one of `modules`."""
     g = torch.nn.modules.module

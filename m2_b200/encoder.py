@@ -258,7 +258,7 @@ class M2BertModel(nn.Module):
         args = (_lib.EncoderLayer * len(layers))()
         keep = []
         for a, y in zip(args, layers):
-            keep.append((y.attention.fill_args(a, L, kind), y.mlp.fill_args(a)))
+            keep.append((y.attention.fill_args(a, L, kind, dev), y.mlp.fill_args(a, dev)))
         e = _lib.EncoderArgs()
         e.batch, e.seq_len, e.d_model, e.inter, e.nblocks = B, L, D, cfg.intermediate_size, cfg.monarch_mlp_nblocks
         e.n_layers, e.kind, e.n_filters = len(layers), kind, 2 if layers[0].attention.residual_long_conv else 1

@@ -10,7 +10,7 @@ import torch
 import torch.nn as nn
 
 from . import _lib, ops
-from ._plan import PlanCache
+from ._plan import PlanCache, expect
 from ._tags import attach, forward_only
 from .blockdiag_linear import BlockdiagLinear, _compute_dtype
 
@@ -38,28 +38,34 @@ class BertGatedLinearUnitMLP(nn.Module):
         self.dropout = nn.Dropout(config.hidden_dropout_prob)
         self.layernorm = nn.LayerNorm(config.hidden_size, eps=config.layer_norm_eps)
 
-    def fill_args(self, a):
+    def fill_args(self, a, dev):
         """Writes the pointers of this module's weights into a (_lib.MlpArgs or _lib.EncoderLayer); returns the tensors
-        that keep them alive."""
+        that keep them alive.  The native call sees pointers only, so what they point to is checked here against the
+        config and the device it runs on."""
+        D, inter, nb = self.config.hidden_size, self.config.intermediate_size, self.config.monarch_mlp_nblocks
+        expect(dev, (self.gated_layers.weight, (nb, 2 * inter // nb, D // nb)), (self.wo.weight, (nb, D // nb, inter // nb)),
+               (self.wo.bias, (D,)), (self.layernorm.weight, (D,)), (self.layernorm.bias, (D,)))
         keep = [self.gated_layers._weight_as(torch.bfloat16), self.wo._weight_as(torch.bfloat16)]
         keep += [ops._f32c(t) for t in (self.wo.bias, self.layernorm.weight, self.layernorm.bias)]
         a.wg, a.wo, a.wo_bias, a.ln_w, a.ln_b = (t.data_ptr() for t in keep)
         a.eps = float(self.layernorm.eps)
         return keep
 
-    def _plan(self):
+    def _plan(self, dev):
         if not hasattr(self, "_plans"):
             self._plans = PlanCache()
 
         def make():
             a = _lib.MlpArgs()
             a.d_model, a.inter, a.nblocks = self.config.hidden_size, self.config.intermediate_size, self.config.monarch_mlp_nblocks
-            return a, self.fill_args(a)
-        return self._plans.get(self, self.wo.bias.device.index, make)
+            return a, self.fill_args(a, dev)
+        return self._plans.get(self, dev.index, make)
 
     def _forward_bf16(self, x, x2, plan, copies_only):
         """The three launches as one call; outputs as in forward()."""
         B, L, D = x.shape
+        if D != self.config.hidden_size:
+            raise AssertionError(f"input has {D} features, the MLP {self.config.hidden_size}")
         m = B * L
         dev = x.device
         if not x2.is_contiguous():
@@ -95,7 +101,7 @@ class BertGatedLinearUnitMLP(nn.Module):
         if x2.dtype != dt:
             x2 = x2.to(dt)
         if dt == torch.bfloat16 and x.dim() == 3 and x2.shape[0] and x.shape[-1] % 256 == 0 and x.shape[-1] <= 2048 and not ops.observed():
-            plan = self._plan()
+            plan = self._plan(x.device)
             if plan is not None:
                 return self._forward_bf16(x, x2, plan, copies_only)
         h = ops.blockdiag_glu_fwd(x2, self.gated_layers._weight_as(dt), cfg.intermediate_size)

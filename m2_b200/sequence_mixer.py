@@ -10,7 +10,7 @@ import torch
 import torch.nn as nn
 
 from . import _lib, ops
-from ._plan import PlanCache
+from ._plan import PlanCache, expect
 from ._tags import copies_of, forward_only, src_dtype_of
 from .hyena_filter import HyenaFilter, _autocast_bf16
 
@@ -99,9 +99,14 @@ class MonarchMixerSequenceMixing(nn.Module):
     def filters(self):
         return [self.filter_fn, self.filter_fn2] if self.residual_long_conv else [self.filter_fn]
 
-    def fill_args(self, a, L, kind):
+    def fill_args(self, a, L, kind, dev):
         """Writes the pointers of this module's weights and filter tables into a (_lib.MixerArgs or _lib.EncoderLayer);
-        returns the tensors that keep them alive."""
+        returns the tensors that keep them alive.  The native call sees pointers only, so what they point to is checked
+        here against d_model and the device it runs on."""
+        D = self.d_model
+        expect(dev, (self.in_linear.weight, (3 * D, D)), (self.in_linear.bias, (3 * D,)), (self.out_linear.weight, (D, D)),
+               (self.out_linear.bias, (D,)), (self.short_filter.weight, (3 * D, 1, 3)), (self.short_filter.bias, (3 * D,)),
+               *((f.bias, (D,)) for f in self.filters()), *((f.implicit_filter[6].weight, (D, None)) for f in self.filters()))
         w_in, w_out = self._weights()
         f32 = [ops._f32c(t) for t in (self.in_linear.bias, self.short_filter.weight, self.short_filter.bias, self.out_linear.bias)]
         a.w_in, a.w_out = w_in.data_ptr(), w_out.data_ptr()
@@ -117,19 +122,21 @@ class MonarchMixerSequenceMixing(nn.Module):
                 keep.append(b)
         return keep
 
-    def _make_plan(self, B, L, kind):
+    def _make_plan(self, B, L, kind, dev):
         a = _lib.MixerArgs()
         Lp = _round_up(L, 8)
         a.batch, a.seq_len, a.pitch, a.out_pitch, a.d_model = B, L, Lp, L, self.d_model
         a.kind, a.n_filters = kind, 2 if self.residual_long_conv else 1
         a.stride, a.u_stride = _round_up(B * Lp, 16), B * Lp
-        return a, self.fill_args(a, L, kind)
+        return a, self.fill_args(a, L, kind, dev)
 
     def _forward_bf16(self, u, ures, kind):
         """bf16 path: the convolution kernels work on channel-major, time-contiguous rows -- in_linear writes (3D, B, L)
         and out_linear reads (D, B, L) through the operand arrangements of m2_linear_fwd, no transposed copy of an
         activation.  Rows are padded to a multiple of 8 steps so that every one starts on a 16-byte boundary."""
         B, L, D = u.shape
+        if D != self.d_model:
+            raise AssertionError(f"input has {D} channels, the mixer {self.d_model}")
         Lp = _round_up(L, 8)
         dev = u.device
         rec = copies_of(u)
@@ -154,7 +161,7 @@ class MonarchMixerSequenceMixing(nn.Module):
         yu_bf16 = ures is not None and src_dtype_of(ures) == torch.bfloat16
         if not hasattr(self, "_plans"):
             self._plans = PlanCache()
-        plan = self._plans.get(self, (B, L, kind, dev.index), lambda: self._make_plan(B, L, kind))
+        plan = self._plans.get(self, (B, L, kind, dev.index), lambda: self._make_plan(B, L, kind, dev))
         stride = _round_up(B * Lp, 16)
         # allocated per call: inside a CUDA-graph capture the buffers then belong to the graph's own pool
         work = torch.empty((4 * D, stride), dtype=torch.bfloat16, device=dev)

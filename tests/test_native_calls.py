@@ -1,0 +1,77 @@
+"""What the modules hand to the one-call entry points (m2_mixer_fwd, m2_mlp_fwd, m2_encoder_fwd), which see pointers and sizes
+and no tensors.  On the CPU with the launch replaced by a recorder: nothing here reaches a GPU."""
+import pytest
+import torch
+import torch.nn as nn
+
+from m2_b200 import BertGatedLinearUnitMLP, MonarchMixerSequenceMixing, ops
+from tests.helpers import Cfg
+
+D, INTER = 256, 512
+
+
+@pytest.fixture
+def calls(monkeypatch):
+    """Names of the launches that would have been made."""
+    names = []
+    monkeypatch.setattr(ops, "_need_cuda", lambda *a: None)
+    monkeypatch.setattr(ops, "_launch", lambda name, *a, **k: names.append(name))
+    return names
+
+
+def mixer(d=D):
+    return MonarchMixerSequenceMixing(d, l_max=128, bidirectional=True, hyena_emb_dim=5, hyena_filter_order=16,
+                                      residual_long_conv=True, hyena_kernel_lr=1e-3).eval()
+
+
+def mlp(d=D, inter=INTER, nblocks=4):
+    return BertGatedLinearUnitMLP(Cfg(hidden_size=d, intermediate_size=inter, monarch_mlp_nblocks=nblocks, layer_norm_eps=1e-12,
+                                      hidden_dropout_prob=0.0)).eval()
+
+
+def mix(m, u, kind=4):
+    with torch.no_grad():
+        return m._forward_bf16(u, u, kind)
+
+
+def feed(m, x):
+    with torch.no_grad():
+        x2 = x.reshape(-1, x.shape[-1]).to(torch.bfloat16)
+        return m._forward_bf16(x, x2, m._plan(x.device), False)
+
+
+def test_right_widths_are_launched(calls):
+    assert mix(mixer(), torch.zeros(2, 128, D)).shape == (2, 128, D) and calls[-1] == "m2_mixer_fwd"
+    assert feed(mlp(), torch.zeros(2, 128, D)).shape == (2, 128, D) and calls[-1] == "m2_mlp_fwd"
+
+
+@pytest.mark.parametrize("width", [D - 8, D + 8, 2 * D])
+def test_another_width_is_refused(calls, width):
+    with pytest.raises(AssertionError):
+        mix(mixer(), torch.zeros(2, 128, width))
+    with pytest.raises(AssertionError):
+        feed(mlp(), torch.zeros(2, 128, width))
+    assert not calls
+
+
+@pytest.mark.parametrize("run,module,edit", [
+    (mix, mixer, lambda m: setattr(m, "in_linear", nn.Linear(D, 3 * D - 3))),
+    (mix, mixer, lambda m: setattr(m, "out_linear", nn.Linear(D - 1, D))),
+    (mix, mixer, lambda m: setattr(m, "short_filter", nn.Conv1d(3 * D, 3 * D, 5, groups=3 * D))),
+    (mix, mixer, lambda m: setattr(m, "filter_fn2", mixer(D // 2).filter_fn)),
+    (feed, mlp, lambda m: setattr(m, "wo", mlp(inter=INTER // 2).wo)),
+    (feed, mlp, lambda m: setattr(m, "gated_layers", mlp(nblocks=2).gated_layers)),
+    (feed, mlp, lambda m: setattr(m, "layernorm", nn.LayerNorm(D // 2)))])
+def test_weights_of_another_shape_are_refused(calls, run, module, edit):
+    m = module()
+    edit(m)
+    with pytest.raises(AssertionError):
+        run(m, torch.zeros(2, 128, D))
+    assert not {"m2_mixer_fwd", "m2_mlp_fwd"} & set(calls)
+
+
+@pytest.mark.parametrize("run,module", [(mix, mixer), (feed, mlp)])
+def test_weights_on_another_device_are_refused(calls, run, module):
+    with pytest.raises(RuntimeError, match="device"):
+        run(module().to("meta"), torch.zeros(2, 128, D))
+    assert not {"m2_mixer_fwd", "m2_mlp_fwd"} & set(calls)
