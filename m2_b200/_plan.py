@@ -71,8 +71,10 @@ class PlanCache:
 
 
 def expect(dev, *tensors):
-    """Raises unless every (tensor, shape) has that shape (None: any size) and lies on `dev`, a CUDA device."""
+    """Raises unless every (tensor, shape) has that shape (None: any size) and lies on `dev`; a missing tensor is not looked at."""
     for t, shape in tensors:
+        if t is None:
+            continue
         if len(t.shape) != len(shape) or any(n is not None and n != m for m, n in zip(t.shape, shape)):
             raise AssertionError(f"weight of shape {tuple(t.shape)} where {shape} is expected")
         if t.device != dev:

@@ -46,8 +46,11 @@ class BertGatedLinearUnitMLP(nn.Module):
         expect(dev, (self.gated_layers.weight, (nb, 2 * inter // nb, D // nb)), (self.wo.weight, (nb, D // nb, inter // nb)),
                (self.wo.bias, (D,)), (self.layernorm.weight, (D,)), (self.layernorm.bias, (D,)))
         keep = [self.gated_layers._weight_as(torch.bfloat16), self.wo._weight_as(torch.bfloat16)]
-        keep += [ops._f32c(t) for t in (self.wo.bias, self.layernorm.weight, self.layernorm.bias)]
-        a.wg, a.wo, a.wo_bias, a.ln_w, a.ln_b = (t.data_ptr() for t in keep)
+        keep += [ops._f32c(t) for t in (self.layernorm.weight, self.layernorm.bias)]
+        a.wg, a.wo, a.ln_w, a.ln_b = (t.data_ptr() for t in keep)
+        if self.wo.bias is not None:
+            keep.append(ops._f32c(self.wo.bias))
+            a.wo_bias = keep[-1].data_ptr()
         a.eps = float(self.layernorm.eps)
         return keep
 

@@ -108,9 +108,13 @@ class MonarchMixerSequenceMixing(nn.Module):
                (self.out_linear.bias, (D,)), (self.short_filter.weight, (3 * D, 1, 3)), (self.short_filter.bias, (3 * D,)),
                *((f.bias, (D,)) for f in self.filters()), *((f.implicit_filter[6].weight, (D, None)) for f in self.filters()))
         w_in, w_out = self._weights()
-        f32 = [ops._f32c(t) for t in (self.in_linear.bias, self.short_filter.weight, self.short_filter.bias, self.out_linear.bias)]
+        f32 = [ops._f32c(self.short_filter.weight), ops._f32c(self.short_filter.bias)]
         a.w_in, a.w_out = w_in.data_ptr(), w_out.data_ptr()
-        a.b_in, a.short_w, a.short_b, a.b_out = (t.data_ptr() for t in f32)
+        a.short_w, a.short_b = (t.data_ptr() for t in f32)
+        for name, bias in (("b_in", self.in_linear.bias), ("b_out", self.out_linear.bias)):
+            if bias is not None:
+                f32.append(ops._f32c(bias))
+                setattr(a, name, f32[-1].data_ptr())
         keep = [w_in, w_out] + f32
         for i, f in enumerate(self.filters()):
             spec = f.spectrum(L, True, kind)

@@ -75,3 +75,14 @@ def test_weights_on_another_device_are_refused(calls, run, module):
     with pytest.raises(RuntimeError, match="device"):
         run(module().to("meta"), torch.zeros(2, 128, D))
     assert not {"m2_mixer_fwd", "m2_mlp_fwd"} & set(calls)
+
+
+def test_linear_layers_without_bias(calls):
+    m, f = mixer(), mlp()
+    m.in_linear, m.out_linear = nn.Linear(D, 3 * D, bias=False), nn.Linear(D, D, bias=False)
+    f.wo.bias = None
+    mix(m, torch.zeros(2, 128, D))
+    feed(f, torch.zeros(2, 128, D))
+    assert calls[-1] == "m2_mlp_fwd" and "m2_mixer_fwd" in calls
+    (a, _), (b, _) = m._make_plan(2, 128, 4, torch.device("cpu")), f._plan(torch.device("cpu"))
+    assert a.b_in is None and a.b_out is None and b.wo_bias is None and a.w_in and b.ln_b
