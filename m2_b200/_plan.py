@@ -1,6 +1,7 @@
 """What the modules lay out once per shape and keep for the next call: kernel arguments with the pointers of weights and
 filter tables filled in.  A plan is used again only while every parameter, buffer and submodule it was made from is the
-same object with the same storage and version counter; activations, workspaces and outputs are never kept.
+same object with the same storage and version counter; activations, workspaces, outputs and copies of parameters are never
+kept.
 """
 from __future__ import annotations
 
@@ -8,6 +9,8 @@ from collections import OrderedDict
 from operator import attrgetter, is_
 
 import torch
+
+from . import ops
 
 _version = attrgetter("_version")
 _ptr = torch.Tensor.data_ptr
@@ -36,6 +39,41 @@ class Watch:
             return False
 
 
+class Plan:
+    """Arguments of a native call with the pointers of weights and filter tables filled in.
+
+    `held` keeps alive what the module's own caches made (bf16 weights, filter tables); registered tensors are not held, as
+    Watch sees when they go.  Where a tensor had to be copied (a parameter that is not contiguous float32) the plan is not
+    `lasting`: the copy then belongs to one call, to its stream and, inside a CUDA-graph capture, to the graph's own pool,
+    and a captured graph never points to what only a plan keeps."""
+
+    def __init__(self, args, **more):
+        self.args, self.held, self.lasting = args, [], True
+        self.__dict__.update(more)
+
+    def cached(self, t):
+        """Pointer of a tensor that a cache of the module holds as long as its source does not change."""
+        self.held.append(t)
+        return t.data_ptr()
+
+    def registered(self, t, source):
+        """Pointer of `t`, the parameter or buffer `source` itself or a copy of it."""
+        if t.data_ptr() != source.data_ptr():
+            self.held.append(t)
+            self.lasting = False
+        return t.data_ptr()
+
+    def f32(self, source):
+        """Pointer of a parameter or buffer as contiguous float32."""
+        return self.registered(ops._f32c(source), source)
+
+    def passing(self, t):
+        """Pointer of a tensor made for this call."""
+        self.held.append(t)
+        self.lasting = False
+        return t.data_ptr()
+
+
 class PlanCache:
     """At most `most` plans of one module, the longest unused dropped first."""
 
@@ -55,6 +93,8 @@ class PlanCache:
         plan = plans.get(key)
         if plan is None:
             plan = make()
+            if not getattr(plan, "lasting", True):
+                return plan
             plans[key] = plan
             while len(plans) > self.most:
                 try:

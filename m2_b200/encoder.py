@@ -19,7 +19,7 @@ import torch
 import torch.nn as nn
 
 from . import _lib, ops
-from ._plan import PlanCache, any_dropping, any_hooks
+from ._plan import Plan, PlanCache, any_dropping, any_hooks
 from ._tags import attach
 from .glu_mlp import BertGatedLinearUnitMLP
 from .hyena_filter import _autocast_bf16
@@ -256,25 +256,24 @@ class M2BertModel(nn.Module):
         if kind < 2:
             return None
         args = (_lib.EncoderLayer * len(layers))()
-        keep = []
-        for a, y in zip(args, layers):
-            keep.append((y.attention.fill_args(a, L, kind, dev), y.mlp.fill_args(a, dev)))
         e = _lib.EncoderArgs()
+        work = _lib.lib().m2_encoder_workspace(B, (L + 7) // 8 * 8, D, cfg.intermediate_size)
+        plan = Plan(e, layers=args, work=work, out=(B, L, D), called=called, dropping=[m for m in called if hasattr(m, "dropout")])
+        for a, y in zip(args, layers):
+            y.attention.fill_args(plan, a, L, kind, dev)
+            y.mlp.fill_args(plan, a, dev)
         e.batch, e.seq_len, e.d_model, e.inter, e.nblocks = B, L, D, cfg.intermediate_size, cfg.monarch_mlp_nblocks
         e.n_layers, e.kind, e.n_filters = len(layers), kind, 2 if layers[0].attention.residual_long_conv else 1
-        tables = [emb.word_embeddings.weight, emb.token_type_embeddings.weight]
+        word, types = emb.word_embeddings.weight, emb.token_type_embeddings.weight
+        e.embed.word_table, e.embed.vocab_rows = plan.f32(word), word.shape[0]
+        e.embed.type_table, e.embed.type_rows = plan.f32(types), types.shape[0]
         if emb.use_positional_encodings:
-            tables.append(emb.position_embeddings.weight)
-        tables = [ops._f32c(t) for t in tables + [emb.LayerNorm.weight, emb.LayerNorm.bias]]
-        e.embed.word_table, e.embed.type_table = tables[0].data_ptr(), tables[1].data_ptr()
-        e.embed.vocab_rows, e.embed.type_rows = tables[0].shape[0], tables[1].shape[0]
-        if emb.use_positional_encodings:
-            e.embed.pos_table, e.embed.pos_rows = tables[2].data_ptr(), tables[2].shape[0]
-        e.embed.weight, e.embed.bias, e.embed.eps = tables[-2].data_ptr(), tables[-1].data_ptr(), float(emb.LayerNorm.eps)
+            pos = emb.position_embeddings.weight
+            e.embed.pos_table, e.embed.pos_rows = plan.f32(pos), pos.shape[0]
+        norm = emb.LayerNorm
+        e.embed.weight, e.embed.bias, e.embed.eps = plan.f32(norm.weight), plan.f32(norm.bias), float(norm.eps)
         e.layers = C.cast(args, C.POINTER(_lib.EncoderLayer))
-        work = _lib.lib().m2_encoder_workspace(B, (L + 7) // 8 * 8, D, cfg.intermediate_size)
-        return dict(args=e, keep=(args, keep, tables), work=work, out=(B, L, D), called=called,
-                    dropping=[m for m in called if hasattr(m, "dropout")])
+        return plan
 
     def _encode_whole(self, input_ids, token_type_ids, position_ids):
         """Embeddings and all layers as one native call: bf16 autocast, no gradients, no hooks on the way.  None where the
@@ -287,15 +286,15 @@ class M2BertModel(nn.Module):
         if not hasattr(self, "_plans"):          # absent from models pickled whole by earlier versions, too
             self._plans = PlanCache()
         plan = self._plans.get(self, (B, L, dev.index), lambda: self._make_plan(B, L, dev))
-        if plan is None or any_hooks(plan["called"]) or any_dropping(plan["dropping"]):
+        if plan is None or any_hooks(plan.called) or any_dropping(plan.dropping):
             return None
 
         def ids64(t):
             return t.expand(B, L).to(torch.long).contiguous() if t is not None else None
         ids = [ids64(input_ids), ids64(token_type_ids), ids64(position_ids)]
-        out = torch.empty(plan["out"], dtype=torch.float32, device=dev)
-        work = torch.empty(plan["work"], dtype=torch.uint8, device=dev)
-        a = _lib.EncoderArgs.from_buffer_copy(plan["args"])
+        out = torch.empty(plan.out, dtype=torch.float32, device=dev)
+        work = torch.empty(plan.work, dtype=torch.uint8, device=dev)
+        a = _lib.EncoderArgs.from_buffer_copy(plan.args)
         a.embed.input_ids = ids[0].data_ptr()
         if ids[1] is not None:
             a.embed.token_type_ids = ids[1].data_ptr()

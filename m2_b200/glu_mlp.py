@@ -10,7 +10,7 @@ import torch
 import torch.nn as nn
 
 from . import _lib, ops
-from ._plan import PlanCache, expect
+from ._plan import Plan, PlanCache, expect
 from ._tags import attach, forward_only
 from .blockdiag_linear import BlockdiagLinear, _compute_dtype
 
@@ -38,21 +38,18 @@ class BertGatedLinearUnitMLP(nn.Module):
         self.dropout = nn.Dropout(config.hidden_dropout_prob)
         self.layernorm = nn.LayerNorm(config.hidden_size, eps=config.layer_norm_eps)
 
-    def fill_args(self, a, dev):
-        """Writes the pointers of this module's weights into a (_lib.MlpArgs or _lib.EncoderLayer); returns the tensors
-        that keep them alive.  The native call sees pointers only, so what they point to is checked here against the
-        config and the device it runs on."""
+    def fill_args(self, plan, a, dev):
+        """Writes the pointers of this module's weights into `a` (a _lib.MlpArgs or _lib.EncoderLayer) of `plan`.  The native
+        call sees pointers only, so what they point to is checked here against the config and the device it runs on."""
         D, inter, nb = self.config.hidden_size, self.config.intermediate_size, self.config.monarch_mlp_nblocks
         expect(dev, (self.gated_layers.weight, (nb, 2 * inter // nb, D // nb)), (self.wo.weight, (nb, D // nb, inter // nb)),
                (self.wo.bias, (D,)), (self.layernorm.weight, (D,)), (self.layernorm.bias, (D,)))
-        keep = [self.gated_layers._weight_as(torch.bfloat16), self.wo._weight_as(torch.bfloat16)]
-        keep += [ops._f32c(t) for t in (self.layernorm.weight, self.layernorm.bias)]
-        a.wg, a.wo, a.ln_w, a.ln_b = (t.data_ptr() for t in keep)
+        for name, lin in (("wg", self.gated_layers), ("wo", self.wo)):
+            w = lin._weight_as(torch.bfloat16)
+            setattr(a, name, plan.registered(w, lin.weight) if lin.weight.dtype == torch.bfloat16 else plan.cached(w))
         if self.wo.bias is not None:
-            keep.append(ops._f32c(self.wo.bias))
-            a.wo_bias = keep[-1].data_ptr()
-        a.eps = float(self.layernorm.eps)
-        return keep
+            a.wo_bias = plan.f32(self.wo.bias)
+        a.ln_w, a.ln_b, a.eps = plan.f32(self.layernorm.weight), plan.f32(self.layernorm.bias), float(self.layernorm.eps)
 
     def _plan(self, dev):
         if not hasattr(self, "_plans"):
@@ -61,7 +58,9 @@ class BertGatedLinearUnitMLP(nn.Module):
         def make():
             a = _lib.MlpArgs()
             a.d_model, a.inter, a.nblocks = self.config.hidden_size, self.config.intermediate_size, self.config.monarch_mlp_nblocks
-            return a, self.fill_args(a, dev)
+            plan = Plan(a)
+            self.fill_args(plan, a, dev)
+            return plan
         return self._plans.get(self, dev.index, make)
 
     def _forward_bf16(self, x, x2, plan, copies_only):
@@ -77,7 +76,7 @@ class BertGatedLinearUnitMLP(nn.Module):
         aug = torch.empty((m, D), dtype=torch.bfloat16, device=dev)
         tm = torch.empty((D, B, L), dtype=torch.float16, device=dev) if L % 8 == 0 else None
         y = aug.view(B, L, D) if copies_only and tm is not None else torch.empty((B, L, D), dtype=torch.float32, device=dev)
-        a = _lib.MlpArgs.from_buffer_copy(plan[0])
+        a = _lib.MlpArgs.from_buffer_copy(plan.args)
         a.m, a.seq_len = m, L
         a.x, a.h = x2.data_ptr(), work.data_ptr()
         a.o = a.h + 2 * m * self.config.intermediate_size

@@ -10,7 +10,7 @@ import torch
 import torch.nn as nn
 
 from . import _lib, ops
-from ._plan import PlanCache, expect
+from ._plan import Plan, PlanCache, expect
 from ._tags import copies_of, forward_only, src_dtype_of
 from .hyena_filter import HyenaFilter, _autocast_bf16
 
@@ -99,32 +99,24 @@ class MonarchMixerSequenceMixing(nn.Module):
     def filters(self):
         return [self.filter_fn, self.filter_fn2] if self.residual_long_conv else [self.filter_fn]
 
-    def fill_args(self, a, L, kind, dev):
-        """Writes the pointers of this module's weights and filter tables into a (_lib.MixerArgs or _lib.EncoderLayer);
-        returns the tensors that keep them alive.  The native call sees pointers only, so what they point to is checked
-        here against d_model and the device it runs on."""
+    def fill_args(self, plan, a, L, kind, dev):
+        """Writes the pointers of this module's weights and filter tables into `a` (a _lib.MixerArgs or _lib.EncoderLayer)
+        of `plan`.  The native call sees pointers only, so what they point to is checked here against d_model and the
+        device it runs on."""
         D = self.d_model
         expect(dev, (self.in_linear.weight, (3 * D, D)), (self.in_linear.bias, (3 * D,)), (self.out_linear.weight, (D, D)),
                (self.out_linear.bias, (D,)), (self.short_filter.weight, (3 * D, 1, 3)), (self.short_filter.bias, (3 * D,)),
                *((f.bias, (D,)) for f in self.filters()), *((f.implicit_filter[6].weight, (D, None)) for f in self.filters()))
-        w_in, w_out = self._weights()
-        f32 = [ops._f32c(self.short_filter.weight), ops._f32c(self.short_filter.bias)]
-        a.w_in, a.w_out = w_in.data_ptr(), w_out.data_ptr()
-        a.short_w, a.short_b = (t.data_ptr() for t in f32)
-        for name, bias in (("b_in", self.in_linear.bias), ("b_out", self.out_linear.bias)):
-            if bias is not None:
-                f32.append(ops._f32c(bias))
-                setattr(a, name, f32[-1].data_ptr())
-        keep = [w_in, w_out] + f32
+        a.w_in, a.w_out = (plan.cached(w) for w in self._weights())
+        a.short_w, a.short_b = plan.f32(self.short_filter.weight), plan.f32(self.short_filter.bias)
+        if self.in_linear.bias is not None:
+            a.b_in = plan.f32(self.in_linear.bias)
+        if self.out_linear.bias is not None:
+            a.b_out = plan.f32(self.out_linear.bias)
         for i, f in enumerate(self.filters()):
-            spec = f.spectrum(L, True, kind)
-            a.spec[i] = spec.data_ptr()
-            keep.append(spec)
+            a.spec[i] = plan.cached(f.spectrum(L, True, kind))
             if kind == 2:
-                b = ops._f32c(f.conv_bias())
-                a.bias[i] = b.data_ptr()
-                keep.append(b)
-        return keep
+                a.bias[i] = plan.f32(f.bias) if f.use_bias else plan.passing(ops._f32c(f.conv_bias()))
 
     def _make_plan(self, B, L, kind, dev):
         a = _lib.MixerArgs()
@@ -132,7 +124,9 @@ class MonarchMixerSequenceMixing(nn.Module):
         a.batch, a.seq_len, a.pitch, a.out_pitch, a.d_model = B, L, Lp, L, self.d_model
         a.kind, a.n_filters = kind, 2 if self.residual_long_conv else 1
         a.stride, a.u_stride = _round_up(B * Lp, 16), B * Lp
-        return a, self.fill_args(a, L, kind, dev)
+        plan = Plan(a)
+        self.fill_args(plan, a, L, kind, dev)
+        return plan
 
     def _forward_bf16(self, u, ures, kind):
         """bf16 path: the convolution kernels work on channel-major, time-contiguous rows -- in_linear writes (3D, B, L)
@@ -172,7 +166,7 @@ class MonarchMixerSequenceMixing(nn.Module):
         y = torch.empty((B, L, D), dtype=torch.bfloat16, device=dev)
         if plan is None or ops.observed():
             return self._launch_singly(x, u_t, work, y, kind, yu_bf16)
-        a = _lib.MixerArgs.from_buffer_copy(plan[0])
+        a = _lib.MixerArgs.from_buffer_copy(plan.args)
         a.x, a.u = x.data_ptr(), u_t.data_ptr() if u_t is not None else None
         a.yu_bf16 = yu_bf16
         a.xin = work.data_ptr()

@@ -84,5 +84,47 @@ def test_linear_layers_without_bias(calls):
     mix(m, torch.zeros(2, 128, D))
     feed(f, torch.zeros(2, 128, D))
     assert calls[-1] == "m2_mlp_fwd" and "m2_mixer_fwd" in calls
-    (a, _), (b, _) = m._make_plan(2, 128, 4, torch.device("cpu")), f._plan(torch.device("cpu"))
+    a, b = m._make_plan(2, 128, 4, torch.device("cpu")).args, f._plan(torch.device("cpu")).args
     assert a.b_in is None and a.b_out is None and b.wo_bias is None and a.w_in and b.ln_b
+
+
+def plans(m):
+    return list(m._plans.plans.values())
+
+
+def test_plans_keep_no_copies_and_no_parameters(calls):
+    """A CUDA graph bakes the addresses of a plan in and outlives it, another stream may use them, and model.cpu() is to free
+    the GPU's memory: so a plan that is kept points to registered tensors and to the module's caches, and holds only the latter."""
+    m, f = mixer(), mlp()
+    mix(m, torch.zeros(2, 128, D))
+    feed(f, torch.zeros(2, 128, D))
+    for module in (m, f):
+        own = {t.data_ptr() for t in module.parameters()}
+        assert len(plans(module)) == 1 and not own & {t.data_ptr() for t in plans(module)[0].held}
+    for module, run in ((m, mix), (f, feed)):
+        module.bfloat16()                            # float32 copies of biases, taps and LayerNorm belong to each call
+        run(module, torch.zeros(2, 128, D))
+        run(module, torch.zeros(2, 128, D))
+        assert not plans(module)
+    m = mixer()
+    m.filter_fn.use_bias = False                     # kind 2 takes a vector of zeros for it
+    mix(m, torch.zeros(2, 256, D)[:, :128], kind=2)
+    assert not plans(m)
+
+
+@pytest.mark.gpu
+def test_a_graph_outlives_the_plans_it_was_captured_with():
+    from m2_b200 import GraphedForward
+    torch.manual_seed(3)
+    m, f = mixer().cuda().bfloat16(), mlp().cuda().bfloat16()
+
+    def layer(u):
+        return f(m(u)[0])
+    u = torch.randn(4, 128, D, device="cuda")
+    graphed = GraphedForward(layer, u)
+    want = graphed(u).clone()
+    with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16):
+        for n in range(1, 20):
+            layer(u[:, :4 * n])
+    junk = [torch.full((n,), 1e30, device="cuda") for n in (D, 3 * D, 9 * D, D, 3 * D) for _ in range(50)]
+    assert torch.equal(graphed(u), want) and len(junk) == 250
