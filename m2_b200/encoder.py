@@ -252,6 +252,8 @@ class M2BertModel(nn.Module):
                  y.attention.residual_long_conv) for y in layers}
         if dims != {(D, D, cfg.intermediate_size, cfg.monarch_mlp_nblocks, layers[0].attention.residual_long_conv)}:
             return None
+        if cfg.intermediate_size % cfg.monarch_mlp_nblocks:        # the last block is shorter: single launches only
+            return None
         kind = ops.longconv_pick(B, L, torch.bfloat16, D)
         if kind < 2:
             return None

@@ -102,7 +102,9 @@ class BertGatedLinearUnitMLP(nn.Module):
         x2 = x.reshape(-1, x.shape[-1])
         if x2.dtype != dt:
             x2 = x2.to(dt)
-        if dt == torch.bfloat16 and x.dim() == 3 and x2.shape[0] and x.shape[-1] % 256 == 0 and x.shape[-1] <= 2048 and not ops.observed():
+        whole = cfg.intermediate_size % cfg.monarch_mlp_nblocks == 0      # else the last block is shorter: single launches only
+        if (dt == torch.bfloat16 and x.dim() == 3 and x2.shape[0] and x.shape[-1] % 256 == 0 and x.shape[-1] <= 2048 and whole
+                and not ops.observed()):
             plan = self._plan(x.device)
             if plan is not None:
                 return self._forward_bf16(x, x2, plan, copies_only)

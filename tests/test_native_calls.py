@@ -4,7 +4,8 @@ import pytest
 import torch
 import torch.nn as nn
 
-from m2_b200 import BertGatedLinearUnitMLP, MonarchMixerSequenceMixing, ops
+from m2_b200 import BertGatedLinearUnitMLP, MonarchMixerSequenceMixing, glu_mlp, ops
+from m2_b200.encoder import M2BertConfig, M2BertModel
 from tests.helpers import Cfg
 
 D, INTER = 256, 512
@@ -86,6 +87,28 @@ def test_linear_layers_without_bias(calls):
     assert calls[-1] == "m2_mlp_fwd" and "m2_mixer_fwd" in calls
     a, b = m._make_plan(2, 128, 4, torch.device("cpu")).args, f._plan(torch.device("cpu")).args
     assert a.b_in is None and a.b_out is None and b.wo_bias is None and a.w_in and b.ln_b
+
+
+def test_a_shorter_last_block_takes_single_launches(calls, monkeypatch):
+    monkeypatch.setattr(glu_mlp, "_compute_dtype", lambda x: torch.bfloat16)
+    f = mlp(inter=INTER + 2)                         # wo.weight (4, 64, 129): 516 columns for 514 features
+    with torch.no_grad():
+        assert f(torch.zeros(2, 128, D)).shape == (2, 128, D)
+    assert calls == ["m2_blockdiag_glu_fwd", "m2_blockdiag_fwd", "m2_add_layernorm_fwd"]
+    model = M2BertModel(M2BertConfig(vocab_size=8, hidden_size=D, intermediate_size=INTER + 2, num_hidden_layers=1, hyena_filter_order=16))
+    assert model._make_plan(2, 128, torch.device("cpu")) is None
+
+
+@pytest.mark.gpu
+def test_mlp_with_a_shorter_last_block():
+    torch.manual_seed(4)
+    f, x = mlp(inter=INTER + 2).cuda(), torch.randn(3, 24, D, device="cuda")
+    with torch.no_grad():
+        want = f(x)
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            got = f(x)
+    # four bf16 roundings (input, weights, h, wo's output) of 2^-9 each on values that LayerNorm brings to 1
+    assert (got - want).norm() / want.norm() < 4 * 2 ** -8
 
 
 def plans(m):
