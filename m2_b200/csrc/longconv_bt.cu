@@ -37,6 +37,7 @@ constexpr int MAX_L = 1024;                     // beyond it the FFT family is f
 constexpr int WROWS = 368;                      // strip rows of two deltas: 2 * 128 + 112
 constexpr int WIN_BYTES = WROWS * 32;
 constexpr int SMEM_MAX = 113 * 1024;            // per CTA with two on an SM
+constexpr long long REACH = 1LL << 33;          // elements from the first to the last of a tensor: offsets are kept as int, in units of 8
 constexpr int YROW = 272;                       // bytes of a 128-step row in the x2 / output buffers (16 of padding)
 
 __host__ __device__ constexpr int tap_count(int nb) { return 256 * nb + 64; }   // fp16 taps of a channel, d = -128 nb ..
@@ -518,6 +519,8 @@ static double bt_us(int batch, int seq_len, int d_model, int nf) {
 // Whether this family beats the FFT family at 128 < L <= 1024, whose waves of 8 sequences per SM take 19 us whatever the
 // length (0.8 of it in the stream of a forward).
 bool longconv_bt_preferred(int batch, int seq_len, int d_model) {
+  // the widest tensor, 3 d_model rows of batch * seq_len steps with their padding (3.7 M tokens at d_model 768)
+  if ((3LL * d_model + 1) * ((long long)batch * ((seq_len + 7) / 8 * 8) + 16) >= bt::REACH) return false;
   const long long waves = ((long long)batch * d_model + 8 * m2_sm_count() - 1) / (8 * m2_sm_count());
   const double bt = bt_us(batch, seq_len, d_model, 2), direct = longconv_direct_us(batch, seq_len, d_model, 2);
   return 0.8 * 19.0 * waves > (bt < direct ? bt : direct);
@@ -564,7 +567,7 @@ int longconv_bt_launch(const m2_longconv_args* a, cudaStream_t st) {
   M2_REQUIRE((long long)P.ntile * P.D < (1LL << 30), M2_ERR_UNSUPPORTED, "m2_longconv_fwd: too many units");
   const long long reach = 3LL * P.D * a->xin_sc + (long long)P.B * a->xin_sb, ureach = (long long)P.D * a->u_sc + (long long)P.B * a->u_sb,
                   oreach = (long long)P.D * a->out_sc + (long long)P.B * a->out_sb;
-  M2_REQUIRE(reach < (1LL << 33) && ureach < (1LL << 33) && oreach < (1LL << 33), M2_ERR_UNSUPPORTED, "m2_longconv_fwd: tensors too large for kind 4");
+  M2_REQUIRE(reach < REACH && ureach < REACH && oreach < REACH, M2_ERR_UNSUPPORTED, "m2_longconv_fwd: tensors too large for kind 4");
   P.units = P.ntile * ((P.D + P.G - 1) / P.G);
   P.ksteps = P.NB == 1 ? (P.L + 15) / 16 : 8;
   P.tcols = 32;

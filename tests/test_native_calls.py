@@ -111,6 +111,16 @@ def test_mlp_with_a_shorter_last_block():
     assert (got - want).norm() / want.norm() < 4 * 2 ** -8
 
 
+@pytest.mark.parametrize("L", [132, 256, 1024])
+@pytest.mark.parametrize("d", [256, 768, 1536])
+def test_family_4_is_not_picked_for_tensors_it_refuses(L, d):
+    limit = 2 ** 33 // (3 * d * L)                   # sequences whose in_linear output the kernel's offsets can reach
+
+    def pick(b):
+        return ops.longconv_pick(b, L, torch.bfloat16, d)
+    assert 4 in map(pick, range(1, 65)) and pick(limit + 1) == pick(2 * limit) == 2
+
+
 def plans(m):
     return list(m._plans.plans.values())
 
