@@ -108,34 +108,67 @@ extern "C" long long m2_encoder_workspace(int batch, int pitch, int d_model, int
   return (long long)m2::layout_of(batch, pitch, d_model, inter).total;
 }
 
+// The mixer of one layer where the convolution runs in float32 (kind 0): token rows throughout, the layer input u float32.
+static int mixer_rows(const m2_encoder_args* a, const m2_encoder_layer& y, const void* x, const float* u, void* xin, void* conv, void* out,
+                      void* stream) {
+  const int rows = a->batch * a->seq_len, D = a->d_model;
+  m2_linear_args p;
+  memset(&p, 0, sizeof(p));
+  p.batch = 1; p.seq_len = rows; p.in_features = D; p.out_features = 3 * D; p.dtype = M2_BF16;
+  p.x = x; p.x_sb = (long long)rows * D; p.x_st = D; p.x_sc = 1;
+  p.w = y.w_in; p.bias = y.b_in;
+  p.out = xin; p.out_sb = 3LL * rows * D; p.out_st = 3LL * D; p.out_sc = 1;
+  int rc;
+  if ((rc = m2_linear_fwd(&p, stream))) return rc;
+  m2_longconv_args c;
+  memset(&c, 0, sizeof(c));
+  c.batch = a->batch; c.seq_len = a->seq_len; c.d_model = D; c.n_filters = a->n_filters; c.kind = 0;
+  c.act_dtype = M2_BF16; c.u_dtype = M2_F32; c.bf16_rounding = 1;
+  c.xin = xin; c.xin_sb = 3LL * a->seq_len * D; c.xin_st = 3LL * D; c.xin_sc = 1;
+  c.u = u; c.u_sb = (long long)a->seq_len * D; c.u_st = D; c.u_sc = 1;
+  c.out = conv; c.out_sb = (long long)a->seq_len * D; c.out_st = D; c.out_sc = 1;
+  c.short_w = y.short_w; c.short_b = y.short_b;
+  for (int f = 0; f < 2; ++f) { c.spec[f] = y.spec[f]; c.bias[f] = y.bias[f]; }
+  if ((rc = m2_longconv_fwd(&c, stream))) return rc;
+  p.x = conv; p.out_features = D; p.w = y.w_out; p.bias = y.b_out;
+  p.out = out; p.out_sb = (long long)rows * D; p.out_st = D;
+  return m2_linear_fwd(&p, stream);
+}
+
 extern "C" int m2_encoder_fwd(const m2_encoder_args* a, void* stream) {
   using namespace m2;
   M2_REQUIRE(a != nullptr, M2_ERR_ARG, "m2_encoder_fwd: args is NULL");
   M2_REQUIRE(a->batch > 0 && a->seq_len > 0 && a->n_layers > 0 && a->d_model > 0 && a->inter > 0, M2_ERR_ARG, "m2_encoder_fwd: bad sizes");
   M2_REQUIRE(a->layers && a->workspace && a->out && m2_aligned(a->workspace, 256), M2_ERR_ARG,
              "m2_encoder_fwd: NULL pointer or workspace not on a 256-byte boundary");
-  const int pitch = (int)round_up(a->seq_len, 8), D = a->d_model;
+  M2_REQUIRE(a->kind == 0 || (a->kind >= 2 && a->kind <= 4), M2_ERR_UNSUPPORTED, "m2_encoder_fwd: kind must be 0, 2, 3 or 4");
+  const bool rows = a->kind == 0;               // float32 convolution: token rows without padding, float32 layer inputs in `out`
+  const int pitch = rows ? a->seq_len : (int)round_up(a->seq_len, 8), D = a->d_model;
   M2_REQUIRE((long long)a->batch * pitch < (1LL << 31) - 512, M2_ERR_UNSUPPORTED, "m2_encoder_fwd: more than 2^31 tokens");
   const Layout l = layout_of(a->batch, pitch, D, a->inter);
   unsigned char* ws = static_cast<unsigned char*>(a->workspace);
   int rc;
   m2_embed_layernorm_args e = a->embed;
-  e.m = (int)l.rows; e.n = D; e.out = nullptr; e.ldo = D;
+  e.m = (int)l.rows; e.n = D; e.out = rows ? a->out : nullptr; e.ldo = D;
   e.out_bf16 = ws + l.aug; e.ld_bf16 = D; e.bf16_pad_cols = 0;
-  e.out_tm_f16 = ws + l.tm; e.tm_sb = pitch; e.tm_sc = l.stride; e.seq_len = pitch; e.valid_len = a->seq_len;
+  e.out_tm_f16 = rows ? nullptr : ws + l.tm; e.tm_sb = pitch; e.tm_sc = l.stride; e.seq_len = pitch; e.valid_len = a->seq_len;
   if ((rc = m2_embed_layernorm_fwd(&e, stream))) return rc;
   for (int i = 0; i < a->n_layers; ++i) {
     const m2_encoder_layer& y = a->layers[i];
-    m2_mixer_args x;
-    memset(&x, 0, sizeof(x));
-    x.batch = a->batch; x.seq_len = a->seq_len; x.pitch = pitch; x.out_pitch = pitch; x.d_model = D;
-    x.kind = a->kind; x.n_filters = a->n_filters;
-    x.x = ws + l.aug; x.u = ws + l.tm; x.u_stride = l.stride;
-    x.w_in = y.w_in; x.b_in = y.b_in; x.short_w = y.short_w; x.short_b = y.short_b;
-    for (int f = 0; f < 2; ++f) { x.spec[f] = y.spec[f]; x.bias[f] = y.bias[f]; }
-    x.w_out = y.w_out; x.b_out = y.b_out;
-    x.xin = ws + l.xin; x.conv = ws + l.conv; x.stride = l.stride; x.out = ws + l.mix;
-    if ((rc = m2_mixer_fwd(&x, stream))) return rc;
+    if (rows) {
+      if ((rc = mixer_rows(a, y, ws + l.aug, a->out, ws + l.xin, ws + l.conv, ws + l.mix, stream))) return rc;
+    } else {
+      m2_mixer_args x;
+      memset(&x, 0, sizeof(x));
+      x.batch = a->batch; x.seq_len = a->seq_len; x.pitch = pitch; x.out_pitch = pitch; x.d_model = D;
+      x.kind = a->kind; x.n_filters = a->n_filters;
+      x.x = ws + l.aug; x.u = ws + l.tm; x.u_stride = l.stride;
+      x.w_in = y.w_in; x.b_in = y.b_in; x.short_w = y.short_w; x.short_b = y.short_b;
+      for (int f = 0; f < 2; ++f) { x.spec[f] = y.spec[f]; x.bias[f] = y.bias[f]; }
+      x.w_out = y.w_out; x.b_out = y.b_out;
+      x.xin = ws + l.xin; x.conv = ws + l.conv; x.stride = l.stride; x.out = ws + l.mix;
+      if ((rc = m2_mixer_fwd(&x, stream))) return rc;
+    }
     m2_mlp_args p;
     memset(&p, 0, sizeof(p));
     const bool last = i + 1 == a->n_layers;
@@ -143,11 +176,9 @@ extern "C" int m2_encoder_fwd(const m2_encoder_args* a, void* stream) {
     p.x = ws + l.mix; p.wg = y.wg; p.wo = y.wo; p.wo_bias = y.wo_bias; p.ln_w = y.ln_w; p.ln_b = y.ln_b; p.eps = y.eps;
     p.h = ws + l.h; p.o = ws + l.o;
     p.seq_len = pitch; p.valid_len = a->seq_len;
-    if (last) {
-      p.out = a->out;
-    } else {                                    // only the next mixer reads this output, through its two copies
-      p.out_bf16 = ws + l.aug; p.out_tm_f16 = ws + l.tm; p.tm_stride = l.stride;
-    }
+    if (last || rows) p.out = a->out;
+    if (!last) p.out_bf16 = ws + l.aug;         // only the next mixer reads this output, through its two copies
+    if (!last && !rows) { p.out_tm_f16 = ws + l.tm; p.tm_stride = l.stride; }
     if ((rc = m2_mlp_fwd(&p, stream))) return rc;
   }
   return M2_OK;

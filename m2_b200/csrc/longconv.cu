@@ -38,9 +38,17 @@ extern "C" int m2_longconv_kind_batch(int batch, int seq_len, m2_dtype act_dtype
 
 extern "C" int m2_longconv_pick(int batch, int seq_len, m2_dtype act_dtype, int d_model) {
   if (act_dtype != M2_BF16 || batch <= 0 || d_model <= 0 || seq_len <= 0 || seq_len > 32768) return 0;
+  // Tensor-core families hold taps (3, 4) or spectra (2) and the residual input in fp16.  They serve the lengths that no other
+  // precision was ever promised for: 65 .. 128 steps of d_model % 128 == 0, batches of 64 and more of 16 .. 128 steps in
+  // multiples of 8, and multiples of 4 beyond 128.  All others are computed in float32 throughout (0): against 64-bit arithmetic
+  // on the same bf16 input (d_model 768, two filters) the float32 result is off by 1.71e-3 at 37 steps and 1.78e-3 at 1531,
+  // nearly all of it the output's own rounding; kinds 3 and 4 by 1.73e-3 at 37, kind 2 by 1.91e-3 at 1531.
+  const bool tz = m2::longconv_tz_supported(batch, seq_len, act_dtype);
   // up to 128 steps both families multiply by the same Toeplitz matrix; kind 3 walks tiles of 128 sequences whatever the
   // batch (34 us at D = 768, L = 128, B = 8 .. 64), kind 4 tiles as narrow as the batch (20 us at 8, 27 at 32, 51 at 64)
-  if (seq_len <= 128) return batch >= 48 ? 3 : 4;
+  if (m2::longconv_tc_supported(seq_len, act_dtype, d_model)) return batch >= 48 ? 3 : 4;
+  if (seq_len <= 128) return tz ? 3 : 0;
+  if (seq_len % 4 != 0) return 0;
   if (m2::longconv_bt_supported(seq_len, act_dtype) && m2::longconv_bt_preferred(batch, seq_len, d_model)) return 4;
   return 2;
 }

@@ -320,7 +320,7 @@ static int next_pow2(int v) { int r = 2; while (r < v) r <<= 1; return r; }
 
 
 bool longconv_f32_supported(const m2_longconv_args* a);           // longconv_f32.cu
-int longconv_f32_launch(ConvParams p, cudaStream_t st);
+int longconv_f32_launch(const m2_longconv_args* a, ConvParams p, cudaStream_t st);
 
 int longconv_simt_launch(const m2_longconv_args* a, cudaStream_t st) {
   ConvParams p;
@@ -347,7 +347,7 @@ int longconv_simt_launch(const m2_longconv_args* a, cudaStream_t st) {
     p.u = a->xin; p.usb = a->xin_sb; p.ust = a->xin_st; p.usc = a->xin_sc;
     p.spec[1] = a->spec[0]; p.bias[1] = a->bias[0];
   } else if (p.nf == 1) { p.u = a->xin; p.usb = p.ust = p.usc = 0; }
-  if (longconv_f32_supported(a)) return longconv_f32_launch(p, st);
+  if (longconv_f32_supported(a)) return longconv_f32_launch(a, p, st);
   const size_t smem = use_cluster ? per_ch / 2 : (size_t)ct * per_ch;
   const bool round = a->bf16_rounding != 0;
   const bool abf = a->act_dtype == M2_BF16, ubf = (p.nf == 2 && !p.plain) ? (a->u_dtype == M2_BF16) : abf;

@@ -107,7 +107,7 @@ class M2BertEmbeddings(nn.Module):
         D = self.word_embeddings.weight.shape[1]
         aug = torch.empty((B * L, D), dtype=torch.bfloat16, device=input_ids.device)
         tm = None
-        if L % 8 == 0:
+        if ops.reads_time_major(B, L, D):
             tm = torch.empty((D, B, L), dtype=torch.float16, device=input_ids.device)
         pos = self.position_embeddings.weight if self.use_positional_encodings else None
         if pos is not None and position_ids is None and L > pos.shape[0]:
@@ -122,7 +122,7 @@ class M2BertEmbeddings(nn.Module):
         B, L, D = e.shape
         aug = torch.empty((B * L, D), dtype=torch.bfloat16, device=e.device)
         tm = None
-        if L % 8 == 0:
+        if ops.reads_time_major(B, L, D):
             tm = torch.empty((D, B, L), dtype=torch.float16, device=e.device)
         y = ops.add_layernorm_fwd(e.reshape(B * L, D), None, self.LayerNorm.weight, self.LayerNorm.bias,
                                   self.LayerNorm.eps, torch.float32, bf16_copy=aug, tm_copy=tm, fill_pad=False)
@@ -254,9 +254,9 @@ class M2BertModel(nn.Module):
             return None
         if cfg.intermediate_size % cfg.monarch_mlp_nblocks:        # the last block is shorter: single launches only
             return None
-        kind = ops.longconv_pick(B, L, torch.bfloat16, D)
-        if kind < 2:
+        if L > 32768:                          # beyond every convolution kernel: the layers raise
             return None
+        kind = ops.longconv_pick(B, L, torch.bfloat16, D)
         args = (_lib.EncoderLayer * len(layers))()
         e = _lib.EncoderArgs()
         work = _lib.lib().m2_encoder_workspace(B, (L + 7) // 8 * 8, D, cfg.intermediate_size)

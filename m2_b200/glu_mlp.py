@@ -74,7 +74,7 @@ class BertGatedLinearUnitMLP(nn.Module):
             x2 = x2.contiguous()
         work = torch.empty((m, self.config.intermediate_size + D), dtype=torch.bfloat16, device=dev)
         aug = torch.empty((m, D), dtype=torch.bfloat16, device=dev)
-        tm = torch.empty((D, B, L), dtype=torch.float16, device=dev) if L % 8 == 0 else None
+        tm = torch.empty((D, B, L), dtype=torch.float16, device=dev) if ops.reads_time_major(B, L, D) else None
         y = aug.view(B, L, D) if copies_only and tm is not None else torch.empty((B, L, D), dtype=torch.float32, device=dev)
         a = _lib.MlpArgs.from_buffer_copy(plan.args)
         a.m, a.seq_len = m, L
@@ -119,7 +119,7 @@ class BertGatedLinearUnitMLP(nn.Module):
             # instead of leaving it to a separate cast pass
             aug = torch.empty((x2.shape[0], x.shape[-1]), dtype=torch.bfloat16, device=x.device)
         tm = None
-        if aug is not None and x.shape[1] % 8 == 0:
+        if aug is not None and ops.reads_time_major(*x.shape):
             # a following mixer of this shape runs a time-contiguous convolution kernel, which reads the
             # layer input as a time-major fp16 tensor: written here too
             tm = torch.empty((x.shape[2], x.shape[0], x.shape[1]), dtype=torch.float16, device=x.device)

@@ -150,6 +150,12 @@ def longconv_pick(batch: int, seq_len: int, act_dtype: torch.dtype, d_model: int
                                        int(d_model))
 
 
+def reads_time_major(batch: int, seq_len: int, d_model: int) -> bool:
+    """Whether a bf16 mixer of this shape reads its input's time-major fp16 copy, as it can come from the LayerNorm before it
+    (rows of whole 16 bytes).  Where the convolution runs in float32 the mixer reads the float32 input itself."""
+    return seq_len % 8 == 0 and longconv_pick(batch, seq_len, torch.bfloat16, d_model) != 0
+
+
 def filter_spectrum(k: torch.Tensor, seq_len: int, kind: int, bias=None) -> torch.Tensor:
     """Spectrum table of one filter for kernel family `kind` (float32, opaque layout).
     Kinds 3 and 4 fold the convolution's bias term into the table: pass it here."""

@@ -115,7 +115,7 @@ class MonarchMixerSequenceMixing(nn.Module):
             a.b_out = plan.f32(self.out_linear.bias)
         for i, f in enumerate(self.filters()):
             a.spec[i] = plan.cached(f.spectrum(L, True, kind))
-            if kind == 2:
+            if kind in (0, 2):                       # kinds 3 and 4 have it inside their tables
                 a.bias[i] = plan.f32(f.bias) if f.use_bias else plan.passing(ops._f32c(f.conv_bias()))
 
     def _make_plan(self, B, L, kind, dev):
@@ -270,7 +270,9 @@ class MonarchMixerSequenceMixing(nn.Module):
             kind = ops.longconv_pick(u.size(0), L, torch.bfloat16, self.d_model)
             if kind and u.size(0):
                 return self._forward_bf16(u, ures, kind), None
-        kind = 0
+        kind = 0                                # float32 convolution on token rows
+        if ures is not None and ures.dtype == torch.float16:
+            ures = ures.float()
         filters = self.filters()
         biases = [f.conv_bias() for f in filters]
         specs = [f.spectrum(L, bf16, kind) for f in filters]
