@@ -96,11 +96,12 @@ class PlanCache:
             if not getattr(plan, "lasting", True):
                 return plan
             plans[key] = plan
+        try:
+            plans.move_to_end(key)
             while len(plans) > self.most:
-                try:
-                    plans.popitem(last=False)
-                except KeyError:             # another thread emptied it
-                    break
+                plans.popitem(last=False)
+        except KeyError:                     # another thread took it out
+            pass
         return plan
 
     def __deepcopy__(self, memo):

@@ -5,6 +5,7 @@ import torch
 import torch.nn as nn
 
 from m2_b200 import BertGatedLinearUnitMLP, MonarchMixerSequenceMixing, glu_mlp, ops
+from m2_b200._plan import PlanCache
 from m2_b200.encoder import M2BertConfig, M2BertModel
 from tests.helpers import Cfg
 
@@ -119,6 +120,13 @@ def test_family_4_is_not_picked_for_tensors_it_refuses(L, d):
     def pick(b):
         return ops.longconv_pick(b, L, torch.bfloat16, d)
     assert 4 in map(pick, range(1, 65)) and pick(limit + 1) == pick(2 * limit) == 2
+
+
+def test_the_longest_unused_plan_is_dropped():
+    m, cache, made = nn.Linear(2, 2), PlanCache(most=2), []
+    for key in "hot", "x", "hot", "y", "hot":
+        cache.get(m, key, lambda: made.append(key) or key)
+    assert made == ["hot", "x", "y"]
 
 
 def plans(m):
