@@ -74,6 +74,9 @@ class Plan:
         return t.data_ptr()
 
 
+REFUSED = object()       # kept in the place of a plan that make() did not give
+
+
 class PlanCache:
     """At most `most` plans of one module, the longest unused dropped first."""
 
@@ -81,7 +84,8 @@ class PlanCache:
         self.most, self.watch, self.plans = most, None, OrderedDict()
 
     def get(self, root, key, make):
-        """The plan of `key`, made by make() when there is none; None when the module's tensors cannot be watched."""
+        """The plan of `key`, made by make() when there is none; None when make() returns that (remembered like a plan) or
+        the module's tensors cannot be watched."""
         if self.watch is None or not self.watch.same():
             self.plans = OrderedDict()
             try:
@@ -95,14 +99,14 @@ class PlanCache:
             plan = make()
             if not getattr(plan, "lasting", True):
                 return plan
-            plans[key] = plan
+            plans[key] = plan = REFUSED if plan is None else plan
         try:
             plans.move_to_end(key)
             while len(plans) > self.most:
                 plans.popitem(last=False)
         except KeyError:                     # another thread took it out
             pass
-        return plan
+        return None if plan is REFUSED else plan
 
     def __deepcopy__(self, memo):
         return PlanCache(self.most)          # a copied module has other tensors

@@ -129,6 +129,13 @@ def test_the_longest_unused_plan_is_dropped():
     assert made == ["hot", "x", "y"]
 
 
+def test_a_refusal_is_remembered_until_something_changes():
+    m, cache, made = nn.Linear(2, 2), PlanCache(), []
+    assert [cache.get(m, 0, lambda: made.append(0)) for _ in range(3)] == [None] * 3 and len(made) == 1
+    m.weight = nn.Parameter(torch.zeros(2, 2))
+    assert cache.get(m, 0, lambda: made.append(0)) is None and len(made) == 2
+
+
 def plans(m):
     return list(m._plans.plans.values())
 
