@@ -5,6 +5,7 @@ kept.
 """
 from __future__ import annotations
 
+import weakref
 from collections import OrderedDict
 from operator import attrgetter, is_
 
@@ -21,6 +22,9 @@ class Watch:
 
     def __init__(self, root):
         mods = list(root.modules())
+        if any(isinstance(v, torch.Tensor) for m in mods for v in vars(m).values()):
+            # weights that are plain attributes (replicas, pruned or functionalised modules) are in no table to be watched
+            raise RuntimeError("tensors outside the modules' parameters and buffers")
         slots = [(d, k, t) for m in mods for d in (m._parameters, m._buffers) for k, t in d.items() if t is not None]
         kids = [(m._modules, k, c) for m in mods for k, c in m._modules.items()]
         self.dicts, self.keys, self.values = zip(*(slots + kids))
@@ -80,8 +84,9 @@ REFUSED = object()       # kept in the place of a plan that make() did not give
 class PlanCache:
     """At most `most` plans of one module, the longest unused dropped first."""
 
-    def __init__(self, most=16):
+    def __init__(self, most=16, owner=None):
         self.most, self.watch, self.plans = most, None, OrderedDict()
+        self.owner = owner and weakref.ref(owner)
 
     def get(self, root, key, make):
         """The plan of `key`, made by make() when there is none; None when make() returns that (remembered like a plan) or
@@ -113,6 +118,15 @@ class PlanCache:
 
     def __reduce__(self):
         return PlanCache, (self.most,)
+
+
+def plans_of(module):
+    """The module's own PlanCache.  One that came with a copied __dict__ (a data-parallel replica, copy.copy) belongs to the
+    module it was made for: plans and Watch of one would answer for the other's tensors."""
+    cache = vars(module).get("_plans")
+    if cache is None or cache.owner is None or cache.owner() is not module:
+        cache = module._plans = PlanCache(owner=module)
+    return cache
 
 
 def expect(dev, *tensors):

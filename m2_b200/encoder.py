@@ -19,7 +19,7 @@ import torch
 import torch.nn as nn
 
 from . import _lib, ops
-from ._plan import Plan, PlanCache, any_dropping, any_hooks
+from ._plan import Plan, any_dropping, any_hooks, plans_of
 from ._tags import attach
 from .glu_mlp import BertGatedLinearUnitMLP
 from .hyena_filter import _autocast_bf16
@@ -285,9 +285,7 @@ class M2BertModel(nn.Module):
             return None
         B, L = input_ids.shape
         dev = input_ids.device
-        if not hasattr(self, "_plans"):          # absent from models pickled whole by earlier versions, too
-            self._plans = PlanCache()
-        plan = self._plans.get(self, (B, L, dev.index), lambda: self._make_plan(B, L, dev))
+        plan = plans_of(self).get(self, (B, L, dev.index), lambda: self._make_plan(B, L, dev))
         if plan is None or any_hooks(plan.called) or any_dropping(plan.dropping):
             return None
 

@@ -10,7 +10,7 @@ import torch
 import torch.nn as nn
 
 from . import _lib, ops
-from ._plan import Plan, PlanCache, expect
+from ._plan import Plan, expect, plans_of
 from ._tags import attach, forward_only
 from .blockdiag_linear import BlockdiagLinear, _compute_dtype
 
@@ -52,16 +52,13 @@ class BertGatedLinearUnitMLP(nn.Module):
         a.ln_w, a.ln_b, a.eps = plan.f32(self.layernorm.weight), plan.f32(self.layernorm.bias), float(self.layernorm.eps)
 
     def _plan(self, dev):
-        if not hasattr(self, "_plans"):
-            self._plans = PlanCache()
-
         def make():
             a = _lib.MlpArgs()
             a.d_model, a.inter, a.nblocks = self.config.hidden_size, self.config.intermediate_size, self.config.monarch_mlp_nblocks
             plan = Plan(a)
             self.fill_args(plan, a, dev)
             return plan
-        return self._plans.get(self, dev.index, make)
+        return plans_of(self).get(self, dev.index, make)
 
     def _forward_bf16(self, x, x2, plan, copies_only):
         """The three launches as one call; outputs as in forward()."""

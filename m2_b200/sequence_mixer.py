@@ -10,7 +10,7 @@ import torch
 import torch.nn as nn
 
 from . import _lib, ops
-from ._plan import Plan, PlanCache, expect
+from ._plan import Plan, expect, plans_of
 from ._tags import copies_of, forward_only, src_dtype_of
 from .hyena_filter import HyenaFilter, _autocast_bf16
 
@@ -157,9 +157,7 @@ class MonarchMixerSequenceMixing(nn.Module):
                 u_t = torch.empty((D, B, Lp), dtype=torch.float16, device=dev)
                 ops.time_major_f16(ures if ures.dtype in (torch.float32, torch.bfloat16) else ures.float(), out=u_t[:, :, :L], rows=rows)
         yu_bf16 = ures is not None and src_dtype_of(ures) == torch.bfloat16
-        if not hasattr(self, "_plans"):
-            self._plans = PlanCache()
-        plan = self._plans.get(self, (B, L, kind, dev.index), lambda: self._make_plan(B, L, kind, dev))
+        plan = plans_of(self).get(self, (B, L, kind, dev.index), lambda: self._make_plan(B, L, kind, dev))
         stride = _round_up(B * Lp, 16)
         # allocated per call: inside a CUDA-graph capture the buffers then belong to the graph's own pool
         work = torch.empty((4 * D, stride), dtype=torch.bfloat16, device=dev)

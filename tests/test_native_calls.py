@@ -1,5 +1,7 @@
 """What the modules hand to the one-call entry points (m2_mixer_fwd, m2_mlp_fwd, m2_encoder_fwd), which see pointers and sizes
 and no tensors.  On the CPU with the launch replaced by a recorder: nothing here reaches a GPU."""
+import copy
+
 import pytest
 import torch
 import torch.nn as nn
@@ -134,6 +136,24 @@ def test_a_refusal_is_remembered_until_something_changes():
     assert [cache.get(m, 0, lambda: made.append(0)) for _ in range(3)] == [None] * 3 and len(made) == 1
     m.weight = nn.Parameter(torch.zeros(2, 2))
     assert cache.get(m, 0, lambda: made.append(0)) is None and len(made) == 2
+
+
+def test_replicas_have_plans_of_their_own(calls):
+    m, u = mixer(), torch.zeros(2, 128, D)
+    mix(m, u)
+    replica = m._replicate_for_data_parallel()       # shares __dict__, its parameters become plain attributes
+    for child in ("in_linear", "out_linear", "short_filter", "filter_fn", "filter_fn2"):
+        replica._modules[child] = m._modules[child]._replicate_for_data_parallel()
+        for k, t in m._modules[child]._parameters.items():
+            setattr(replica._modules[child], k, t.detach().clone())
+    for f in ("filter_fn", "filter_fn2"):
+        replica._modules[f]._modules.update(m._modules[f]._modules)
+    mix(replica, u)
+    assert replica._plans is not m._plans and not plans(replica) and plans(m)
+    assert "m2_linear_fwd" in calls[-3:]             # tensors that cannot be watched: single launches
+    twin = copy.copy(m)
+    mix(twin, u)
+    assert twin._plans is not m._plans and m._plans.owner() is m and plans(m)
 
 
 def plans(m):
