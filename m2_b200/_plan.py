@@ -18,28 +18,31 @@ _ptr = torch.Tensor.data_ptr
 
 
 class Watch:
-    """The parameters, buffers and submodules below `root` as they are now; `same()` says whether they still are."""
+    """The parameters, buffers, submodules and settings below `root` as they are now; `same()` says whether they still are."""
 
     def __init__(self, root):
         mods = list(root.modules())
         if any(isinstance(v, torch.Tensor) for m in mods for v in vars(m).values()):
             # weights that are plain attributes (replicas, pruned or functionalised modules) are in no table to be watched
             raise RuntimeError("tensors outside the modules' parameters and buffers")
-        slots = [(d, k, t) for m in mods for d in (m._parameters, m._buffers) for k, t in d.items() if t is not None]
+        slots = [(d, k, t) for m in mods for d in (m._parameters, m._buffers) for k, t in d.items()]   # None: no such tensor
         kids = [(m._modules, k, c) for m in mods for k, c in m._modules.items()]
         self.dicts, self.keys, self.values = zip(*(slots + kids))
-        self.tensors = [t for _, _, t in slots]
+        self.tensors = [t for _, _, t in slots if t is not None]
         self.versions = list(map(_version, self.tensors))      # RuntimeError for tensors made under inference_mode
         self.ptrs = list(map(_ptr, self.tensors))
-        self.norms = [m for m in mods if isinstance(m, torch.nn.LayerNorm)]
-        self.eps = [m.eps for m in self.norms]
+        # plain attributes that plans are made from: those a module's class names in `plan_attrs`, and eps
+        names = [(m, type(m).plan_attrs if hasattr(type(m), "plan_attrs") else ("eps",) if isinstance(m, torch.nn.LayerNorm) else ())
+                 for m in mods]
+        self.attrs = [(m, attrgetter(*n)) for m, n in names if n]
+        self.attr_values = [get(m) for m, get in self.attrs]
 
     def same(self):
         try:
             return (all(map(is_, map(dict.__getitem__, self.dicts, self.keys), self.values))
                     and list(map(_version, self.tensors)) == self.versions and list(map(_ptr, self.tensors)) == self.ptrs
-                    and [m.eps for m in self.norms] == self.eps)
-        except KeyError:
+                    and [get(m) for m, get in self.attrs] == self.attr_values)
+        except (KeyError, AttributeError):
             return False
 
 

@@ -64,6 +64,8 @@ class M2BertConfig:
 class M2BertEmbeddings(nn.Module):
     """word + token-type (+ learned position) embeddings, LayerNorm, dropout."""
 
+    plan_attrs = ("use_positional_encodings", "LayerNorm.eps")
+
     def __init__(self, config):
         super().__init__()
         self.word_embeddings = nn.Embedding(config.vocab_size, config.hidden_size,

@@ -24,6 +24,8 @@ class BertGatedLinearUnitMLP(nn.Module):
     materialised: the gated GEMM applies GELU and the product in its epilogue.
     """
 
+    plan_attrs = ("config", "config.hidden_size", "config.intermediate_size", "config.monarch_mlp_nblocks", "layernorm.eps")
+
     def __init__(self, config):
         super().__init__()
         self.config = config

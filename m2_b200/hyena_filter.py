@@ -103,6 +103,8 @@ class HyenaFilter(OptimModule):
     (B, d_model, L) input (hyena_utils.py:219-248).
     """
 
+    plan_attrs = ("use_bias",)
+
     def __init__(self, d_model, emb_dim=3, order=16, seq_len=1024, lr=1e-3, lr_pos_emb=1e-5,
                  dropout=0.0, w=1, w_mod=1, wd=0, bias=True, num_inner_mlps=2,
                  linear_mixer=False, modulate: bool = True, normalized=False,

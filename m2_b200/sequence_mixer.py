@@ -55,6 +55,8 @@ class MonarchMixerSequenceMixing(nn.Module):
     where the reference's PyTorch ops would.
     """
 
+    plan_attrs = ("d_model", "residual_long_conv", "hyena_training_additions")
+
     def __init__(self, d_model, l_max=128, dropout=0.0, hyena_kernel_lr=None, bidirectional=False,
                  hyena_lr_pos_emb=1e-5, hyena_w=10, hyena_w_mod=1, hyena_wd=0.1, hyena_emb_dim=3,
                  hyena_filter_dropout=0.0, hyena_filter_order=16, residual_long_conv=False,

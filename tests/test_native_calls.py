@@ -1,13 +1,14 @@
 """What the modules hand to the one-call entry points (m2_mixer_fwd, m2_mlp_fwd, m2_encoder_fwd), which see pointers and sizes
 and no tensors.  On the CPU with the launch replaced by a recorder: nothing here reaches a GPU."""
 import copy
+import dataclasses
 
 import pytest
 import torch
 import torch.nn as nn
 
 from m2_b200 import BertGatedLinearUnitMLP, MonarchMixerSequenceMixing, glu_mlp, ops
-from m2_b200._plan import PlanCache
+from m2_b200._plan import PlanCache, Watch
 from m2_b200.encoder import M2BertConfig, M2BertModel
 from tests.helpers import Cfg
 
@@ -154,6 +155,60 @@ def test_replicas_have_plans_of_their_own(calls):
     twin = copy.copy(m)
     mix(twin, u)
     assert twin._plans is not m._plans and m._plans.owner() is m and plans(m)
+
+
+def small_model():
+    return M2BertModel(M2BertConfig(vocab_size=8, hidden_size=D, intermediate_size=INTER, num_hidden_layers=2, hyena_filter_order=16)).eval()
+
+
+SETTINGS = [(lambda m: setattr(m.encoder.layer[1].attention.filter_fn, "use_bias", False)),
+            (lambda m: setattr(m.encoder.layer[0].attention, "residual_long_conv", False)),
+            (lambda m: setattr(m.encoder.layer[0].attention, "hyena_training_additions", True)),
+            (lambda m: setattr(m.encoder.layer[0].attention, "d_model", D // 2)),
+            (lambda m: setattr(m.embeddings, "use_positional_encodings", False)),
+            (lambda m: setattr(m.embeddings.LayerNorm, "eps", 0.5)),
+            (lambda m: setattr(m.encoder.layer[1].mlp.layernorm, "eps", 0.5)),
+            (lambda m: setattr(m.encoder.layer[0].mlp.config, "intermediate_size", INTER // 2)),
+            (lambda m: setattr(m.encoder.layer[0].mlp, "config", dataclasses.replace(m.config, monarch_mlp_nblocks=2)))]
+
+
+@pytest.mark.parametrize("change", SETTINGS)
+def test_settings_that_plans_are_made_from_are_watched(change):
+    m = small_model()
+    w = Watch(m)
+    assert w.same()
+    change(m)
+    assert not w.same()
+
+
+def test_a_tensor_that_was_not_there_is_watched():
+    m = nn.Linear(2, 2, bias=False)
+    w = Watch(m)
+    assert w.same()
+    m.bias = nn.Parameter(torch.zeros(2))
+    assert not w.same()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("L", [37, 72, 256])
+@pytest.mark.parametrize("change", [SETTINGS[0], SETTINGS[4], SETTINGS[6],
+                                    lambda m: [setattr(y.attention, "residual_long_conv", False) for y in m.encoder.layer]])
+def test_planned_and_single_launches_agree_after_a_setting_changed(change, L):
+    torch.manual_seed(6)
+    m = M2BertModel(M2BertConfig(vocab_size=8, hidden_size=D, intermediate_size=INTER, num_hidden_layers=2, hyena_filter_order=16,
+                                 max_position_embeddings=256, long_conv_l_max=256)).eval().cuda()
+    ids = torch.randint(0, 8, (3, L), device="cuda")
+
+    def out():
+        with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16):
+            return m(ids)[0]
+    before = out()
+    change(m)
+    after = out()
+    handle = m.encoder.register_forward_hook(lambda *a: None)
+    single = out()
+    handle.remove()
+    assert not torch.equal(before, after) and torch.equal(after, single)
 
 
 def plans(m):
