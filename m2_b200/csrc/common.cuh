@@ -73,7 +73,9 @@ __device__ int m2_dev_status_word = 0;
 
 // ---- device helpers -----------------------------------------------------------------
 // The next kernel of the stream may be launched; then wait for the kernels before this one.  Every thread of a kernel
-// started by m2_launch calls it before it reads or writes global memory.
+// started by m2_launch calls it before it reads or writes global memory.  A kernel that uses tensor memory triggers only
+// when its block holds it (after the barrier behind the allocation): were the next kernel let in while an allocation waits
+// for the kernel before, it could take what that one frees and keep it, waiting for this one, which waits for its memory.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait_only() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() {

@@ -95,16 +95,18 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     tc::tmem_alloc2(tmem_slot, 512);
     tc::tmem_relinquish2();
   }
-  pdl_wait();
-  float* sbias = reinterpret_cast<float*>(smem + OFF_BIAS);
-  const bool bias_smem = MODE != CHANNELS && P.bias != nullptr && P.n_rows <= BIAS_MAX;
-  if (bias_smem)
-    for (int i = threadIdx.x; i < ((P.n_rows + 15) & ~15); i += THREADS) sbias[i] = i < P.n_rows ? bf16r(__ldg(P.bias + i)) : 0.f;
   tc::tc_fence_before();
   __syncthreads();
   tc::cluster_sync();                       // the peer's barriers and tensor memory exist before anything touches them
   tc::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
+  float* sbias = reinterpret_cast<float*>(smem + OFF_BIAS);
+  const bool bias_smem = MODE != CHANNELS && P.bias != nullptr && P.n_rows <= BIAS_MAX;
+  if (bias_smem) {
+    for (int i = threadIdx.x; i < ((P.n_rows + 15) & ~15); i += THREADS) sbias[i] = i < P.n_rows ? bf16r(__ldg(P.bias + i)) : 0.f;
+    __syncthreads();
+  }
 
   auto decode = [&](int tile, int& mp, int& nt, int& kb) {
     // the weight-side tile index runs fastest, so the pairs working at the same moment share one token tile

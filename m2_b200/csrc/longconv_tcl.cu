@@ -712,13 +712,6 @@ longconv_tcl_kernel(const Params P) {
     *abort_flag = 0;
     tc::mbar_fence_init();
   }
-  pdl_wait();
-  {
-    const uint4* src = reinterpret_cast<const uint4*>(P.spec[0]);
-    uint4* dst = reinterpret_cast<uint4*>(hdrb);
-    for (int i = tid; i < G::HDR_BYTES / 16; i += G::THREADS) dst[i] = __ldg(src + i);
-    tc::fence_proxy_async_smem();
-  }
   if (warp == 0) {
     tc::tmem_alloc(tmem_slot, G::TCOLS);
     tc::tmem_relinquish();
@@ -726,6 +719,14 @@ longconv_tcl_kernel(const Params P) {
   tc::tc_fence_before();
   __syncthreads();
   tc::tc_fence_after();
+  pdl_wait();
+  {
+    const uint4* src = reinterpret_cast<const uint4*>(P.spec[0]);
+    uint4* dst = reinterpret_cast<uint4*>(hdrb);
+    for (int i = tid; i < G::HDR_BYTES / 16; i += G::THREADS) dst[i] = __ldg(src + i);
+    tc::fence_proxy_async_smem();
+  }
+  __syncthreads();
   uint64_t* bar_ops = bars + 3 * slot;
   uint64_t* bar_mma = bar_ops + 1;
   uint64_t* bar_w = bar_ops + 2;

@@ -2,6 +2,8 @@
 and no tensors.  On the CPU with the launch replaced by a recorder: nothing here reaches a GPU."""
 import copy
 import dataclasses
+import re
+from pathlib import Path
 
 import pytest
 import torch
@@ -209,6 +211,34 @@ def test_planned_and_single_launches_agree_after_a_setting_changed(change, L):
     single = out()
     handle.remove()
     assert not torch.equal(before, after) and torch.equal(after, single)
+
+
+def test_the_next_kernel_is_let_in_after_tensor_memory_is_allocated():
+    """Kernels that are launched while the one before them runs wait for it; one that holds tensor memory while the kernel
+    before it still waits for some would never end.  Source order of allocation, block barrier and trigger."""
+    seen = 0
+    for path in sorted((Path(ops.__file__).parent / "csrc").glob("*.cu")):
+        code = "\n".join(line.split("//")[0] for line in path.read_text().splitlines())
+        for kernel in code.split("__global__")[1:]:
+            alloc, trigger = re.search(r"tmem_alloc2?\(", kernel), re.search(r"pdl_(wait|trigger)\(\)", kernel)
+            if alloc and trigger:
+                seen += 1
+                assert alloc.start() < trigger.start() and "__syncthreads()" in kernel[alloc.end():trigger.start()], path.name
+    assert seen >= 6
+
+
+@pytest.mark.gpu
+def test_families_one_after_the_other_on_one_stream():
+    """Short launches that overlap: kinds 4 and 2 and a GEMM in turn, each with tensor memory of its own."""
+    from tests.test_gpu_precision import mixer as built, run as conv
+    m, xin, u = built(132, 64, 2)
+    w = torch.randn(192, 64, device="cuda").bfloat16()
+    first = None
+    for _ in range(20):
+        y = [conv(m, 4, xin, u), conv(m, 2, xin, u), conv(m, 4, xin, u), ops.linear_fwd(u.bfloat16(), w, None), conv(m, 2, xin, u)]
+        first = first or y
+        assert all(torch.equal(a, b) for a, b in zip(first, y))
+    assert ops.device_status() == 0
 
 
 def plans(m):
