@@ -241,6 +241,32 @@ def test_families_one_after_the_other_on_one_stream():
     assert ops.device_status() == 0
 
 
+def test_shapes_of_token_type_ids():
+    t = torch.arange(6, dtype=torch.int32)
+    assert ops.token_ids(None, 2, 3) is None
+    for same in (t, t.view(2, 3), t.view(6, 1), t.view(2, 3).t().contiguous().t()):
+        assert ops.token_ids(same, 2, 3).view(2, 3).tolist() == [[0, 1, 2], [3, 4, 5]]
+    assert ops.token_ids(t[:3].view(1, 3), 2, 3).view(2, 3).tolist() == [[0, 1, 2]] * 2
+    for wrong in (t[:4], t[:2].view(1, 2), t[:4].view(2, 2)):
+        with pytest.raises(RuntimeError):
+            ops.token_ids(wrong, 2, 3)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("hooked", [False, True])
+def test_token_type_ids_of_any_accepted_shape(hooked):
+    model = small_model().cuda()
+    if hooked:                                       # layer by layer
+        model.encoder.register_forward_hook(lambda *a: None)
+    ids, types = torch.randint(0, 8, (3, 40), device="cuda"), torch.randint(0, 2, (1, 40), device="cuda")
+
+    def out(t):
+        with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16):
+            return model(ids, token_type_ids=t)[0]
+    want = out(types.expand(3, 40))
+    assert torch.equal(out(types), want) and torch.equal(out(types.repeat(3, 1).view(-1)), want)
+
+
 def plans(m):
     return list(m._plans.plans.values())
 
