@@ -266,6 +266,8 @@ class MonarchMixerSequenceMixing(nn.Module):
             u = u.unsqueeze(0)
         u_orig = u
         ures = u_orig if self.residual_long_conv else None
+        if ures is not None:
+            ops._dt(ures)                       # the residual filter reads the input itself: TypeError for float64 or integers
         if bf16:
             kind = ops.longconv_pick(u.size(0), L, torch.bfloat16, self.d_model)
             if kind and u.size(0):

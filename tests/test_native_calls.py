@@ -9,12 +9,21 @@ import pytest
 import torch
 import torch.nn as nn
 
-from m2_b200 import BertGatedLinearUnitMLP, MonarchMixerSequenceMixing, glu_mlp, ops
+from m2_b200 import BertGatedLinearUnitMLP, MonarchMixerSequenceMixing, glu_mlp, ops, sequence_mixer
 from m2_b200._plan import PlanCache, Watch
 from m2_b200.encoder import M2BertConfig, M2BertModel
 from tests.helpers import Cfg
 
 D, INTER = 256, 512
+
+
+class CudaLike(torch.Tensor):
+    """A CPU tensor that says it is on a GPU."""
+
+    def __new__(cls, t):
+        return t.as_subclass(cls)
+
+    is_cuda = True
 
 
 @pytest.fixture
@@ -265,6 +274,19 @@ def test_token_type_ids_of_any_accepted_shape(hooked):
             return model(ids, token_type_ids=t)[0]
     want = out(types.expand(3, 40))
     assert torch.equal(out(types), want) and torch.equal(out(types.repeat(3, 1).view(-1)), want)
+
+
+@pytest.mark.parametrize("dtype", [torch.float64, torch.int64])
+@pytest.mark.parametrize("L", [16, 128])
+def test_residual_inputs_of_other_types_are_refused(calls, monkeypatch, dtype, L):
+    monkeypatch.setattr(sequence_mixer, "_autocast_bf16", lambda: True)
+    m, u = mixer(), CudaLike(torch.zeros((2, L, D), dtype=dtype))
+    with torch.no_grad(), pytest.raises(TypeError):
+        m(u)
+    assert "m2_mixer_fwd" not in calls
+    m.residual_long_conv = False                     # nothing but its bf16 copy is read then
+    with torch.no_grad():
+        m(u)
 
 
 def plans(m):
