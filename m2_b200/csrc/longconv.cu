@@ -116,6 +116,9 @@ extern "C" int m2_longconv_fwd(const m2_longconv_args* a, void* stream) {
              "m2_longconv_fwd: NULL tensor pointer");
   M2_REQUIRE(a->n_filters == 1 || (a->u && a->spec[1] && (folded || a->bias[1])), M2_ERR_ARG,
              "m2_longconv_fwd: residual filter requested but u/spec[1]/bias[1] is NULL");
+  M2_REQUIRE(a->act_dtype == M2_F32 || a->act_dtype == M2_BF16, M2_ERR_UNSUPPORTED, "m2_longconv_fwd: xin and out are float32 or bf16");
+  M2_REQUIRE(a->n_filters == 1 || a->u_dtype == M2_F32 || a->u_dtype == M2_BF16 || (a->u_dtype == M2_F16 && a->kind >= 2), M2_ERR_UNSUPPORTED,
+             "m2_longconv_fwd: u is float32 or bf16, fp16 for kinds 2, 3 and 4 only");
   M2_REQUIRE(a->xin_st == 1 || a->xin_sc == 1, M2_ERR_UNSUPPORTED,
              "m2_longconv_fwd: xin must be contiguous along time or along channels");
   M2_REQUIRE(a->batch <= 65535, M2_ERR_UNSUPPORTED, "m2_longconv_fwd: batch > 65535");

@@ -1,6 +1,7 @@
 """What the modules hand to the one-call entry points (m2_mixer_fwd, m2_mlp_fwd, m2_encoder_fwd), which see pointers and sizes
 and no tensors.  On the CPU with the launch replaced by a recorder: nothing here reaches a GPU."""
 import copy
+import ctypes
 import dataclasses
 import re
 from pathlib import Path
@@ -9,7 +10,7 @@ import pytest
 import torch
 import torch.nn as nn
 
-from m2_b200 import BertGatedLinearUnitMLP, MonarchMixerSequenceMixing, glu_mlp, ops, sequence_mixer
+from m2_b200 import BertGatedLinearUnitMLP, MonarchMixerSequenceMixing, _lib, glu_mlp, ops, sequence_mixer
 from m2_b200._plan import PlanCache, Watch
 from m2_b200.encoder import M2BertConfig, M2BertModel
 from tests.helpers import Cfg
@@ -287,6 +288,21 @@ def test_residual_inputs_of_other_types_are_refused(calls, monkeypatch, dtype, L
     m.residual_long_conv = False                     # nothing but its bf16 copy is read then
     with torch.no_grad():
         m(u)
+
+
+@pytest.mark.parametrize("kind,act,u", [(0, _lib.M2_BF16, _lib.M2_F16), (0, _lib.M2_F32, _lib.M2_F16), (1, _lib.M2_BF16, _lib.M2_F16),
+                                        (0, _lib.M2_F16, _lib.M2_F32)])
+def test_half_operands_are_refused_where_no_kernel_reads_them(kind, act, u):
+    """Sizes of another type would have the kernels read past the end; the check comes before any launch."""
+    a = _lib.LongconvArgs()
+    a.batch, a.seq_len, a.d_model, a.n_filters, a.kind, a.act_dtype, a.u_dtype = 1, 128, 128, 2, kind, act, u
+    host = ctypes.create_string_buffer(64)
+    at = (ctypes.addressof(host) + 15) // 16 * 16
+    a.xin = a.u = a.out = a.short_w = a.short_b = at
+    a.xin_sc = a.u_sc = a.out_sc = 1
+    for i in range(2):
+        a.spec[i] = a.bias[i] = at
+    assert _lib.lib().m2_longconv_fwd(ctypes.byref(a), None) == 2 and b"float32 or bf16" in _lib.lib().m2_last_error()
 
 
 def plans(m):
