@@ -19,8 +19,9 @@
 // cheaper (the A slab is shared by more of them) but leave room for one CTA.  Against the FFT family at the same
 // shapes (18.9 kclk of shared-memory traffic per sequence whatever its length up to 2048): see m2_longconv_pick.
 //
-// The range and rounding of the operands are those of family 3: v * x1 is a bf16 value converted exactly to fp16, the
-// residual input an fp16 copy, taps fp16 after a per-channel power-of-two scaling with the bias folded into h(0),
+// The range and rounding of the operands are those of family 3: v * x1 is a bf16 value converted to fp16 (exactly between
+// 2^-14 and 65504, saturating beyond; the direct kernel of longconv_direct.cu sums it as it is), the residual input an fp16
+// copy, taps fp16 after a per-channel power-of-two scaling with the bias folded into h(0),
 // float32 accumulation in TMEM.  Every mbarrier wait is bounded.
 //
 // Computation replaced: bert/src/mm/monarch_mixer_sequence_mixer.py:109-149 and
@@ -135,6 +136,12 @@ __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t (&r)[4
 __device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, const uint32_t (&r)[4]) {
   asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};"
                ::"r"(addr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory");
+}
+// bf16x2 -> fp16x2, exact inside fp16's range and its largest value beyond, as family 3 has it (a NaN stays one)
+__device__ __forceinline__ uint32_t bf2_to_h2_sat(uint32_t v) {
+  uint32_t r;
+  asm("cvt.rn.satfinite.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(lcl::bf_hi(v)), "f"(lcl::bf_lo(v)));
+  return r;
 }
 // barrier of the worker warps, true where `v` is for all of them
 __device__ __forceinline__ bool workers_and(bool v) {
@@ -291,7 +298,7 @@ longconv_bt_kernel(const Params P) {
             h[0] = v.x; h[1] = v.y; h[2] = v.z; h[3] = v.w;
             if (!P.u_f16) {
 #pragma unroll
-              for (int j = 0; j < 4; ++j) h[j] = bf2_to_h2(h[j]);
+              for (int j = 0; j < 4; ++j) h[j] = bf2_to_h2_sat(h[j]);
             }
             mask_tail(h, 8 * okc, q.w);
           }
@@ -348,7 +355,7 @@ longconv_bt_kernel(const Params P) {
               float cx0, cv0, cx1, cv1;
               f2_unpack(y0, cx0, cv0);
               f2_unpack(y1, cx1, cv1);
-              h[j] = bf2_to_h2(bf2_mul(pack_bf2(cv0, cv1), pack_bf2(cx0, cx1)));
+              h[j] = bf2_to_h2_sat(bf2_mul(pack_bf2(cv0, cv1), pack_bf2(cx0, cx1)));
             }
             mask_tail(h, 8 * okc, lim[i]);
             sts128(a1 + okc * LBO + (8 + g * gcols + k0 + 16 * i + orow) * 16, h[0], h[1], h[2], h[3]);

@@ -133,3 +133,31 @@ def test_mixer_takes_half_inputs_at_float32_lengths():
     m, _, u = mixer(37, 256, 2)
     with torch.no_grad(), torch.autocast("cuda", dtype=torch.bfloat16):
         assert torch.equal(m(u.half())[0], m(u.half().float())[0])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind,L,D,B", [(3, 128, 128, 64), (4, 128, 128, 2), (4, 128, 256, 40), (4, 128, 128, 64), (4, 256, 768, 8)])
+def test_operands_beyond_fp16(kind, L, D, B):
+    """v * x1 and the residual input saturate at 65504 in the Toeplitz families: nothing finite becomes Inf, whichever kernel the
+    batch takes; where they stay below, the result is the float32 family's; and a NaN does not get lost."""
+    m, xin, u = mixer(L, D, B)
+    with torch.no_grad():
+        m.short_filter.weight.zero_()
+        m.short_filter.weight[:, 0, 2] = 1.0
+        m.short_filter.bias.zero_()
+    xin = xin.contiguous()
+    # at step 5 the product of channel 0 is beyond fp16 and that of channel 1 just inside it
+    xin[:, 5, 0], xin[:, 5, 2 * D] = 512.0, 256.0
+    xin[:, 5, 1], xin[:, 5, 2 * D + 1] = 255.0, 256.0
+    u[:, 7, 2] = 1e5                                      # saturates in the fp16 copy
+    y, ref = run(m, kind, xin, u).float(), run(m, 0, xin, u).float()
+    assert torch.isfinite(y).all() and torch.isfinite(ref).all()
+    keep = [c for c in range(D) if c not in (0, 2)]
+    # taps that differ by 2^-12 make some of the three bf16 roundings fall the other way, a step of 2^-8 of the value each; where
+    # a few large steps make up a channel's norm all three may do so on them
+    err = (y - ref)[..., keep].norm(dim=1) / ref[..., keep].norm(dim=1)
+    assert err.max() < 3 * 2 ** -8
+    xin[0, 5, 3] = float("nan")
+    y = run(m, kind, xin, u).float()
+    assert torch.isnan(y[0, :, 3]).any() and torch.isfinite(y[..., 4:]).all()
+    assert ops.device_status() == 0
