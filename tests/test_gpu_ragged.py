@@ -1,5 +1,5 @@
-"""Convolution families on padded time-contiguous rows of any length: the block-Toeplitz family (kind 4) and the long-row
-family (kind 2) at lengths that are no multiple of 8, against the float32 CUDA-core family.  What lies between a row's end
+"""Convolution families on padded time-contiguous rows of any length: the block-Toeplitz family (kind 4), the Toeplitz family
+(kind 3) and the long-row family (kind 2) at lengths that are no multiple of 8, against the float32 CUDA-core family.  What lies between a row's end
 and the next row holds NaNs in the inputs and must stay untouched in the output.  Tolerance: the path's 2e-2 per operator
 (bf16 rounding points shared by both families, one differing flip moves a value by 2^-8 of itself)."""
 import pytest
@@ -36,7 +36,7 @@ def run_both(kind, L, D, B, residual, u_dtype, seed):
         buf = torch.full((D, B, Lp), float("nan"), dtype=torch.bfloat16, device=DEV)
         out = buf[:, :, :L].permute(1, 2, 0)
         ops.longconv_fwd(xin, u if residual else None, m.short_filter.weight, m.short_filter.bias,
-                         [f.spectrum(L, True, kind) for f in filters], None if kind == 4 else biases, kind=kind,
+                         [f.spectrum(L, True, kind) for f in filters], None if kind in (3, 4) else biases, kind=kind,
                          bf16_rounding=True, out=out, yu_bf16=yu)
     torch.cuda.synchronize()
     assert ops.device_status() == 0
@@ -51,6 +51,15 @@ def run_both(kind, L, D, B, residual, u_dtype, seed):
 def test_block_toeplitz_family(L, D, B, residual, u_dtype):
     e = run_both(4, L, D, B, residual, u_dtype, 91)
     print("kind4-vs-kind0: %.3e" % e)
+    assert e < TOL_BF16, e
+
+
+@pytest.mark.parametrize("L", [1, 7, 8, 9, 15, 17, 33, 65, 100, 127, 128])
+@pytest.mark.parametrize("B", [1, 48, 63, 129])
+@pytest.mark.parametrize("residual", [True, False])
+def test_toeplitz_family_at_any_length(L, B, residual):
+    e = run_both(3, L, 16, B, residual, torch.float16, 94)
+    print("kind3-vs-kind0: %.3e" % e)
     assert e < TOL_BF16, e
 
 
