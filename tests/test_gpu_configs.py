@@ -56,7 +56,7 @@ def check_layers(model, sdt, ids, want_kind, final_factor):
     """Per-layer parity on the stock-op path's own inputs, then the free-running model."""
     B, L = ids.shape
     D = model.config.hidden_size
-    assert ops.longconv_kind_batch(B, L, torch.bfloat16, D) == want_kind
+    assert ops.longconv_pick(B, L, torch.bfloat16, D) == want_kind
     worst = 0.0
     with torch.autocast("cuda", dtype=torch.bfloat16):
         h_ref = T.embeddings_forward(sdt, ids)

@@ -295,7 +295,7 @@ def test_encoder_small_fp32_and_bf16():
 @pytest.mark.parametrize("B", [16, 64])
 def test_encoder_80m_shape_bf16(B):
     """Two 80M-shaped layers at the benchmark's L against the stock-op path (batch 16 runs the
-    FFT tensor-core convolution, batch 64 the Toeplitz-GEMM one).
+    block-Toeplitz convolution, batch 64 the Toeplitz-GEMM one).
 
     The path's tolerance (2e-2) is a per-layer statement: each layer is checked on the SAME
     input the stock-op path saw.  Run free, the differences of layer 1 (single bf16 rounding
@@ -304,7 +304,7 @@ def test_encoder_80m_shape_bf16(B):
     """
     cfg = dict(kind="encoder", seed=43, B=B, L=128, D=768, I=3072, layers=2, vocab=30528, order=128)
     model, sd = _encoder(cfg, DEV)
-    assert ops.longconv_kind_batch(B, 128, torch.bfloat16, 768) == (3 if B >= 64 else 1)
+    assert ops.longconv_pick(B, 128, torch.bfloat16, 768) == (3 if B >= 64 else 4)
     ids_t = torch.from_numpy(np.random.default_rng(1).integers(0, 30528, size=(B, 128))).to(DEV)
     sdt = to_torch(sd, DEV)
     with torch.autocast("cuda", dtype=torch.bfloat16):
