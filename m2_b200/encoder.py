@@ -291,8 +291,8 @@ class M2BertModel(nn.Module):
         if plan is None or any_hooks(plan.called) or any_dropping(plan.dropping):
             return None
 
-        ids = [ops.token_ids(input_ids, B, L), ops.token_ids(token_type_ids, B, L),
-               ops.token_ids(position_ids.expand(B, L), B, L) if position_ids is not None else None]
+        ids = [ops.token_ids(input_ids, B, L, dev), ops.token_ids(token_type_ids, B, L, dev),
+               ops.token_ids(position_ids.expand(B, L), B, L, dev) if position_ids is not None else None]
         out = torch.empty(plan.out, dtype=torch.float32, device=dev)
         work = torch.empty(plan.work, dtype=torch.uint8, device=dev)
         a = _lib.EncoderArgs.from_buffer_copy(plan.args)

@@ -334,11 +334,13 @@ def add_layernorm_fwd(a2d, b2d, weight, bias, eps, out_dtype, bf16_copy=None, tm
     return out
 
 
-def token_ids(t, B, L):
-    """(B, L) ids as the embedding kernel reads them: int64, packed.  A tensor of one row, or of one id per row, stands for
-    all of them; B * L ids in any shape are taken in order; None stays None."""
+def token_ids(t, B, L, device):
+    """(B, L) ids as the embedding kernel on `device` reads them: int64, packed.  A tensor of one row, or of one id per row,
+    stands for all of them; B * L ids in any shape are taken in order; None stays None."""
     if t is None:
         return None
+    if t.device != device:
+        raise RuntimeError(f"m2_b200 kernels need ids on one device: {t.device} and {device}")
     return (t.reshape(-1) if t.numel() == B * L else t.expand(B, L)).to(torch.long).contiguous()
 
 
@@ -353,8 +355,9 @@ def embed_layernorm_fwd(input_ids, word_table, type_table, pos_table, weight, bi
     n = word_table.shape[1]
     m = B * L
 
-    keep = [token_ids(input_ids, B, L), token_ids(token_type_ids, B, L),
-            token_ids(position_ids.expand(B, L), B, L) if position_ids is not None else None,
+    dev = input_ids.device
+    keep = [token_ids(input_ids, B, L, dev), token_ids(token_type_ids, B, L, dev),
+            token_ids(position_ids.expand(B, L), B, L, dev) if position_ids is not None else None,
             _f32c(word_table), _f32c(type_table), _f32c(pos_table) if pos_table is not None else None,
             _f32c(weight), _f32c(bias)]
     out = torch.empty((B, L, n), dtype=torch.float32, device=input_ids.device)

@@ -253,13 +253,16 @@ def test_families_one_after_the_other_on_one_stream():
 
 def test_shapes_of_token_type_ids():
     t = torch.arange(6, dtype=torch.int32)
-    assert ops.token_ids(None, 2, 3) is None
+    cpu = torch.device("cpu")
+    assert ops.token_ids(None, 2, 3, cpu) is None
     for same in (t, t.view(2, 3), t.view(6, 1), t.view(2, 3).t().contiguous().t()):
-        assert ops.token_ids(same, 2, 3).view(2, 3).tolist() == [[0, 1, 2], [3, 4, 5]]
-    assert ops.token_ids(t[:3].view(1, 3), 2, 3).view(2, 3).tolist() == [[0, 1, 2]] * 2
+        assert ops.token_ids(same, 2, 3, cpu).view(2, 3).tolist() == [[0, 1, 2], [3, 4, 5]]
+    assert ops.token_ids(t[:3].view(1, 3), 2, 3, cpu).view(2, 3).tolist() == [[0, 1, 2]] * 2
     for wrong in (t[:4], t[:2].view(1, 2), t[:4].view(2, 2)):
         with pytest.raises(RuntimeError):
-            ops.token_ids(wrong, 2, 3)
+            ops.token_ids(wrong, 2, 3, cpu)
+    with pytest.raises(RuntimeError, match="one device"):      # a host pointer in a kernel's arguments otherwise
+        ops.token_ids(t, 2, 3, torch.device("meta"))
 
 
 @pytest.mark.gpu
