@@ -34,14 +34,14 @@ class Watch:
         # plain attributes that plans are made from: those a module's class names in `plan_attrs`, and eps
         names = [(m, type(m).plan_attrs if hasattr(type(m), "plan_attrs") else ("eps",) if isinstance(m, torch.nn.LayerNorm) else ())
                  for m in mods]
-        self.attrs = [(m, attrgetter(*n)) for m, n in names if n]
-        self.attr_values = [get(m) for m, get in self.attrs]
+        self.attrs = [(weakref.ref(m), attrgetter(*n)) for m, n in names if n]     # weak: root holds this, and would hold itself
+        self.attr_values = [get(m()) for m, get in self.attrs]
 
     def same(self):
         try:
             return (all(map(is_, map(dict.__getitem__, self.dicts, self.keys), self.values))
                     and list(map(_version, self.tensors)) == self.versions and list(map(_ptr, self.tensors)) == self.ptrs
-                    and [get(m) for m, get in self.attrs] == self.attr_values)
+                    and [get(m()) for m, get in self.attrs] == self.attr_values)
         except (KeyError, AttributeError):
             return False
 

@@ -3,7 +3,9 @@ and no tensors.  On the CPU with the launch replaced by a recorder: nothing here
 import copy
 import ctypes
 import dataclasses
+import gc
 import re
+import weakref
 from pathlib import Path
 
 import pytest
@@ -11,7 +13,7 @@ import torch
 import torch.nn as nn
 
 from m2_b200 import BertGatedLinearUnitMLP, MonarchMixerSequenceMixing, _lib, glu_mlp, ops, sequence_mixer
-from m2_b200._plan import PlanCache, Watch
+from m2_b200._plan import PlanCache, Watch, plans_of
 from m2_b200.encoder import M2BertConfig, M2BertModel
 from tests.helpers import Cfg
 
@@ -306,6 +308,23 @@ def test_half_operands_are_refused_where_no_kernel_reads_them(kind, act, u):
     for i in range(2):
         a.spec[i] = a.bias[i] = at
     assert _lib.lib().m2_longconv_fwd(ctypes.byref(a), None) == 2 and b"float32 or bf16" in _lib.lib().m2_last_error()
+
+
+def test_modules_with_plans_are_freed_without_the_collector(calls):
+    """A module that its own plans keep alive would keep its GPU memory until the next garbage collection."""
+    gc.collect()
+    gc.disable()
+    try:
+        m, f, model = mixer(), mlp(), small_model()
+        mix(m, torch.zeros(2, 128, D))
+        feed(f, torch.zeros(2, 128, D))
+        plans_of(model).get(model, 0, lambda: model._make_plan(2, 128, torch.device("cpu")))
+        assert plans(m) and plans(f) and plans(model)
+        dead = [weakref.ref(x) for x in (m, f, model)]
+        del m, f, model
+        assert [x() for x in dead] == [None] * 3
+    finally:
+        gc.enable()
 
 
 def plans(m):
