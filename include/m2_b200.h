@@ -98,22 +98,24 @@ int m2_hyena_filter(const m2_filter_args* args, void* stream);
 /* ---------------------------------------------------------------------------------------
  * Filter spectrum in the layout the long-convolution kernel consumes.
  * Replaces `k_f = torch.fft.rfft(k, n=2L) / (2L)`, bert/src/mm/hyena_utils.py:23-24.
- * m2_longconv_kind() names the kernel family used for (seq_len, act_dtype, d_model): 0 = float32
- * arithmetic on CUDA cores (any shape; fastest on channel-contiguous rows of up to 2048 steps), 1 = tcgen05 tensor cores (bf16, 64 < seq_len <= 128,
- * d_model a multiple of 128, channel-contiguous tensors), 2 = tcgen05 tensor cores for long rows
- * (bf16, 128 < seq_len <= 32768, transform length 4096 / 16384 / 65536 for
- * seq_len up to 2048 / 8192 / 32768; needs time-contiguous tensors, i.e. xin_st == u_st ==
- * out_st == 1; when u is a 2-byte type and every row of xin, u and out starts on a 16-byte boundary,
- * the kernel copies its rows into shared memory asynchronously, ahead of their use -- same results bit
- * for bit, 15-35 % less time);
- * 3 = tcgen05 Toeplitz GEMMs with the batch as the M dimension (bf16, seq_len <= 128, any batch,
- * meant for 48 and more; time-contiguous tensors, the residual input as fp16 from m2_time_major_f16); 4 = tcgen05 block-Toeplitz GEMMs, direct float32 sums for a few short rows (bf16, seq_len <= 1024, any
- * batch; time-contiguous tensors, u as fp16 or bf16).  m2_longconv_kind() never returns 3; m2_longconv_kind_batch() does when
- * the batch is large enough to fill the 128-row tiles.  Both answer for tensors whose rows are seq_len steps
- * apart: kind 2 for multiples of 4 only, never 4.  m2_longconv_pick() is the choice for a caller that lays
- * its time-contiguous rows out itself, every row on a 16-byte boundary and readable up to the next multiple of
- * 8 steps (what lies there is never used; kinds 2, 3 and 4 write nothing at or beyond seq_len): 0 where the other two
- * say 0 (the length is computed in float32, on tensors of any layout), else the fastest of 2, 3 and 4.
+ * Kernel families: 0 = float32 arithmetic on CUDA cores (any shape and layout; fastest on channel-contiguous rows of
+ * up to 2048 steps); 1 = tcgen05 FFT (bf16, 64 < seq_len <= 128, d_model a multiple of 128, channel-contiguous
+ * tensors; no module of the package asks for it any more, it stays for callers of this interface); 2 = tcgen05 FFT for
+ * long rows (bf16, 128 < seq_len <= 32768, transform length 4096 / 16384 / 65536 for seq_len up to 2048 / 8192 / 32768;
+ * time-contiguous tensors, i.e. xin_st == u_st == out_st == 1; when u is a 2-byte type and every row of xin, u and
+ * out starts on a 16-byte boundary, the kernel copies its rows into shared memory asynchronously, ahead of their use
+ * -- same results bit for bit, 15-35 % less time); 3 = tcgen05 Toeplitz GEMMs with the batch as the M dimension (bf16,
+ * seq_len <= 128, any batch, meant for 48 and more; time-contiguous tensors, u as fp16 from m2_time_major_f16);
+ * 4 = tcgen05 block-Toeplitz GEMMs, direct float32 sums for a few short rows (bf16, seq_len <= 1024, any batch;
+ * time-contiguous tensors, u as fp16 or bf16).  In fp16: the spectra and the signal between stages in 1 and 2, the taps
+ * and u in 3 and 4; nothing in 0.
+ * m2_longconv_pick() is the choice for a caller that lays its time-contiguous rows out itself, every row on a 16-byte
+ * boundary and readable up to the next multiple of 8 steps (what lies there is never used; kinds 2, 3 and 4 write
+ * nothing at or beyond seq_len): 0 where the length is computed in float32, else the fastest of 2, 3 and 4.  What the
+ * modules ask.
+ * m2_longconv_kind() and m2_longconv_kind_batch() answer for tensors whose rows are seq_len steps apart: 0, 1 (channel-
+ * contiguous), 2 (multiples of 4) and, the latter, 3 (batch >= 64, 16 <= seq_len <= 128, a multiple of 8); never 4.
+ * MonarchMixerSequenceMixing.forward_channels asks the first.
  * m2_filter_spectrum_floats() is the number of float32 the spectrum of one filter takes.
  * m2_filter_spectrum_bias() is m2_filter_spectrum() with the convolution's bias term (the
  * `+ u * bias` of fftconv_ref, bert/src/mm/hyena_utils.py:35-36; float32 (d_model), device, or
@@ -167,7 +169,7 @@ int m2_linear_fwd(const m2_linear_args* args, void* stream);
  *   xin : device, in_linear output; element (b, t, ch), ch in [0, 3*d_model) ordered x1|x2|v,
  *         at xin[b*xin_sb + t*xin_st + ch*xin_sc]; either xin_st == 1 or xin_sc == 1.
  *   u   : device, raw layer input (b, t, c) with its own strides and dtype (float32 or bf16; kinds 2
- *         and 3 also take the fp16 copy written by m2_time_major_f16 / m2_add_layernorm_fwd); used
+ *         to 4 also take the fp16 copy written by m2_time_major_f16 / m2_add_layernorm_fwd); used
  *         only when n_filters == 2.
  *   out : device, (b, t, c) with its own strides, dtype act_dtype: the tensor out_linear
  *         consumes.

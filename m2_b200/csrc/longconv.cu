@@ -45,7 +45,8 @@ extern "C" int m2_longconv_pick(int batch, int seq_len, m2_dtype act_dtype, int 
   // nearly all of it the output's own rounding; kinds 3 and 4 by 1.73e-3 at 37, kind 2 by 1.91e-3 at 1531.
   const bool tz = m2::longconv_tz_supported(batch, seq_len, act_dtype);
   // up to 128 steps both families multiply by the same Toeplitz matrix; kind 3 walks tiles of 128 sequences whatever the
-  // batch (34 us at D = 768, L = 128, B = 8 .. 64), kind 4 tiles as narrow as the batch (20 us at 8, 27 at 32, 51 at 64)
+  // batch (34 us at D = 768, L = 128, B = 8 .. 64), kind 4 tiles as narrow as the batch (20 us at 8, 27 at 32, 51 at 64;
+  // all launched alone with the L2 flushed)
   if (m2::longconv_tc_supported(seq_len, act_dtype, d_model)) return batch >= 48 ? 3 : 4;
   if (seq_len <= 128) return tz ? 3 : 0;
   if (seq_len % 4 != 0) return 0;

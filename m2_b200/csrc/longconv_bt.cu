@@ -13,11 +13,12 @@
 // at different start rows.  The strip is built in shared memory from the channel's 2 L fp16 taps, two deltas (368
 // rows) at a time, while the tensor core works on the two before.
 //
-// Bound: up to NB = 4 (L = 512) by the memory traffic of 10 bytes per step and channel, beyond it by the MMAs (N = 128:
-// 64 clocks each, at 16 blocks of 8 sequences 40 on average because a 4 KB A slab takes 32 to fetch).  Two CTAs share
-// an SM and overlap one's loads and epilogue with the other's MMAs; more than 128 columns per CTA would make the MMAs
-// cheaper (the A slab is shared by more of them) but leave room for one CTA.  Against the FFT family at the same
-// shapes (18.9 kclk of shared-memory traffic per sequence whatever its length up to 2048): see m2_longconv_pick.
+// Bound: few rows by one unit's chain of phases (load, 2 NB strip windows with a hand-over each, gate, write); many short ones
+// (NB <= 4) by the memory traffic of 10 bytes per step and channel.  Beyond that it is neither that nor the MMAs: 16 x 1024 at
+// 768 channels takes 123 us (ncu, caches cold), of which the 240 MMAs of a unit, 40 to 65 clocks each, are some 35 and the
+// traffic 20; two CTAs share an SM and overlap one's phases with the other's, no more.  More than 128 columns per CTA would share
+// a unit's strips among more data but leave room for one CTA.  The FFT family at the same shapes moves 18.9 kclk of
+// shared-memory traffic per sequence whatever its length up to 2048: longconv_bt_preferred draws the line.
 //
 // The range and rounding of the operands are those of family 3: v * x1 is a bf16 value converted to fp16 (exactly between
 // 2^-14 and 65504, saturating beyond; the direct kernel of longconv_direct.cu sums it as it is), the residual input an fp16
@@ -513,9 +514,10 @@ int longconv_bt_supported(int seq_len, m2_dtype act_dtype) {
   return act_dtype == M2_BF16 && seq_len >= 1 && seq_len <= bt::MAX_L;
 }
 
-// Time of the block-Toeplitz kernel in us.  It runs in waves of two units per SM; measured at D = 768, L = 256 .. 1024,
-// B = 1 .. 64, a wave takes 0.25 us per column and 2 us per block, and in the stream of a forward 0.8 of that (D = 768, one
-// sequence to eight: 12 us at 128 steps, 18 at 256, 40 at 384; D = 1536: 28, 34, 58).
+// Time of the block-Toeplitz kernel in us.  It runs in waves of two units per SM; launched alone with the L2 flushed (D = 768,
+// L = 256 .. 1024, B = 1 .. 64) a wave takes 0.25 us per column and 2 us per block, and in the stream of a forward, its start
+// overlapped and its operands in L2, 0.8 of that (D = 768, one sequence to eight: 12 us at 128 steps, 18 at 256, 40 at 384;
+// D = 1536: 28, 34, 58).  The same launch at 8 x 128 is 20 us alone and 16.5 under ncu, which runs it alone with other clocks.
 static double bt_us(int batch, int seq_len, int d_model, int nf) {
   const bt::Shape s = bt::shape_of(seq_len, batch);
   const int g = bt::group_of(s, batch, d_model, nf), sms = m2_sm_count();

@@ -12,8 +12,8 @@
 //
 // Bound by the float32 pipe and shared memory together; the tables (16 bytes a point and channel) come from L2.  Measured
 // at 768 channels, two filters (us, L2 flushed; the stage-by-stage kernel first): 8 x 128 115 -> 33, 4 x 512 283 -> 109,
-// 8 x 1024 797 -> 254, 4 x 2048 920 -> 326, 3 x 500 210 -> 64, 1 x 64 49 -> 21.  On bf16 rows a forward of twelve such layers
-// at 6 x 1531 takes 5.95 ms; with the stage-by-stage kernel and one launch after the other from the host it took 15.5.
+// 8 x 1024 797 -> 254, 4 x 2048 920 -> 326, 3 x 500 210 -> 64, 1 x 64 49 -> 21.  On bf16 rows (float32
+// residual input): 6 x 1531 1163 -> 393, 2 x 514 277 -> 91, 47 x 64 150 -> 86, 8 x 64 57 -> 37, 1 x 37 45 -> 18.
 //
 // Computation replaced: bert/src/mm/monarch_mixer_sequence_mixer.py:109-149 and bert/src/mm/hyena_utils.py:16-42, :219-248
 // of the reference, float32.

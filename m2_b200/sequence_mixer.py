@@ -200,7 +200,8 @@ class MonarchMixerSequenceMixing(nn.Module):
         channel over several GPUs: short convolution, gates and long convolutions are independent per
         channel, in_linear contributes its rows c, D + c, 2D + c, and only out_linear mixes channels (it is
         not part of a shard).  Shards computed on different GPUs and concatenated along the last axis equal
-        forward_channels(u, 0, d_model) bit for bit.  The reference has no counterpart (its parallelism is
+        forward_channels(u, 0, d_model) bit for bit (forward() itself may run another convolution family, whose results agree
+        within the mode's tolerance).  The reference has no counterpart (its parallelism is
         data parallel only); this follows bert/src/mm/monarch_mixer_sequence_mixer.py:108-149 per channel."""
         if not (u.is_cuda and _autocast_bf16()):
             raise RuntimeError("forward_channels runs on CUDA tensors under torch.autocast('cuda', dtype=torch.bfloat16)")
