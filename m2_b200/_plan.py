@@ -64,14 +64,14 @@ class Plan:
         return t.data_ptr()
 
     def registered(self, t, source):
-        """Pointer of `t`, the parameter or buffer `source` itself or a copy of it."""
-        if t.data_ptr() != source.data_ptr():
-            self.held.append(t)
-            self.lasting = False
-        return t.data_ptr()
+        """Pointer of `t`, the parameter `source` itself or a copy of it.  A source that is no parameter (a parametrized module
+        computes it on every access) is held like a copy."""
+        if t.data_ptr() == source.data_ptr() and isinstance(source, torch.nn.Parameter):
+            return t.data_ptr()
+        return self.passing(t)
 
     def f32(self, source):
-        """Pointer of a parameter or buffer as contiguous float32."""
+        """Pointer of a parameter as contiguous float32."""
         return self.registered(ops._f32c(source), source)
 
     def passing(self, t):

@@ -11,6 +11,7 @@ from pathlib import Path
 import pytest
 import torch
 import torch.nn as nn
+from torch.nn.utils import parametrize
 
 from m2_b200 import BertGatedLinearUnitMLP, MonarchMixerSequenceMixing, _lib, glu_mlp, ops, sequence_mixer
 from m2_b200._plan import PlanCache, Watch, plans_of
@@ -151,6 +152,22 @@ def test_a_refusal_is_remembered_until_something_changes():
     assert [cache.get(m, 0, lambda: made.append(0)) for _ in range(3)] == [None] * 3 and len(made) == 1
     m.weight = nn.Parameter(torch.zeros(2, 2))
     assert cache.get(m, 0, lambda: made.append(0)) is None and len(made) == 2
+
+
+class Doubled(nn.Module):
+    def forward(self, t):
+        return 2 * t
+
+
+def test_computed_parameters_are_held_for_the_call(calls):
+    """A parametrized bias is another tensor on every access: its pointer is good while somebody holds that one."""
+    m, f = mixer(), mlp()
+    parametrize.register_parametrization(m.out_linear, "bias", Doubled())
+    parametrize.register_parametrization(f.layernorm, "weight", Doubled())
+    for plan, pointer in ((m._make_plan(2, 128, 4, torch.device("cpu")), "b_out"), (f._plan(torch.device("cpu")), "ln_w")):
+        assert getattr(plan.args, pointer) in [t.data_ptr() for t in plan.held] and not plan.lasting
+    mix(m, torch.zeros(2, 128, D))
+    assert not plans(m) and not plans(f)
 
 
 def test_replicas_have_plans_of_their_own(calls):
