@@ -254,8 +254,6 @@ class M2BertModel(nn.Module):
                  y.attention.residual_long_conv) for y in layers}
         if dims != {(D, D, cfg.intermediate_size, cfg.monarch_mlp_nblocks, layers[0].attention.residual_long_conv)}:
             return None
-        if cfg.intermediate_size % cfg.monarch_mlp_nblocks:        # the last block is shorter: single launches only
-            return None
         if L > 32768:                          # beyond every convolution kernel: the layers raise
             return None
         kind = ops.longconv_pick(B, L, torch.bfloat16, D)
@@ -265,7 +263,8 @@ class M2BertModel(nn.Module):
         plan = Plan(e, layers=args, work=work, out=(B, L, D), called=called, dropping=[m for m in called if hasattr(m, "dropout")])
         for a, y in zip(args, layers):
             y.attention.fill_args(plan, a, L, kind, dev)
-            y.mlp.fill_args(plan, a, dev)
+            if not y.mlp.fill_args(plan, a, dev):
+                return None
         e.batch, e.seq_len, e.d_model, e.inter, e.nblocks = B, L, D, cfg.intermediate_size, cfg.monarch_mlp_nblocks
         e.n_layers, e.kind, e.n_filters = len(layers), kind, 2 if layers[0].attention.residual_long_conv else 1
         word, types = emb.word_embeddings.weight, emb.token_type_embeddings.weight

@@ -41,9 +41,12 @@ class BertGatedLinearUnitMLP(nn.Module):
         self.layernorm = nn.LayerNorm(config.hidden_size, eps=config.layer_norm_eps)
 
     def fill_args(self, plan, a, dev):
-        """Writes the pointers of this module's weights into `a` (a _lib.MlpArgs or _lib.EncoderLayer) of `plan`.  The native
-        call sees pointers only, so what they point to is checked here against the config and the device it runs on."""
+        """Writes the pointers of this module's weights into `a` (a _lib.MlpArgs or _lib.EncoderLayer) of `plan`; False where
+        the native call, which knows one block count and whole blocks only, does not compute what the weights say.  It sees
+        pointers and no tensors, so what they point to is checked here against the config and the device it runs on."""
         D, inter, nb = self.config.hidden_size, self.config.intermediate_size, self.config.monarch_mlp_nblocks
+        if self.gated_layers.weight.shape != (nb, 2 * inter // nb, D // nb) or self.wo.weight.shape != (nb, D // nb, inter // nb):
+            return False
         expect(dev, (self.gated_layers.weight, (nb, 2 * inter // nb, D // nb)), (self.wo.weight, (nb, D // nb, inter // nb)),
                (self.wo.bias, (D,)), (self.layernorm.weight, (D,)), (self.layernorm.bias, (D,)))
         for name, lin in (("wg", self.gated_layers), ("wo", self.wo)):
@@ -52,14 +55,14 @@ class BertGatedLinearUnitMLP(nn.Module):
         if self.wo.bias is not None:
             a.wo_bias = plan.f32(self.wo.bias)
         a.ln_w, a.ln_b, a.eps = plan.f32(self.layernorm.weight), plan.f32(self.layernorm.bias), float(self.layernorm.eps)
+        return True
 
     def _plan(self, dev):
         def make():
             a = _lib.MlpArgs()
             a.d_model, a.inter, a.nblocks = self.config.hidden_size, self.config.intermediate_size, self.config.monarch_mlp_nblocks
             plan = Plan(a)
-            self.fill_args(plan, a, dev)
-            return plan
+            return plan if self.fill_args(plan, a, dev) else None
         return plans_of(self).get(self, dev.index, make)
 
     def _forward_bf16(self, x, x2, plan, copies_only):
@@ -101,9 +104,7 @@ class BertGatedLinearUnitMLP(nn.Module):
         x2 = x.reshape(-1, x.shape[-1])
         if x2.dtype != dt:
             x2 = x2.to(dt)
-        whole = cfg.intermediate_size % cfg.monarch_mlp_nblocks == 0      # else the last block is shorter: single launches only
-        if (dt == torch.bfloat16 and x.dim() == 3 and x2.shape[0] and x.shape[-1] % 256 == 0 and x.shape[-1] <= 2048 and whole
-                and not ops.observed()):
+        if dt == torch.bfloat16 and x.dim() == 3 and x2.shape[0] and x.shape[-1] % 256 == 0 and x.shape[-1] <= 2048 and not ops.observed():
             plan = self._plan(x.device)
             if plan is not None:
                 return self._forward_bf16(x, x2, plan, copies_only)

@@ -79,8 +79,6 @@ def test_another_width_is_refused(calls, width):
     (mix, mixer, lambda m: setattr(m, "out_linear", nn.Linear(D - 1, D))),
     (mix, mixer, lambda m: setattr(m, "short_filter", nn.Conv1d(3 * D, 3 * D, 5, groups=3 * D))),
     (mix, mixer, lambda m: setattr(m, "filter_fn2", mixer(D // 2).filter_fn)),
-    (feed, mlp, lambda m: setattr(m, "wo", mlp(inter=INTER // 2).wo)),
-    (feed, mlp, lambda m: setattr(m, "gated_layers", mlp(nblocks=2).gated_layers)),
     (feed, mlp, lambda m: setattr(m, "layernorm", nn.LayerNorm(D // 2)))])
 def test_weights_of_another_shape_are_refused(calls, run, module, edit):
     m = module()
@@ -108,20 +106,28 @@ def test_linear_layers_without_bias(calls):
     assert a.b_in is None and a.b_out is None and b.wo_bias is None and a.w_in and b.ln_b
 
 
-def test_a_shorter_last_block_takes_single_launches(calls, monkeypatch):
+@pytest.mark.parametrize("f", [lambda: mlp(inter=INTER + 2),      # wo.weight (4, 64, 129): 516 columns for 514 features
+                               lambda: other_blocks(mlp(), "gated_layers"), lambda: other_blocks(mlp(), "wo")])
+def test_weights_of_other_blocks_take_single_launches(calls, monkeypatch, f):
     monkeypatch.setattr(glu_mlp, "_compute_dtype", lambda x: torch.bfloat16)
-    f = mlp(inter=INTER + 2)                         # wo.weight (4, 64, 129): 516 columns for 514 features
+    f, model = f(), small_model()
     with torch.no_grad():
         assert f(torch.zeros(2, 128, D)).shape == (2, 128, D)
     assert calls == ["m2_blockdiag_glu_fwd", "m2_blockdiag_fwd", "m2_add_layernorm_fwd"]
-    model = M2BertModel(M2BertConfig(vocab_size=8, hidden_size=D, intermediate_size=INTER + 2, num_hidden_layers=1, hyena_filter_order=16))
+    model.encoder.layer[1].mlp = f
     assert model._make_plan(2, 128, torch.device("cpu")) is None
 
 
+def other_blocks(f, name):
+    setattr(f, name, getattr(mlp(nblocks=2), name))
+    return f
+
+
 @pytest.mark.gpu
-def test_mlp_with_a_shorter_last_block():
+@pytest.mark.parametrize("f", [lambda: mlp(inter=INTER + 2), lambda: other_blocks(mlp(), "gated_layers"), lambda: other_blocks(mlp(), "wo")])
+def test_mlp_with_other_blocks(f):
     torch.manual_seed(4)
-    f, x = mlp(inter=INTER + 2).cuda(), torch.randn(3, 24, D, device="cuda")
+    f, x = f().cuda(), torch.randn(3, 24, D, device="cuda")
     with torch.no_grad():
         want = f(x)
         with torch.autocast("cuda", dtype=torch.bfloat16):
