@@ -17,14 +17,17 @@ _version = attrgetter("_version")
 _ptr = torch.Tensor.data_ptr
 
 
+WEIGHTS = ("weight", "bias", "freq", "z", "t", "deltas")       # names of the tensors that plans and filter tables are made from
+
+
 class Watch:
     """The parameters, buffers, submodules and settings below `root` as they are now; `same()` says whether they still are."""
 
     def __init__(self, root):
         mods = list(root.modules())
-        if any(isinstance(v, torch.Tensor) for m in mods for v in vars(m).values()):
+        if any(isinstance(vars(m).get(name), torch.Tensor) for m in mods for name in WEIGHTS):
             # weights that are plain attributes (replicas, pruned or functionalised modules) are in no table to be watched
-            raise RuntimeError("tensors outside the modules' parameters and buffers")
+            raise RuntimeError("weights outside the modules' parameters and buffers")
         slots = [(d, k, t) for m in mods for d in (m._parameters, m._buffers) for k, t in d.items()]   # None: no such tensor
         kids = [(m._modules, k, c) for m in mods for k, c in m._modules.items()]
         self.dicts, self.keys, self.values = zip(*(slots + kids))

@@ -160,6 +160,16 @@ def test_a_refusal_is_remembered_until_something_changes():
     assert cache.get(m, 0, lambda: made.append(0)) is None and len(made) == 2
 
 
+def test_other_tensors_on_a_module_do_not_matter():
+    m = small_model()
+    m.temperature = torch.ones(())
+    assert Watch(m).same()
+    m.encoder.layer[0].attention.in_linear._parameters.pop("bias")
+    m.encoder.layer[0].attention.in_linear.bias = torch.zeros(3 * D)
+    with pytest.raises(RuntimeError):
+        Watch(m)
+
+
 class Doubled(nn.Module):
     def forward(self, t):
         return 2 * t
