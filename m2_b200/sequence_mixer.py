@@ -103,9 +103,9 @@ class MonarchMixerSequenceMixing(nn.Module):
 
     def fill_args(self, plan, a, L, kind, dev):
         """Writes the pointers of this module's weights and filter tables into `a` (a _lib.MixerArgs or _lib.EncoderLayer)
-        of `plan`.  The native call sees pointers only, so what they point to is checked here against d_model and the
-        device it runs on."""
-        D = self.d_model
+        of `plan`.  The native call sees pointers only, so what they point to is checked here against in_linear's width and
+        the device it runs on."""
+        D = self.in_linear.weight.shape[-1]
         expect(dev, (self.in_linear.weight, (3 * D, D)), (self.in_linear.bias, (3 * D,)), (self.out_linear.weight, (D, D)),
                (self.out_linear.bias, (D,)), (self.short_filter.weight, (3 * D, 1, 3)), (self.short_filter.bias, (3 * D,)),
                *((f.bias, (D,)) for f in self.filters()), *((f.implicit_filter[6].weight, (D, None)) for f in self.filters()))
@@ -123,7 +123,7 @@ class MonarchMixerSequenceMixing(nn.Module):
     def _make_plan(self, B, L, kind, dev):
         a = _lib.MixerArgs()
         Lp = _round_up(L, 8)
-        a.batch, a.seq_len, a.pitch, a.out_pitch, a.d_model = B, L, Lp, L, self.d_model
+        a.batch, a.seq_len, a.pitch, a.out_pitch, a.d_model = B, L, Lp, L, self.in_linear.weight.shape[-1]
         a.kind, a.n_filters = kind, 2 if self.residual_long_conv else 1
         a.stride, a.u_stride = _round_up(B * Lp, 16), B * Lp
         plan = Plan(a)
@@ -135,8 +135,8 @@ class MonarchMixerSequenceMixing(nn.Module):
         and out_linear reads (D, B, L) through the operand arrangements of m2_linear_fwd, no transposed copy of an
         activation.  Rows are padded to a multiple of 8 steps so that every one starts on a 16-byte boundary."""
         B, L, D = u.shape
-        if D != self.d_model:
-            raise AssertionError(f"input has {D} channels, the mixer {self.d_model}")
+        if D != self.in_linear.weight.shape[-1]:
+            raise AssertionError(f"input has {D} channels, the mixer {self.in_linear.weight.shape[-1]}")
         Lp = _round_up(L, 8)
         dev = u.device
         rec = copies_of(u)

@@ -88,6 +88,13 @@ def test_weights_of_another_shape_are_refused(calls, run, module, edit):
     assert not {"m2_mixer_fwd", "m2_mlp_fwd"} & set(calls)
 
 
+def test_the_weights_decide_the_width(calls):
+    m = mixer()
+    m.d_model = D // 2                               # nothing but the choice of a kernel family reads it
+    assert mix(m, torch.zeros(2, 128, D)).shape == (2, 128, D)
+    assert m._plans.plans.popitem()[1].args.d_model == D
+
+
 @pytest.mark.parametrize("run,module", [(mix, mixer), (feed, mlp)])
 def test_weights_on_another_device_are_refused(calls, run, module):
     with pytest.raises(RuntimeError, match="device"):
