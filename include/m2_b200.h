@@ -26,7 +26,7 @@
 extern "C" {
 #endif
 
-#define M2_B200_ABI_VERSION 4
+#define M2_B200_ABI_VERSION 5
 
 typedef enum { M2_F32 = 0, M2_BF16 = 1, M2_F16 = 2 /* only where an entry point says so */ } m2_dtype;
 
@@ -155,9 +155,16 @@ typedef struct {
   const float* bias;
   void* out; long long out_sb, out_st, out_sc;
   int force_simt;      /* != 0: always the CUDA-core kernel (cross-checks) */
+  const void* w_split; /* float32 only: NULL (one chain of float32 additions in ascending k), or `w` as m2_split_weights writes it:
+                          tensor cores on pairs of fp16 values, float32 results, where rows of x are packed in 16-byte units */
 } m2_linear_args;
 
 int m2_linear_fwd(const m2_linear_args* args, void* stream);
+
+/* Rows of float32 weights (rows, p), each scaled by a power of two and written as pairs of fp16 values that keep 22 bits: the
+ * operand of float32 layers on the tensor cores.  `out` has m2_split_weights_bytes(rows, p) bytes on a 16-byte boundary. */
+size_t m2_split_weights_bytes(long long rows, int p);
+int m2_split_weights(const float* w, long long rows, int p, void* out, void* stream);
 
 /* ---------------------------------------------------------------------------------------
  * Fused gated long convolution: everything between in_linear and out_linear.
@@ -238,7 +245,8 @@ typedef struct {
   const float* bias;
   void* out; long long ldo;
   int variant;   /* 0: the library picks the kernel; 2: CTA-pair tiles (the kernel of m2_linear_fwd) where they apply --
-                    results are bit-identical, kept selectable for cross-checks */
+                    results are bit-identical, kept selectable for cross-checks; float32 ignores it */
+  const void* w_split;   /* as in m2_linear_args */
 } m2_blockdiag_args;
 
 int m2_blockdiag_fwd(const m2_blockdiag_args* args, void* stream);
@@ -261,6 +269,7 @@ typedef struct {
                     1: always the kernel that streams x and wg tiles through shared memory (the general one);
                     3: CTA pairs with resident x slices where they apply.  Results are bit-identical; the variants are
                     selectable for cross-checks */
+  const void* wg_split;  /* as w_split in m2_linear_args */
 } m2_glu_args;
 
 int m2_blockdiag_glu_fwd(const m2_glu_args* args, void* stream);
@@ -340,6 +349,8 @@ int m2_embed_layernorm_fwd(const m2_embed_layernorm_args* args, void* stream);
  *   xin, conv : workspace, bf16 (3 d_model, stride) and (d_model, stride), stride a multiple of 16 >= batch * pitch.
  *   out  : bf16, packed rows, out_pitch = pitch or seq_len of them per sequence.
  *   kind : 2, 3 or 4, from m2_longconv_pick(); spec and bias as m2_longconv_fwd takes them for that kind.
+ *   f32  : != 0 without autocast: x, w_in, w_out, xin, conv and out are float32 on packed token rows (pitch, out_pitch =
+ *          seq_len), x is the residual input too (u is not read), kind is 0, w_in_split and w_out_split as in m2_linear_args.
  * ------------------------------------------------------------------------------------- */
 typedef struct {
   int batch, seq_len, pitch, out_pitch, d_model, kind, n_filters, yu_bf16;
@@ -351,13 +362,15 @@ typedef struct {
   const void* w_out; const float* b_out;     /* bf16 (d_model, d_model), float32 (d_model) */
   void* xin; void* conv; long long stride;
   void* out;
+  int f32; const void* w_in_split; const void* w_out_split;
 } m2_mixer_args;
 
 int m2_mixer_fwd(const m2_mixer_args* args, void* stream);
 
 /* BertGatedLinearUnitMLP.forward under bf16 autocast (bert/src/bert_layers.py:482-508): GLU GEMM, wo GEMM, add + LayerNorm.
  * x bf16 (m, d_model); h, o workspace bf16 (m, inter), (m, d_model); outputs as in m2_add_layernorm_fwd: `out` float32 or
- * NULL, out_bf16 (m, d_model) and out_tm_f16 (d_model, m / seq_len, seq_len) with channels tm_stride apart, or NULL. */
+ * NULL, out_bf16 (m, d_model) and out_tm_f16 (d_model, m / seq_len, seq_len) with channels tm_stride apart, or NULL.
+ * f32 != 0: x, weights, h, o and out float32, no other outputs; wg_split and wo_split as in m2_linear_args. */
 typedef struct {
   int m, d_model, inter, nblocks;
   const void* x;
@@ -366,6 +379,7 @@ typedef struct {
   void* h; void* o;
   float* out; void* out_bf16; void* out_tm_f16; long long tm_stride;
   int seq_len, valid_len;
+  int f32; const void* wg_split; const void* wo_split;
 } m2_mlp_args;
 
 int m2_mlp_fwd(const m2_mlp_args* args, void* stream);
@@ -375,12 +389,15 @@ int m2_mlp_fwd(const m2_mlp_args* args, void* stream);
  *   embed : tables, ids, LayerNorm of the embeddings as m2_embed_layernorm_fwd takes them (ids packed, batch * seq_len);
  *           its outputs and sizes are filled in here.
  *   kind  : 0, 2, 3 or 4, from m2_longconv_pick(); spec and bias of each layer as m2_longconv_fwd takes them for that kind.
- *   workspace : m2_encoder_workspace() bytes on a 256-byte boundary, pitch = seq_len rounded up to a multiple of 8. */
+ *   workspace : m2_encoder_workspace() bytes on a 256-byte boundary, pitch = seq_len rounded up to a multiple of 8.
+ *   f32   : != 0 without autocast: the layers alone (6 n_layers launches), from the embeddings' float32 output x; kind 0, float32
+ *           weights, m2_encoder_workspace_f32() bytes. */
 typedef struct {
   const void* w_in; const float* b_in; const float* short_w; const float* short_b;
   const float* spec[2]; const float* bias[2];
   const void* w_out; const float* b_out;
   const void* wg; const void* wo; const float* wo_bias; const float* ln_w; const float* ln_b; float eps;
+  const void* w_in_split; const void* w_out_split; const void* wg_split; const void* wo_split;   /* f32 only */
 } m2_encoder_layer;
 
 typedef struct {
@@ -389,9 +406,11 @@ typedef struct {
   const m2_encoder_layer* layers;            /* host memory */
   void* workspace;
   float* out;
+  int f32; const float* x;
 } m2_encoder_args;
 
 long long m2_encoder_workspace(int batch, int pitch, int d_model, int inter);
+long long m2_encoder_workspace_f32(int batch, int seq_len, int d_model, int inter);
 int m2_encoder_fwd(const m2_encoder_args* args, void* stream);
 
 #ifdef __cplusplus

@@ -10,7 +10,7 @@ import os
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libm2b200.so")
-ABI_VERSION = 4
+ABI_VERSION = 5
 
 M2_F32, M2_BF16, M2_F16 = 0, 1, 2
 
@@ -57,7 +57,7 @@ class BlockdiagArgs(C.Structure):
         ("m", C.c_int), ("nblocks", C.c_int), ("p", C.c_int), ("q", C.c_int),
         ("in_features", C.c_int), ("out_features", C.c_int), ("dtype", C.c_int),
         ("x", C.c_void_p), ("ldx", C.c_longlong), ("w", C.c_void_p), ("bias", C.c_void_p),
-        ("out", C.c_void_p), ("ldo", C.c_longlong), ("variant", C.c_int),
+        ("out", C.c_void_p), ("ldo", C.c_longlong), ("variant", C.c_int), ("w_split", C.c_void_p),
     ]
 
 
@@ -66,7 +66,7 @@ class GluArgs(C.Structure):
         ("m", C.c_int), ("d_model", C.c_int), ("inter", C.c_int), ("nblocks", C.c_int),
         ("dtype", C.c_int),
         ("x", C.c_void_p), ("ldx", C.c_longlong), ("wg", C.c_void_p),
-        ("h", C.c_void_p), ("ldh", C.c_longlong), ("variant", C.c_int),
+        ("h", C.c_void_p), ("ldh", C.c_longlong), ("variant", C.c_int), ("wg_split", C.c_void_p),
     ]
 
 
@@ -77,7 +77,7 @@ class LinearArgs(C.Structure):
         ("x", C.c_void_p), ("x_sb", C.c_longlong), ("x_st", C.c_longlong), ("x_sc", C.c_longlong),
         ("w", C.c_void_p), ("bias", C.c_void_p),
         ("out", C.c_void_p), ("out_sb", C.c_longlong), ("out_st", C.c_longlong), ("out_sc", C.c_longlong),
-        ("force_simt", C.c_int),
+        ("force_simt", C.c_int), ("w_split", C.c_void_p),
     ]
 
 
@@ -116,6 +116,7 @@ class MixerArgs(C.Structure):
         ("w_in", C.c_void_p), ("b_in", C.c_void_p), ("short_w", C.c_void_p), ("short_b", C.c_void_p),
         ("spec", C.c_void_p * 2), ("bias", C.c_void_p * 2), ("w_out", C.c_void_p), ("b_out", C.c_void_p),
         ("xin", C.c_void_p), ("conv", C.c_void_p), ("stride", C.c_longlong), ("out", C.c_void_p),
+        ("f32", C.c_int), ("w_in_split", C.c_void_p), ("w_out_split", C.c_void_p),
     ]
 
 
@@ -127,6 +128,7 @@ class MlpArgs(C.Structure):
         ("h", C.c_void_p), ("o", C.c_void_p),
         ("out", C.c_void_p), ("out_bf16", C.c_void_p), ("out_tm_f16", C.c_void_p), ("tm_stride", C.c_longlong),
         ("seq_len", C.c_int), ("valid_len", C.c_int),
+        ("f32", C.c_int), ("wg_split", C.c_void_p), ("wo_split", C.c_void_p),
     ]
 
 
@@ -136,6 +138,7 @@ class EncoderLayer(C.Structure):
         ("spec", C.c_void_p * 2), ("bias", C.c_void_p * 2), ("w_out", C.c_void_p), ("b_out", C.c_void_p),
         ("wg", C.c_void_p), ("wo", C.c_void_p), ("wo_bias", C.c_void_p),
         ("ln_w", C.c_void_p), ("ln_b", C.c_void_p), ("eps", C.c_float),
+        ("w_in_split", C.c_void_p), ("w_out_split", C.c_void_p), ("wg_split", C.c_void_p), ("wo_split", C.c_void_p),
     ]
 
 
@@ -144,6 +147,7 @@ class EncoderArgs(C.Structure):
         ("batch", C.c_int), ("seq_len", C.c_int), ("d_model", C.c_int), ("inter", C.c_int), ("nblocks", C.c_int),
         ("n_layers", C.c_int), ("kind", C.c_int), ("n_filters", C.c_int),
         ("embed", EmbedLayernormArgs), ("layers", C.POINTER(EncoderLayer)), ("workspace", C.c_void_p), ("out", C.c_void_p),
+        ("f32", C.c_int), ("x", C.c_void_p),
     ]
 
 
@@ -162,6 +166,8 @@ SYMBOLS = {
     "m2_longconv_pick": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_int]),
     "m2_filter_spectrum_bias": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
     "m2_linear_fwd": (C.c_int, [C.POINTER(LinearArgs), C.c_void_p]),
+    "m2_split_weights_bytes": (C.c_size_t, [C.c_longlong, C.c_int]),
+    "m2_split_weights": (C.c_int, [C.c_void_p, C.c_longlong, C.c_int, C.c_void_p, C.c_void_p]),
     "m2_longconv_fwd": (C.c_int, [C.POINTER(LongconvArgs), C.c_void_p]),
     "m2_time_major_f16": (C.c_int, [C.POINTER(TimeMajorArgs), C.c_void_p]),
     "m2_blockdiag_fwd": (C.c_int, [C.POINTER(BlockdiagArgs), C.c_void_p]),
@@ -171,6 +177,7 @@ SYMBOLS = {
     "m2_mixer_fwd": (C.c_int, [C.POINTER(MixerArgs), C.c_void_p]),
     "m2_mlp_fwd": (C.c_int, [C.POINTER(MlpArgs), C.c_void_p]),
     "m2_encoder_workspace": (C.c_longlong, [C.c_int, C.c_int, C.c_int, C.c_int]),
+    "m2_encoder_workspace_f32": (C.c_longlong, [C.c_int, C.c_int, C.c_int, C.c_int]),
     "m2_encoder_fwd": (C.c_int, [C.POINTER(EncoderArgs), C.c_void_p]),
 }
 

@@ -15,33 +15,62 @@ struct Layout {
   long long rows, stride;                       // padded tokens; distance of two channels of a time-contiguous tensor
   size_t aug, tm, xin, conv, mix, h, o, total;
 };
-static Layout layout_of(int batch, int pitch, int d_model, int inter) {
+static Layout layout_of(int batch, int pitch, int d_model, int inter, bool f32) {
   Layout l;
   l.rows = (long long)batch * pitch;
   l.stride = round_up(l.rows, 16);
   size_t at = 0;
-  auto take = [&](long long elements) { const size_t p = at; at += (size_t)round_up(2 * elements, 256); return p; };
-  l.aug = take(l.rows * d_model);
-  l.tm = take(l.stride * d_model);
+  const int size = f32 ? 4 : 2;
+  auto take = [&](long long elements) { const size_t p = at; at += (size_t)round_up(size * elements, 256); return p; };
+  l.aug = take(f32 ? 0 : l.rows * d_model);      // float32 layers read each other's output as it is
+  l.tm = take(f32 ? 0 : l.stride * d_model);
   l.mix = take(l.rows * d_model);
   l.o = take(l.rows * d_model);
   l.xin = l.h = at;                             // in_linear's and the conv's results are dead when the GLU writes h
   take(3 * l.stride * d_model);
   l.conv = take(l.stride * d_model);
-  const size_t h_end = l.h + (size_t)round_up(2 * l.rows * inter, 256);
+  const size_t h_end = l.h + (size_t)round_up(size * l.rows * inter, 256);
   l.total = at > h_end ? at : h_end;
   return l;
+}
+
+// The mixer on float32 token rows.
+static int mixer_f32(const m2_mixer_args* a, void* stream) {
+  const int L = a->seq_len, D = a->d_model;
+  m2_linear_args p;
+  memset(&p, 0, sizeof(p));
+  p.batch = a->batch; p.seq_len = L; p.in_features = D; p.out_features = 3 * D; p.dtype = M2_F32;
+  p.x = a->x; p.x_sb = (long long)L * D; p.x_st = D; p.x_sc = 1;
+  p.w = a->w_in; p.bias = a->b_in; p.w_split = a->w_in_split;
+  p.out = a->xin; p.out_sb = 3LL * L * D; p.out_st = 3LL * D; p.out_sc = 1;
+  int rc;
+  if ((rc = m2_linear_fwd(&p, stream))) return rc;
+  m2_longconv_args c;
+  memset(&c, 0, sizeof(c));
+  c.batch = a->batch; c.seq_len = L; c.d_model = D; c.n_filters = a->n_filters; c.kind = 0;
+  c.act_dtype = M2_F32; c.u_dtype = M2_F32;
+  c.xin = a->xin; c.xin_sb = 3LL * L * D; c.xin_st = 3LL * D; c.xin_sc = 1;
+  c.u = a->x; c.u_sb = (long long)L * D; c.u_st = D; c.u_sc = 1;
+  c.out = a->conv; c.out_sb = (long long)L * D; c.out_st = D; c.out_sc = 1;
+  c.short_w = a->short_w; c.short_b = a->short_b;
+  for (int f = 0; f < 2; ++f) { c.spec[f] = a->spec[f]; c.bias[f] = a->bias[f]; }
+  if ((rc = m2_longconv_fwd(&c, stream))) return rc;
+  p.x = a->conv; p.out_features = D; p.w = a->w_out; p.bias = a->b_out; p.w_split = a->w_out_split;
+  p.out = a->out; p.out_sb = (long long)L * D; p.out_st = D;
+  return m2_linear_fwd(&p, stream);
 }
 
 }  // namespace m2
 
 extern "C" int m2_mixer_fwd(const m2_mixer_args* a, void* stream) {
   M2_REQUIRE(a != nullptr, M2_ERR_ARG, "m2_mixer_fwd: args is NULL");
-  M2_REQUIRE(a->batch >= 0 && a->seq_len > 0 && a->d_model > 0 && a->pitch >= a->seq_len && a->pitch % 8 == 0 &&
+  M2_REQUIRE(a->batch >= 0 && a->seq_len > 0 && a->d_model > 0 && (a->f32 ? a->pitch == a->seq_len : a->pitch >= a->seq_len && a->pitch % 8 == 0) &&
              (a->out_pitch == a->pitch || a->out_pitch == a->seq_len) && a->stride >= (long long)a->batch * a->pitch, M2_ERR_ARG,
              "m2_mixer_fwd: bad sizes batch=%d seq_len=%d pitch=%d out_pitch=%d d_model=%d", a->batch, a->seq_len, a->pitch, a->out_pitch, a->d_model);
-  M2_REQUIRE(a->kind >= 2 && a->kind <= 4, M2_ERR_UNSUPPORTED, "m2_mixer_fwd: kind must be 2, 3 or 4 (time-contiguous rows)");
+  M2_REQUIRE(a->f32 ? a->kind == 0 : a->kind >= 2 && a->kind <= 4, M2_ERR_UNSUPPORTED,
+             "m2_mixer_fwd: kind must be 2, 3 or 4 (time-contiguous rows), or 0 in float32");
   if (a->batch == 0) return M2_OK;
+  if (a->f32) return m2::mixer_f32(a, stream);
   const int rows = a->batch * a->pitch;
   int rc;
   m2_linear_args in;
@@ -79,21 +108,22 @@ extern "C" int m2_mlp_fwd(const m2_mlp_args* a, void* stream) {
   M2_REQUIRE(a->d_model % a->nblocks == 0 && a->inter % a->nblocks == 0, M2_ERR_UNSUPPORTED,
              "m2_mlp_fwd: d_model and inter must be multiples of nblocks");
   if (a->m == 0) return M2_OK;
+  const m2_dtype dtype = a->f32 ? M2_F32 : M2_BF16;
   int rc;
   m2_glu_args g;
   memset(&g, 0, sizeof(g));
-  g.m = a->m; g.d_model = a->d_model; g.inter = a->inter; g.nblocks = a->nblocks; g.dtype = M2_BF16;
-  g.x = a->x; g.ldx = a->d_model; g.wg = a->wg; g.h = a->h; g.ldh = a->inter;
+  g.m = a->m; g.d_model = a->d_model; g.inter = a->inter; g.nblocks = a->nblocks; g.dtype = dtype;
+  g.x = a->x; g.ldx = a->d_model; g.wg = a->wg; g.h = a->h; g.ldh = a->inter; g.wg_split = a->f32 ? a->wg_split : nullptr;
   if ((rc = m2_blockdiag_glu_fwd(&g, stream))) return rc;
   m2_blockdiag_args w;
   memset(&w, 0, sizeof(w));
   w.m = a->m; w.nblocks = a->nblocks; w.p = a->inter / a->nblocks; w.q = a->d_model / a->nblocks;
-  w.in_features = a->inter; w.out_features = a->d_model; w.dtype = M2_BF16;
+  w.in_features = a->inter; w.out_features = a->d_model; w.dtype = dtype; w.w_split = a->f32 ? a->wo_split : nullptr;
   w.x = a->h; w.ldx = a->inter; w.w = a->wo; w.bias = a->wo_bias; w.out = a->o; w.ldo = a->d_model;
   if ((rc = m2_blockdiag_fwd(&w, stream))) return rc;
   m2_add_layernorm_args n;
   memset(&n, 0, sizeof(n));
-  n.m = a->m; n.n = a->d_model; n.in_dtype = M2_BF16; n.out_dtype = M2_F32;
+  n.m = a->m; n.n = a->d_model; n.in_dtype = dtype; n.out_dtype = M2_F32;
   n.a = a->o; n.lda = a->d_model; n.b = a->x; n.ldb = a->d_model;
   n.weight = a->ln_w; n.bias = a->ln_b; n.eps = a->eps;
   n.out = a->out; n.ldo = a->d_model;
@@ -105,7 +135,42 @@ extern "C" int m2_mlp_fwd(const m2_mlp_args* a, void* stream) {
 
 extern "C" long long m2_encoder_workspace(int batch, int pitch, int d_model, int inter) {
   if (batch <= 0 || pitch <= 0 || d_model <= 0 || inter <= 0) return 0;
-  return (long long)m2::layout_of(batch, pitch, d_model, inter).total;
+  return (long long)m2::layout_of(batch, pitch, d_model, inter, false).total;
+}
+
+extern "C" long long m2_encoder_workspace_f32(int batch, int seq_len, int d_model, int inter) {
+  if (batch <= 0 || seq_len <= 0 || d_model <= 0 || inter <= 0) return 0;
+  return (long long)m2::layout_of(batch, seq_len, d_model, inter, true).total;
+}
+
+// The layers in float32, from the embeddings' output.
+static int encoder_f32(const m2_encoder_args* a, void* stream) {
+  using namespace m2;
+  M2_REQUIRE(a->x && a->kind == 0, M2_ERR_ARG, "m2_encoder_fwd: float32 layers need x and kind 0");
+  M2_REQUIRE((long long)a->batch * a->seq_len < (1LL << 31) - 512, M2_ERR_UNSUPPORTED, "m2_encoder_fwd: more than 2^31 tokens");
+  const Layout l = layout_of(a->batch, a->seq_len, a->d_model, a->inter, true);
+  unsigned char* ws = static_cast<unsigned char*>(a->workspace);
+  const float* in = a->x;
+  for (int i = 0; i < a->n_layers; ++i, in = a->out) {         // a layer's input is dead when its MLP writes the output
+    const m2_encoder_layer& y = a->layers[i];
+    m2_mixer_args x;
+    memset(&x, 0, sizeof(x));
+    x.batch = a->batch; x.seq_len = x.pitch = x.out_pitch = a->seq_len; x.d_model = a->d_model; x.n_filters = a->n_filters; x.f32 = 1;
+    x.x = in; x.w_in = y.w_in; x.b_in = y.b_in; x.w_in_split = y.w_in_split; x.short_w = y.short_w; x.short_b = y.short_b;
+    for (int f = 0; f < 2; ++f) { x.spec[f] = y.spec[f]; x.bias[f] = y.bias[f]; }
+    x.w_out = y.w_out; x.b_out = y.b_out; x.w_out_split = y.w_out_split;
+    x.xin = ws + l.xin; x.conv = ws + l.conv; x.stride = l.stride; x.out = ws + l.mix;
+    int rc;
+    if ((rc = m2_mixer_fwd(&x, stream))) return rc;
+    m2_mlp_args p;
+    memset(&p, 0, sizeof(p));
+    p.m = (int)l.rows; p.d_model = a->d_model; p.inter = a->inter; p.nblocks = a->nblocks; p.f32 = 1;
+    p.x = ws + l.mix; p.wg = y.wg; p.wo = y.wo; p.wo_bias = y.wo_bias; p.ln_w = y.ln_w; p.ln_b = y.ln_b; p.eps = y.eps;
+    p.wg_split = y.wg_split; p.wo_split = y.wo_split;
+    p.h = ws + l.h; p.o = ws + l.o; p.out = a->out;
+    if ((rc = m2_mlp_fwd(&p, stream))) return rc;
+  }
+  return M2_OK;
 }
 
 // The mixer of one layer where the convolution runs in float32 (kind 0): token rows throughout, the layer input u float32.
@@ -141,11 +206,12 @@ extern "C" int m2_encoder_fwd(const m2_encoder_args* a, void* stream) {
   M2_REQUIRE(a->batch > 0 && a->seq_len > 0 && a->n_layers > 0 && a->d_model > 0 && a->inter > 0, M2_ERR_ARG, "m2_encoder_fwd: bad sizes");
   M2_REQUIRE(a->layers && a->workspace && a->out && m2_aligned(a->workspace, 256), M2_ERR_ARG,
              "m2_encoder_fwd: NULL pointer or workspace not on a 256-byte boundary");
+  if (a->f32) return encoder_f32(a, stream);
   M2_REQUIRE(a->kind == 0 || (a->kind >= 2 && a->kind <= 4), M2_ERR_UNSUPPORTED, "m2_encoder_fwd: kind must be 0, 2, 3 or 4");
   const bool rows = a->kind == 0;               // float32 convolution: token rows without padding, float32 layer inputs in `out`
   const int pitch = rows ? a->seq_len : (int)round_up(a->seq_len, 8), D = a->d_model;
   M2_REQUIRE((long long)a->batch * pitch < (1LL << 31) - 512, M2_ERR_UNSUPPORTED, "m2_encoder_fwd: more than 2^31 tokens");
-  const Layout l = layout_of(a->batch, pitch, D, a->inter);
+  const Layout l = layout_of(a->batch, pitch, D, a->inter, false);
   unsigned char* ws = static_cast<unsigned char*>(a->workspace);
   int rc;
   m2_embed_layernorm_args e = a->embed;

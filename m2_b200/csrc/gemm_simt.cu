@@ -354,6 +354,7 @@ extern "C" int m2_blockdiag_fwd(const m2_blockdiag_args* a, void* stream) {
   if (blockdiag_pair_supported(a)) return blockdiag_pair_launch(a, st);
   dim3 grid((a->q + GT - 1) / GT, (a->m + GT - 1) / GT, a->nblocks);
   M2_REQUIRE(grid.y <= 65535 && grid.z <= 65535, M2_ERR_UNSUPPORTED, "m2_blockdiag_fwd: too many row tiles");
+  if (blockdiag_split_supported(a)) return blockdiag_split_launch(a, st);
   if (blockdiag_f32_supported(a)) return blockdiag_f32_launch(a, st);
   if (a->dtype == M2_BF16)
     blockdiag_simt_kernel<__nv_bfloat16, true><<<grid, 256, 0, st>>>(
@@ -388,6 +389,7 @@ extern "C" int m2_blockdiag_glu_fwd(const m2_glu_args* a, void* stream) {
   const int p = a->d_model / a->nblocks, q = 2 * a->inter / a->nblocks;
   dim3 grid((q + GT - 1) / GT, (a->m + GT - 1) / GT, a->nblocks / 2);
   M2_REQUIRE(grid.y <= 65535, M2_ERR_UNSUPPORTED, "m2_blockdiag_glu_fwd: too many row tiles");
+  if (glu_split_supported(a)) return glu_split_launch(a, st);
   if (glu_f32_supported(a)) return glu_f32_launch(a, st);
   if (a->dtype == M2_BF16)
     blockdiag_glu_simt_kernel<__nv_bfloat16, true><<<grid, 256, 0, st>>>(

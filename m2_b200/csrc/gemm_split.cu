@@ -1,0 +1,542 @@
+// Linear and block-diagonal layers on float32 activations as tcgen05 GEMMs over pairs of fp16 values, with float32 results.
+//
+// Every 64 columns of a row of x are scaled by a power of two that brings the largest of them to [2^14, 2^15) and written as
+// hi + lo, two fp16 values that keep 22 bits of it; a weight row is scaled and split once as a whole.  x . w is then
+// lo.hi + hi.lo + hi.hi on the tensor cores (lo.lo is below 2^-24 of it), summed over 64 columns in tensor memory, small
+// terms first.  Each such sum is scaled back and added to a float32 register, rounded to nearest: the tensor core's own
+// accumulation drops what does not fit, always towards zero, so a chain of K / 16 of its additions would be further from the
+// exact sum than a float32 chain; four of them are nearer (N(0, 1) operands, 768 columns, relative 2-norm against 64 bits: chain
+// 5.0e-7; sums in tensor memory over 768 columns 2.6e-6, 256 8.4e-7, 128 3.8e-7, 64 1.5e-7).
+//
+// A row whose largest value is beyond 2^90 (or infinite) marks its tile, a weight row its output column; their non-finite
+// results are summed again as the ascending float32 chain of gemm_f32.cu.  NaNs stay NaNs by themselves.
+//
+// Roles: warp 0 brings float32 rows of x and split rows of w to shared memory by TMA, warps 12-19 convert (a thread owns a row
+// of x; four warps take the even K blocks, four the odd ones) and leave hi and lo in tensor memory, from where the MMAs take
+// them as their A operand, warp 1 issues the MMAs, warps 4-11 add up.
+//
+// Bound: 64 columns of a 128 x 128 tile bring 64 KB to the SM, 1700 clocks at the 38 bytes a clock that TMA tile loads reach in every
+// GEMM here; shared memory is busy for 1150 of them (64 KB written, 32 read by the conversion, 48 by the 12 MMAs of 64 clocks).
+// Splitting x too before the launch would cost a pass and move as many bytes; converting both operands in place in shared memory
+// took 2.3 times as long there.  Few rows: the first loads and one K block after the other.
+// Measured (us, L2 flushed; the float32 chain of gemm_f32.cu first): 768 -> 2304 at 64 / 1024 / 2048 / 8192 tokens 38 / 94 / 180 /
+// 684 -> 16 / 23 / 36 / 111; 768 -> 768 37 / 57 / 87 at 64 / 1024 / 2048 -> 16 / 19 / 23; GLU 768 -> 3072 at 2048 158 -> 45; wo 88 -> 25.
+// A tile's scales and biases come through shared memory and the accumulators are several: with scalar loads in the epilogue and
+// two accumulators 8192 tokens took 137 us and the GLU 61.
+//
+// Computation replaced: nn.Linear of bert/src/mm/monarch_mixer_sequence_mixer.py:100-154, bert/src/mm/blockdiag_multiply.py:49-60,
+// bert/src/mm/structured_linear.py:52-70, bert/src/bert_layers.py:492-506 of the reference, float32.
+#include "tc_common.cuh"
+
+namespace m2 {
+namespace f32s {
+
+constexpr int BM = 128, BK = 64;
+constexpr int FLUSH0 = 4, FLUSH_WARPS = 8, CONV0 = 12, CONV_WARPS = 4, THREADS = 32 * (CONV0 + 2 * CONV_WARPS);
+constexpr int NA = 4;                      // buffers of hi and lo in tensor memory, 64 columns each
+constexpr int SLOTS = 16;                  // K blocks whose scales are kept: more than can be between a conversion and its sum
+constexpr float HUGE_ROW = 1.2379400392853803e27f;   // 2^90
+constexpr int X_BYTES = BM * 256;          // two boxes of 32 float32 columns
+
+template <int BN> struct Geo {
+  static constexpr int STAGE = X_BYTES + BN * 256;                   // rows of x, then hi and lo of the rows of w
+  static constexpr int NST = BN == 128 ? 3 : (BN == 64 ? 4 : 5);
+  static constexpr int OFF_SCALE = NST * STAGE;                      // [SLOTS][BM] floats
+  static constexpr int OFF_HUGE = OFF_SCALE + SLOTS * BM * 4;        // [SLOTS][CONV_WARPS] ints
+  static constexpr int NACC = BN == 128 ? 2 : 4;                     // accumulators
+  static constexpr int OFF_COLS = OFF_HUGE + SLOTS * CONV_WARPS * 4; // [2] of a tile's columns: inverse scales (of both halves of a GLU), bias
+  static constexpr int OFF_BAR = OFF_COLS + 2 * 2 * BN * 4;
+  static constexpr int NBARS = 2 * NST + SLOTS + 2 * NA + 2 * NACC + 4;
+  static constexpr int SMEM = OFF_BAR + NBARS * 8 + 16 + 1024;
+  static constexpr uint32_t TCOLS = 512;                             // accumulators and buffers of hi and lo: 384 columns at least
+  static_assert(SMEM <= 227 * 1024, "shared memory budget");
+};
+
+struct Params {
+  const float* x; long long ldx;           // row t of x, block kb: x + t * ldx + kb * p
+  const float* w;                          // [block][q][p]
+  const __half* ws; const float* winv;     // the same rows split, and the inverse of each row's scale
+  const float* bias;
+  float* out; long long osb, ost, osc;     // token t at (t / L) * osb + (t % L) * ost
+  int tokens, L, p, q, steps;
+  int partner;                             // GLU: block kb is gated, block kb + partner is its factor
+  int n_tiles, m_tiles, total;
+  int vec;                                 // 32-byte stores are legal for eight neighbouring columns
+};
+
+// the largest magnitude's biased exponent -> scale that brings it to [2^14, 2^15), and its inverse
+__device__ __forceinline__ float split_scale(uint32_t ex) { return __uint_as_float((268u - ex) << 23); }
+__device__ __forceinline__ float split_inverse(uint32_t ex) { return __uint_as_float((ex - 14u) << 23); }
+__device__ __forceinline__ uint32_t split_exponent(float m) { return max(27u, __float_as_uint(m) >> 23); }
+__device__ __forceinline__ void split_pair(float y0, float y1, uint32_t& hi, uint32_t& lo) {
+  const __half2 h = __floats2half2_rn(y0, y1);
+  const float2 hf = __half22float2(h);
+  const __half2 l = __floats2half2_rn(y0 - hf.x, y1 - hf.y);
+  hi = *reinterpret_cast<const uint32_t*>(&h);
+  lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+
+// weight rows: per 64 columns hi, then lo; zeros up to the next multiple of 64.  A warp per row.
+__global__ void __launch_bounds__(256)
+split_weights_kernel(const float* __restrict__ w, int rows, int p, int steps, __half* __restrict__ ws, float* __restrict__ winv) {
+  const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (row >= rows) return;
+  const float* r = w + (size_t)row * p;
+  float m = 0.f;
+  for (int k = lane; k < p; k += 32) m = fmaxf(m, fabsf(r[k]));
+  for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+  const uint32_t ex = split_exponent(m);
+  const float s = split_scale(ex);
+  uint32_t* o = reinterpret_cast<uint32_t*>(ws) + (size_t)row * steps * BK;
+  for (int k = 2 * lane; k < steps * BK; k += 64) {
+    uint32_t hi, lo;
+    split_pair(k < p ? r[k] * s : 0.f, k + 1 < p ? r[k + 1] * s : 0.f, hi, lo);
+    const int at = (k / BK) * BK + (k % BK) / 2;
+    o[at] = hi;
+    o[at + BK / 2] = lo;
+  }
+  if (lane == 0) winv[row] = m >= HUGE_ROW ? __int_as_float(0x7fffffff) : split_inverse(ex);   // NaN: the column is summed again
+}
+
+// D[tmem] (+)= A[tmem] * B[smem desc]
+__device__ __forceinline__ void mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}\n"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+               ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// the sum as the float32 kernels have it: one chain of fused multiply-adds in ascending k
+__device__ __noinline__ float chain(const float* x, const float* w, int p) {
+  float s = 0.f;
+  for (int k = 0; k < p; ++k) s = fmaf(__ldg(x + k), __ldg(w + k), s);
+  return s;
+}
+
+template <int BN, bool GLU>
+__global__ void __launch_bounds__(THREADS, 1)
+gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const Params P) {
+  using G = Geo<BN>;
+  constexpr int NST = G::NST, NACC = G::NACC, CPW = BN / 2;          // accumulator columns of a flush warp
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  float* scales = reinterpret_cast<float*>(smem + G::OFF_SCALE);
+  float* cvals = reinterpret_cast<float*>(smem + G::OFF_COLS);
+  int* huge = reinterpret_cast<int*>(smem + G::OFF_HUGE);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + G::OFF_BAR);
+  uint64_t* full = bars;                   // [NST] boxes have landed
+  uint64_t* empty = full + NST;            // [NST] x has been read by the converters, w by the MMAs
+  uint64_t* sfull = empty + NST;           // [SLOTS] scales of a K block are written
+  uint64_t* afull = sfull + SLOTS;         // [NA] hi and lo of x are in tensor memory
+  uint64_t* aempty = afull + NA;           // [NA] and have been read
+  uint64_t* tfull = aempty + NA;           // [NACC] the K block's sums are complete
+  uint64_t* tempty = tfull + NACC;         // [NACC] the sums have been read
+  uint64_t* cfull = tempty + NACC;         // [2] a tile's column values are there
+  uint64_t* cempty = cfull + 2;            // [2] and have been used
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + G::NBARS);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int warp = tc::uniform_warp_id(), lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < NST; ++s) { tc::mbar_init(full + s, 1); tc::mbar_init(empty + s, CONV_WARPS + 1); }
+    for (int s = 0; s < SLOTS; ++s) tc::mbar_init(sfull + s, CONV_WARPS);
+    for (int b = 0; b < NA; ++b) { tc::mbar_init(afull + b, CONV_WARPS); tc::mbar_init(aempty + b, 1); }
+    for (int b = 0; b < 2; ++b) { tc::mbar_init(cfull + b, 32); tc::mbar_init(cempty + b, FLUSH_WARPS); }
+    for (int b = 0; b < NACC; ++b) { tc::mbar_init(tfull + b, 1); tc::mbar_init(tempty + b, FLUSH_WARPS); }
+    *abort_flag = 0;
+    tc::mbar_fence_init();
+    tc::tma_prefetch_desc(&tmX);
+    tc::tma_prefetch_desc(&tmW);
+  }
+  if (warp == 1) {
+    tc::tmem_alloc(tmem_slot, G::TCOLS);
+    tc::tmem_relinquish();
+  }
+  tc::tc_fence_before();
+  __syncthreads();
+  tc::tc_fence_after();
+  const uint32_t tmem = *tmem_slot, tmem_a = tmem + NACC * BN;       // buffer b: hi at 64 b, lo at 64 b + 32
+  pdl_wait();
+
+  const int blocks = GLU ? 2 * P.steps : P.steps;    // K blocks of a tile; those of the GLU's factor follow those of its gate
+  auto decode = [&](int tile, int& mt, int& nt, int& kb) {
+    nt = tile % P.n_tiles;
+    const int r = tile / P.n_tiles;
+    mt = r % P.m_tiles;
+    kb = r / P.m_tiles;
+  };
+
+  if (warp == 0) {
+    // ---- TMA producer ----
+    if (tc::elect_one()) {
+      int stage = 0; uint32_t phase = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < P.total && ok; tile += gridDim.x) {
+        int mt, nt, kb;
+        decode(tile, mt, nt, kb);
+        for (int c = 0; c < blocks; ++c) {
+          ok = tc::mbar_wait(empty + stage, phase ^ 1, abort_flag, tc::ST_TIMEOUT_EMPTY);
+          if (!ok) break;
+          const bool second = GLU && c >= P.steps;
+          const int b = second ? kb + P.partner : kb, s = second ? c - P.steps : c;
+          unsigned char* st = smem + stage * G::STAGE;
+          tc::mbar_expect_tx(full + stage, G::STAGE);
+          tc::tma_load_3d(st, &tmX, full + stage, s * BK, b, mt * BM);
+          tc::tma_load_3d(st + BM * 128, &tmX, full + stage, s * BK + 32, b, mt * BM);
+          tc::tma_load_2d(st + X_BYTES, &tmW, full + stage, s * 2 * BK, b * P.q + nt * BN);
+          tc::tma_load_2d(st + X_BYTES + BN * 128, &tmW, full + stage, s * 2 * BK + BK, b * P.q + nt * BN);
+          if (++stage == NST) { stage = 0; phase ^= 1; }
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // ---- MMA issue ----
+    if (tc::elect_one()) {
+      constexpr uint32_t idesc = tc::make_idesc(BM, BN, 0);
+      const uint64_t b_hi = tc::smem_desc_k_sw128(tc::smem_u32(smem + X_BYTES)), b_lo = tc::desc_advance(b_hi, BN * 128 >> 4);
+      int stage = 0; uint32_t phase = 0, it = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < P.total && ok; tile += gridDim.x) {
+        for (int c = 0; c < blocks; ++c, ++it) {
+          const int buf = it % NACC, ab = it % NA;
+          ok = tc::mbar_wait(full + stage, phase, abort_flag, tc::ST_TIMEOUT_TMA) &&
+               tc::mbar_wait(tempty + buf, ((it / NACC) & 1) ^ 1, abort_flag, tc::ST_TIMEOUT_MMA) &&
+               tc::mbar_wait(afull + ab, (it / NA) & 1, abort_flag, tc::ST_TIMEOUT_MMA);
+          if (!ok) break;
+          tc::tc_fence_after();
+          const uint32_t acc = tmem + buf * BN, a = tmem_a + ab * 64, off = (uint32_t)(stage * (G::STAGE >> 4));
+#pragma unroll
+          for (int kk = 0; kk < BK / 16; ++kk) mma_ts(acc, a + 32 + 8 * kk, tc::desc_advance(b_hi, off + 2 * kk), idesc, kk ? 1u : 0u);
+#pragma unroll
+          for (int kk = 0; kk < BK / 16; ++kk) mma_ts(acc, a + 8 * kk, tc::desc_advance(b_lo, off + 2 * kk), idesc, 1u);
+#pragma unroll
+          for (int kk = 0; kk < BK / 16; ++kk) mma_ts(acc, a + 8 * kk, tc::desc_advance(b_hi, off + 2 * kk), idesc, 1u);
+          tc::mma_commit(empty + stage);
+          tc::mma_commit(aempty + ab);
+          tc::mma_commit(tfull + buf);
+          if (++stage == NST) { stage = 0; phase ^= 1; }
+        }
+      }
+    }
+  } else if (warp == 2) {
+    // ---- column values of the tiles ----
+    uint32_t n = 0;
+    for (int tile = blockIdx.x; tile < P.total; tile += gridDim.x, ++n) {
+      int mt, nt, kb;
+      decode(tile, mt, nt, kb);
+      bool ok = tc::mbar_wait(cempty + (n & 1), ((n >> 1) & 1) ^ 1, abort_flag, tc::ST_TIMEOUT_EMPTY);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      float* dst = cvals + (n & 1) * 2 * BN;
+      for (int j = lane; j < BN; j += 32) {
+        const bool in = nt * BN + j < P.q;
+        const long long c = (long long)kb * P.q + nt * BN + j;
+        dst[j] = in ? __ldg(P.winv + c) : 0.f;
+        dst[BN + j] = !in ? 0.f : GLU ? __ldg(P.winv + c + (long long)P.partner * P.q) : P.bias ? __ldg(P.bias + c) : 0.f;
+      }
+      tc::mbar_arrive(cfull + (n & 1));
+    }
+  } else if (warp >= CONV0) {
+    // ---- conversion: a thread owns one row of x ----
+    const int group = (warp - CONV0) / CONV_WARPS, cw = warp & 3, r = cw * 32 + lane, sw = (r & 7) * 16;
+    const uint32_t tq = tmem_a + ((uint32_t)(cw * 32) << 16);
+    uint32_t it = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < P.total && ok; tile += gridDim.x) {
+      for (int c = 0; c < blocks; ++c, ++it) {
+        if ((int)(it & 1) != group) continue;
+        const uint32_t stage = it % NST;
+        ok = tc::mbar_wait(full + stage, (it / NST) & 1, abort_flag, tc::ST_TIMEOUT_TMA);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        const int slot = it & (SLOTS - 1);
+        const unsigned char* p0 = smem + stage * G::STAGE + r * 128;
+        float4 v[16];
+        float m = 0.f;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          v[j] = *reinterpret_cast<const float4*>(p0 + (j < 8 ? 0 : BM * 128) + (((j & 7) * 16) ^ sw));
+          m = fmaxf(m, fmaxf(fmaxf(fabsf(v[j].x), fabsf(v[j].y)), fmaxf(fabsf(v[j].z), fabsf(v[j].w))));
+        }
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(empty + stage);
+        const uint32_t ex = split_exponent(m);
+        const f32x2 s = f2_splat(split_scale(ex));
+        scales[slot * BM + r] = split_inverse(ex);
+        const bool any = __any_sync(0xffffffffu, m >= HUGE_ROW);
+        if (lane == 0) huge[slot * CONV_WARPS + cw] = any;
+        const uint32_t ab = it % NA, ta = tq + ab * 64;
+        ok = tc::mbar_wait(aempty + ab, ((it / NA) & 1) ^ 1, abort_flag, tc::ST_TIMEOUT_MMA);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        tc::tc_fence_after();
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {                  // 16 columns: eight tensor-memory columns of pairs
+          uint32_t hi[8], lo[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const float4& q = v[4 * j + (i >> 1)];
+            float y0, y1;
+            f2_unpack(f2_mul((i & 1) ? f2_pack(q.z, q.w) : f2_pack(q.x, q.y), s), y0, y1);
+            split_pair(y0, y1, hi[i], lo[i]);
+          }
+          tmem_st8(ta + 8 * j, hi);
+          tmem_st8(ta + 32 + 8 * j, lo);
+        }
+        tmem_st_wait();
+        tc::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          tc::mbar_arrive(afull + ab);
+          tc::mbar_arrive(sfull + slot);
+        }
+      }
+    }
+  } else if (warp >= FLUSH0) {
+    // ---- K-block sums to float32 registers, then the tile's results ----
+    const int quarter = warp & 3, half = (warp - FLUSH0) >> 2;
+    const uint32_t tl = tmem + ((uint32_t)(quarter * 32) << 16) + half * CPW;
+    uint32_t it = 0, n = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < P.total && ok; tile += gridDim.x, ++n) {
+      int mt, nt, kb;
+      decode(tile, mt, nt, kb);
+      f32x2 acc[GLU ? 2 : 1][CPW / 2];
+      int big = 0;
+#pragma unroll
+      for (int g = 0; g < (GLU ? 2 : 1); ++g) {
+#pragma unroll
+        for (int j = 0; j < CPW / 2; ++j) acc[g][j] = 0;
+        for (int c = 0; c < P.steps; ++c, ++it) {
+          const int buf = it % NACC, slot = it & (SLOTS - 1);
+          ok = ok && tc::mbar_wait(sfull + slot, (it / SLOTS) & 1, abort_flag, tc::ST_TIMEOUT_EPI) &&
+               tc::mbar_wait(tfull + buf, (it / NACC) & 1, abort_flag, tc::ST_TIMEOUT_EPI);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          tc::tc_fence_after();
+          const f32x2 rs = f2_splat(scales[slot * BM + quarter * 32 + lane]);
+          const int4 h = *reinterpret_cast<const int4*>(huge + slot * CONV_WARPS);
+          big |= h.x | h.y | h.z | h.w;
+#pragma unroll
+          for (int c0 = 0; c0 < CPW; c0 += 16) {
+            uint32_t t[16];
+            tc::tmem_ld16(tl + buf * BN + c0, t);
+            tc::tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              acc[g][c0 / 2 + j] = f2_fma(f2_pack(__uint_as_float(t[2 * j]), __uint_as_float(t[2 * j + 1])), rs, acc[g][c0 / 2 + j]);
+          }
+          tc::tc_fence_before();
+          __syncwarp();
+          if (lane == 0) tc::mbar_arrive(tempty + buf);
+        }
+      }
+      if (!ok) break;
+      ok = tc::mbar_wait(cfull + (n & 1), (n >> 1) & 1, abort_flag, tc::ST_TIMEOUT_EPI);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      const int t = mt * BM + quarter * 32 + lane, c0 = nt * BN + half * CPW;
+      const long long base = (long long)(t / P.L) * P.osb + (long long)(t % P.L) * P.ost;
+      const float* cv = cvals + (n & 1) * 2 * BN + half * CPW;
+      float* orow = P.out + base + ((long long)kb * P.q + c0) * P.osc;
+      bool again = big != 0;
+#pragma unroll
+      for (int j8 = 0; j8 < CPW; j8 += 8) {
+        uint32_t v[8];
+#pragma unroll
+        for (int j = 0; j < 8; j += 4) {
+          const float4 w = *reinterpret_cast<const float4*>(cv + j8 + j), b = *reinterpret_cast<const float4*>(cv + BN + j8 + j);
+          again |= !(w.x + w.y + w.z + w.w < 3e38f);
+          float a0, a1, a2, a3;
+          if (GLU) {
+            again |= !(b.x + b.y + b.z + b.w < 3e38f);
+            float n0, n1, n2, n3;
+            f2_unpack(f2_mul(acc[0][(j8 + j) / 2], f2_pack(w.x, w.y)), a0, a1);
+            f2_unpack(f2_mul(acc[0][(j8 + j) / 2 + 1], f2_pack(w.z, w.w)), a2, a3);
+            f2_unpack(f2_mul(acc[GLU ? 1 : 0][(j8 + j) / 2], f2_pack(b.x, b.y)), n0, n1);
+            f2_unpack(f2_mul(acc[GLU ? 1 : 0][(j8 + j) / 2 + 1], f2_pack(b.z, b.w)), n2, n3);
+            a0 = gelu_erf(a0) * n0; a1 = gelu_erf(a1) * n1; a2 = gelu_erf(a2) * n2; a3 = gelu_erf(a3) * n3;
+          } else {
+            // the scale is a power of two: one rounding, as in a sum followed by the bias
+            f2_unpack(f2_fma(acc[0][(j8 + j) / 2], f2_pack(w.x, w.y), f2_pack(b.x, b.y)), a0, a1);
+            f2_unpack(f2_fma(acc[0][(j8 + j) / 2 + 1], f2_pack(w.z, w.w), f2_pack(b.z, b.w)), a2, a3);
+          }
+          v[j] = __float_as_uint(a0); v[j + 1] = __float_as_uint(a1); v[j + 2] = __float_as_uint(a2); v[j + 3] = __float_as_uint(a3);
+        }
+        if (t >= P.tokens) continue;
+        if (P.vec && c0 + j8 + 8 <= P.q) {
+          stg256(orow + j8, v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            if (c0 + j8 + j < P.q) orow[(j8 + j) * P.osc] = __uint_as_float(v[j]);
+        }
+      }
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(cempty + (n & 1));
+      if (again && t < P.tokens) {
+        const float* xr = P.x + (long long)t * P.ldx + (long long)kb * P.p;
+        for (int j = 0; j < CPW && c0 + j < P.q; ++j) {
+          const long long c = (long long)kb * P.q + c0 + j;
+          float* po = P.out + base + c * P.osc;
+          if (fabsf(*po) <= 3.402823466e38f) continue;
+          float v = chain(xr, P.w + c * P.p, P.p);
+          if (GLU) v = gelu_erf(v) * chain(xr + (long long)P.partner * P.p, P.w + (c + (long long)P.partner * P.q) * P.p, P.p);
+          else if (P.bias) v += __ldg(P.bias + c);
+          *po = v;
+        }
+      }
+    }
+  }
+  __syncthreads();
+  if (*abort_flag && threadIdx.x == 0) {
+    // loads issued before the abort get a bounded time to land
+    for (int s = 0; s < NST; ++s)
+      for (uint32_t i = 0; i < 4096 && !tc::mbar_try_wait(full + s, 0) && !tc::mbar_try_wait(full + s, 1); ++i) {}
+  }
+  tc::tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc::tc_fence_after();
+    tc::tmem_dealloc(tmem, G::TCOLS);
+  }
+}
+
+// float32 rows {p (contiguous), nb blocks, tokens}, box 32 x 1 x 128, 128-byte swizzle, zeros out of range
+static int make_tmap_rows(CUtensorMap* map, const void* base, uint64_t p, uint64_t nb, uint64_t tokens, uint64_t ld) {
+  m2_encode_tiled_fn enc;
+  int rc = m2_get_encode_fn(&enc);
+  if (rc) return rc;
+  cuuint64_t dims[3] = {p, nb, tokens};
+  cuuint64_t strides[2] = {p * 4, ld * 4};
+  cuuint32_t box[3] = {32, 1, BM};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<void*>(base), dims, strides, box, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return m2_set_error(M2_ERR_CUDA, "cuTensorMapEncodeTiled (float32) failed with code %d", (int)r);
+  return M2_OK;
+}
+
+template <int BN, bool GLU>
+static int launch(Params& P, int nblocks, cudaStream_t st) {
+  CUtensorMap tmX, tmW;
+  int rc;
+  const uint64_t rows = (uint64_t)nblocks * P.q, pitch = (uint64_t)P.steps * 2 * BK;
+  if ((rc = make_tmap_rows(&tmX, P.x, P.p, nblocks, P.tokens, P.ldx))) return rc;
+  // 16-bit elements are moved as they are: the bf16 map serves fp16
+  if ((rc = m2_make_tmap_bf16_2d(&tmW, P.ws, rows, pitch, pitch, BN))) return rc;
+  P.n_tiles = (P.q + BN - 1) / BN;
+  P.m_tiles = (P.tokens + BM - 1) / BM;
+  P.total = P.n_tiles * P.m_tiles * (GLU ? nblocks / 2 : nblocks);
+  auto kern = gemm_split_kernel<BN, GLU>;
+  constexpr int SMEM = Geo<BN>::SMEM;
+  M2_SMEM_ONCE(kern, SMEM);
+  const int sms = m2_sm_count();
+  return m2_launch("gemm_split_kernel", (long long)P.tokens * P.p * nblocks, kern, P.total < sms ? P.total : sms, THREADS, SMEM, st, tmX, tmW, P);
+}
+
+// Columns of a tile: a K block of 64 costs some 1150 clocks at 128 columns, 750 at 64, 600 at 32.
+static int pick_bn(const Params& P, int blocks) {
+  const int sms = m2_sm_count();
+  auto cost = [&](int bn, double per) {
+    const long long tiles = (long long)((P.tokens + BM - 1) / BM) * ((P.q + bn - 1) / bn) * blocks;
+    return (double)((tiles + sms - 1) / sms) * P.steps * per;
+  };
+  const double c128 = cost(128, 1150), c64 = cost(64, 750), c32 = cost(32, 600);
+  return c128 <= c64 && c128 <= c32 ? 128 : (c64 <= c32 ? 64 : 32);
+}
+
+// What the TMA loads need: rows that start on 16-byte boundaries; `ws` as m2_split_weights writes it.  Below 128 products a
+// chain is about as exact (68 columns: 1.3e-7 of the result both) and as fast (36 columns, 100 rows: 10.3 us both).
+static bool rows_ok(const void* x, long long ld, const void* ws, int p) {
+  return ws && p >= 2 * BK && p % 4 == 0 && ld % 4 == 0 && m2_aligned(x, 16) && m2_aligned(ws, 16);
+}
+static size_t split_halves(long long rows, int p) { return (size_t)rows * ((p + BK - 1) / BK) * 2 * BK; }
+static void set_weights(Params& P, const void* w, const void* ws, long long rows) {
+  P.w = (const float*)w;
+  P.ws = (const __half*)ws;
+  P.winv = reinterpret_cast<const float*>(P.ws + split_halves(rows, P.p));
+  P.steps = (P.p + BK - 1) / BK;
+}
+
+static int run(Params& P, int blocks, cudaStream_t st) {
+  const int bn = pick_bn(P, blocks);
+  if (bn == 128) return launch<128, false>(P, blocks, st);
+  if (bn == 64) return launch<64, false>(P, blocks, st);
+  return launch<32, false>(P, blocks, st);
+}
+
+}  // namespace f32s
+
+bool linear_split_supported(const m2_linear_args* a) {
+  return a->dtype == M2_F32 && !a->force_simt && a->x_sc == 1 && (a->batch == 1 || a->x_sb == (long long)a->seq_len * a->x_st) &&
+         a->x_st >= a->in_features && f32s::rows_ok(a->x, a->x_st, a->w_split, a->in_features);
+}
+
+int linear_split_launch(const m2_linear_args* a, cudaStream_t st) {
+  f32s::Params P = {};
+  P.x = (const float*)a->x; P.ldx = a->x_st;
+  P.bias = a->bias;
+  P.out = (float*)a->out; P.osb = a->out_sb; P.ost = a->out_st; P.osc = a->out_sc;
+  P.tokens = a->batch * a->seq_len; P.L = a->seq_len; P.p = a->in_features; P.q = a->out_features;
+  f32s::set_weights(P, a->w, a->w_split, P.q);
+  P.vec = a->out_sc == 1 && m2_aligned(a->out, 32) && a->out_st % 8 == 0 && (a->batch == 1 || a->out_sb % 8 == 0);
+  return f32s::run(P, 1, st);
+}
+
+bool blockdiag_split_supported(const m2_blockdiag_args* a) {
+  return a->dtype == M2_F32 && a->in_features == a->nblocks * a->p && a->out_features == a->nblocks * a->q && a->ldx >= a->in_features &&
+         f32s::rows_ok(a->x, a->ldx, a->w_split, a->p);
+}
+
+int blockdiag_split_launch(const m2_blockdiag_args* a, cudaStream_t st) {
+  f32s::Params P = {};
+  P.x = (const float*)a->x; P.ldx = a->ldx;
+  P.bias = a->bias;
+  P.out = (float*)a->out; P.ost = a->ldo; P.osc = 1;
+  P.tokens = P.L = a->m; P.p = a->p; P.q = a->q;
+  f32s::set_weights(P, a->w, a->w_split, (long long)a->nblocks * a->q);
+  P.vec = m2_aligned(a->out, 32) && a->ldo % 8 == 0 && a->q % 8 == 0;
+  return f32s::run(P, a->nblocks, st);
+}
+
+bool glu_split_supported(const m2_glu_args* a) {
+  return a->dtype == M2_F32 && a->ldx >= a->d_model && f32s::rows_ok(a->x, a->ldx, a->wg_split, a->d_model / a->nblocks);
+}
+
+int glu_split_launch(const m2_glu_args* a, cudaStream_t st) {
+  f32s::Params P = {};
+  P.x = (const float*)a->x; P.ldx = a->ldx;
+  P.out = (float*)a->h; P.ost = a->ldh; P.osc = 1;
+  P.tokens = P.L = a->m; P.p = a->d_model / a->nblocks; P.q = 2 * a->inter / a->nblocks;
+  P.partner = a->nblocks / 2;
+  f32s::set_weights(P, a->wg, a->wg_split, (long long)a->nblocks * P.q);
+  P.vec = m2_aligned(a->h, 32) && a->ldh % 8 == 0 && P.q % 8 == 0;
+  return f32s::launch<64, true>(P, a->nblocks, st);
+}
+
+}  // namespace m2
+
+extern "C" size_t m2_split_weights_bytes(long long rows, int p) {
+  if (rows <= 0 || p <= 0) return 0;
+  return m2::f32s::split_halves(rows, p) * 2 + (size_t)rows * 4;
+}
+
+extern "C" int m2_split_weights(const float* w, long long rows, int p, void* out, void* stream) {
+  using namespace m2::f32s;
+  M2_REQUIRE(rows > 0 && rows < (1LL << 31) - 8 && p > 0, M2_ERR_ARG, "m2_split_weights: bad sizes rows=%lld p=%d", rows, p);
+  M2_REQUIRE(w && out, M2_ERR_ARG, "m2_split_weights: NULL pointer");
+  M2_REQUIRE(m2_aligned(out, 16), M2_ERR_ALIGN, "m2_split_weights: out must be 16-byte aligned");
+  __half* ws = static_cast<__half*>(out);
+  split_weights_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      w, (int)rows, p, (p + BK - 1) / BK, ws, reinterpret_cast<float*>(ws + split_halves(rows, p)));
+  M2_LAUNCH_CHECK("split_weights_kernel");
+  return M2_OK;
+}

@@ -460,6 +460,7 @@ extern "C" int m2_linear_fwd(const m2_linear_args* a, void* stream) {
   if (!tc_ok) {
     dim3 grid((N + 63) / 64, (unsigned)((tokens + 63) / 64));
     M2_REQUIRE(grid.y <= 65535, M2_ERR_UNSUPPORTED, "m2_linear_fwd: too many tokens for the CUDA-core kernel");
+    if (linear_split_supported(a)) return linear_split_launch(a, st);
     if (linear_f32_supported(a)) return linear_f32_launch(a, st);
     if (a->dtype == M2_BF16)
       lin::linear_simt_kernel<__nv_bfloat16, true><<<grid, 256, 0, st>>>(

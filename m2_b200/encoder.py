@@ -238,7 +238,7 @@ class M2BertModel(nn.Module):
             ms += [layer, layer.attention, layer.mlp]
         return ms
 
-    def _make_plan(self, B, L, dev):
+    def _make_plan(self, B, L, dev, f32=False):
         """Arguments of one m2_encoder_fwd for (B, L), or None where the modules are not what that call computes."""
         emb, layers = self.embeddings, list(self.encoder.layer)
         D = emb.word_embeddings.weight.shape[1]
@@ -256,17 +256,22 @@ class M2BertModel(nn.Module):
             return None
         if L > 32768:                          # beyond every convolution kernel: the layers raise
             return None
-        kind = ops.longconv_pick(B, L, torch.bfloat16, D)
+        kind = 0 if f32 else ops.longconv_pick(B, L, torch.bfloat16, D)
         args = (_lib.EncoderLayer * len(layers))()
         e = _lib.EncoderArgs()
-        work = _lib.lib().m2_encoder_workspace(B, (L + 7) // 8 * 8, D, cfg.intermediate_size)
+        work = (_lib.lib().m2_encoder_workspace_f32(B, L, D, cfg.intermediate_size) if f32 else
+                _lib.lib().m2_encoder_workspace(B, (L + 7) // 8 * 8, D, cfg.intermediate_size))
         plan = Plan(e, layers=args, work=work, out=(B, L, D), called=called, dropping=[m for m in called if hasattr(m, "dropout")])
         for a, y in zip(args, layers):
-            y.attention.fill_args(plan, a, L, kind, dev)
-            if not y.mlp.fill_args(plan, a, dev):
+            y.attention.fill_args(plan, a, L, kind, dev, f32)
+            if not y.mlp.fill_args(plan, a, dev, f32):
                 return None
         e.batch, e.seq_len, e.d_model, e.inter, e.nblocks = B, L, D, cfg.intermediate_size, cfg.monarch_mlp_nblocks
         e.n_layers, e.kind, e.n_filters = len(layers), kind, 2 if layers[0].attention.residual_long_conv else 1
+        e.f32 = f32
+        e.layers = C.cast(args, C.POINTER(_lib.EncoderLayer))
+        if f32:                                # the embeddings are modules of their own there
+            return plan
         word, types = emb.word_embeddings.weight, emb.token_type_embeddings.weight
         e.embed.word_table, e.embed.vocab_rows = plan.f32(word), word.shape[0]
         e.embed.type_table, e.embed.type_rows = plan.f32(types), types.shape[0]
@@ -275,7 +280,6 @@ class M2BertModel(nn.Module):
             e.embed.pos_table, e.embed.pos_rows = plan.f32(pos), pos.shape[0]
         norm = emb.LayerNorm
         e.embed.weight, e.embed.bias, e.embed.eps = plan.f32(norm.weight), plan.f32(norm.bias), float(norm.eps)
-        e.layers = C.cast(args, C.POINTER(_lib.EncoderLayer))
         return plan
 
     def _encode_whole(self, input_ids, token_type_ids, position_ids):
@@ -304,12 +308,33 @@ class M2BertModel(nn.Module):
         ops._launch("m2_encoder_fwd", out, _lib.lib().m2_encoder_fwd, C.byref(a), launches=1 + 6 * a.n_layers)
         return out
 
+    def _layers_f32(self, h):
+        """All layers on the float32 embeddings as one native call: no autocast, no gradients, no hooks on the way.  None where
+        the layers have to be called one by one."""
+        if not (h.is_cuda and h.dim() == 3 and h.dtype == torch.float32 and not torch.is_grad_enabled()
+                and not torch.is_autocast_enabled("cuda") and h.shape[0] > 0 and h.shape[1] > 0) or ops.observed():
+            return None
+        B, L, D = h.shape
+        plan = plans_of(self).get(self, (B, L, "f32", h.device.index), lambda: self._make_plan(B, L, h.device, f32=True))
+        if plan is None or plan.out != (B, L, D) or any_hooks(plan.called) or any_dropping(plan.dropping):
+            return None
+        h = h.contiguous()
+        out = torch.empty(plan.out, dtype=torch.float32, device=h.device)
+        work = torch.empty(plan.work, dtype=torch.uint8, device=h.device)
+        a = _lib.EncoderArgs.from_buffer_copy(plan.args)
+        a.x, a.workspace, a.out = h.data_ptr(), work.data_ptr(), out.data_ptr()
+        ops._launch("m2_encoder_fwd", out, _lib.lib().m2_encoder_fwd, C.byref(a), launches=6 * a.n_layers)
+        return out
+
     def forward(self, input_ids, token_type_ids=None, attention_mask=None, position_ids=None,
                 output_all_encoded_layers=False):
         whole = None if output_all_encoded_layers else self._encode_whole(input_ids, token_type_ids, position_ids)
         if whole is not None:
             return self._finish([whole], attention_mask, False)
         h = self.embeddings(input_ids, token_type_ids, position_ids)
+        whole = None if output_all_encoded_layers else self._layers_f32(h)
+        if whole is not None:
+            return self._finish([whole], attention_mask, False)
         return self._finish(self.encoder(h, attention_mask, output_all_encoded_layers), attention_mask, output_all_encoded_layers)
 
     def _finish(self, outs, attention_mask, output_all_encoded_layers):

@@ -40,7 +40,7 @@ class BertGatedLinearUnitMLP(nn.Module):
         self.dropout = nn.Dropout(config.hidden_dropout_prob)
         self.layernorm = nn.LayerNorm(config.hidden_size, eps=config.layer_norm_eps)
 
-    def fill_args(self, plan, a, dev):
+    def fill_args(self, plan, a, dev, f32=False):
         """Writes the pointers of this module's weights into `a` (a _lib.MlpArgs or _lib.EncoderLayer) of `plan`; False where
         the native call, which knows one block count and whole blocks only, does not compute what the weights say.  It sees
         pointers and no tensors, so what they point to is checked here against the config and the device it runs on."""
@@ -50,6 +50,10 @@ class BertGatedLinearUnitMLP(nn.Module):
         expect(dev, (self.gated_layers.weight, (nb, 2 * inter // nb, D // nb)), (self.wo.weight, (nb, D // nb, inter // nb)),
                (self.wo.bias, (D,)), (self.layernorm.weight, (D,)), (self.layernorm.bias, (D,)))
         for name, lin in (("wg", self.gated_layers), ("wo", self.wo)):
+            if f32:
+                setattr(a, name, plan.f32(lin.weight))
+                setattr(a, name + "_split", plan.split(lin._splitter(), lin.weight))
+                continue
             w = lin._weight_as(torch.bfloat16)
             setattr(a, name, plan.registered(w, lin.weight) if lin.weight.dtype == torch.bfloat16 else plan.cached(w))
         if self.wo.bias is not None:
@@ -57,13 +61,14 @@ class BertGatedLinearUnitMLP(nn.Module):
         a.ln_w, a.ln_b, a.eps = plan.f32(self.layernorm.weight), plan.f32(self.layernorm.bias), float(self.layernorm.eps)
         return True
 
-    def _plan(self, dev):
+    def _plan(self, dev, f32=False):
         def make():
             a = _lib.MlpArgs()
+            a.f32 = f32
             a.d_model, a.inter, a.nblocks = self.config.hidden_size, self.config.intermediate_size, self.config.monarch_mlp_nblocks
             plan = Plan(a)
-            return plan if self.fill_args(plan, a, dev) else None
-        return plans_of(self).get(self, dev.index, make)
+            return plan if self.fill_args(plan, a, dev, f32) else None
+        return plans_of(self).get(self, (dev.index, f32), make)
 
     def _forward_bf16(self, x, x2, plan, copies_only):
         """The three launches as one call; outputs as in forward()."""
@@ -90,6 +95,22 @@ class BertGatedLinearUnitMLP(nn.Module):
         ops._launch("m2_mlp_fwd", aug, _lib.lib().m2_mlp_fwd, C.byref(a), launches=3)
         return attach(y, bf16=aug, tm=tm, src_dtype=torch.float32)
 
+    def _forward_f32(self, x, x2, plan):
+        """The three launches on float32 activations as one call."""
+        D, inter = self.config.hidden_size, self.config.intermediate_size
+        if x2.shape[-1] != D:
+            raise AssertionError(f"input has {x2.shape[-1]} features, the MLP {D}")
+        x2 = x2.contiguous()
+        m = x2.shape[0]
+        work = torch.empty((m, inter + D), dtype=torch.float32, device=x2.device)
+        y = torch.empty(x.shape, dtype=torch.float32, device=x2.device)
+        a = _lib.MlpArgs.from_buffer_copy(plan.args)
+        a.m = m
+        a.x, a.h, a.out = x2.data_ptr(), work.data_ptr(), y.data_ptr()
+        a.o = a.h + 4 * m * inter
+        ops._launch("m2_mlp_fwd", y, _lib.lib().m2_mlp_fwd, C.byref(a), launches=3)
+        return y
+
     @forward_only
     def forward(self, hidden_states: torch.Tensor, copies_only: bool = False) -> torch.Tensor:
         """copies_only (used by M2BertEncoder between layers): when the next mixer of this shape
@@ -108,9 +129,13 @@ class BertGatedLinearUnitMLP(nn.Module):
             plan = self._plan(x.device)
             if plan is not None:
                 return self._forward_bf16(x, x2, plan, copies_only)
-        h = ops.blockdiag_glu_fwd(x2, self.gated_layers._weight_as(dt), cfg.intermediate_size)
+        if dt == torch.float32 and x.is_cuda and x2.shape[0] and not ops.observed():
+            plan = self._plan(x.device, f32=True)
+            if plan is not None:
+                return self._forward_f32(x, x2, plan)
+        h = ops.blockdiag_glu_fwd(x2, self.gated_layers._weight_as(dt), cfg.intermediate_size, w_split=self.gated_layers._split(dt))
         o = ops.blockdiag_fwd(h, self.wo._weight_as(dt), self.wo.bias, cfg.intermediate_size,
-                              cfg.hidden_size)
+                              cfg.hidden_size, w_split=self.wo._split(dt))
         # under autocast LayerNorm runs in float32 and returns float32
         out_dtype = torch.float32 if dt == torch.bfloat16 else dt
         aug = None

@@ -230,13 +230,14 @@ def longconv_fwd(xin, u, short_w, short_b, specs, biases, *, kind, bf16_rounding
     return out
 
 
-def linear_fwd(x, w, bias, out=None, *, force_simt=False):
+def linear_fwd(x, w, bias, out=None, *, force_simt=False, w_split=None):
     """nn.Linear on strided activations: y[b, t, n] = sum_k x[b, t, k] w[n, k] + bias[n].
 
     x (B, L, K) and out (B, L, N) are torch VIEWS with any strides that keep either the feature axis or the
     time axis contiguous (a permuted (B, K, L) or channel-major (K, B, L) buffer is passed as its (B, L, K)
     view); w (N, K) contiguous, dtype of x; bias float32-convertible (N) or None.  Returns `out` (allocated
-    row-major when not given)."""
+    row-major when not given).  w_split: split_weights(w), for float32
+    products on the tensor cores."""
     _need_cuda(x, w)
     B, L, K = x.shape
     N = w.shape[0]
@@ -252,11 +253,24 @@ def linear_fwd(x, w, bias, out=None, *, force_simt=False):
     a.bias = b.data_ptr() if b is not None else None
     a.out, (a.out_sb, a.out_st, a.out_sc) = out.data_ptr(), out.stride()
     a.force_simt = int(bool(force_simt))
+    a.w_split = w_split.data_ptr() if w_split is not None else None
     _launch("m2_linear_fwd", x, _lib.lib().m2_linear_fwd, C.byref(a))
     return out
 
 
-def blockdiag_fwd(x2d, w, bias, in_features, out_features, variant=0):
+def split_weights(w):
+    """float32 weights (..., p) as the tensor cores take them in float32 layers: the w_split of linear_fwd, blockdiag_fwd and
+    blockdiag_glu_fwd."""
+    _need_cuda(w)
+    w = _f32c(w)
+    p = w.shape[-1]
+    rows = w.numel() // p
+    out = torch.empty(_lib.lib().m2_split_weights_bytes(rows, p), dtype=torch.uint8, device=w.device)
+    _launch("m2_split_weights", w, _lib.lib().m2_split_weights, w.data_ptr(), rows, p, out.data_ptr())
+    return out
+
+
+def blockdiag_fwd(x2d, w, bias, in_features, out_features, variant=0, w_split=None):
     """x2d (m, in_features) @ blockdiag(w)^T (+ bias) -> (m, out_features), dtype of x2d.  variant=2 asks for
     the CTA-pair kernel (bit-identical results; for cross-checks)."""
     _need_cuda(x2d, w)
@@ -272,12 +286,13 @@ def blockdiag_fwd(x2d, w, bias, in_features, out_features, variant=0):
     a.x, a.ldx, a.w = x2d.data_ptr(), x2d.stride(0) if m > 1 else max(x2d.stride(0), in_features), w.data_ptr()
     a.bias = b.data_ptr() if b is not None else None
     a.out, a.ldo, a.variant = out.data_ptr(), out.stride(0), int(variant)
+    a.w_split = w_split.data_ptr() if w_split is not None else None
     assert w.dtype == x2d.dtype and w.is_contiguous()
     _launch("m2_blockdiag_fwd", x2d, _lib.lib().m2_blockdiag_fwd, C.byref(a))
     return out
 
 
-def blockdiag_glu_fwd(x2d, wg, inter, variant=0):
+def blockdiag_glu_fwd(x2d, wg, inter, variant=0, w_split=None):
     """h = gelu(G[:, :inter]) * G[:, inter:], G = x2d @ blockdiag(wg)^T, without writing G.  variant=1 forces
     the general streaming kernel, variant=3 the CTA-pair kernel (bit-identical results; for cross-checks)."""
     _need_cuda(x2d, wg)
@@ -291,6 +306,7 @@ def blockdiag_glu_fwd(x2d, wg, inter, variant=0):
     a.m, a.d_model, a.inter, a.nblocks, a.dtype = m, d_model, int(inter), nb, _dt(x2d)
     a.x, a.ldx, a.wg = x2d.data_ptr(), max(x2d.stride(0), d_model), wg.data_ptr()
     a.h, a.ldh, a.variant = h.data_ptr(), h.stride(0), int(variant)
+    a.wg_split = w_split.data_ptr() if w_split is not None else None
     _launch("m2_blockdiag_glu_fwd", x2d, _lib.lib().m2_blockdiag_glu_fwd, C.byref(a))
     return h
 

@@ -10,7 +10,7 @@ import torch
 import torch.nn as nn
 
 from . import _lib, ops
-from ._plan import Plan, expect, plans_of
+from ._plan import Plan, SplitWeight, expect, plans_of
 from ._tags import copies_of, forward_only, src_dtype_of
 from .hyena_filter import HyenaFilter, _autocast_bf16
 
@@ -98,10 +98,15 @@ class MonarchMixerSequenceMixing(nn.Module):
             self._w_in, self._w_out = _Bf16Linear(), _Bf16Linear()
         return self._w_in.get(self.in_linear), self._w_out.get(self.out_linear)
 
+    def _splitters(self):
+        if not hasattr(self, "_s_in"):
+            self._s_in, self._s_out = SplitWeight(), SplitWeight()
+        return self._s_in, self._s_out
+
     def filters(self):
         return [self.filter_fn, self.filter_fn2] if self.residual_long_conv else [self.filter_fn]
 
-    def fill_args(self, plan, a, L, kind, dev):
+    def fill_args(self, plan, a, L, kind, dev, f32=False):
         """Writes the pointers of this module's weights and filter tables into `a` (a _lib.MixerArgs or _lib.EncoderLayer)
         of `plan`.  The native call sees pointers only, so what they point to is checked here against in_linear's width and
         the device it runs on."""
@@ -109,25 +114,33 @@ class MonarchMixerSequenceMixing(nn.Module):
         expect(dev, (self.in_linear.weight, (3 * D, D)), (self.in_linear.bias, (3 * D,)), (self.out_linear.weight, (D, D)),
                (self.out_linear.bias, (D,)), (self.short_filter.weight, (3 * D, 1, 3)), (self.short_filter.bias, (3 * D,)),
                *((f.bias, (D,)) for f in self.filters()), *((f.implicit_filter[6].weight, (D, None)) for f in self.filters()))
-        a.w_in, a.w_out = (plan.cached(w) for w in self._weights())
+        if f32:
+            for lin in (self.in_linear, self.out_linear):
+                if lin.weight.dtype != torch.float32 or not lin.weight.is_contiguous():
+                    raise AssertionError("float32 inputs need contiguous float32 weights")
+            a.w_in, a.w_out = plan.f32(self.in_linear.weight), plan.f32(self.out_linear.weight)
+            a.w_in_split, a.w_out_split = (plan.split(s, lin.weight) for s, lin in zip(self._splitters(), (self.in_linear, self.out_linear)))
+        else:
+            a.w_in, a.w_out = (plan.cached(w) for w in self._weights())
         a.short_w, a.short_b = plan.f32(self.short_filter.weight), plan.f32(self.short_filter.bias)
         if self.in_linear.bias is not None:
             a.b_in = plan.f32(self.in_linear.bias)
         if self.out_linear.bias is not None:
             a.b_out = plan.f32(self.out_linear.bias)
         for i, f in enumerate(self.filters()):
-            a.spec[i] = plan.cached(f.spectrum(L, True, kind))
+            a.spec[i] = plan.cached(f.spectrum(L, not f32, kind))
             if kind in (0, 2):                       # kinds 3 and 4 have it inside their tables
                 a.bias[i] = plan.f32(f.bias) if f.use_bias else plan.passing(ops._f32c(f.conv_bias()))
 
-    def _make_plan(self, B, L, kind, dev):
+    def _make_plan(self, B, L, kind, dev, f32=False):
         a = _lib.MixerArgs()
-        Lp = _round_up(L, 8)
+        Lp = L if f32 else _round_up(L, 8)
+        a.f32 = f32
         a.batch, a.seq_len, a.pitch, a.out_pitch, a.d_model = B, L, Lp, L, self.in_linear.weight.shape[-1]
         a.kind, a.n_filters = kind, 2 if self.residual_long_conv else 1
         a.stride, a.u_stride = _round_up(B * Lp, 16), B * Lp
         plan = Plan(a)
-        self.fill_args(plan, a, L, kind, dev)
+        self.fill_args(plan, a, L, kind, dev, f32)
         return plan
 
     def _forward_bf16(self, u, ures, kind):
@@ -171,6 +184,23 @@ class MonarchMixerSequenceMixing(nn.Module):
         a.yu_bf16 = yu_bf16
         a.xin = work.data_ptr()
         a.conv, a.out = a.xin + 2 * 3 * D * stride, y.data_ptr()
+        ops._launch("m2_mixer_fwd", y, _lib.lib().m2_mixer_fwd, C.byref(a), launches=3)
+        return y
+
+    def _forward_f32(self, u):
+        """The float32 mixer on contiguous token rows as one native call; None where single launches have to do it."""
+        B, L, D = u.shape
+        if D != self.in_linear.weight.shape[-1] or not u.is_contiguous() or ops.observed():
+            return None
+        dev = u.device
+        plan = plans_of(self).get(self, (B, L, "f32", dev.index), lambda: self._make_plan(B, L, 0, dev, f32=True))
+        if plan is None:
+            return None
+        work = torch.empty((B * L, 4 * D), dtype=torch.float32, device=dev)
+        y = torch.empty((B, L, D), dtype=torch.float32, device=dev)
+        a = _lib.MixerArgs.from_buffer_copy(plan.args)
+        a.x, a.out, a.xin = u.data_ptr(), y.data_ptr(), work.data_ptr()
+        a.conv = a.xin + 4 * 3 * D * B * L
         ops._launch("m2_mixer_fwd", y, _lib.lib().m2_mixer_fwd, C.byref(a), launches=3)
         return y
 
@@ -273,6 +303,10 @@ class MonarchMixerSequenceMixing(nn.Module):
             kind = ops.longconv_pick(u.size(0), L, torch.bfloat16, self.d_model)
             if kind and u.size(0):
                 return self._forward_bf16(u, ures, kind), None
+        elif u.size(0):
+            y = self._forward_f32(u)
+            if y is not None:
+                return y, None
         kind = 0                                # float32 convolution on token rows
         if ures is not None and ures.dtype == torch.float16:
             ures = ures.float()
@@ -281,10 +315,12 @@ class MonarchMixerSequenceMixing(nn.Module):
         specs = [f.spectrum(L, bf16, kind) for f in filters]
         if bf16:
             w_in, w_out = self._weights()
+            s_out = None
             xin = ops.linear_fwd(bf16_input(u), w_in, self.in_linear.bias)
         else:
             w_in, w_out = self.in_linear.weight.detach(), self.out_linear.weight.detach()
-            xin = ops.linear_fwd(u, w_in, self.in_linear.bias)
+            s_in, s_out = (s.get(lin.weight) for s, lin in zip(self._splitters(), (self.in_linear, self.out_linear)))
+            xin = ops.linear_fwd(u, w_in, self.in_linear.bias, w_split=s_in)
         y = ops.longconv_fwd(xin, ures, self.short_filter.weight, self.short_filter.bias, specs, biases,
                              kind=kind, bf16_rounding=bf16)
-        return ops.linear_fwd(y, w_out, self.out_linear.bias), None
+        return ops.linear_fwd(y, w_out, self.out_linear.bias, w_split=s_out), None
