@@ -203,9 +203,15 @@ typedef struct {
   int yu_bf16;              /* with an fp16 u (kind 3 always, kinds 2 and 4 optionally): != 0 rounds the residual
                                convolution to bf16 before the final add, as the reference does when the
                                layer input is bf16 (with a float32 / bf16 u this follows from u_dtype) */
+  int rows_padded;          /* kind 0, time-contiguous tensors: != 0 says that rows of xin and u start on 16-byte boundaries and may be
+                               read up to a multiple of 8 steps (what lies there is never used) */
 } m2_longconv_args;
 
 int m2_longconv_fwd(const m2_longconv_args* args, void* stream);
+
+/* Whether kind 0 of m2_longconv_fwd wants bf16 activations of this shape as time-contiguous rows with rows_padded set (and u as
+ * float32 rows of the same kind) rather than as token rows. */
+int m2_longconv_padded(int batch, int seq_len, int d_model);
 
 /* ---------------------------------------------------------------------------------------
  * dst[c, b, t] = fp16(src[b, t, c]) (saturating): the time-contiguous fp16 copy of the raw
@@ -221,6 +227,7 @@ typedef struct {
   const void* src; long long src_sb, src_st, src_sc;
   void* dst;       long long dst_sb, dst_sc;
   void* rows_bf16; long long rows_sb, rows_st;  /* optional: the same values as bf16 rows, (b, t, c) at b*rows_sb + t*rows_st + c */
+  int dst_f32;                                  /* != 0: dst is float32 */
 } m2_time_major_args;
 
 int m2_time_major_f16(const m2_time_major_args* args, void* stream);
@@ -305,6 +312,7 @@ typedef struct {
                           its bias (a multiple of 8, at most 256) */
   int valid_len;       /* 0, or the steps of each seq_len-row sequence that are not padding: `out` then has
                           batch * valid_len rows, packed (a, b and the copies keep seq_len rows per sequence) */
+  int tm_f32;          /* != 0: out_tm_f16 is float32 (on a 32-byte boundary) */
 } m2_add_layernorm_args;
 
 int m2_add_layernorm_fwd(const m2_add_layernorm_args* args, void* stream);
@@ -333,6 +341,7 @@ typedef struct {
   void* out_tm_f16; long long tm_sb, tm_sc; int seq_len;
   long long vocab_rows, type_rows, pos_rows;
   int valid_len;      /* as in m2_add_layernorm_args; input_ids, token_type_ids and position_ids are packed too */
+  int tm_f32;
 } m2_embed_layernorm_args;
 
 int m2_embed_layernorm_fwd(const m2_embed_layernorm_args* args, void* stream);
@@ -345,10 +354,11 @@ int m2_embed_layernorm_fwd(const m2_embed_layernorm_args* args, void* stream);
  *   Activations are token rows, `pitch` (a multiple of 8, >= seq_len) rows per sequence; what the rows at and beyond
  *   seq_len hold is never used.
  *   x    : bf16 (batch * pitch, d_model), packed rows.
- *   u    : fp16 (d_model, batch, pitch), channels u_stride elements apart (a multiple of 8); n_filters == 2 only.
+ *   u    : fp16 (kind 0: float32) (d_model, batch, pitch), channels u_stride elements apart (a multiple of 8); n_filters == 2 only.
  *   xin, conv : workspace, bf16 (3 d_model, stride) and (d_model, stride), stride a multiple of 16 >= batch * pitch.
  *   out  : bf16, packed rows, out_pitch = pitch or seq_len of them per sequence.
- *   kind : 2, 3 or 4, from m2_longconv_pick(); spec and bias as m2_longconv_fwd takes them for that kind.
+ *   kind : from m2_longconv_pick(), 0 only where m2_longconv_padded() says so; spec and bias as m2_longconv_fwd takes them for
+ *          that kind.
  *   f32  : != 0 without autocast: x, w_in, w_out, xin, conv and out are float32 on packed token rows (pitch, out_pitch =
  *          seq_len), x is the residual input too (u is not read), kind is 0, w_in_split and w_out_split as in m2_linear_args.
  * ------------------------------------------------------------------------------------- */
@@ -380,6 +390,7 @@ typedef struct {
   float* out; void* out_bf16; void* out_tm_f16; long long tm_stride;
   int seq_len, valid_len;
   int f32; const void* wg_split; const void* wo_split;
+  int tm_f32;          /* as in m2_add_layernorm_args */
 } m2_mlp_args;
 
 int m2_mlp_fwd(const m2_mlp_args* args, void* stream);
@@ -389,7 +400,8 @@ int m2_mlp_fwd(const m2_mlp_args* args, void* stream);
  *   embed : tables, ids, LayerNorm of the embeddings as m2_embed_layernorm_fwd takes them (ids packed, batch * seq_len);
  *           its outputs and sizes are filled in here.
  *   kind  : 0, 2, 3 or 4, from m2_longconv_pick(); spec and bias of each layer as m2_longconv_fwd takes them for that kind.
- *   workspace : m2_encoder_workspace() bytes on a 256-byte boundary, pitch = seq_len rounded up to a multiple of 8.
+ *   workspace : m2_encoder_workspace_kind() bytes on a 256-byte boundary (m2_encoder_workspace() with pitch = seq_len rounded up
+ *           to a multiple of 8 is enough for kinds 2, 3 and 4).
  *   f32   : != 0 without autocast: the layers alone (6 n_layers launches), from the embeddings' float32 output x; kind 0, float32
  *           weights, m2_encoder_workspace_f32() bytes. */
 typedef struct {
@@ -409,6 +421,7 @@ typedef struct {
   int f32; const float* x;
 } m2_encoder_args;
 
+long long m2_encoder_workspace_kind(int kind, int batch, int seq_len, int d_model, int inter);
 long long m2_encoder_workspace(int batch, int pitch, int d_model, int inter);
 long long m2_encoder_workspace_f32(int batch, int seq_len, int d_model, int inter);
 int m2_encoder_fwd(const m2_encoder_args* args, void* stream);

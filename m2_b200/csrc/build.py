@@ -11,7 +11,7 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 OUT = os.path.join(os.path.dirname(HERE), "libm2b200.so")
 SOURCES = ["m2_b200.cu"]   # single translation unit that includes the other .cu parts
-PARTS = ["abi.cu", "filter.cu", "longconv_simt.cu", "longconv_f32.cu", "longconv_tc.cu", "longconv_tcl.cu", "longconv_tz.cu", "longconv_direct.cu", "longconv_bt.cu", "longconv.cu",
+PARTS = ["abi.cu", "filter.cu", "longconv_simt.cu", "longconv_f32.cu", "longconv_tc.cu", "longconv_tcl.cu", "longconv_tz.cu", "longconv_direct.cu", "longconv_bt.cu", "longconv_bts.cu", "longconv.cu",
          "gemm_f32.cu", "gemm_split.cu", "gemm_tc.cu", "linear_tc.cu", "glu_pair.cu", "gemm_simt.cu", "forward.cu", "selftest.cu", "common.cuh", "tc_common.cuh", "m2_b200.cu",
          os.path.join("..", "..", "include", "m2_b200.h")]
 

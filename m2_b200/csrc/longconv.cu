@@ -22,6 +22,12 @@ bool longconv_bt_preferred(int batch, int seq_len, int d_model);
 size_t spectrum_kind4_floats(int D, int L);
 int spectrum_kind4_launch(int D, int L, const float* k, const float* bias, float* spec, cudaStream_t st);
 int longconv_bt_launch(const m2_longconv_args* a, cudaStream_t st);
+bool longconv_bts_f32_preferred(int batch, int seq_len, int d_model);
+bool longconv_bts_f32_supported(const m2_longconv_args* a);
+size_t taps_f32_offset(int D, int L);
+size_t taps_f32_floats(int D, int L);
+int taps_f32_launch(int D, int L, const float* k, float* taps, cudaStream_t st);
+int longconv_bts_f32_launch(const m2_longconv_args* a, cudaStream_t st);
 int time_major_f16_launch(const m2_time_major_args* a, cudaStream_t st);
 }  // namespace m2
 
@@ -54,14 +60,17 @@ extern "C" int m2_longconv_pick(int batch, int seq_len, m2_dtype act_dtype, int 
   return 2;
 }
 
+extern "C" int m2_longconv_padded(int batch, int seq_len, int d_model) {
+  return batch > 0 && seq_len > 0 && d_model > 0 && m2::longconv_bts_f32_preferred(batch, seq_len, d_model);
+}
+
 extern "C" size_t m2_filter_spectrum_floats(int kind, int d_model, int seq_len) {
   if (d_model <= 0 || seq_len <= 0) return 0;
   if (kind == 3) return m2::spectrum_kind3_floats(d_model, seq_len);
   if (kind == 4) return m2::spectrum_kind4_floats(d_model, seq_len);
   if (kind == 1) return m2::spectrum_kind1_floats(d_model, seq_len);
   if (kind == 2) return m2::spectrum_kind2_floats(d_model, seq_len);
-  const size_t M = (size_t)m2_filter_row_len(seq_len) / 2;
-  return M + 4 * M * (size_t)d_model;
+  return m2::taps_f32_offset(d_model, seq_len) + m2::taps_f32_floats(d_model, seq_len);
 }
 
 extern "C" int m2_filter_spectrum_bias(int kind, int d_model, int seq_len, const float* k, const float* bias,
@@ -99,7 +108,10 @@ extern "C" int m2_filter_spectrum(int kind, int d_model, int seq_len, const floa
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (kind == 3) return m2::spectrum_kind3_launch(d_model, seq_len, k, nullptr, spec_out, st);
   if (kind == 4) return m2::spectrum_kind4_launch(d_model, seq_len, k, nullptr, spec_out, st);
-  if (kind == 0) return m2::spectrum_kind0_launch(d_model, seq_len, k, spec_out, st);
+  if (kind == 0) {
+    const int rc = m2::spectrum_kind0_launch(d_model, seq_len, k, spec_out, st);
+    return rc ? rc : m2::taps_f32_launch(d_model, seq_len, k, spec_out + m2::taps_f32_offset(d_model, seq_len), st);
+  }
   if (kind == 1) return m2::spectrum_kind1_launch(d_model, seq_len, k, spec_out, st);
   if (kind == 2) return m2::spectrum_kind2_launch(d_model, seq_len, k, spec_out, st);
   return m2_set_error(M2_ERR_ARG, "m2_filter_spectrum: unknown kind %d", kind);
@@ -126,6 +138,7 @@ extern "C" int m2_longconv_fwd(const m2_longconv_args* a, void* stream) {
   M2_REQUIRE(m2_aligned(a->spec[0], 16) && (a->n_filters == 1 || m2_aligned(a->spec[1], 16)), M2_ERR_ALIGN,
              "m2_longconv_fwd: spectrum tables must be 16-byte aligned");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (a->kind == 0 && m2::longconv_bts_f32_supported(a)) return m2::longconv_bts_f32_launch(a, st);
   if (a->kind == 0 || a->plain) return m2::longconv_simt_launch(a, st);
   if (a->kind == 1) return m2::longconv_tc_launch(a, st);
   if (a->kind == 2) return m2::longconv_tcl_launch(a, st);

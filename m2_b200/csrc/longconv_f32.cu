@@ -241,13 +241,22 @@ bool longconv_f32_supported(const m2_longconv_args* a) {
          (a->n_filters == 1 || (a->u_sc == 1 && (a->u_dtype == M2_F32 || (bf16 && a->u_dtype == M2_BF16))));
 }
 
-int longconv_f32_launch(const m2_longconv_args* a, ConvParams p, cudaStream_t st) {
-  // channels per CTA: 32 make a warp's access one 128-byte line (64 bytes of bf16), fewer leave room for more CTAs; 64 KB of
-  // rows let three CTAs share an SM, and two CTAs per SM should exist
-  const size_t row = (size_t)(p.M + 1) * sizeof(float2);
+// channels per CTA: 32 make a warp's access one 128-byte line (64 bytes of bf16), fewer leave room for more CTAs; 64 KB of
+// rows let three CTAs share an SM, and two CTAs per SM should exist
+static int longconv_f32_channels(int B, int M, int D) {
+  const size_t row = (size_t)(M + 1) * sizeof(float2);
   int ct = 32;
-  while (ct > 8 && (ct * row > 66 * 1024 || (long long)((p.D + ct - 1) / ct) * p.B < 2 * m2_sm_count())) ct >>= 1;
-  p.CT = ct;
+  while (ct > 8 && (ct * row > 66 * 1024 || (long long)((D + ct - 1) / ct) * B < 2 * m2_sm_count())) ct >>= 1;
+  return ct;
+}
+long long longconv_f32_ctas(int B, int L, int D) {
+  const int ct = longconv_f32_channels(B, m2_filter_row_len(L) / 2, D);
+  return (long long)((D + ct - 1) / ct) * B;
+}
+
+int longconv_f32_launch(const m2_longconv_args* a, ConvParams p, cudaStream_t st) {
+  const size_t row = (size_t)(p.M + 1) * sizeof(float2);
+  const int ct = p.CT = longconv_f32_channels(p.B, p.M, p.D);
   const size_t smem = ct * row + (size_t)(p.M / 2) * sizeof(float2);
   const int threads = smem > 100 * 1024 ? 512 : 256;                         // the one CTA of an SM brings 16 warps
   if (a->act_dtype == M2_F32) return f32c::launch_stages<float, float, false>(p, threads, smem, st);

@@ -260,7 +260,7 @@ class M2BertModel(nn.Module):
         args = (_lib.EncoderLayer * len(layers))()
         e = _lib.EncoderArgs()
         work = (_lib.lib().m2_encoder_workspace_f32(B, L, D, cfg.intermediate_size) if f32 else
-                _lib.lib().m2_encoder_workspace(B, (L + 7) // 8 * 8, D, cfg.intermediate_size))
+                _lib.lib().m2_encoder_workspace_kind(kind, B, L, D, cfg.intermediate_size))
         plan = Plan(e, layers=args, work=work, out=(B, L, D), called=called, dropping=[m for m in called if hasattr(m, "dropout")])
         for a, y in zip(args, layers):
             y.attention.fill_args(plan, a, L, kind, dev, f32)
