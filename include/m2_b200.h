@@ -26,7 +26,7 @@
 extern "C" {
 #endif
 
-#define M2_B200_ABI_VERSION 5
+#define M2_B200_ABI_VERSION 6
 
 typedef enum { M2_F32 = 0, M2_BF16 = 1, M2_F16 = 2 /* only where an entry point says so */ } m2_dtype;
 
@@ -165,6 +165,8 @@ int m2_linear_fwd(const m2_linear_args* args, void* stream);
  * operand of float32 layers on the tensor cores.  `out` has m2_split_weights_bytes(rows, p) bytes on a 16-byte boundary. */
 size_t m2_split_weights_bytes(long long rows, int p);
 int m2_split_weights(const float* w, long long rows, int p, void* out, void* stream);
+/* Whether the float32 GEMMs take split weights of p columns at all (where not, w_split changes nothing). */
+int m2_split_weights_used(int p);
 
 /* ---------------------------------------------------------------------------------------
  * Fused gated long convolution: everything between in_linear and out_linear.
@@ -360,7 +362,8 @@ int m2_embed_layernorm_fwd(const m2_embed_layernorm_args* args, void* stream);
  *   kind : from m2_longconv_pick(), 0 only where m2_longconv_padded() says so; spec and bias as m2_longconv_fwd takes them for
  *          that kind.
  *   f32  : != 0 without autocast: x, w_in, w_out, xin, conv and out are float32 on packed token rows (pitch, out_pitch =
- *          seq_len), x is the residual input too (u is not read), kind is 0, w_in_split and w_out_split as in m2_linear_args.
+ *          seq_len), x is the residual input too (u is not read), kind is 0.  split: workspace of m2_mixer_split_bytes() bytes on
+ *          a 16-byte boundary, to which every call writes its weights as m2_split_weights does, or NULL (float32 chains).
  * ------------------------------------------------------------------------------------- */
 typedef struct {
   int batch, seq_len, pitch, out_pitch, d_model, kind, n_filters, yu_bf16;
@@ -372,15 +375,16 @@ typedef struct {
   const void* w_out; const float* b_out;     /* bf16 (d_model, d_model), float32 (d_model) */
   void* xin; void* conv; long long stride;
   void* out;
-  int f32; const void* w_in_split; const void* w_out_split;
+  int f32; void* split;
 } m2_mixer_args;
 
+long long m2_mixer_split_bytes(int d_model);
 int m2_mixer_fwd(const m2_mixer_args* args, void* stream);
 
 /* BertGatedLinearUnitMLP.forward under bf16 autocast (bert/src/bert_layers.py:482-508): GLU GEMM, wo GEMM, add + LayerNorm.
  * x bf16 (m, d_model); h, o workspace bf16 (m, inter), (m, d_model); outputs as in m2_add_layernorm_fwd: `out` float32 or
  * NULL, out_bf16 (m, d_model) and out_tm_f16 (d_model, m / seq_len, seq_len) with channels tm_stride apart, or NULL.
- * f32 != 0: x, weights, h, o and out float32, no other outputs; wg_split and wo_split as in m2_linear_args. */
+ * f32 != 0: x, weights, h, o and out float32, no other outputs; split as in m2_mixer_args, m2_mlp_split_bytes() bytes. */
 typedef struct {
   int m, d_model, inter, nblocks;
   const void* x;
@@ -389,10 +393,11 @@ typedef struct {
   void* h; void* o;
   float* out; void* out_bf16; void* out_tm_f16; long long tm_stride;
   int seq_len, valid_len;
-  int f32; const void* wg_split; const void* wo_split;
+  int f32; void* split;
   int tm_f32;          /* as in m2_add_layernorm_args */
 } m2_mlp_args;
 
+long long m2_mlp_split_bytes(int d_model, int inter, int nblocks);
 int m2_mlp_fwd(const m2_mlp_args* args, void* stream);
 
 /* The encoder (bert/src/bert_layers.py:186-252 embeddings, :552-813 layers) from token ids to the last layer's float32
@@ -402,14 +407,13 @@ int m2_mlp_fwd(const m2_mlp_args* args, void* stream);
  *   kind  : 0, 2, 3 or 4, from m2_longconv_pick(); spec and bias of each layer as m2_longconv_fwd takes them for that kind.
  *   workspace : m2_encoder_workspace_kind() bytes on a 256-byte boundary (m2_encoder_workspace() with pitch = seq_len rounded up
  *           to a multiple of 8 is enough for kinds 2, 3 and 4).
- *   f32   : != 0 without autocast: the layers alone (6 n_layers launches), from the embeddings' float32 output x; kind 0, float32
+ *   f32   : != 0 without autocast: the layers alone (7 n_layers launches at most), from the embeddings' float32 output x; kind 0, float32
  *           weights, m2_encoder_workspace_f32() bytes. */
 typedef struct {
   const void* w_in; const float* b_in; const float* short_w; const float* short_b;
   const float* spec[2]; const float* bias[2];
   const void* w_out; const float* b_out;
   const void* wg; const void* wo; const float* wo_bias; const float* ln_w; const float* ln_b; float eps;
-  const void* w_in_split; const void* w_out_split; const void* wg_split; const void* wo_split;   /* f32 only */
 } m2_encoder_layer;
 
 typedef struct {
@@ -423,7 +427,7 @@ typedef struct {
 
 long long m2_encoder_workspace_kind(int kind, int batch, int seq_len, int d_model, int inter);
 long long m2_encoder_workspace(int batch, int pitch, int d_model, int inter);
-long long m2_encoder_workspace_f32(int batch, int seq_len, int d_model, int inter);
+long long m2_encoder_workspace_f32(int batch, int seq_len, int d_model, int inter, int nblocks);
 int m2_encoder_fwd(const m2_encoder_args* args, void* stream);
 
 #ifdef __cplusplus

@@ -10,7 +10,7 @@ import os
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libm2b200.so")
-ABI_VERSION = 5
+ABI_VERSION = 6
 
 M2_F32, M2_BF16, M2_F16 = 0, 1, 2
 
@@ -116,7 +116,7 @@ class MixerArgs(C.Structure):
         ("w_in", C.c_void_p), ("b_in", C.c_void_p), ("short_w", C.c_void_p), ("short_b", C.c_void_p),
         ("spec", C.c_void_p * 2), ("bias", C.c_void_p * 2), ("w_out", C.c_void_p), ("b_out", C.c_void_p),
         ("xin", C.c_void_p), ("conv", C.c_void_p), ("stride", C.c_longlong), ("out", C.c_void_p),
-        ("f32", C.c_int), ("w_in_split", C.c_void_p), ("w_out_split", C.c_void_p),
+        ("f32", C.c_int), ("split", C.c_void_p),
     ]
 
 
@@ -128,7 +128,7 @@ class MlpArgs(C.Structure):
         ("h", C.c_void_p), ("o", C.c_void_p),
         ("out", C.c_void_p), ("out_bf16", C.c_void_p), ("out_tm_f16", C.c_void_p), ("tm_stride", C.c_longlong),
         ("seq_len", C.c_int), ("valid_len", C.c_int),
-        ("f32", C.c_int), ("wg_split", C.c_void_p), ("wo_split", C.c_void_p), ("tm_f32", C.c_int),
+        ("f32", C.c_int), ("split", C.c_void_p), ("tm_f32", C.c_int),
     ]
 
 
@@ -138,7 +138,6 @@ class EncoderLayer(C.Structure):
         ("spec", C.c_void_p * 2), ("bias", C.c_void_p * 2), ("w_out", C.c_void_p), ("b_out", C.c_void_p),
         ("wg", C.c_void_p), ("wo", C.c_void_p), ("wo_bias", C.c_void_p),
         ("ln_w", C.c_void_p), ("ln_b", C.c_void_p), ("eps", C.c_float),
-        ("w_in_split", C.c_void_p), ("w_out_split", C.c_void_p), ("wg_split", C.c_void_p), ("wo_split", C.c_void_p),
     ]
 
 
@@ -167,6 +166,7 @@ SYMBOLS = {
     "m2_filter_spectrum_bias": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
     "m2_linear_fwd": (C.c_int, [C.POINTER(LinearArgs), C.c_void_p]),
     "m2_split_weights_bytes": (C.c_size_t, [C.c_longlong, C.c_int]),
+    "m2_split_weights_used": (C.c_int, [C.c_int]),
     "m2_split_weights": (C.c_int, [C.c_void_p, C.c_longlong, C.c_int, C.c_void_p, C.c_void_p]),
     "m2_longconv_fwd": (C.c_int, [C.POINTER(LongconvArgs), C.c_void_p]),
     "m2_time_major_f16": (C.c_int, [C.POINTER(TimeMajorArgs), C.c_void_p]),
@@ -179,7 +179,9 @@ SYMBOLS = {
     "m2_encoder_workspace": (C.c_longlong, [C.c_int, C.c_int, C.c_int, C.c_int]),
     "m2_encoder_workspace_kind": (C.c_longlong, [C.c_int, C.c_int, C.c_int, C.c_int, C.c_int]),
     "m2_longconv_padded": (C.c_int, [C.c_int, C.c_int, C.c_int]),
-    "m2_encoder_workspace_f32": (C.c_longlong, [C.c_int, C.c_int, C.c_int, C.c_int]),
+    "m2_encoder_workspace_f32": (C.c_longlong, [C.c_int, C.c_int, C.c_int, C.c_int, C.c_int]),
+    "m2_mixer_split_bytes": (C.c_longlong, [C.c_int]),
+    "m2_mlp_split_bytes": (C.c_longlong, [C.c_int, C.c_int, C.c_int]),
     "m2_encoder_fwd": (C.c_int, [C.POINTER(EncoderArgs), C.c_void_p]),
 }
 

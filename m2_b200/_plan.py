@@ -77,13 +77,6 @@ class Plan:
         """Pointer of a parameter as contiguous float32."""
         return self.registered(ops._f32c(source), source)
 
-    def split(self, cache, source):
-        """Pointer of the split of a parameter, from the module's SplitWeight; None where there is none."""
-        t = cache.get(source)
-        if t is None:
-            return None
-        return self.cached(t) if cache.entry is not None and cache.entry[3] is t else self.passing(t)
-
     def passing(self, t):
         """Pointer of a tensor made for this call."""
         self.held.append(t)
@@ -92,30 +85,7 @@ class Plan:
 
 
 class SplitWeight:
-    """A float32 weight as pairs of fp16 values (ops.split_weights), made again when the parameter is another one or changes."""
-
-    def __init__(self):
-        self.entry = None                    # replaced as a whole: threads that share it read one weight's or the other's
-
-    def get(self, w):
-        """The split of `w`, or None where it could not be told whether one is still true (tensors made under inference_mode) or
-        there is none (other types)."""
-        if w.dtype != torch.float32 or w.is_inference():
-            return None
-        entry = self.entry
-        if entry is not None and entry[0]() is w and entry[1:3] == (w._version, w.data_ptr()):
-            return entry[3]
-        t = ops.split_weights(w)
-        if not torch.cuda.is_current_stream_capturing():       # what a capture makes belongs to its graph
-            torch.cuda.current_stream(w.device).synchronize()  # once per weight: any stream may read it from now on
-            self.entry = (weakref.ref(w), w._version, w.data_ptr(), t)
-        return t
-
-    def __deepcopy__(self, memo):
-        return SplitWeight()
-
-    def __reduce__(self):
-        return SplitWeight, ()
+    """Modules saved with pickle may hold one from when they kept split weights; nothing reads it."""
 
 
 REFUSED = object()       # kept in the place of a plan that make() did not give

@@ -13,7 +13,6 @@ import torch.nn as nn
 from torch.nn import init
 
 from . import ops
-from ._plan import SplitWeight
 from ._tags import forward_only
 from .hyena_filter import _autocast_bf16
 
@@ -149,15 +148,6 @@ class BlockdiagLinear(StructuredLinear):
             return w.contiguous()
         return self._w_cache.get(self.weight) if dt == torch.bfloat16 else w.to(dt)
 
-    def _splitter(self):
-        if "_w_split" not in self.__dict__:
-            self._w_split = SplitWeight()
-        return self._w_split
-
-    def _split(self, dt):
-        """The weight as float32 layers take it on the tensor cores, None in other types."""
-        return self._splitter().get(self.weight) if dt == torch.float32 else None
-
     @forward_only
     def forward_matmul(self, x):
         return self._run(x, None)
@@ -171,7 +161,8 @@ class BlockdiagLinear(StructuredLinear):
         x2 = x.reshape(-1, x.shape[-1])
         if x2.dtype != dt:
             x2 = x2.to(dt)
-        out = ops.blockdiag_fwd(x2, self._weight_as(dt), bias, x2.shape[-1], self.out_features, w_split=self._split(dt))
+        w = self._weight_as(dt)
+        out = ops.blockdiag_fwd(x2, w, bias, x2.shape[-1], self.out_features, w_split=ops.split_of(w))
         return out.reshape(*x.shape[:-1], self.out_features)
 
     @forward_only

@@ -76,10 +76,21 @@ __device__ __forceinline__ void split_pair(float y0, float y1, uint32_t& hi, uin
   lo = *reinterpret_cast<const uint32_t*>(&l);
 }
 
-// weight rows: per 64 columns hi, then lo; zeros up to the next multiple of 64.  A warp per row.
+// weight rows: per 64 columns hi, then lo; zeros up to the next multiple of 64.  A warp per row, up to four matrices a launch.
+struct SplitJobs {
+  struct { const float* w; __half* ws; float* winv; int rows, p, steps, first; } job[4];   // first: its first block of eight rows
+  int n;
+};
 __global__ void __launch_bounds__(256)
-split_weights_kernel(const float* __restrict__ w, int rows, int p, int steps, __half* __restrict__ ws, float* __restrict__ winv) {
-  const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+split_weights_kernel(const SplitJobs J) {
+  pdl_wait();
+  int j = 0;
+  while (j + 1 < J.n && (int)blockIdx.x >= J.job[j + 1].first) ++j;
+  const float* __restrict__ w = J.job[j].w;
+  __half* __restrict__ ws = J.job[j].ws;
+  float* __restrict__ winv = J.job[j].winv;
+  const int rows = J.job[j].rows, p = J.job[j].p, steps = J.job[j].steps;
+  const int row = (blockIdx.x - J.job[j].first) * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (row >= rows) return;
   const float* r = w + (size_t)row * p;
   float m = 0.f;
@@ -453,10 +464,12 @@ static int pick_bn(const Params& P, int blocks) {
   return c128 <= c64 && c128 <= c32 ? 128 : (c64 <= c32 ? 64 : 32);
 }
 
-// What the TMA loads need: rows that start on 16-byte boundaries; `ws` as m2_split_weights writes it.  Below 128 products a
-// chain is about as exact (68 columns: 1.3e-7 of the result both) and as fast (36 columns, 100 rows: 10.3 us both).
+// Below 128 products a chain is about as exact (68 columns: 1.3e-7 of the result both) and as fast (36 columns, 100 rows: 10.3 us
+// both).
+static bool columns_ok(int p) { return p >= 2 * BK && p % 4 == 0; }
+// What the TMA loads need: rows that start on 16-byte boundaries; `ws` as m2_split_weights writes it.
 static bool rows_ok(const void* x, long long ld, const void* ws, int p) {
-  return ws && p >= 2 * BK && p % 4 == 0 && ld % 4 == 0 && m2_aligned(x, 16) && m2_aligned(ws, 16);
+  return ws && columns_ok(p) && ld % 4 == 0 && m2_aligned(x, 16) && m2_aligned(ws, 16);
 }
 static size_t split_halves(long long rows, int p) { return (size_t)rows * ((p + BK - 1) / BK) * 2 * BK; }
 static void set_weights(Params& P, const void* w, const void* ws, long long rows) {
@@ -522,6 +535,27 @@ int glu_split_launch(const m2_glu_args* a, cudaStream_t st) {
   return f32s::launch<64, true>(P, a->nblocks, st);
 }
 
+struct WeightRows { const void* w; long long rows; int p; void* out; };
+// One launch for up to four matrices; `elements` as in m2_launch.
+static int split_weights_launch(const WeightRows* rows, int n, long long elements, cudaStream_t st) {
+  using namespace f32s;
+  SplitJobs J = {};
+  long long blocks = 0;
+  for (int i = 0; i < n; ++i) {
+    const WeightRows& r = rows[i];
+    M2_REQUIRE(r.rows > 0 && r.rows < (1LL << 31) - 8 && r.p > 0, M2_ERR_ARG, "m2_split_weights: bad sizes rows=%lld p=%d", r.rows, r.p);
+    M2_REQUIRE(r.w && r.out, M2_ERR_ARG, "m2_split_weights: NULL pointer");
+    M2_REQUIRE(m2_aligned(r.out, 16), M2_ERR_ALIGN, "m2_split_weights: out must be 16-byte aligned");
+    __half* ws = static_cast<__half*>(r.out);
+    J.job[i] = {static_cast<const float*>(r.w), ws, reinterpret_cast<float*>(ws + split_halves(r.rows, r.p)), (int)r.rows, r.p,
+                (r.p + BK - 1) / BK, (int)blocks};
+    blocks += (r.rows + 7) / 8;
+  }
+  M2_REQUIRE(blocks < (1LL << 31), M2_ERR_UNSUPPORTED, "m2_split_weights: too many rows");
+  J.n = n;
+  return m2_launch("split_weights_kernel", elements, split_weights_kernel, (unsigned)blocks, 256, 0, st, J);
+}
+
 }  // namespace m2
 
 extern "C" size_t m2_split_weights_bytes(long long rows, int p) {
@@ -529,14 +563,9 @@ extern "C" size_t m2_split_weights_bytes(long long rows, int p) {
   return m2::f32s::split_halves(rows, p) * 2 + (size_t)rows * 4;
 }
 
+extern "C" int m2_split_weights_used(int p) { return m2::f32s::columns_ok(p); }
+
 extern "C" int m2_split_weights(const float* w, long long rows, int p, void* out, void* stream) {
-  using namespace m2::f32s;
-  M2_REQUIRE(rows > 0 && rows < (1LL << 31) - 8 && p > 0, M2_ERR_ARG, "m2_split_weights: bad sizes rows=%lld p=%d", rows, p);
-  M2_REQUIRE(w && out, M2_ERR_ARG, "m2_split_weights: NULL pointer");
-  M2_REQUIRE(m2_aligned(out, 16), M2_ERR_ALIGN, "m2_split_weights: out must be 16-byte aligned");
-  __half* ws = static_cast<__half*>(out);
-  split_weights_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      w, (int)rows, p, (p + BK - 1) / BK, ws, reinterpret_cast<float*>(ws + split_halves(rows, p)));
-  M2_LAUNCH_CHECK("split_weights_kernel");
-  return M2_OK;
+  const m2::WeightRows r = {w, rows, p, out};
+  return m2::split_weights_launch(&r, 1, rows * p, static_cast<cudaStream_t>(stream));
 }

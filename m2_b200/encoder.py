@@ -259,14 +259,16 @@ class M2BertModel(nn.Module):
         kind = 0 if f32 else ops.longconv_pick(B, L, torch.bfloat16, D)
         args = (_lib.EncoderLayer * len(layers))()
         e = _lib.EncoderArgs()
-        work = (_lib.lib().m2_encoder_workspace_f32(B, L, D, cfg.intermediate_size) if f32 else
+        nb = cfg.monarch_mlp_nblocks
+        work = (_lib.lib().m2_encoder_workspace_f32(B, L, D, cfg.intermediate_size, nb) if f32 else
                 _lib.lib().m2_encoder_workspace_kind(kind, B, L, D, cfg.intermediate_size))
-        plan = Plan(e, layers=args, work=work, out=(B, L, D), called=called, dropping=[m for m in called if hasattr(m, "dropout")])
+        plan = Plan(e, layers=args, work=work, out=(B, L, D), called=called, dropping=[m for m in called if hasattr(m, "dropout")],
+                    per_layer=6 + (f32 and ops.split_used(D, D // nb, cfg.intermediate_size // nb)))
         for a, y in zip(args, layers):
             y.attention.fill_args(plan, a, L, kind, dev, f32)
             if not y.mlp.fill_args(plan, a, dev, f32):
                 return None
-        e.batch, e.seq_len, e.d_model, e.inter, e.nblocks = B, L, D, cfg.intermediate_size, cfg.monarch_mlp_nblocks
+        e.batch, e.seq_len, e.d_model, e.inter, e.nblocks = B, L, D, cfg.intermediate_size, nb
         e.n_layers, e.kind, e.n_filters = len(layers), kind, 2 if layers[0].attention.residual_long_conv else 1
         e.f32 = f32
         e.layers = C.cast(args, C.POINTER(_lib.EncoderLayer))
@@ -323,7 +325,7 @@ class M2BertModel(nn.Module):
         work = torch.empty(plan.work, dtype=torch.uint8, device=h.device)
         a = _lib.EncoderArgs.from_buffer_copy(plan.args)
         a.x, a.workspace, a.out = h.data_ptr(), work.data_ptr(), out.data_ptr()
-        ops._launch("m2_encoder_fwd", out, _lib.lib().m2_encoder_fwd, C.byref(a), launches=6 * a.n_layers)
+        ops._launch("m2_encoder_fwd", out, _lib.lib().m2_encoder_fwd, C.byref(a), launches=plan.per_layer * a.n_layers)
         return out
 
     def forward(self, input_ids, token_type_ids=None, attention_mask=None, position_ids=None,

@@ -52,7 +52,6 @@ class BertGatedLinearUnitMLP(nn.Module):
         for name, lin in (("wg", self.gated_layers), ("wo", self.wo)):
             if f32:
                 setattr(a, name, plan.f32(lin.weight))
-                setattr(a, name + "_split", plan.split(lin._splitter(), lin.weight))
                 continue
             w = lin._weight_as(torch.bfloat16)
             setattr(a, name, plan.registered(w, lin.weight) if lin.weight.dtype == torch.bfloat16 else plan.cached(w))
@@ -66,7 +65,8 @@ class BertGatedLinearUnitMLP(nn.Module):
             a = _lib.MlpArgs()
             a.f32 = f32
             a.d_model, a.inter, a.nblocks = self.config.hidden_size, self.config.intermediate_size, self.config.monarch_mlp_nblocks
-            plan = Plan(a)
+            split = _lib.lib().m2_mlp_split_bytes(a.d_model, a.inter, a.nblocks) if f32 else 0
+            plan = Plan(a, split=split, launches=3 + (f32 and ops.split_used(a.d_model // a.nblocks, a.inter // a.nblocks)))
             return plan if self.fill_args(plan, a, dev, f32) else None
         return plans_of(self).get(self, (dev.index, f32), make)
 
@@ -96,19 +96,20 @@ class BertGatedLinearUnitMLP(nn.Module):
         return attach(y, bf16=aug, tm=tm, src_dtype=torch.float32)
 
     def _forward_f32(self, x, x2, plan):
-        """The three launches on float32 activations as one call."""
+        """The launches on float32 activations (the split of the weights, two GEMMs, LayerNorm) as one call."""
         D, inter = self.config.hidden_size, self.config.intermediate_size
         if x2.shape[-1] != D:
             raise AssertionError(f"input has {x2.shape[-1]} features, the MLP {D}")
         x2 = x2.contiguous()
         m = x2.shape[0]
         work = torch.empty((m, inter + D), dtype=torch.float32, device=x2.device)
+        split = torch.empty(plan.split, dtype=torch.uint8, device=x2.device)
         y = torch.empty(x.shape, dtype=torch.float32, device=x2.device)
         a = _lib.MlpArgs.from_buffer_copy(plan.args)
         a.m = m
         a.x, a.h, a.out = x2.data_ptr(), work.data_ptr(), y.data_ptr()
-        a.o = a.h + 4 * m * inter
-        ops._launch("m2_mlp_fwd", y, _lib.lib().m2_mlp_fwd, C.byref(a), launches=3)
+        a.o, a.split = a.h + 4 * m * inter, split.data_ptr()
+        ops._launch("m2_mlp_fwd", y, _lib.lib().m2_mlp_fwd, C.byref(a), launches=plan.launches)
         return y
 
     @forward_only
@@ -133,9 +134,9 @@ class BertGatedLinearUnitMLP(nn.Module):
             plan = self._plan(x.device, f32=True)
             if plan is not None:
                 return self._forward_f32(x, x2, plan)
-        h = ops.blockdiag_glu_fwd(x2, self.gated_layers._weight_as(dt), cfg.intermediate_size, w_split=self.gated_layers._split(dt))
-        o = ops.blockdiag_fwd(h, self.wo._weight_as(dt), self.wo.bias, cfg.intermediate_size,
-                              cfg.hidden_size, w_split=self.wo._split(dt))
+        wg, wo = self.gated_layers._weight_as(dt), self.wo._weight_as(dt)
+        h = ops.blockdiag_glu_fwd(x2, wg, cfg.intermediate_size, w_split=ops.split_of(wg))
+        o = ops.blockdiag_fwd(h, wo, self.wo.bias, cfg.intermediate_size, cfg.hidden_size, w_split=ops.split_of(wo))
         # under autocast LayerNorm runs in float32 and returns float32
         out_dtype = torch.float32 if dt == torch.bfloat16 else dt
         aug = None

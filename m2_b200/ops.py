@@ -276,6 +276,16 @@ def split_weights(w):
     return out
 
 
+def split_used(*columns) -> bool:
+    """Whether any float32 weight with one of these column counts goes to the tensor cores."""
+    return any(_lib.lib().m2_split_weights_used(int(p)) for p in columns)
+
+
+def split_of(w):
+    """split_weights(w) for this call where the float32 GEMMs read it, else None.  Nothing keeps it: the weight may change."""
+    return split_weights(w) if w.dtype == torch.float32 and w.is_cuda and w.numel() and split_used(w.shape[-1]) else None
+
+
 def blockdiag_fwd(x2d, w, bias, in_features, out_features, variant=0, w_split=None):
     """x2d (m, in_features) @ blockdiag(w)^T (+ bias) -> (m, out_features), dtype of x2d.  variant=2 asks for
     the CTA-pair kernel (bit-identical results; for cross-checks)."""

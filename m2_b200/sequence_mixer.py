@@ -10,7 +10,7 @@ import torch
 import torch.nn as nn
 
 from . import _lib, ops
-from ._plan import Plan, SplitWeight, expect, plans_of
+from ._plan import Plan, expect, plans_of
 from ._tags import copies_of, forward_only, src_dtype_of
 from .hyena_filter import HyenaFilter, _autocast_bf16
 
@@ -98,11 +98,6 @@ class MonarchMixerSequenceMixing(nn.Module):
             self._w_in, self._w_out = _Bf16Linear(), _Bf16Linear()
         return self._w_in.get(self.in_linear), self._w_out.get(self.out_linear)
 
-    def _splitters(self):
-        if not hasattr(self, "_s_in"):
-            self._s_in, self._s_out = SplitWeight(), SplitWeight()
-        return self._s_in, self._s_out
-
     def filters(self):
         return [self.filter_fn, self.filter_fn2] if self.residual_long_conv else [self.filter_fn]
 
@@ -119,7 +114,6 @@ class MonarchMixerSequenceMixing(nn.Module):
                 if lin.weight.dtype != torch.float32 or not lin.weight.is_contiguous():
                     raise AssertionError("float32 inputs need contiguous float32 weights")
             a.w_in, a.w_out = plan.f32(self.in_linear.weight), plan.f32(self.out_linear.weight)
-            a.w_in_split, a.w_out_split = (plan.split(s, lin.weight) for s, lin in zip(self._splitters(), (self.in_linear, self.out_linear)))
         else:
             a.w_in, a.w_out = (plan.cached(w) for w in self._weights())
         a.short_w, a.short_b = plan.f32(self.short_filter.weight), plan.f32(self.short_filter.bias)
@@ -139,7 +133,7 @@ class MonarchMixerSequenceMixing(nn.Module):
         a.batch, a.seq_len, a.pitch, a.out_pitch, a.d_model = B, L, Lp, L, self.in_linear.weight.shape[-1]
         a.kind, a.n_filters = kind, 2 if self.residual_long_conv else 1
         a.stride, a.u_stride = _round_up(B * Lp, 16), B * Lp
-        plan = Plan(a)
+        plan = Plan(a, split=_lib.lib().m2_mixer_split_bytes(a.d_model) if f32 else 0, launches=3 + (f32 and ops.split_used(a.d_model)))
         self.fill_args(plan, a, L, kind, dev, f32)
         return plan
 
@@ -197,11 +191,12 @@ class MonarchMixerSequenceMixing(nn.Module):
         if plan is None:
             return None
         work = torch.empty((B * L, 4 * D), dtype=torch.float32, device=dev)
+        split = torch.empty(plan.split, dtype=torch.uint8, device=dev)
         y = torch.empty((B, L, D), dtype=torch.float32, device=dev)
         a = _lib.MixerArgs.from_buffer_copy(plan.args)
-        a.x, a.out, a.xin = u.data_ptr(), y.data_ptr(), work.data_ptr()
+        a.x, a.out, a.xin, a.split = u.data_ptr(), y.data_ptr(), work.data_ptr(), split.data_ptr()
         a.conv = a.xin + 4 * 3 * D * B * L
-        ops._launch("m2_mixer_fwd", y, _lib.lib().m2_mixer_fwd, C.byref(a), launches=3)
+        ops._launch("m2_mixer_fwd", y, _lib.lib().m2_mixer_fwd, C.byref(a), launches=plan.launches)
         return y
 
     def _launch_singly(self, x, u_t, work, y, kind, yu_bf16):
@@ -315,12 +310,10 @@ class MonarchMixerSequenceMixing(nn.Module):
         specs = [f.spectrum(L, bf16, kind) for f in filters]
         if bf16:
             w_in, w_out = self._weights()
-            s_out = None
             xin = ops.linear_fwd(bf16_input(u), w_in, self.in_linear.bias)
         else:
             w_in, w_out = self.in_linear.weight.detach(), self.out_linear.weight.detach()
-            s_in, s_out = (s.get(lin.weight) for s, lin in zip(self._splitters(), (self.in_linear, self.out_linear)))
-            xin = ops.linear_fwd(u, w_in, self.in_linear.bias, w_split=s_in)
+            xin = ops.linear_fwd(u, w_in, self.in_linear.bias, w_split=ops.split_of(w_in))
         y = ops.longconv_fwd(xin, ures, self.short_filter.weight, self.short_filter.bias, specs, biases,
                              kind=kind, bf16_rounding=bf16)
-        return ops.linear_fwd(y, w_out, self.out_linear.bias, w_split=s_out), None
+        return ops.linear_fwd(y, w_out, self.out_linear.bias, w_split=ops.split_of(w_out)), None
