@@ -405,8 +405,10 @@ int m2_mlp_fwd(const m2_mlp_args* args, void* stream);
  *   embed : tables, ids, LayerNorm of the embeddings as m2_embed_layernorm_fwd takes them (ids packed, batch * seq_len);
  *           its outputs and sizes are filled in here.
  *   kind  : 0, 2, 3 or 4, from m2_longconv_pick(); spec and bias of each layer as m2_longconv_fwd takes them for that kind.
- *   workspace : m2_encoder_workspace_kind() bytes on a 256-byte boundary (m2_encoder_workspace() with pitch = seq_len rounded up
- *           to a multiple of 8 is enough for kinds 2, 3 and 4).
+ *   padded : kind 0 only: != 0 for padded time-contiguous rows with a float32 copy of the layer input, where m2_longconv_padded()
+ *           says so; 0 for token rows, at any length.
+ *   workspace : m2_encoder_workspace_kind() bytes for this kind and layout on a 256-byte boundary, or m2_encoder_workspace() with
+ *           pitch = seq_len rounded up to a multiple of 8, which is enough for all of them.
  *   f32   : != 0 without autocast: the layers alone (7 n_layers launches at most), from the embeddings' float32 output x; kind 0, float32
  *           weights, m2_encoder_workspace_f32() bytes. */
 typedef struct {
@@ -423,9 +425,10 @@ typedef struct {
   void* workspace;
   float* out;
   int f32; const float* x;
+  int padded;
 } m2_encoder_args;
 
-long long m2_encoder_workspace_kind(int kind, int batch, int seq_len, int d_model, int inter);
+long long m2_encoder_workspace_kind(int kind, int padded, int batch, int seq_len, int d_model, int inter);
 long long m2_encoder_workspace(int batch, int pitch, int d_model, int inter);
 long long m2_encoder_workspace_f32(int batch, int seq_len, int d_model, int inter, int nblocks);
 int m2_encoder_fwd(const m2_encoder_args* args, void* stream);

@@ -146,7 +146,7 @@ class EncoderArgs(C.Structure):
         ("batch", C.c_int), ("seq_len", C.c_int), ("d_model", C.c_int), ("inter", C.c_int), ("nblocks", C.c_int),
         ("n_layers", C.c_int), ("kind", C.c_int), ("n_filters", C.c_int),
         ("embed", EmbedLayernormArgs), ("layers", C.POINTER(EncoderLayer)), ("workspace", C.c_void_p), ("out", C.c_void_p),
-        ("f32", C.c_int), ("x", C.c_void_p),
+        ("f32", C.c_int), ("x", C.c_void_p), ("padded", C.c_int),
     ]
 
 
@@ -177,7 +177,7 @@ SYMBOLS = {
     "m2_mixer_fwd": (C.c_int, [C.POINTER(MixerArgs), C.c_void_p]),
     "m2_mlp_fwd": (C.c_int, [C.POINTER(MlpArgs), C.c_void_p]),
     "m2_encoder_workspace": (C.c_longlong, [C.c_int, C.c_int, C.c_int, C.c_int]),
-    "m2_encoder_workspace_kind": (C.c_longlong, [C.c_int, C.c_int, C.c_int, C.c_int, C.c_int]),
+    "m2_encoder_workspace_kind": (C.c_longlong, [C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int]),
     "m2_longconv_padded": (C.c_int, [C.c_int, C.c_int, C.c_int]),
     "m2_encoder_workspace_f32": (C.c_longlong, [C.c_int, C.c_int, C.c_int, C.c_int, C.c_int]),
     "m2_mixer_split_bytes": (C.c_longlong, [C.c_int]),

@@ -185,14 +185,15 @@ extern "C" long long m2_mlp_split_bytes(int d_model, int inter, int nblocks) {
   return d_model > 0 && inter > 0 && nblocks > 0 ? (long long)m2::mlp_split_bytes(d_model, inter, nblocks) : 0;
 }
 
+// enough for every kind and layout: the largest has a float32 copy of the layer input on padded rows
 extern "C" long long m2_encoder_workspace(int batch, int pitch, int d_model, int inter) {
   if (batch <= 0 || pitch <= 0 || d_model <= 0 || inter <= 0) return 0;
-  return (long long)m2::layout_of(batch, pitch, d_model, inter, false).total;
+  return (long long)m2::layout_of(batch, pitch, d_model, inter, false, true).total;
 }
 
-extern "C" long long m2_encoder_workspace_kind(int kind, int batch, int seq_len, int d_model, int inter) {
+extern "C" long long m2_encoder_workspace_kind(int kind, int padded, int batch, int seq_len, int d_model, int inter) {
   if (batch <= 0 || seq_len <= 0 || d_model <= 0 || inter <= 0) return 0;
-  const bool tm_f32 = kind == 0 && m2_longconv_padded(batch, seq_len, d_model);
+  const bool tm_f32 = kind == 0 && padded;
   return (long long)m2::layout_of(batch, kind == 0 && !tm_f32 ? seq_len : (int)m2::round_up(seq_len, 8), d_model, inter, false, tm_f32).total;
 }
 
@@ -281,8 +282,9 @@ extern "C" int m2_encoder_fwd(const m2_encoder_args* a, void* stream) {
   if (a->f32) return encoder_f32(a, stream);
   M2_REQUIRE(a->kind == 0 || (a->kind >= 2 && a->kind <= 4), M2_ERR_UNSUPPORTED, "m2_encoder_fwd: kind must be 0, 2, 3 or 4");
   // float32 convolution: token rows without padding and float32 layer inputs in `out`, or padded time-contiguous rows as for the
-  // other kinds with a float32 copy of the layer input
-  const bool rows = a->kind == 0 && !m2_longconv_padded(a->batch, a->seq_len, a->d_model), tm_f32 = a->kind == 0 && !rows;
+  // other kinds with a float32 copy of the layer input.  The caller says which, as the workspace is laid out for it: what
+  // m2_longconv_padded says depends on the device that is current when it is asked.
+  const bool rows = a->kind == 0 && !a->padded, tm_f32 = a->kind == 0 && !rows;
   const int pitch = rows ? a->seq_len : (int)round_up(a->seq_len, 8), D = a->d_model;
   M2_REQUIRE((long long)a->batch * pitch < (1LL << 31) - 512, M2_ERR_UNSUPPORTED, "m2_encoder_fwd: more than 2^31 tokens");
   const Layout l = layout_of(a->batch, pitch, D, a->inter, false, tm_f32);

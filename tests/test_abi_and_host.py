@@ -340,3 +340,12 @@ def test_copies_record_is_dropped_after_an_in_place_edit():
     t.add_(1.0)
     assert _tags.copies_of(t) is None and _tags.src_dtype_of(t) == torch.float32
     assert _tags.copies_of(torch.zeros(1)) is None
+
+
+@pytest.mark.parametrize("B,L,D,I", [(6, 1531, 768, 3072), (1, 1, 256, 512), (40, 301, 256, 512), (16, 2047, 1536, 6144), (2, 1024, 256, 256)])
+def test_encoder_workspace_is_enough_for_every_kind(B, L, D, I):
+    lib = _lib.lib()
+    most = lib.m2_encoder_workspace(B, (L + 7) // 8 * 8, D, I)
+    assert all(0 < lib.m2_encoder_workspace_kind(kind, padded, B, L, D, I) <= most for kind in (0, 2, 3, 4) for padded in (0, 1))
+    # the float32 copy is twice as large as the fp16 one
+    assert lib.m2_encoder_workspace_kind(0, 1, B, L, D, I) >= lib.m2_encoder_workspace_kind(2, 0, B, L, D, I) + 2 * B * L * D
