@@ -145,12 +145,7 @@ __device__ __forceinline__ uint32_t bf2_to_h2_sat(uint32_t v) {
   return r;
 }
 // barrier of the worker warps, true where `v` is for all of them
-__device__ __forceinline__ bool workers_and(bool v) {
-  uint32_t r;
-  asm volatile("{\n\t.reg .pred P, Q;\n\tsetp.ne.u32 P, %1, 0;\n\tbarrier.cta.red.and.pred Q, 1, %2, P;\n\tselp.u32 %0, 1, 0, Q;\n\t}"
-               : "=r"(r) : "r"((uint32_t)v), "n"(WORKERS) : "memory");
-  return r != 0;
-}
+__device__ __forceinline__ bool workers_and(bool v) { return tc::group_and<1, WORKERS>(v); }
 __device__ __forceinline__ void workers_sync() { asm volatile("barrier.cta.sync 1, %0;" ::"n"(WORKERS) : "memory"); }
 
 // A unit is G channels x Bt sequences (G > 1 only where one channel's columns leave most of the CTA idle and there are

@@ -235,16 +235,16 @@ longconv_bts_kernel(const Params P) {
       tc::bulk_load(smem + LY.raw, P.spec[f] + c * (TB / 2), 2 * TB, hfull);
     };
     fetch_taps(0);
-    for (int unit = u0; unit < u1 && ok; ++unit, ++n) {
+    bool go = true;                                  // the same for all warps of the role, `ok` is the warp's own
+    for (int unit = u0; unit < u1 && go; ++unit, ++n) {
       const int c = unit / P.ntile;
-      for (int f = 0; f < P.nf && ok; ++f, ++seg) {
+      for (int f = 0; f < P.nf && go; ++f, ++seg) {
         const uint32_t tb = taps + (seg & 1) * PL * TB;
         const int slot = f * SLOTS + (n & (SLOTS - 1));
         const uint32_t T = base + LY.raw;
         const float m0 = __ldg(P.spec[f] + (size_t)P.D * (TB / 2) + c), hb = __ldg(P.bias[f] + c);
-        ok = tc::mbar_wait(hfull, seg & 1, abort_flag, tc::ST_TIMEOUT_TMA);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
+        go = ok = tc::group_and<2, 32 * BUILD_WARPS>(ok && tc::mbar_wait(hfull, seg & 1, abort_flag, tc::ST_TIMEOUT_TMA));
+        if (!go) break;
         const float h0 = __uint_as_float(lds32(T + 4 * 128 * NB)) + hb;
         const float m = m0 <= 3.402823466e38f && fabsf(h0) <= 3.402823466e38f ? fmaxf(m0, fabsf(h0)) : __int_as_float(0x7f800000);
         const float sc = row_scale(m);
@@ -265,7 +265,7 @@ longconv_bts_kernel(const Params P) {
           const uint32_t wn = 128 * (dhi - dlo + 1) + 112;
           ok = tc::mbar_wait(wempty + (w & 1), ((w >> 1) & 1) ^ 1, abort_flag, tc::ST_TIMEOUT_MMA);
           ok = __all_sync(0xffffffffu, ok);
-          if (!ok) break;
+          if (!ok) break;                            // this warp; the others hear of it at the next segment's barrier
           // strip row m: taps h(i - m + 112 - 128 dlo), i = 0 .. 15, the first and the last eight in planes of their own
           const int pbase = 112 - 128 * dlo + 128 * NB;
 #pragma unroll
@@ -358,10 +358,9 @@ longconv_bts_kernel(const Params P) {
             }
           }
           if (k0 == 0) {                             // the first loads are on their way
-            ok = tc::mbar_wait(opempty, (n & 1) ^ 1, abort_flag, tc::ST_TIMEOUT_EMPTY);
-            ok = __all_sync(0xffffffffu, ok);
+            // (the maxima are cleared when all are here)
+            ok = tc::group_and<1, 16 * LOAD_WARPS>(tc::mbar_wait(opempty, (n & 1) ^ 1, abort_flag, tc::ST_TIMEOUT_EMPTY));
             if (!ok) break;
-            group_sync<1, 16 * LOAD_WARPS>();        // the maxima are cleared
           }
 #pragma unroll
           for (int i = 0; i < U; ++i) {
@@ -430,10 +429,8 @@ longconv_bts_kernel(const Params P) {
             }
           }
           if (k0 == 0) {
-            ok = tc::mbar_wait(opempty + 1, (n & 1) ^ 1, abort_flag, tc::ST_TIMEOUT_EMPTY);
-            ok = __all_sync(0xffffffffu, ok);
+            ok = tc::group_and<3, 16 * LOAD_WARPS>(tc::mbar_wait(opempty + 1, (n & 1) ^ 1, abort_flag, tc::ST_TIMEOUT_EMPTY));
             if (!ok) break;
-            group_sync<3, 16 * LOAD_WARPS>();
           }
 #pragma unroll
           for (int i = 0; i < U; ++i) {

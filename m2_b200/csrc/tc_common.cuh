@@ -93,6 +93,16 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return mbar_wait_ns(bar, parity, abort_flag, why, WAIT_LIMIT_NS);
 }
 
+// Barrier ID of N threads that also tells whether `v` holds for all of them.  Warps of one role that wait on mbarriers one by one
+// meet here before they act on what their waits said: one may give up where the next one's wait completes, and a warp that
+// left its loop alone would leave the others in a barrier that has no limit.
+template <int ID, int N> __device__ __forceinline__ bool group_and(bool v) {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred P, Q;\n\tsetp.ne.u32 P, %1, 0;\n\tbarrier.cta.red.and.pred Q, %2, %3, P;\n\tselp.u32 %0, 1, 0, Q;\n\t}"
+               : "=r"(r) : "r"((uint32_t)v), "n"(ID), "n"(N) : "memory");
+  return r != 0;
+}
+
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
