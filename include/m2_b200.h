@@ -205,14 +205,18 @@ typedef struct {
   int yu_bf16;              /* with an fp16 u (kind 3 always, kinds 2 and 4 optionally): != 0 rounds the residual
                                convolution to bf16 before the final add, as the reference does when the
                                layer input is bf16 (with a float32 / bf16 u this follows from u_dtype) */
-  int rows_padded;          /* kind 0, time-contiguous tensors: != 0 says that rows of xin and u start on 16-byte boundaries and may be
-                               read up to a multiple of 8 steps (what lies there is never used) */
+  int rows_padded;          /* kind 0, bf16 activations on time-contiguous rows of up to 2048 steps: != 0 says that rows of xin and u start
+                               on 16-byte boundaries and may be read up to a multiple of 8 steps (what lies there is never used),
+                               and asks for tensor-core products of fp16 pairs: taps and u keep 22 bits and the sums, before
+                               they are rounded to bf16, are off by up to some 3e-6 of the result (the float32 transform that
+                               kind 0 is otherwise: 1.5e-7) */
 } m2_longconv_args;
 
 int m2_longconv_fwd(const m2_longconv_args* args, void* stream);
 
-/* Whether kind 0 of m2_longconv_fwd wants bf16 activations of this shape as time-contiguous rows with rows_padded set (and u as
- * float32 rows of the same kind) rather than as token rows. */
+/* Whether kind 0 of m2_longconv_fwd is faster on bf16 activations of this shape with rows_padded, on padded time-contiguous rows and
+ * with u as float32 rows of the same kind, than on token rows.  Nothing else in this library asks for it: m2_longconv_pick's kind 0
+ * stands for float32 throughout. */
 int m2_longconv_padded(int batch, int seq_len, int d_model);
 
 /* ---------------------------------------------------------------------------------------
@@ -229,7 +233,6 @@ typedef struct {
   const void* src; long long src_sb, src_st, src_sc;
   void* dst;       long long dst_sb, dst_sc;
   void* rows_bf16; long long rows_sb, rows_st;  /* optional: the same values as bf16 rows, (b, t, c) at b*rows_sb + t*rows_st + c */
-  int dst_f32;                                  /* != 0: dst is float32 */
 } m2_time_major_args;
 
 int m2_time_major_f16(const m2_time_major_args* args, void* stream);
@@ -314,7 +317,6 @@ typedef struct {
                           its bias (a multiple of 8, at most 256) */
   int valid_len;       /* 0, or the steps of each seq_len-row sequence that are not padding: `out` then has
                           batch * valid_len rows, packed (a, b and the copies keep seq_len rows per sequence) */
-  int tm_f32;          /* != 0: out_tm_f16 is float32 (on a 32-byte boundary) */
 } m2_add_layernorm_args;
 
 int m2_add_layernorm_fwd(const m2_add_layernorm_args* args, void* stream);
@@ -343,7 +345,6 @@ typedef struct {
   void* out_tm_f16; long long tm_sb, tm_sc; int seq_len;
   long long vocab_rows, type_rows, pos_rows;
   int valid_len;      /* as in m2_add_layernorm_args; input_ids, token_type_ids and position_ids are packed too */
-  int tm_f32;
 } m2_embed_layernorm_args;
 
 int m2_embed_layernorm_fwd(const m2_embed_layernorm_args* args, void* stream);
@@ -356,11 +357,10 @@ int m2_embed_layernorm_fwd(const m2_embed_layernorm_args* args, void* stream);
  *   Activations are token rows, `pitch` (a multiple of 8, >= seq_len) rows per sequence; what the rows at and beyond
  *   seq_len hold is never used.
  *   x    : bf16 (batch * pitch, d_model), packed rows.
- *   u    : fp16 (kind 0: float32) (d_model, batch, pitch), channels u_stride elements apart (a multiple of 8); n_filters == 2 only.
+ *   u    : fp16 (d_model, batch, pitch), channels u_stride elements apart (a multiple of 8); n_filters == 2 only.
  *   xin, conv : workspace, bf16 (3 d_model, stride) and (d_model, stride), stride a multiple of 16 >= batch * pitch.
  *   out  : bf16, packed rows, out_pitch = pitch or seq_len of them per sequence.
- *   kind : from m2_longconv_pick(), 0 only where m2_longconv_padded() says so; spec and bias as m2_longconv_fwd takes them for
- *          that kind.
+ *   kind : 2, 3 or 4, from m2_longconv_pick(); spec and bias as m2_longconv_fwd takes them for that kind.
  *   f32  : != 0 without autocast: x, w_in, w_out, xin, conv and out are float32 on packed token rows (pitch, out_pitch =
  *          seq_len), x is the residual input too (u is not read), kind is 0.  split: workspace of m2_mixer_split_bytes() bytes on
  *          a 16-byte boundary, to which every call writes its weights as m2_split_weights does, or NULL (float32 chains).
@@ -394,7 +394,6 @@ typedef struct {
   float* out; void* out_bf16; void* out_tm_f16; long long tm_stride;
   int seq_len, valid_len;
   int f32; void* split;
-  int tm_f32;          /* as in m2_add_layernorm_args */
 } m2_mlp_args;
 
 long long m2_mlp_split_bytes(int d_model, int inter, int nblocks);
@@ -405,10 +404,7 @@ int m2_mlp_fwd(const m2_mlp_args* args, void* stream);
  *   embed : tables, ids, LayerNorm of the embeddings as m2_embed_layernorm_fwd takes them (ids packed, batch * seq_len);
  *           its outputs and sizes are filled in here.
  *   kind  : 0, 2, 3 or 4, from m2_longconv_pick(); spec and bias of each layer as m2_longconv_fwd takes them for that kind.
- *   padded : kind 0 only: != 0 for padded time-contiguous rows with a float32 copy of the layer input, where m2_longconv_padded()
- *           says so; 0 for token rows, at any length.
- *   workspace : m2_encoder_workspace_kind() bytes for this kind and layout on a 256-byte boundary, or m2_encoder_workspace() with
- *           pitch = seq_len rounded up to a multiple of 8, which is enough for all of them.
+ *   workspace : m2_encoder_workspace() bytes on a 256-byte boundary, pitch = seq_len rounded up to a multiple of 8.
  *   f32   : != 0 without autocast: the layers alone (7 n_layers launches at most), from the embeddings' float32 output x; kind 0, float32
  *           weights, m2_encoder_workspace_f32() bytes. */
 typedef struct {
@@ -425,10 +421,8 @@ typedef struct {
   void* workspace;
   float* out;
   int f32; const float* x;
-  int padded;
 } m2_encoder_args;
 
-long long m2_encoder_workspace_kind(int kind, int padded, int batch, int seq_len, int d_model, int inter);
 long long m2_encoder_workspace(int batch, int pitch, int d_model, int inter);
 long long m2_encoder_workspace_f32(int batch, int seq_len, int d_model, int inter, int nblocks);
 int m2_encoder_fwd(const m2_encoder_args* args, void* stream);

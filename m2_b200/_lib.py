@@ -48,7 +48,7 @@ class TimeMajorArgs(C.Structure):
         ("batch", C.c_int), ("seq_len", C.c_int), ("d_model", C.c_int), ("src_dtype", C.c_int),
         ("src", C.c_void_p), ("src_sb", C.c_longlong), ("src_st", C.c_longlong), ("src_sc", C.c_longlong),
         ("dst", C.c_void_p), ("dst_sb", C.c_longlong), ("dst_sc", C.c_longlong),
-        ("rows_bf16", C.c_void_p), ("rows_sb", C.c_longlong), ("rows_st", C.c_longlong), ("dst_f32", C.c_int),
+        ("rows_bf16", C.c_void_p), ("rows_sb", C.c_longlong), ("rows_st", C.c_longlong),
     ]
 
 
@@ -89,7 +89,7 @@ class AddLayernormArgs(C.Structure):
         ("out", C.c_void_p), ("ldo", C.c_longlong),
         ("out_bf16", C.c_void_p), ("ld_bf16", C.c_longlong),
         ("out_tm_f16", C.c_void_p), ("tm_sb", C.c_longlong), ("tm_sc", C.c_longlong), ("seq_len", C.c_int),
-        ("bf16_pad_cols", C.c_int), ("valid_len", C.c_int), ("tm_f32", C.c_int),
+        ("bf16_pad_cols", C.c_int), ("valid_len", C.c_int),
     ]
 
 
@@ -104,7 +104,7 @@ class EmbedLayernormArgs(C.Structure):
         ("out_bf16", C.c_void_p), ("ld_bf16", C.c_longlong), ("bf16_pad_cols", C.c_int),
         ("out_tm_f16", C.c_void_p), ("tm_sb", C.c_longlong), ("tm_sc", C.c_longlong), ("seq_len", C.c_int),
         ("vocab_rows", C.c_longlong), ("type_rows", C.c_longlong), ("pos_rows", C.c_longlong),
-        ("valid_len", C.c_int), ("tm_f32", C.c_int),
+        ("valid_len", C.c_int),
     ]
 
 
@@ -128,7 +128,7 @@ class MlpArgs(C.Structure):
         ("h", C.c_void_p), ("o", C.c_void_p),
         ("out", C.c_void_p), ("out_bf16", C.c_void_p), ("out_tm_f16", C.c_void_p), ("tm_stride", C.c_longlong),
         ("seq_len", C.c_int), ("valid_len", C.c_int),
-        ("f32", C.c_int), ("split", C.c_void_p), ("tm_f32", C.c_int),
+        ("f32", C.c_int), ("split", C.c_void_p),
     ]
 
 
@@ -146,7 +146,7 @@ class EncoderArgs(C.Structure):
         ("batch", C.c_int), ("seq_len", C.c_int), ("d_model", C.c_int), ("inter", C.c_int), ("nblocks", C.c_int),
         ("n_layers", C.c_int), ("kind", C.c_int), ("n_filters", C.c_int),
         ("embed", EmbedLayernormArgs), ("layers", C.POINTER(EncoderLayer)), ("workspace", C.c_void_p), ("out", C.c_void_p),
-        ("f32", C.c_int), ("x", C.c_void_p), ("padded", C.c_int),
+        ("f32", C.c_int), ("x", C.c_void_p),
     ]
 
 
@@ -177,7 +177,6 @@ SYMBOLS = {
     "m2_mixer_fwd": (C.c_int, [C.POINTER(MixerArgs), C.c_void_p]),
     "m2_mlp_fwd": (C.c_int, [C.POINTER(MlpArgs), C.c_void_p]),
     "m2_encoder_workspace": (C.c_longlong, [C.c_int, C.c_int, C.c_int, C.c_int]),
-    "m2_encoder_workspace_kind": (C.c_longlong, [C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int]),
     "m2_longconv_padded": (C.c_int, [C.c_int, C.c_int, C.c_int]),
     "m2_encoder_workspace_f32": (C.c_longlong, [C.c_int, C.c_int, C.c_int, C.c_int, C.c_int]),
     "m2_mixer_split_bytes": (C.c_longlong, [C.c_int]),

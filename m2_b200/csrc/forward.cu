@@ -22,7 +22,7 @@ static size_t mlp_split_bytes(int d_model, int inter, int nblocks) {
   return split_bytes(2LL * inter, d_model / nblocks) + split_bytes(d_model, inter / nblocks);
 }
 
-static Layout layout_of(int batch, int pitch, int d_model, int inter, bool f32, bool tm_f32 = false) {
+static Layout layout_of(int batch, int pitch, int d_model, int inter, bool f32) {
   Layout l;
   l.rows = (long long)batch * pitch;
   l.stride = round_up(l.rows, 16);
@@ -30,7 +30,7 @@ static Layout layout_of(int batch, int pitch, int d_model, int inter, bool f32, 
   const int size = f32 ? 4 : 2;
   auto take = [&](long long elements) { const size_t p = at; at += (size_t)round_up(size * elements, 256); return p; };
   l.aug = take(f32 ? 0 : l.rows * d_model);      // float32 layers read each other's output as it is
-  l.tm = take(f32 ? 0 : (tm_f32 ? 2 : 1) * l.stride * d_model);
+  l.tm = take(f32 ? 0 : l.stride * d_model);
   l.mix = take(l.rows * d_model);
   l.o = take(l.rows * d_model);
   l.xin = l.h = at;                             // in_linear's and the conv's results are dead when the GLU writes h
@@ -114,7 +114,7 @@ static int mlp_run(const m2_mlp_args* a, const m2_glu_args& g, const m2_blockdia
   n.out = a->out; n.ldo = a->d_model;
   n.out_bf16 = a->out_bf16; n.ld_bf16 = a->d_model;
   n.out_tm_f16 = a->out_tm_f16; n.tm_sb = a->seq_len; n.tm_sc = a->tm_stride;
-  n.seq_len = a->seq_len; n.valid_len = a->valid_len; n.tm_f32 = a->tm_f32;
+  n.seq_len = a->seq_len; n.valid_len = a->valid_len;
   return m2_add_layernorm_fwd(&n, stream);
 }
 
@@ -125,7 +125,8 @@ extern "C" int m2_mixer_fwd(const m2_mixer_args* a, void* stream) {
   M2_REQUIRE(a->batch >= 0 && a->seq_len > 0 && a->d_model > 0 && (a->f32 ? a->pitch == a->seq_len : a->pitch >= a->seq_len && a->pitch % 8 == 0) &&
              (a->out_pitch == a->pitch || a->out_pitch == a->seq_len) && a->stride >= (long long)a->batch * a->pitch, M2_ERR_ARG,
              "m2_mixer_fwd: bad sizes batch=%d seq_len=%d pitch=%d out_pitch=%d d_model=%d", a->batch, a->seq_len, a->pitch, a->out_pitch, a->d_model);
-  M2_REQUIRE(a->kind == 0 || (!a->f32 && a->kind >= 2 && a->kind <= 4), M2_ERR_UNSUPPORTED, "m2_mixer_fwd: kind must be 0, 2, 3 or 4");
+  M2_REQUIRE(a->f32 ? a->kind == 0 : a->kind >= 2 && a->kind <= 4, M2_ERR_UNSUPPORTED,
+             "m2_mixer_fwd: kind must be 2, 3 or 4 (time-contiguous rows), or 0 in float32");
   if (a->batch == 0) return M2_OK;
   if (a->f32) {
     m2::SplitWork work;
@@ -146,12 +147,12 @@ extern "C" int m2_mixer_fwd(const m2_mixer_args* a, void* stream) {
   m2_longconv_args c;
   memset(&c, 0, sizeof(c));
   c.batch = a->batch; c.seq_len = a->seq_len; c.d_model = a->d_model; c.n_filters = a->n_filters; c.kind = a->kind;
-  c.act_dtype = M2_BF16; c.u_dtype = a->kind == 0 ? M2_F32 : M2_F16; c.bf16_rounding = 1; c.rows_padded = 1;
+  c.act_dtype = M2_BF16; c.u_dtype = M2_F16; c.bf16_rounding = 1;
   c.xin = a->xin; c.xin_sb = a->pitch; c.xin_st = 1; c.xin_sc = a->stride;
   c.u = a->u; c.u_sb = a->pitch; c.u_st = 1; c.u_sc = a->u_stride;
   c.out = a->conv; c.out_sb = a->pitch; c.out_st = 1; c.out_sc = a->stride;
   c.short_w = a->short_w; c.short_b = a->short_b;
-  for (int f = 0; f < 2; ++f) { c.spec[f] = a->spec[f]; c.bias[f] = a->kind == 2 || a->kind == 0 ? a->bias[f] : nullptr; }
+  for (int f = 0; f < 2; ++f) { c.spec[f] = a->spec[f]; c.bias[f] = a->kind == 2 ? a->bias[f] : nullptr; }
   c.yu_bf16 = a->yu_bf16;
   if ((rc = m2_longconv_fwd(&c, stream))) return rc;
   m2_linear_args out;
@@ -185,16 +186,9 @@ extern "C" long long m2_mlp_split_bytes(int d_model, int inter, int nblocks) {
   return d_model > 0 && inter > 0 && nblocks > 0 ? (long long)m2::mlp_split_bytes(d_model, inter, nblocks) : 0;
 }
 
-// enough for every kind and layout: the largest has a float32 copy of the layer input on padded rows
 extern "C" long long m2_encoder_workspace(int batch, int pitch, int d_model, int inter) {
   if (batch <= 0 || pitch <= 0 || d_model <= 0 || inter <= 0) return 0;
-  return (long long)m2::layout_of(batch, pitch, d_model, inter, false, true).total;
-}
-
-extern "C" long long m2_encoder_workspace_kind(int kind, int padded, int batch, int seq_len, int d_model, int inter) {
-  if (batch <= 0 || seq_len <= 0 || d_model <= 0 || inter <= 0) return 0;
-  const bool tm_f32 = kind == 0 && padded;
-  return (long long)m2::layout_of(batch, kind == 0 && !tm_f32 ? seq_len : (int)m2::round_up(seq_len, 8), d_model, inter, false, tm_f32).total;
+  return (long long)m2::layout_of(batch, pitch, d_model, inter, false).total;
 }
 
 // behind the activations the split weights of one layer, written again for the next
@@ -281,19 +275,16 @@ extern "C" int m2_encoder_fwd(const m2_encoder_args* a, void* stream) {
              "m2_encoder_fwd: NULL pointer or workspace not on a 256-byte boundary");
   if (a->f32) return encoder_f32(a, stream);
   M2_REQUIRE(a->kind == 0 || (a->kind >= 2 && a->kind <= 4), M2_ERR_UNSUPPORTED, "m2_encoder_fwd: kind must be 0, 2, 3 or 4");
-  // float32 convolution: token rows without padding and float32 layer inputs in `out`, or padded time-contiguous rows as for the
-  // other kinds with a float32 copy of the layer input.  The caller says which, as the workspace is laid out for it: what
-  // m2_longconv_padded says depends on the device that is current when it is asked.
-  const bool rows = a->kind == 0 && !a->padded, tm_f32 = a->kind == 0 && !rows;
+  const bool rows = a->kind == 0;               // float32 convolution: token rows without padding, float32 layer inputs in `out`
   const int pitch = rows ? a->seq_len : (int)round_up(a->seq_len, 8), D = a->d_model;
   M2_REQUIRE((long long)a->batch * pitch < (1LL << 31) - 512, M2_ERR_UNSUPPORTED, "m2_encoder_fwd: more than 2^31 tokens");
-  const Layout l = layout_of(a->batch, pitch, D, a->inter, false, tm_f32);
+  const Layout l = layout_of(a->batch, pitch, D, a->inter, false);
   unsigned char* ws = static_cast<unsigned char*>(a->workspace);
   int rc;
   m2_embed_layernorm_args e = a->embed;
   e.m = (int)l.rows; e.n = D; e.out = rows ? a->out : nullptr; e.ldo = D;
   e.out_bf16 = ws + l.aug; e.ld_bf16 = D; e.bf16_pad_cols = 0;
-  e.out_tm_f16 = rows ? nullptr : ws + l.tm; e.tm_sb = pitch; e.tm_sc = l.stride; e.seq_len = pitch; e.valid_len = a->seq_len; e.tm_f32 = tm_f32;
+  e.out_tm_f16 = rows ? nullptr : ws + l.tm; e.tm_sb = pitch; e.tm_sc = l.stride; e.seq_len = pitch; e.valid_len = a->seq_len;
   if ((rc = m2_embed_layernorm_fwd(&e, stream))) return rc;
   for (int i = 0; i < a->n_layers; ++i) {
     const m2_encoder_layer& y = a->layers[i];
@@ -320,7 +311,7 @@ extern "C" int m2_encoder_fwd(const m2_encoder_args* a, void* stream) {
     p.seq_len = pitch; p.valid_len = a->seq_len;
     if (last || rows) p.out = a->out;
     if (!last) p.out_bf16 = ws + l.aug;         // only the next mixer reads this output, through its two copies
-    if (!last && !rows) { p.out_tm_f16 = ws + l.tm; p.tm_stride = l.stride; p.tm_f32 = tm_f32; }
+    if (!last && !rows) { p.out_tm_f16 = ws + l.tm; p.tm_stride = l.stride; }
     if ((rc = m2_mlp_fwd(&p, stream))) return rc;
   }
   return M2_OK;

@@ -166,14 +166,13 @@ __device__ __forceinline__ long long clamp_row(long long id, long long rows, boo
   return id;
 }
 
-// TM: type of the time-major copy, fp16 or float32
-template <typename TI, typename TO, int VI, typename TM>
+template <typename TI, typename TO, int VI>
 __global__ void __launch_bounds__(512)
 add_layernorm_warp_kernel(const TI* a, long long lda, const TI* b, long long ldb, const LnGather gt,
                           const float* __restrict__ w, const float* __restrict__ bias, float eps, TO* out,
                           long long ldo, __nv_bfloat16* out2, long long ld2, int m,
-                          TM* out_tm, long long tm_sb, long long tm_sc, int seq_len, int valid, int rpw, int pad2) {
-  extern __shared__ __align__(16) __half ln_tile[];   // [rows of the block][n] fp16 or float32, only with out_tm
+                          __half* out_tm, long long tm_sb, long long tm_sc, int seq_len, int valid, int rpw, int pad2) {
+  extern __shared__ __half ln_tile[];   // [rows of the block][n] fp16, only with out_tm
   pdl_wait_only();
   const int wib = threadIdx.x >> 5, nw = blockDim.x >> 5, lane = threadIdx.x & 31;
   constexpr int n = VI * 256;
@@ -271,11 +270,7 @@ add_layernorm_warp_kernel(const TI* a, long long lda, const TI* b, long long ldb
           make_uint4(pk[0], pk[1], pk[2], pk[3]);
     }
     if (out2) *reinterpret_cast<uint4*>(out2 + (long long)warp * ld2 + c0) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-    if constexpr (sizeof(TM) == 4) {
-      float4* q = reinterpret_cast<float4*>(reinterpret_cast<float*>(ln_tile) + (size_t)trow * n + c0);
-      q[0] = make_float4(y[0], y[1], y[2], y[3]);
-      q[1] = make_float4(y[4], y[5], y[6], y[7]);
-    } else if (out_tm) {
+    if (out_tm) {
       uint32_t hk[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -293,16 +288,6 @@ add_layernorm_warp_kernel(const TI* a, long long lda, const TI* b, long long ldb
     __syncthreads();
     const int rows = nw * rpw;
     const long long row0 = (long long)blockIdx.x * rows;
-    if constexpr (sizeof(TM) == 4) {    // eight rows: a channel's run is one 32-byte sector
-      float* dst = out_tm + (row0 / seq_len) * tm_sb + (row0 % seq_len);
-      const uint32_t* tile = reinterpret_cast<const uint32_t*>(ln_tile);
-      for (int c = threadIdx.x; c < n; c += blockDim.x) {
-        uint32_t q[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) q[j] = tile[(size_t)j * n + c];
-        stg256(dst + (long long)c * tm_sc, q[0], q[1], q[2], q[3], q[4], q[5], q[6], q[7]);
-      }
-    } else {
     __half* dst = out_tm + (row0 / seq_len) * tm_sb + (row0 % seq_len);
     const uint32_t* tile32 = reinterpret_cast<const uint32_t*>(ln_tile);
     const bool wide = (rows % 16 == 0) && ((reinterpret_cast<uintptr_t>(dst) & 31) == 0) && (tm_sc % 16 == 0);
@@ -331,7 +316,6 @@ add_layernorm_warp_kernel(const TI* a, long long lda, const TI* b, long long ldb
           }
         }
       }
-    }
     }
   }
 }
@@ -447,7 +431,7 @@ extern "C" int m2_embed_layernorm_fwd(const m2_embed_layernorm_args* e, void* st
   a.a = e->word_table; a.lda = e->n; a.b = e->pos_table; a.ldb = e->n;
   a.weight = e->weight; a.bias = e->bias; a.eps = e->eps;
   a.out = e->out; a.ldo = e->ldo; a.out_bf16 = e->out_bf16; a.ld_bf16 = e->ld_bf16; a.bf16_pad_cols = e->bf16_pad_cols;
-  a.out_tm_f16 = e->out_tm_f16; a.tm_sb = e->tm_sb; a.tm_sc = e->tm_sc; a.tm_f32 = e->tm_f32; a.seq_len = e->seq_len; a.valid_len = e->valid_len;
+  a.out_tm_f16 = e->out_tm_f16; a.tm_sb = e->tm_sb; a.tm_sc = e->tm_sc; a.seq_len = e->seq_len; a.valid_len = e->valid_len;
   const m2::LnGather g = {e->input_ids, e->pos_table ? e->position_ids : nullptr, e->pos_table && !e->position_ids ? steps : 0,
                           e->type_table, e->n, e->token_type_ids, e->vocab_rows, e->pos_rows, e->type_rows};
   return add_layernorm_core(&a, g, stream);
@@ -477,8 +461,7 @@ static int add_layernorm_core(const m2_add_layernorm_args* a, const m2::LnGather
                "m2_add_layernorm_fwd: the time-major copy needs n a multiple of 256 (<= 2048), 16-byte aligned rows and bf16 inputs (or float32 inputs with a float32 output)");
     M2_REQUIRE(a->seq_len > 0 && a->seq_len % 8 == 0 && a->m % a->seq_len == 0, M2_ERR_ARG,
                "m2_add_layernorm_fwd: the time-major copy needs m = batch * seq_len rows with seq_len a multiple of 8");
-    M2_REQUIRE(!a->tm_f32 || a->out_dtype == M2_F32, M2_ERR_UNSUPPORTED, "m2_add_layernorm_fwd: a float32 time-major copy comes with float32 results");
-    M2_REQUIRE(m2_aligned(a->out_tm_f16, a->tm_f32 ? 32 : 16) && a->tm_sb % 8 == 0 && a->tm_sc % 8 == 0, M2_ERR_ALIGN,
+    M2_REQUIRE(m2_aligned(a->out_tm_f16, 16) && a->tm_sb % 8 == 0 && a->tm_sc % 8 == 0, M2_ERR_ALIGN,
                "m2_add_layernorm_fwd: the time-major copy needs 16-byte aligned rows");
   }
   M2_REQUIRE(a->valid_len >= 0 && (a->valid_len == 0 || (a->seq_len > 0 && a->valid_len <= a->seq_len && a->m % a->seq_len == 0)),
@@ -489,22 +472,21 @@ static int add_layernorm_core(const m2_add_layernorm_args* a, const m2::LnGather
     // run of them one 32-byte sector, 32 steps two.  Few rows take short blocks all the same: 128 rows are four blocks
     // of 32 (11 us) or 16 of 8; from one and a half blocks per SM on the runs decide.
     int rows = 8, threads = 256, rpw = 1;
-    if (a->out_tm_f16 && !a->tm_f32) {
+    if (a->out_tm_f16) {
       const int sms = m2_sm_count();
       rows = a->seq_len % 32 == 0 && a->n <= 768 && a->m >= 48 * sms ? 32 : a->seq_len % 16 == 0 && a->m >= 24 * sms ? 16 : 8;
       threads = rows >= 16 ? 512 : 256;
       rpw = rows / (threads / 32);
     }
     const int blocks = (a->m + rows - 1) / rows;
-    const size_t tile = a->out_tm_f16 ? (size_t)rows * a->n * (a->tm_f32 ? 4 : 2) : 0;
+    const size_t tile = a->out_tm_f16 ? (size_t)rows * a->n * 2 : 0;
 #define M2_LNW(TO, VI) do { if (a->in_dtype == M2_F32) M2_LNW2(float, float, VI); else M2_LNW2(__nv_bfloat16, TO, VI); } while (0)
-#define M2_LNW2(TI, TO, VI) do { if (a->out_tm_f16 && a->tm_f32) M2_LNW3(TI, float, VI, float); else M2_LNW3(TI, TO, VI, __half); } while (0)
-#define M2_LNW3(TI, TO, VI, TM) do { \
-      if (tile > 48 * 1024) M2_SMEM_ONCE((add_layernorm_warp_kernel<TI, TO, VI, TM>), 64 * 1024); /* at most 16 x 2048 x 2 or 8 x 2048 x 4 bytes */ \
-      return m2_launch("add_layernorm_warp_kernel", (long long)a->m * a->n, add_layernorm_warp_kernel<TI, TO, VI, TM>, blocks, threads, tile, st, \
+#define M2_LNW2(TI, TO, VI) do { \
+      if (tile > 48 * 1024) M2_SMEM_ONCE((add_layernorm_warp_kernel<TI, TO, VI>), 64 * 1024); /* at most 16 x 2048 x 2 bytes */ \
+      return m2_launch("add_layernorm_warp_kernel", (long long)a->m * a->n, add_layernorm_warp_kernel<TI, TO, VI>, blocks, threads, tile, st, \
       (const TI*)a->a, a->lda, (const TI*)a->b, a->ldb, gather, a->weight, a->bias, a->eps, \
       (TO*)a->out, a->ldo, (__nv_bfloat16*)a->out_bf16, a->ld_bf16, a->m, \
-      (TM*)a->out_tm_f16, a->tm_sb, a->tm_sc, a->seq_len, a->valid_len > 0 ? a->valid_len : a->seq_len, rpw, a->bf16_pad_cols); } while (0)
+      (__half*)a->out_tm_f16, a->tm_sb, a->tm_sc, a->seq_len, a->valid_len > 0 ? a->valid_len : a->seq_len, rpw, a->bf16_pad_cols); } while (0)
 #define M2_LNW_VI(TO) switch (a->n / 256) { case 1: M2_LNW(TO, 1); break; case 2: M2_LNW(TO, 2); break; \
       case 3: M2_LNW(TO, 3); break; case 4: M2_LNW(TO, 4); break; case 5: M2_LNW(TO, 5); break; \
       case 6: M2_LNW(TO, 6); break; case 7: M2_LNW(TO, 7); break; default: M2_LNW(TO, 8); break; }
@@ -512,7 +494,6 @@ static int add_layernorm_core(const m2_add_layernorm_args* a, const m2::LnGather
 #undef M2_LNW_VI
 #undef M2_LNW
 #undef M2_LNW2
-#undef M2_LNW3
   }
   M2_REQUIRE(!gather.ids_a && !gather.c, M2_ERR_UNSUPPORTED, "m2_embed_layernorm_fwd: shape not covered by the vectorised kernel");
   M2_REQUIRE(a->out != nullptr && a->out_bf16 == nullptr && a->out_tm_f16 == nullptr, M2_ERR_UNSUPPORTED,

@@ -110,15 +110,12 @@ spectrum_kind3_kernel(const float* __restrict__ kfilt, const float* __restrict__
 // (b, t, c) tensor of float32 / bf16 -> fp16 copy with time contiguous (the layout the
 // residual filter's A operand is loaded from)
 // ---------------------------------------------------------------------------------------
-template <typename TD> __device__ __forceinline__ TD copied(float v);
-template <> __device__ __forceinline__ __half copied<__half>(float v) { return __float2half_rn(fminf(fmaxf(v, -65504.f), 65504.f)); }
-template <> __device__ __forceinline__ float copied<float>(float v) { return v; }
-template <typename TS, typename TD>
+template <typename TS>
 __global__ void __launch_bounds__(256)
-time_major_kernel(const TS* __restrict__ src, long long ssb, long long sst, long long ssc,
-                  TD* __restrict__ dst, long long dsb, long long dsc, __nv_bfloat16* __restrict__ rows, long long rsb, long long rst,
-                  int L, int D) {
-  __shared__ TD tile[64][sizeof(TD) == 2 ? 66 : 65];
+time_major_f16_kernel(const TS* __restrict__ src, long long ssb, long long sst, long long ssc,
+                      __half* __restrict__ dst, long long dsb, long long dsc, __nv_bfloat16* __restrict__ rows, long long rsb, long long rst,
+                      int L, int D) {
+  __shared__ __half tile[64][66];
   const int t0 = blockIdx.x * 64, c0 = blockIdx.y * 64, b = blockIdx.z;
   const int tx = threadIdx.x & 63, ty = threadIdx.x >> 6;
   float v[16];                                             // all loads of the thread in flight at once
@@ -134,7 +131,7 @@ time_major_kernel(const TS* __restrict__ src, long long ssb, long long sst, long
       if (t0 + ty + 4 * i < L && c0 + tx < D) rows[b * rsb + (long long)(t0 + ty + 4 * i) * rst + c0 + tx] = __float2bfloat16_rn(v[i]);
   }
 #pragma unroll
-  for (int i = 0; i < 16; ++i) tile[ty + 4 * i][tx] = copied<TD>(v[i]);
+  for (int i = 0; i < 16; ++i) tile[ty + 4 * i][tx] = __float2half_rn(fminf(fmaxf(v[i], -65504.f), 65504.f));
   __syncthreads();
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
@@ -622,23 +619,21 @@ int longconv_tz_launch(const m2_longconv_args* a, cudaStream_t st) {
 int time_major_f16_launch(const m2_time_major_args* a, cudaStream_t st) {
   dim3 grid((a->seq_len + 63) / 64, (a->d_model + 63) / 64, a->batch);
   __nv_bfloat16* rows = (__nv_bfloat16*)a->rows_bf16;
-  const bool vec = !a->dst_f32 && a->src_dtype == M2_F32 && a->src_sc == 1 && a->d_model % 4 == 0 && m2_aligned(a->src, 16) && a->src_sb % 4 == 0 &&
+  const bool vec = a->src_dtype == M2_F32 && a->src_sc == 1 && a->d_model % 4 == 0 && m2_aligned(a->src, 16) && a->src_sb % 4 == 0 &&
                    a->src_st % 4 == 0 && m2_aligned(a->dst, 16) && a->dst_sb % 8 == 0 && a->dst_sc % 8 == 0 &&
                    m2_aligned(rows, 16) && (!rows || (a->rows_sb % 8 == 0 && a->rows_st % 8 == 0));
-  if (vec) {
+  if (vec)
     tz::row_copies_kernel<<<grid, 256, 0, st>>>((const float*)a->src, a->src_sb, a->src_st, (__half*)a->dst, a->dst_sb, a->dst_sc,
                                                 rows, a->rows_sb, a->rows_st, a->seq_len, a->d_model);
-  } else {
-    auto launch = [&](auto ts, auto td) {
-      using TS = decltype(ts);
-      using TD = decltype(td);
-      tz::time_major_kernel<TS, TD><<<grid, 256, 0, st>>>((const TS*)a->src, a->src_sb, a->src_st, a->src_sc, (TD*)a->dst, a->dst_sb,
-                                                          a->dst_sc, rows, a->rows_sb, a->rows_st, a->seq_len, a->d_model);
-    };
-    if (a->src_dtype == M2_F32) a->dst_f32 ? launch(0.f, 0.f) : launch(0.f, __half());
-    else a->dst_f32 ? launch(__nv_bfloat16(), 0.f) : launch(__nv_bfloat16(), __half());
-  }
-  M2_LAUNCH_CHECK("time_major_kernel");
+  else if (a->src_dtype == M2_F32)
+    tz::time_major_f16_kernel<float><<<grid, 256, 0, st>>>((const float*)a->src, a->src_sb, a->src_st, a->src_sc,
+                                                            (__half*)a->dst, a->dst_sb, a->dst_sc, rows, a->rows_sb, a->rows_st,
+                                                            a->seq_len, a->d_model);
+  else
+    tz::time_major_f16_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>((const __nv_bfloat16*)a->src, a->src_sb, a->src_st,
+                                                                    a->src_sc, (__half*)a->dst, a->dst_sb, a->dst_sc,
+                                                                    rows, a->rows_sb, a->rows_st, a->seq_len, a->d_model);
+  M2_LAUNCH_CHECK("time_major_f16_kernel");
   return M2_OK;
 }
 

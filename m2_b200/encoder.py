@@ -259,10 +259,9 @@ class M2BertModel(nn.Module):
         kind = 0 if f32 else ops.longconv_pick(B, L, torch.bfloat16, D)
         args = (_lib.EncoderLayer * len(layers))()
         e = _lib.EncoderArgs()
-        padded = not f32 and kind == 0 and ops.longconv_padded(B, L, D)
         nb = cfg.monarch_mlp_nblocks
         work = (_lib.lib().m2_encoder_workspace_f32(B, L, D, cfg.intermediate_size, nb) if f32 else
-                _lib.lib().m2_encoder_workspace_kind(kind, padded, B, L, D, cfg.intermediate_size))
+                _lib.lib().m2_encoder_workspace(B, (L + 7) // 8 * 8, D, cfg.intermediate_size))
         plan = Plan(e, layers=args, work=work, out=(B, L, D), called=called, dropping=[m for m in called if hasattr(m, "dropout")],
                     per_layer=6 + (f32 and ops.split_used(D, D // nb, cfg.intermediate_size // nb)))
         for a, y in zip(args, layers):
@@ -271,7 +270,7 @@ class M2BertModel(nn.Module):
                 return None
         e.batch, e.seq_len, e.d_model, e.inter, e.nblocks = B, L, D, cfg.intermediate_size, nb
         e.n_layers, e.kind, e.n_filters = len(layers), kind, 2 if layers[0].attention.residual_long_conv else 1
-        e.f32, e.padded = f32, padded
+        e.f32 = f32
         e.layers = C.cast(args, C.POINTER(_lib.EncoderLayer))
         if f32:                                # the embeddings are modules of their own there
             return plan

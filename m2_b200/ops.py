@@ -176,23 +176,22 @@ def filter_spectrum(k: torch.Tensor, seq_len: int, kind: int, bias=None) -> torc
 
 
 def longconv_padded(batch: int, seq_len: int, d_model: int) -> bool:
-    """Whether kind 0 wants bf16 activations of this shape as padded time-contiguous rows."""
+    """Whether kind 0 is faster on bf16 activations of this shape with rows_padded.  The modules do not ask for it."""
     return bool(_lib.lib().m2_longconv_padded(int(batch), int(seq_len), int(d_model)))
 
 
 def time_major_f16(u: torch.Tensor, out=None, rows=None) -> torch.Tensor:
     """fp16 copy of u (B, L, D) laid out (D, B, L): the residual-filter operand of kind 3.  rows: optional (B, L, D) bf16
-    tensor with contiguous channels that receives u rounded to bf16 in the same pass.  A float32 `out` receives u as it is."""
+    tensor with contiguous channels that receives u rounded to bf16 in the same pass."""
     _need_cuda(u)
     B, L, D = u.shape
     if out is None:
         out = torch.empty((D, B, L), dtype=torch.float16, device=u.device)
-    assert out.dtype in (torch.float16, torch.float32) and out.shape == (D, B, L) and out.stride(2) == 1
+    assert out.dtype == torch.float16 and out.shape == (D, B, L) and out.stride(2) == 1
     a = _lib.TimeMajorArgs()
     a.batch, a.seq_len, a.d_model, a.src_dtype = B, L, D, _dt(u)
     a.src, (a.src_sb, a.src_st, a.src_sc) = u.data_ptr(), u.stride()
     a.dst, a.dst_sc, a.dst_sb = out.data_ptr(), out.stride(0), out.stride(1)
-    a.dst_f32 = int(out.dtype == torch.float32)
     if rows is not None:
         assert rows.dtype == torch.bfloat16 and rows.shape == (B, L, D) and rows.stride(2) == 1
         a.rows_bf16, a.rows_sb, a.rows_st = rows.data_ptr(), rows.stride(0), rows.stride(1)

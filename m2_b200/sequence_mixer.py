@@ -150,7 +150,7 @@ class MonarchMixerSequenceMixing(nn.Module):
         x = rec.bf16 if rec is not None else None                                # (B*L, D) from the LayerNorm
         rows = None                              # bf16 rows to be written together with the time-major copy below
         if x is None or L != Lp or x.shape != (B * L, D) or x.device != dev or not x.is_contiguous():
-            if ures is u and u.dtype == torch.float32 and (rec is None or rec.tm is None or L != Lp or not kind):
+            if ures is u and u.dtype == torch.float32 and (rec is None or rec.tm is None or L != Lp):
                 x = torch.empty((B, Lp, D), dtype=torch.bfloat16, device=dev)
                 rows = x[:, :L]
             elif L == Lp:
@@ -161,9 +161,9 @@ class MonarchMixerSequenceMixing(nn.Module):
         u_t = None
         if ures is not None:
             rec = copies_of(ures)
-            u_t = rec.tm if rec is not None and kind else None                   # (D, B, L) fp16 from the LayerNorm
+            u_t = rec.tm if rec is not None else None                            # (D, B, L) fp16 from the LayerNorm
             if rows is not None or u_t is None or u_t.shape != (D, B, Lp) or L != Lp or u_t.device != dev or not u_t.is_contiguous():
-                u_t = torch.empty((D, B, Lp), dtype=torch.float16 if kind else torch.float32, device=dev)
+                u_t = torch.empty((D, B, Lp), dtype=torch.float16, device=dev)
                 ops.time_major_f16(ures if ures.dtype in (torch.float32, torch.bfloat16) else ures.float(), out=u_t[:, :, :L], rows=rows)
         yu_bf16 = ures is not None and src_dtype_of(ures) == torch.bfloat16
         plan = plans_of(self).get(self, (B, L, kind, dev.index), lambda: self._make_plan(B, L, kind, dev))
@@ -212,8 +212,8 @@ class MonarchMixerSequenceMixing(nn.Module):
         fs = self.filters()
         ops.longconv_fwd(rows(work[:3 * D]), u_t[:, :, :L].permute(1, 2, 0) if u_t is not None else None,
                          self.short_filter.weight, self.short_filter.bias, [f.spectrum(L, True, kind) for f in fs],
-                         [f.conv_bias() for f in fs] if kind in (0, 2) else None, kind=kind, bf16_rounding=True,
-                         out=rows(work[3 * D:]), yu_bf16=yu_bf16, rows_padded=True)
+                         [f.conv_bias() for f in fs] if kind == 2 else None, kind=kind, bf16_rounding=True,
+                         out=rows(work[3 * D:]), yu_bf16=yu_bf16)
         if L == Lp:
             return ops.linear_fwd(work[3 * D:, :n].t().unsqueeze(0), w_out, self.out_linear.bias, out=y.view(1, n, D)).view(B, L, D)
         return ops.linear_fwd(rows(work[3 * D:]), w_out, self.out_linear.bias, out=y)
@@ -296,7 +296,7 @@ class MonarchMixerSequenceMixing(nn.Module):
             ops._dt(ures)                       # the residual filter reads the input itself: TypeError for float64 or integers
         if bf16:
             kind = ops.longconv_pick(u.size(0), L, torch.bfloat16, self.d_model)
-            if u.size(0) and (kind or ops.longconv_padded(u.size(0), L, self.in_linear.weight.shape[-1])):
+            if kind and u.size(0):
                 return self._forward_bf16(u, ures, kind), None
         elif u.size(0):
             y = self._forward_f32(u)

@@ -342,10 +342,8 @@ def test_copies_record_is_dropped_after_an_in_place_edit():
     assert _tags.copies_of(torch.zeros(1)) is None
 
 
-@pytest.mark.parametrize("B,L,D,I", [(6, 1531, 768, 3072), (1, 1, 256, 512), (40, 301, 256, 512), (16, 2047, 1536, 6144), (2, 1024, 256, 256)])
-def test_encoder_workspace_is_enough_for_every_kind(B, L, D, I):
-    lib = _lib.lib()
-    most = lib.m2_encoder_workspace(B, (L + 7) // 8 * 8, D, I)
-    assert all(0 < lib.m2_encoder_workspace_kind(kind, padded, B, L, D, I) <= most for kind in (0, 2, 3, 4) for padded in (0, 1))
-    # the float32 copy is twice as large as the fp16 one
-    assert lib.m2_encoder_workspace_kind(0, 1, B, L, D, I) >= lib.m2_encoder_workspace_kind(2, 0, B, L, D, I) + 2 * B * L * D
+@pytest.mark.parametrize("kind,f32", [(0, 0), (1, 0), (5, 0), (2, 1), (4, 1)])
+def test_mixer_refuses_kinds_that_it_does_not_run(kind, f32):
+    a = _lib.MixerArgs()
+    a.batch, a.seq_len, a.pitch, a.out_pitch, a.d_model, a.stride, a.kind, a.n_filters, a.f32 = 6, 1536, 1536, 1536, 768, 6 * 1536, kind, 2, f32
+    assert _lib.lib().m2_mixer_fwd(C.byref(a), None) == 2 and b"kind must be" in _lib.lib().m2_last_error()
