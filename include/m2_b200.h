@@ -208,8 +208,8 @@ typedef struct {
   int rows_padded;          /* kind 0, bf16 activations on time-contiguous rows of up to 2048 steps: != 0 says that rows of xin and u start
                                on 16-byte boundaries and may be read up to a multiple of 8 steps (what lies there is never used),
                                and asks for tensor-core products of fp16 pairs: taps and u keep 22 bits and the sums, before
-                               they are rounded to bf16, are off by up to some 3e-6 of the result (the float32 transform that
-                               kind 0 is otherwise: 1.5e-7) */
+                               they are rounded to bf16, fall short by up to 3.5e-6 of the result, 1.7e-5 where all products
+                               have one sign (the float32 transform that kind 0 is otherwise: 1.5e-7) */
 } m2_longconv_args;
 
 int m2_longconv_fwd(const m2_longconv_args* args, void* stream);

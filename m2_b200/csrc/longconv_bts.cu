@@ -1,5 +1,6 @@
 // Fused gated long convolution of family 0 (float32 taps and residual input) on bf16 activations in time-contiguous rows, up to 2048
-// steps: block-Toeplitz GEMMs over pairs of fp16 values, with a warp for every part of the work.
+// steps: block-Toeplitz GEMMs over pairs of fp16 values, with a warp for every part of the work.  For callers that ask for it
+// (rows_padded): the modules take the float32 transform at these lengths, whatever the batch.
 //
 // The product is that of longconv_bt.cu: a sequence is cut into NB = ceil(L / 128) blocks, the Toeplitz block of a distance
 // delta is the MMA's A operand, all (block, sequence) pairs of a tile of Bt sequences its columns:
@@ -12,8 +13,11 @@
 // Taps h (bias folded into h(0)) and the residual input u are float32.  Each is scaled by a power of two (taps
 // per channel, u per channel and sequence, as is v * x1) that brings its largest value to [2^14, 2^15) and written as hi + lo, two
 // fp16 values that keep 22 bits; v * x1 is a bf16 value, which one fp16 value holds exactly down to 2^-31 of the largest.  The products are
-// lo.hi + hi.hi for v * x1 and lo.hi + hi.lo + hi.hi for u, accumulated in float32, the small terms apart (an accumulation
-// in tensor memory drops what does not fit).  Any non-finite value makes all outputs of its row NaN, as in a transform.
+// lo.hi + hi.hi for v * x1 and lo.hi + hi.lo + hi.hi for u, accumulated in float32, the small terms apart.  An accumulation
+// in tensor memory drops what does not fit, always towards zero, and up to 128 follow one another: before the rounding to bf16 the
+// sums are off by 2.2e-7 / 1.7e-6 / 2.6e-6 / 3.5e-6 of the result at 129 / 1000 / 1531 / 2045 steps of random data, 1.7e-5 at 2045
+// where inputs and taps have one sign (the transform: 0.8e-7 to 1.5e-7).  Taken out of tensor memory and added up in float32 every
+// 64 steps they were off by 1.2e-7 to 2.5e-7, and 6 x 1531 through twelve layers took 6048 us (transform 5950).  Any non-finite value makes all outputs of its row NaN, as in a transform.
 //
 // Bound: the MMAs, which shared memory feeds: each reads 4 KB of strip and 32 bytes a column, 56 to 60 clocks beside the other warps'
 // traffic (6 x 1531 at 768 channels: 920 a unit, 55 of its 63 thousand clocks); units that fill the SMs unevenly (five or six each);
@@ -39,9 +43,6 @@ constexpr int REGION = 256;                     // accumulator columns of a filt
 constexpr int BATCHES = 8;                      // of eight columns in an epilogue warp, two warps to a quarter of the lanes
 constexpr int MAXCOLS = 16 * BATCHES;
 constexpr int SMALL = 128;                      // where the columns of the small terms start in a region
-// What an addition in tensor memory drops on average, towards zero: 4.6e-8 of the final sum where products differ in sign (sums of 48
-// additions were short by 2.2e-6).  With up to 128 of them per output it is put back before the rounding to bf16.
-constexpr float DROPPED = 4.6e-8f;
 
 __host__ __device__ constexpr int tap_count(int nb) { return 256 * nb + 64; }   // taps of a channel, d = -128 nb ..
 __host__ __device__ constexpr int window_rows(int nb) { return nb == 1 ? 240 : WROWS; }
@@ -248,7 +249,7 @@ longconv_bts_kernel(const Params P) {
         const float h0 = __uint_as_float(lds32(T + 4 * 128 * NB)) + hb;
         const float m = m0 <= 3.402823466e38f && fabsf(h0) <= 3.402823466e38f ? fmaxf(m0, fabsf(h0)) : __int_as_float(0x7f800000);
         const float sc = row_scale(m);
-        if (bt == 0) tinv[slot] = row_inverse(m) * (1.0f + DROPPED * NB * P.ksteps);
+        if (bt == 0) tinv[slot] = row_inverse(m);
         for (uint32_t i = 2 * bt; i < TB / 2; i += 2 * 32 * BUILD_WARPS) {
           uint32_t t0, t1, hi, lo;
           asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(t0), "=r"(t1) : "r"(T + 4 * i));

@@ -71,6 +71,23 @@ def test_values_of_any_size():
         assert error(y[b], ref[b].double()) < 1e-2 ** 0.5 * 2 ** -8
 
 
+@pytest.mark.parametrize("L", [129, 1531])
+def test_exact_sums_stay_exact(L):
+    """A filter of one tap, at values half way between two bf16 values: whatever scaled the sums would push them over."""
+    m, xin, u = mixer(L, 8, 6)
+    k = torch.zeros_like(m.filter_fn.time_filter(L, True))
+    k[:, 0] = 1.0
+    spec, zero = ops.filter_spectrum(k, L, 0), torch.zeros(8, device=DEV)
+    u.copy_(1 + 2.0 ** -8)
+    u[:, ::2].mul_(-1)
+    rows = torch.zeros((4 * 8, 6, (L + 7) // 8 * 8), dtype=torch.bfloat16, device=DEV)
+    t = rows[:, :, :L].permute(1, 2, 0)                       # the gate is zero: the residual convolution alone
+    y = ops.longconv_fwd(t[..., :3 * 8], rows.new_zeros((8, 6, rows.shape[2]), dtype=torch.float32)[:, :, :L].copy_(u.permute(2, 0, 1)).permute(1, 2, 0),
+                         m.short_filter.weight, torch.zeros_like(m.short_filter.bias), [spec, spec], [zero, zero], kind=0, bf16_rounding=True,
+                         out=t[..., 3 * 8:], rows_padded=True)
+    assert torch.equal(y.float(), u.sign())
+
+
 @pytest.mark.parametrize("B,L", [(6, 1531), (40, 301)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_module_takes_padded_rows(B, L, dtype):
