@@ -205,6 +205,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
           if (++stage == NST) { stage = 0; phase ^= 1; }
         }
       }
+      tc::drain_loads(full, NST, tc::ring_parities(stage, phase));
     }
   } else if (warp == 1) {
     // ---- MMA issue ----
@@ -404,12 +405,6 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         }
       }
     }
-  }
-  __syncthreads();
-  if (*abort_flag && threadIdx.x == 0) {
-    // loads issued before the abort get a bounded time to land
-    for (int s = 0; s < NST; ++s)
-      for (uint32_t i = 0; i < 4096 && !tc::mbar_try_wait(full + s, 0) && !tc::mbar_try_wait(full + s, 1); ++i) {}
   }
   tc::tc_fence_before();
   __syncthreads();

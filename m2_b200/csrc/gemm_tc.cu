@@ -180,6 +180,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           if (++stage == C::NSTAGES) { stage = 0; phase ^= 1; }
         }
       }
+      tc::drain_loads(full, C::NSTAGES, tc::ring_parities(stage, phase));
     }
   } else if (warp >= 1 && warp <= C::NACC) {
     // ------------------------------- MMA issuers --------------------------------
@@ -275,12 +276,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   }
 
   // ------------------------------- teardown -------------------------------------
-  __syncthreads();
-  if (*abort_flag && threadIdx.x == 0) {
-    // give loads that were issued before the abort a bounded time to land
-    for (int s = 0; s < C::NSTAGES; ++s)
-      for (uint32_t i = 0; i < 4096 && !tc::mbar_try_wait(full + s, 0) && !tc::mbar_try_wait(full + s, 1); ++i) {}
-  }
   __syncthreads();
   if (warp == 1) {
     tc::tc_fence_after();
@@ -394,6 +389,7 @@ glu_res_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
           }
         }
       }
+      tc::drain_loads(b_full, NSTB, tc::ring_parities(stage, phase));
     }
   } else if (warp == 1 || warp == 2) {
     // ------------------------------- MMA issuers: warp 1 gate, warp 2 linear ----------------------
@@ -456,11 +452,6 @@ glu_res_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   }
 
   // ------------------------------- teardown -------------------------------------
-  __syncthreads();
-  if (*abort_flag && threadIdx.x == 0) {
-    for (int s = 0; s < NSTB; ++s)
-      for (uint32_t i = 0; i < 4096 && !tc::mbar_try_wait(b_full + s, 0) && !tc::mbar_try_wait(b_full + s, 1); ++i) {}
-  }
   __syncthreads();
   if (warp == 1) {
     tc::tc_fence_after();

@@ -124,6 +124,7 @@ glu_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
           }
         }
       }
+      if (rank == 0) tc::drain_loads(b_full, NSTB, tc::ring_parities(stage, phase));       // both CTAs' loads of every stage it armed
     }
   } else if (warp == 1 || warp == 2) {
     // ------------------------------- MMA issuers (leader CTA): warp 1 gate, warp 2 linear -------------------------------
@@ -218,10 +219,7 @@ glu_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 
   // ------------------------------- teardown -------------------------------------
   __syncthreads();
-  if (*abort_flag && threadIdx.x == 0 && rank == 0) {
-    for (int s = 0; s < NSTB; ++s)
-      for (uint32_t i = 0; i < 4096 && !tc::mbar_try_wait(b_full + s, 0) && !tc::mbar_try_wait(b_full + s, 1); ++i) {}
-  }
+  if (*abort_flag && threadIdx.x == 0 && rank != 0) tc::pause_ns(1000000);       // a load takes a thousandth of it
   tc::tc_fence_before();
   tc::cluster_sync();
   if (warp == 1) {

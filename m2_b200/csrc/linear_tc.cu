@@ -147,6 +147,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
           if (++stage == NST) { stage = 0; phase ^= 1; }
         }
       }
+      if (rank == 0) tc::drain_loads(full, NST, tc::ring_parities(stage, phase));          // both CTAs' loads of every stage it armed
     }
   } else if (warp == 1) {
     // ------------------------------- MMA issue (leader CTA only) -------------------------------
@@ -295,11 +296,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
 
   // ------------------------------- teardown -------------------------------------
   __syncthreads();
-  if (*abort_flag && threadIdx.x == 0 && rank == 0) {
-    // give loads that were issued before the abort a bounded time to land
-    for (int s = 0; s < NST; ++s)
-      for (uint32_t i = 0; i < 4096 && !tc::mbar_try_wait(full + s, 0) && !tc::mbar_try_wait(full + s, 1); ++i) {}
-  }
+  if (*abort_flag && threadIdx.x == 0 && rank != 0) tc::pause_ns(1000000);       // a load takes a thousandth of it
   tc::tc_fence_before();
   tc::cluster_sync();                       // nobody leaves while the peer may still signal it or read its operands
   if (warp == 1) {

@@ -228,9 +228,11 @@ longconv_bts_kernel(const Params P) {
     uint32_t w = 0, n = 0, seg = 0;
     bool ok = true;
     // the taps of a segment (one filter of one unit) are fetched while the strips of the one before are built
+    uint32_t fetched = 1u;                           // parity of the last fetch
     auto fetch_taps = [&](uint32_t s) {
       const uint32_t k = s / P.nf, f = s - k * P.nf;
       if (bt != 0 || u0 + (int)k >= u1) return;
+      fetched = s & 1u;
       const size_t c = (u0 + k) / P.ntile;
       tc::mbar_expect_tx(hfull, 2 * TB);
       tc::bulk_load(smem + LY.raw, P.spec[f] + c * (TB / 2), 2 * TB, hfull);
@@ -295,6 +297,7 @@ longconv_bts_kernel(const Params P) {
         }
       }
     }
+    if (bt == 0) tc::drain_loads(hfull, 1, fetched);
   } else if (warp < EPI0) {
     // ---- operands: four warps for v * x1, four for the residual input; a warp covers 64 bytes of eight rows, a quarter warp writes
     // one core matrix ----
@@ -568,11 +571,6 @@ longconv_bts_kernel(const Params P) {
         if (lane == 0) tc::mbar_arrive(tempty + f);
       }
     }
-  }
-  __syncthreads();
-  if (*abort_flag && tid == 0) {
-    // taps on their way before the abort get a bounded time to land
-    for (uint32_t i = 0; i < 4096 && !tc::mbar_try_wait(hfull, 0) && !tc::mbar_try_wait(hfull, 1); ++i) {}
   }
   tc::tc_fence_before();
   __syncthreads();

@@ -281,6 +281,7 @@ longconv_tz_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
     // ------------------------- TMA: strips, raw x1 / v, residual operand -------------------------
     if (tc::elect_one()) {
       int it = 0, epoch = -1, prev_c = -1;
+      uint32_t strips = 3u;                                // parities of the strips' loads
       bool ok = true;
       for (int unit = u_first; unit < u_last && ok; ++unit) {
         const int c = unit / P.nbt, b0 = (unit % P.nbt) * TB;
@@ -288,6 +289,7 @@ longconv_tz_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
           prev_c = c; ++epoch;
           const int p = epoch & 1;
           if (!tc::mbar_wait(strip_empty + p, ((epoch >> 1) & 1) ^ 1, abort_flag, tc::ST_TIMEOUT_EMPTY)) break;
+          strips = (strips & ~(1u << p)) | ((uint32_t)(epoch >> 1) & 1u) << p;
           tc::mbar_expect_tx(strip_full + p, P.nf * STRIP_BYTES);
           for (int f = 0; f < P.nf; ++f)
             tc::bulk_load(smem + OFF_STRIP + (2 * p + f) * STRIP_BYTES, (f ? P.spec[1] : P.spec[0]) + (size_t)c * STRIP_FLOATS,
@@ -302,12 +304,15 @@ longconv_tz_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
           tc::tma_load_3d(st + RAW_BYTES, &tmX, full_main + s, TW * j - HALO, b0, 2 * P.D + c);
         }
       }
+      tc::drain_loads(strip_full, 2, strips);
+      tc::drain_loads(full_main, NST, tc::ring_parities(it % NST, (it / NST) & 1));
     }
   } else if (warp == 2) {
     // ------------------------- TMA: raw x2 rows for the epilogue -------------------------
     if (tc::elect_one()) {
       bool ok = true;
       int ui = 0, it = 0;
+      uint32_t x2 = ~0u;                                   // parities of the x2 rows' loads
       for (int unit = u_first; unit < u_last && ok; ++unit, ++ui) {
         const int c = unit / P.nbt, b0 = (unit % P.nbt) * TB;
         // the residual operand of the unit in tiles of 64 steps, rows of 128 bytes (a 16-byte-row
@@ -323,10 +328,13 @@ longconv_tz_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
         for (int j = 0; j < P.nsub; ++j) {
           const int sl = 4 * (ui % XSETS) + j;             // units rotate through the slot sets
           if (!tc::mbar_wait(x2_empty + sl, ((ui / XSETS) & 1) ^ 1, abort_flag, tc::ST_TIMEOUT_EMPTY)) { ok = false; break; }
+          x2 = (x2 & ~(1u << sl)) | ((uint32_t)(ui / XSETS) & 1u) << sl;
           tc::mbar_expect_tx(x2_full + sl, RAW_BYTES);
           tc::tma_load_3d(smem + OFF_X2 + sl * RAW_BYTES, &tmX, x2_full + sl, TW * j - HALO, b0, P.D + c);
         }
       }
+      tc::drain_loads(u_full, NU, tc::ring_parities(it % NU, (it / NU) & 1));
+      tc::drain_loads(x2_full, NX2, x2);
     }
   } else if (warp == 1) {
     // ------------------------- MMA issuer -------------------------
@@ -515,16 +523,6 @@ longconv_tz_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constan
   }
 
   // ------------------------- teardown -------------------------
-  __syncthreads();
-  if (*abort_flag && threadIdx.x == 0) {
-    // give loads that were issued before the abort a bounded time to land
-    for (int s = 0; s < NST; ++s)
-      for (uint32_t i = 0; i < 4096 && !tc::mbar_try_wait(full_main + s, 0) && !tc::mbar_try_wait(full_main + s, 1); ++i) {}
-    for (int s = 0; s < NU; ++s)
-      for (uint32_t i = 0; i < 4096 && !tc::mbar_try_wait(u_full + s, 0) && !tc::mbar_try_wait(u_full + s, 1); ++i) {}
-    for (int j = 0; j < NX2; ++j)
-      for (uint32_t i = 0; i < 4096 && !tc::mbar_try_wait(x2_full + j, 0) && !tc::mbar_try_wait(x2_full + j, 1); ++i) {}
-  }
   __syncthreads();
   if (warp == 1) {
     tc::tc_fence_after();

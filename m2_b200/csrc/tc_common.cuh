@@ -93,6 +93,30 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return mbar_wait_ns(bar, parity, abort_flag, why, WAIT_LIMIT_NS);
 }
 
+// The last act of a thread that issues loads: those it has in flight land (or the limit runs out) before its role, and with it the
+// CTA, can end, also where another role gave up and nobody is going to read them.  Bit s of `parities` is the parity of the
+// phase that the last load into stage s completes, 1 where there was none (a barrier's phase before the first has parity 1).
+__device__ __forceinline__ bool drain_loads(uint64_t* full, int stages, uint32_t parities, unsigned long long limit_ns = WAIT_LIMIT_NS) {
+  const unsigned long long t0 = global_timer_ns();
+  for (int s = 0; s < stages; ++s)
+    while (!mbar_try_wait(full + s, (parities >> s) & 1u))
+      if (global_timer_ns() - t0 > limit_ns) {
+        atomicOr(&m2_dev_status_word, ST_TIMEOUT_TMA);
+        return false;
+      }
+  return true;
+}
+// `parities` of a ring whose next load would go to `stage` in a round of parity `phase`
+__device__ __forceinline__ uint32_t ring_parities(int stage, uint32_t phase) {
+  const uint32_t low = (1u << stage) - 1u;
+  return phase ? low : ~low;
+}
+// What a CTA waits whose loads signal another CTA's barriers, which it cannot poll.
+__device__ __forceinline__ void pause_ns(unsigned long long ns) {
+  const unsigned long long t0 = global_timer_ns();
+  while (global_timer_ns() - t0 < ns) {}
+}
+
 // Barrier ID of N threads that also tells whether `v` holds for all of them.  Warps of one role that wait on mbarriers one by one
 // meet here before they act on what their waits said: one may give up where the next one's wait completes, and a warp that
 // left its loop alone would leave the others in a barrier that has no limit.
