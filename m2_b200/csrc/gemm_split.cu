@@ -39,14 +39,19 @@ constexpr float HUGE_ROW = 1.2379400392853803e27f;   // 2^90
 constexpr int X_BYTES = BM * 256;          // two boxes of 32 float32 columns
 
 template <int BN> struct Geo {
-  static constexpr int STAGE = X_BYTES + BN * 256;                   // rows of x, then hi and lo of the rows of w
-  static constexpr int NST = BN == 128 ? 3 : (BN == 64 ? 4 : 5);
-  static constexpr int OFF_SCALE = NST * STAGE;                      // [SLOTS][BM] floats
+  static constexpr int W_BYTES = BN * 256;                           // hi, then lo of 64 columns of the rows of w
+  // K blocks of x and of w in shared memory: x is free when it is converted, w when it is multiplied.  The two groups of conversion
+  // warps take the K blocks in turn, so the stages of x are even in number: then a stage is always the same group's, which sees
+  // every phase of its barrier.  (A wait on a parity cannot tell a phase from the one two before.)
+  static constexpr int NX = BN == 128 ? 2 : 4, NW = BN == 128 ? 4 : 5;
+  static_assert(NX % 2 == 0, "a stage of x belongs to one group");
+  static constexpr int OFF_W = NX * X_BYTES;
+  static constexpr int OFF_SCALE = OFF_W + NW * W_BYTES;             // [SLOTS][BM] floats
   static constexpr int OFF_HUGE = OFF_SCALE + SLOTS * BM * 4;        // [SLOTS][CONV_WARPS] ints
   static constexpr int NACC = BN == 128 ? 2 : 4;                     // accumulators
   static constexpr int OFF_COLS = OFF_HUGE + SLOTS * CONV_WARPS * 4; // [2] of a tile's columns: inverse scales (of both halves of a GLU), bias
   static constexpr int OFF_BAR = OFF_COLS + 2 * 2 * BN * 4;
-  static constexpr int NBARS = 2 * NST + SLOTS + 2 * NA + 2 * NACC + 4;
+  static constexpr int NBARS = 2 * NX + 2 * NW + SLOTS + 2 * NA + 2 * NACC + 4;
   static constexpr int SMEM = OFF_BAR + NBARS * 8 + 16 + 1024;
   static constexpr uint32_t TCOLS = 512;                             // accumulators and buffers of hi and lo: 384 columns at least
   static_assert(SMEM <= 227 * 1024, "shared memory budget");
@@ -135,16 +140,18 @@ template <int BN, bool GLU>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const Params P) {
   using G = Geo<BN>;
-  constexpr int NST = G::NST, NACC = G::NACC, CPW = BN / 2;          // accumulator columns of a flush warp
+  constexpr int NX = G::NX, NW = G::NW, NACC = G::NACC, CPW = BN / 2;          // accumulator columns of a flush warp
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   float* scales = reinterpret_cast<float*>(smem + G::OFF_SCALE);
   float* cvals = reinterpret_cast<float*>(smem + G::OFF_COLS);
   int* huge = reinterpret_cast<int*>(smem + G::OFF_HUGE);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + G::OFF_BAR);
-  uint64_t* full = bars;                   // [NST] boxes have landed
-  uint64_t* empty = full + NST;            // [NST] x has been read by the converters, w by the MMAs
-  uint64_t* sfull = empty + NST;           // [SLOTS] scales of a K block are written
+  uint64_t* xfull = bars;                  // [NX] x has landed
+  uint64_t* xempty = xfull + NX;           // [NX] and has been read by the converters
+  uint64_t* wfull = xempty + NX;           // [NW] w has landed
+  uint64_t* wempty = wfull + NW;           // [NW] and has been read by the MMAs
+  uint64_t* sfull = wempty + NW;           // [SLOTS] scales of a K block are written
   uint64_t* afull = sfull + SLOTS;         // [NA] hi and lo of x are in tensor memory
   uint64_t* aempty = afull + NA;           // [NA] and have been read
   uint64_t* tfull = aempty + NA;           // [NACC] the K block's sums are complete
@@ -155,7 +162,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   const int warp = tc::uniform_warp_id(), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < NST; ++s) { tc::mbar_init(full + s, 1); tc::mbar_init(empty + s, CONV_WARPS + 1); }
+    for (int s = 0; s < NX; ++s) { tc::mbar_init(xfull + s, 1); tc::mbar_init(xempty + s, CONV_WARPS); }
+    for (int s = 0; s < NW; ++s) { tc::mbar_init(wfull + s, 1); tc::mbar_init(wempty + s, 1); }
     for (int s = 0; s < SLOTS; ++s) tc::mbar_init(sfull + s, CONV_WARPS);
     for (int b = 0; b < NA; ++b) { tc::mbar_init(afull + b, CONV_WARPS); tc::mbar_init(aempty + b, 1); }
     for (int b = 0; b < 2; ++b) { tc::mbar_init(cfull + b, 32); tc::mbar_init(cempty + b, FLUSH_WARPS); }
@@ -186,53 +194,59 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
   if (warp == 0) {
     // ---- TMA producer ----
     if (tc::elect_one()) {
-      int stage = 0; uint32_t phase = 0;
+      int xs = 0, ws = 0; uint32_t xphase = 0, wphase = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < P.total && ok; tile += gridDim.x) {
         int mt, nt, kb;
         decode(tile, mt, nt, kb);
         for (int c = 0; c < blocks; ++c) {
-          ok = tc::mbar_wait(empty + stage, phase ^ 1, abort_flag, tc::ST_TIMEOUT_EMPTY);
-          if (!ok) break;
           const bool second = GLU && c >= P.steps;
           const int b = second ? kb + P.partner : kb, s = second ? c - P.steps : c;
-          unsigned char* st = smem + stage * G::STAGE;
-          tc::mbar_expect_tx(full + stage, G::STAGE);
-          tc::tma_load_3d(st, &tmX, full + stage, s * BK, b, mt * BM);
-          tc::tma_load_3d(st + BM * 128, &tmX, full + stage, s * BK + 32, b, mt * BM);
-          tc::tma_load_2d(st + X_BYTES, &tmW, full + stage, s * 2 * BK, b * P.q + nt * BN);
-          tc::tma_load_2d(st + X_BYTES + BN * 128, &tmW, full + stage, s * 2 * BK + BK, b * P.q + nt * BN);
-          if (++stage == NST) { stage = 0; phase ^= 1; }
+          ok = tc::mbar_wait(xempty + xs, xphase ^ 1, abort_flag, tc::ST_TIMEOUT_EMPTY);
+          if (!ok) break;
+          unsigned char* sx = smem + xs * X_BYTES;
+          tc::mbar_expect_tx(xfull + xs, X_BYTES);
+          tc::tma_load_3d(sx, &tmX, xfull + xs, s * BK, b, mt * BM);
+          tc::tma_load_3d(sx + BM * 128, &tmX, xfull + xs, s * BK + 32, b, mt * BM);
+          if (++xs == NX) { xs = 0; xphase ^= 1; }
+          ok = tc::mbar_wait(wempty + ws, wphase ^ 1, abort_flag, tc::ST_TIMEOUT_EMPTY);
+          if (!ok) break;
+          unsigned char* sw = smem + G::OFF_W + ws * G::W_BYTES;
+          tc::mbar_expect_tx(wfull + ws, G::W_BYTES);
+          tc::tma_load_2d(sw, &tmW, wfull + ws, s * 2 * BK, b * P.q + nt * BN);
+          tc::tma_load_2d(sw + BN * 128, &tmW, wfull + ws, s * 2 * BK + BK, b * P.q + nt * BN);
+          if (++ws == NW) { ws = 0; wphase ^= 1; }
         }
       }
-      tc::drain_loads(full, NST, tc::ring_parities(stage, phase));
+      tc::drain_loads(xfull, NX, tc::ring_parities(xs, xphase));
+      tc::drain_loads(wfull, NW, tc::ring_parities(ws, wphase));
     }
   } else if (warp == 1) {
     // ---- MMA issue ----
     if (tc::elect_one()) {
       constexpr uint32_t idesc = tc::make_idesc(BM, BN, 0);
-      const uint64_t b_hi = tc::smem_desc_k_sw128(tc::smem_u32(smem + X_BYTES)), b_lo = tc::desc_advance(b_hi, BN * 128 >> 4);
+      const uint64_t b_hi = tc::smem_desc_k_sw128(tc::smem_u32(smem + G::OFF_W)), b_lo = tc::desc_advance(b_hi, BN * 128 >> 4);
       int stage = 0; uint32_t phase = 0, it = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < P.total && ok; tile += gridDim.x) {
         for (int c = 0; c < blocks; ++c, ++it) {
           const int buf = it % NACC, ab = it % NA;
-          ok = tc::mbar_wait(full + stage, phase, abort_flag, tc::ST_TIMEOUT_TMA) &&
+          ok = tc::mbar_wait(wfull + stage, phase, abort_flag, tc::ST_TIMEOUT_TMA) &&
                tc::mbar_wait(tempty + buf, ((it / NACC) & 1) ^ 1, abort_flag, tc::ST_TIMEOUT_MMA) &&
                tc::mbar_wait(afull + ab, (it / NA) & 1, abort_flag, tc::ST_TIMEOUT_MMA);
           if (!ok) break;
           tc::tc_fence_after();
-          const uint32_t acc = tmem + buf * BN, a = tmem_a + ab * 64, off = (uint32_t)(stage * (G::STAGE >> 4));
+          const uint32_t acc = tmem + buf * BN, a = tmem_a + ab * 64, off = (uint32_t)(stage * (G::W_BYTES >> 4));
 #pragma unroll
           for (int kk = 0; kk < BK / 16; ++kk) mma_ts(acc, a + 32 + 8 * kk, tc::desc_advance(b_hi, off + 2 * kk), idesc, kk ? 1u : 0u);
 #pragma unroll
           for (int kk = 0; kk < BK / 16; ++kk) mma_ts(acc, a + 8 * kk, tc::desc_advance(b_lo, off + 2 * kk), idesc, 1u);
 #pragma unroll
           for (int kk = 0; kk < BK / 16; ++kk) mma_ts(acc, a + 8 * kk, tc::desc_advance(b_hi, off + 2 * kk), idesc, 1u);
-          tc::mma_commit(empty + stage);
+          tc::mma_commit(wempty + stage);
           tc::mma_commit(aempty + ab);
           tc::mma_commit(tfull + buf);
-          if (++stage == NST) { stage = 0; phase ^= 1; }
+          if (++stage == NW) { stage = 0; phase ^= 1; }
         }
       }
     }
@@ -263,12 +277,12 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
     for (int tile = blockIdx.x; tile < P.total && ok; tile += gridDim.x) {
       for (int c = 0; c < blocks; ++c, ++it) {
         if ((int)(it & 1) != group) continue;
-        const uint32_t stage = it % NST;
-        ok = tc::mbar_wait(full + stage, (it / NST) & 1, abort_flag, tc::ST_TIMEOUT_TMA);
+        const uint32_t stage = it % NX;
+        ok = tc::mbar_wait(xfull + stage, (it / NX) & 1, abort_flag, tc::ST_TIMEOUT_TMA);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         const int slot = it & (SLOTS - 1);
-        const unsigned char* p0 = smem + stage * G::STAGE + r * 128;
+        const unsigned char* p0 = smem + stage * X_BYTES + r * 128;
         float4 v[16];
         float m = 0.f;
 #pragma unroll
@@ -276,13 +290,16 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
           v[j] = *reinterpret_cast<const float4*>(p0 + (j < 8 ? 0 : BM * 128) + (((j & 7) * 16) ^ sw));
           m = fmaxf(m, fmaxf(fmaxf(fabsf(v[j].x), fabsf(v[j].y)), fmaxf(fabsf(v[j].z), fabsf(v[j].w))));
         }
-        __syncwarp();
-        if (lane == 0) tc::mbar_arrive(empty + stage);
+        // The vote needs every lane's values, the store the vote: the arrival behind it finds all loads complete.  (Right behind the
+        // loads it overtook them, and the next rows landed under those that were still waiting for shared memory.)
+        const bool any = __any_sync(0xffffffffu, m >= HUGE_ROW);
+        if (lane == 0) {
+          huge[slot * CONV_WARPS + cw] = any;
+          tc::mbar_arrive(xempty + stage);
+        }
         const uint32_t ex = split_exponent(m);
         const f32x2 s = f2_splat(split_scale(ex));
         scales[slot * BM + r] = split_inverse(ex);
-        const bool any = __any_sync(0xffffffffu, m >= HUGE_ROW);
-        if (lane == 0) huge[slot * CONV_WARPS + cw] = any;
         const uint32_t ab = it % NA, ta = tq + ab * 64;
         ok = tc::mbar_wait(aempty + ab, ((it / NA) & 1) ^ 1, abort_flag, tc::ST_TIMEOUT_MMA);
         ok = __all_sync(0xffffffffu, ok);

@@ -110,3 +110,13 @@ def test_modules(B, L):
         assert not torch.equal(after, whole[0])
         mixer.in_linear.weight = torch.nn.Parameter(2 * mixer.in_linear.weight)
         assert torch.equal(mixer(u)[0], whole[0])
+
+
+@pytest.mark.parametrize("m,nb,p,q", [(2048, 4, 192, 1536), (2048, 4, 768, 192), (2048, 2, 384, 768), (100, 2, 320, 64)])
+def test_many_tiles_a_block(m, nb, p, q):
+    """Launches right behind one another, several tiles to a thread block, K blocks in odd and even numbers: the same bits every time."""
+    x, w = rand(m, nb * p), rand(nb, q, p, seed=2, scale=p ** -0.5)
+    ws = ops.split_weights(w)
+    for f in (lambda: ops.blockdiag_fwd(x, w, None, nb * p, nb * q, w_split=ws), lambda: ops.blockdiag_glu_fwd(x, w, nb * q // 2, w_split=ws)):
+        y = [f() for _ in range(30)]
+        assert all(torch.equal(t, y[0]) for t in y)
