@@ -156,12 +156,12 @@ typedef struct {
   void* out; long long out_sb, out_st, out_sc;
   int force_simt;      /* != 0: always the CUDA-core kernel (cross-checks) */
   const void* w_split; /* float32 only: NULL (one chain of float32 additions in ascending k), or `w` as m2_split_weights writes it:
-                          tensor cores on pairs of fp16 values, float32 results, where rows of x are packed in 16-byte units */
+                          tensor cores on three bf16 parts of every value, float32 results, where rows of x are packed in 16-byte units */
 } m2_linear_args;
 
 int m2_linear_fwd(const m2_linear_args* args, void* stream);
 
-/* Rows of float32 weights (rows, p), each scaled by a power of two and written as pairs of fp16 values that keep 22 bits: the
+/* Rows of float32 weights (rows, p), each value written as three bf16 parts that keep its 24 bits (down to 2^-110): the
  * operand of float32 layers on the tensor cores.  `out` has m2_split_weights_bytes(rows, p) bytes on a 16-byte boundary. */
 size_t m2_split_weights_bytes(long long rows, int p);
 int m2_split_weights(const float* w, long long rows, int p, void* out, void* stream);

@@ -1,28 +1,31 @@
-// Linear and block-diagonal layers on float32 activations as tcgen05 GEMMs over pairs of fp16 values, with float32 results.
+// Linear and block-diagonal layers on float32 activations as tcgen05 GEMMs over triples of bf16 values, with float32 results.
 //
-// Every 64 columns of a row of x are scaled by a power of two that brings the largest of them to [2^14, 2^15) and written as
-// hi + lo, two fp16 values that keep 22 bits of it; a weight row is scaled and split once as a whole.  x . w is then
-// lo.hi + hi.lo + hi.hi on the tensor cores (lo.lo is below 2^-24 of it), summed over 64 columns in tensor memory, small
-// terms first.  Each such sum is scaled back and added to a float32 register, rounded to nearest: the tensor core's own
+// Every value of x and w is written as hi + mid + lo, three bf16 values of eight bits each: rounded to nearest, they hold the 24 bits
+// of a float32 exactly (down to 2^-110, where lo leaves the range), whatever its neighbours are.  x . w is then lo.hi + hi.lo + mid.mid +
+// mid.hi + hi.mid + hi.hi on the tensor cores (mid.lo and lo.mid are at most 2^-25 of |x||w| each), summed over 64 columns in tensor
+// memory, small terms first.  Each such sum is added to a float32 register, rounded to nearest: the tensor core's own
 // accumulation drops what does not fit, always towards zero, so a chain of K / 16 of its additions would be further from the
-// exact sum than a float32 chain; four of them are nearer (N(0, 1) operands, 768 columns, relative 2-norm against 64 bits: chain
-// 5.0e-7; sums in tensor memory over 768 columns 2.6e-6, 256 8.4e-7, 128 3.8e-7, 64 1.5e-7).
+// exact sum than a float32 chain; the four of the large terms are nearer.  Relative 2-norm against 64 bits, chain / this: N(0, 1)
+// operands 128 columns 2.0e-7 / 0.8e-7, 768 5.0e-7 / 1.0e-7; of one sign 1.7e-7 / 0.9e-7, 3.7e-7 / 1.0e-7.  Results that are one large
+// product are truncated, up to 2^-23, where a chain rounds them (2.6e-8 / 9.3e-8).
+// Two fp16 values with a scale for 64 columns take half the MMAs and a sixth less time, but keep 22 bits, and fewer of what is below
+// 2^-17 of the largest beside it: with one column in 64 scaled by 2^24 in x and by 2^-24 in w the result was 1.4e-5 off (here it is the
+// same bits as without), and operands of one sign in 128 columns 2.1e-7.
 //
-// A row whose largest value is beyond 2^90 (or infinite) marks its tile, a weight row its output column; their non-finite
-// results are summed again as the ascending float32 chain of gemm_f32.cu.  NaNs stay NaNs by themselves.
+// A result that is not finite is summed again as the ascending float32 chain of gemm_f32.cu: products of infinities with the parts of
+// a value, and values that round up to an infinite hi, end here.
 //
 // Roles: warp 0 brings float32 rows of x and split rows of w to shared memory by TMA, warps 12-19 convert (a thread owns a row
-// of x; four warps take the even K blocks, four the odd ones) and leave hi and lo in tensor memory, from where the MMAs take
+// of x; four warps take the even K blocks, four the odd ones) and leave the three parts in tensor memory, from where the MMAs take
 // them as their A operand, warp 1 issues the MMAs, warps 4-11 add up.
 //
-// Bound: 64 columns of a 128 x 128 tile bring 64 KB to the SM, 1700 clocks at the 38 bytes a clock that TMA tile loads reach in every
-// GEMM here; shared memory is busy for 1150 of them (64 KB written, 32 read by the conversion, 48 by the 12 MMAs of 64 clocks).
-// Splitting x too before the launch would cost a pass and move as many bytes; converting both operands in place in shared memory
-// took 2.3 times as long there.  Few rows: the first loads and one K block after the other.
-// Measured (us, L2 flushed; the float32 chain of gemm_f32.cu first): 768 -> 2304 at 64 / 1024 / 2048 / 8192 tokens 38 / 94 / 180 /
-// 684 -> 16 / 23 / 36 / 111; 768 -> 768 37 / 57 / 87 at 64 / 1024 / 2048 -> 16 / 19 / 23; GLU 768 -> 3072 at 2048 158 -> 45; wo 88 -> 25.
-// A tile's scales and biases come through shared memory and the accumulators are several: with scalar loads in the epilogue and
-// two accumulators 8192 tokens took 137 us and the GLU 61.
+// Bound: 64 columns of a 128 x 128 tile bring 80 KB to the SM, 2150 of its 2300 clocks at the 38 bytes a clock that TMA tile loads reach
+// in every GEMM here; the 24 MMAs of 64 clocks take 1540, shared memory is busy for 1650 (80 KB written, 32 read by the conversion, 96
+// by the MMAs).  Splitting x too before the launch would cost a pass and move more bytes.  Few rows: the first loads and one K block
+// after the other.
+// Measured (us, L2 flushed; the float32 chain of gemm_f32.cu / fp16 pairs / this): 768 -> 2304 at 64 tokens 38 / 15 / 15, 1024 94 / 23 / 27,
+// 2048 180 / 35 / 41, 8192 684 / 107 / 130; 768 -> 768 at 64 37 / 15 / 14, 1024 57 / 16 / 18, 2048 87 / 23 / 25; GLU 768 -> 3072 at 2048
+// 158 / 44 / 46; wo 88 / 25 / 25.
 //
 // Computation replaced: nn.Linear of bert/src/mm/monarch_mixer_sequence_mixer.py:100-154, bert/src/mm/blockdiag_multiply.py:49-60,
 // bert/src/mm/structured_linear.py:52-70, bert/src/bert_layers.py:492-506 of the reference, float32.
@@ -33,34 +36,31 @@ namespace f32s {
 
 constexpr int BM = 128, BK = 64;
 constexpr int FLUSH0 = 4, FLUSH_WARPS = 8, CONV0 = 12, CONV_WARPS = 4, THREADS = 32 * (CONV0 + 2 * CONV_WARPS);
-constexpr int NA = 4;                      // buffers of hi and lo in tensor memory, 64 columns each
-constexpr int SLOTS = 16;                  // K blocks whose scales are kept: more than can be between a conversion and its sum
-constexpr float HUGE_ROW = 1.2379400392853803e27f;   // 2^90
+constexpr int PARTS = 3, A_COLS = PARTS * BK / 2;       // tensor-memory columns of a K block of x: hi, mid, lo, 32 each
 constexpr int X_BYTES = BM * 256;          // two boxes of 32 float32 columns
 
 template <int BN> struct Geo {
-  static constexpr int W_BYTES = BN * 256;                           // hi, then lo of 64 columns of the rows of w
+  static constexpr int W_BYTES = BN * PARTS * 128;                   // hi, mid, lo of 64 columns of the rows of w
   // K blocks of x and of w in shared memory: x is free when it is converted, w when it is multiplied.  The two groups of conversion
-  // warps take the K blocks in turn, so the stages of x are even in number: then a stage is always the same group's, which sees
-  // every phase of its barrier.  (A wait on a parity cannot tell a phase from the one two before.)
-  static constexpr int NX = BN == 128 ? 2 : 4, NW = BN == 128 ? 4 : 5;
-  static_assert(NX % 2 == 0, "a stage of x belongs to one group");
+  // warps take the K blocks in turn, so the stages of x and its buffers in tensor memory are even in number: then each is always the
+  // same group's, which sees every phase of its barrier.  (A wait on a parity cannot tell a phase from the one two before.)
+  static constexpr int NX = BN == 128 ? 2 : 4, NW = BN == 128 ? 3 : BN == 64 ? 4 : 5;
+  static constexpr int NACC = BN == 32 ? 4 : 2, NA = BN == 128 ? 2 : 4;   // accumulators, buffers of x
+  static_assert(NX % 2 == 0 && NA % 2 == 0, "a stage and a buffer of x belong to one group");
   static constexpr int OFF_W = NX * X_BYTES;
-  static constexpr int OFF_SCALE = OFF_W + NW * W_BYTES;             // [SLOTS][BM] floats
-  static constexpr int OFF_HUGE = OFF_SCALE + SLOTS * BM * 4;        // [SLOTS][CONV_WARPS] ints
-  static constexpr int NACC = BN == 128 ? 2 : 4;                     // accumulators
-  static constexpr int OFF_COLS = OFF_HUGE + SLOTS * CONV_WARPS * 4; // [2] of a tile's columns: inverse scales (of both halves of a GLU), bias
-  static constexpr int OFF_BAR = OFF_COLS + 2 * 2 * BN * 4;
-  static constexpr int NBARS = 2 * NX + 2 * NW + SLOTS + 2 * NA + 2 * NACC + 4;
+  static constexpr int OFF_COLS = OFF_W + NW * W_BYTES;              // [2] a tile's bias
+  static constexpr int OFF_BAR = OFF_COLS + 2 * BN * 4;
+  static constexpr int NBARS = 2 * NX + 2 * NW + 2 * NA + 2 * NACC + 4;
   static constexpr int SMEM = OFF_BAR + NBARS * 8 + 16 + 1024;
-  static constexpr uint32_t TCOLS = 512;                             // accumulators and buffers of hi and lo: 384 columns at least
+  static constexpr uint32_t TCOLS = 512;
+  static_assert(NACC * BN + NA * A_COLS <= (int)TCOLS && NACC * BN + NA * A_COLS > 256, "tensor memory");
   static_assert(SMEM <= 227 * 1024, "shared memory budget");
 };
 
 struct Params {
   const float* x; long long ldx;           // row t of x, block kb: x + t * ldx + kb * p
   const float* w;                          // [block][q][p]
-  const __half* ws; const float* winv;     // the same rows split, and the inverse of each row's scale
+  const __nv_bfloat16* ws;                 // the same rows split
   const float* bias;
   float* out; long long osb, ost, osc;     // token t at (t / L) * osb + (t % L) * ost
   int tokens, L, p, q, steps;
@@ -69,21 +69,22 @@ struct Params {
   int vec;                                 // 32-byte stores are legal for eight neighbouring columns
 };
 
-// the largest magnitude's biased exponent -> scale that brings it to [2^14, 2^15), and its inverse
-__device__ __forceinline__ float split_scale(uint32_t ex) { return __uint_as_float((268u - ex) << 23); }
-__device__ __forceinline__ float split_inverse(uint32_t ex) { return __uint_as_float((ex - 14u) << 23); }
-__device__ __forceinline__ uint32_t split_exponent(float m) { return max(27u, __float_as_uint(m) >> 23); }
-__device__ __forceinline__ void split_pair(float y0, float y1, uint32_t& hi, uint32_t& lo) {
-  const __half2 h = __floats2half2_rn(y0, y1);
-  const float2 hf = __half22float2(h);
-  const __half2 l = __floats2half2_rn(y0 - hf.x, y1 - hf.y);
-  hi = *reinterpret_cast<const uint32_t*>(&h);
-  lo = *reinterpret_cast<const uint32_t*>(&l);
+__device__ __forceinline__ uint32_t bf16_pair(float y0, float y1) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(y0, y1);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
+// two values as pairs of their parts; what is left after each is exact
+__device__ __forceinline__ void split_triple(float y0, float y1, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  hi = bf16_pair(y0, y1);
+  y0 -= __uint_as_float(hi << 16);
+  y1 -= __uint_as_float(hi & 0xffff0000u);
+  mid = bf16_pair(y0, y1);
+  lo = bf16_pair(y0 - __uint_as_float(mid << 16), y1 - __uint_as_float(mid & 0xffff0000u));
 }
 
-// weight rows: per 64 columns hi, then lo; zeros up to the next multiple of 64.  A warp per row, up to four matrices a launch.
+// weight rows: per 64 columns hi, mid, lo; zeros up to the next multiple of 64.  A warp per row, up to four matrices a launch.
 struct SplitJobs {
-  struct { const float* w; __half* ws; float* winv; int rows, p, steps, first; } job[4];   // first: its first block of eight rows
+  struct { const float* w; __nv_bfloat16* ws; int rows, p, steps, first, vec; } job[4];   // first: its first block of eight rows
   int n;
 };
 __global__ void __launch_bounds__(256)
@@ -92,26 +93,30 @@ split_weights_kernel(const SplitJobs J) {
   int j = 0;
   while (j + 1 < J.n && (int)blockIdx.x >= J.job[j + 1].first) ++j;
   const float* __restrict__ w = J.job[j].w;
-  __half* __restrict__ ws = J.job[j].ws;
-  float* __restrict__ winv = J.job[j].winv;
-  const int rows = J.job[j].rows, p = J.job[j].p, steps = J.job[j].steps;
+  const int rows = J.job[j].rows, p = J.job[j].p, steps = J.job[j].steps, vec = J.job[j].vec;
   const int row = (blockIdx.x - J.job[j].first) * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (row >= rows) return;
   const float* r = w + (size_t)row * p;
-  float m = 0.f;
-  for (int k = lane; k < p; k += 32) m = fmaxf(m, fabsf(r[k]));
-  for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  const uint32_t ex = split_exponent(m);
-  const float s = split_scale(ex);
-  uint32_t* o = reinterpret_cast<uint32_t*>(ws) + (size_t)row * steps * BK;
-  for (int k = 2 * lane; k < steps * BK; k += 64) {
-    uint32_t hi, lo;
-    split_pair(k < p ? r[k] * s : 0.f, k + 1 < p ? r[k + 1] * s : 0.f, hi, lo);
-    const int at = (k / BK) * BK + (k % BK) / 2;
-    o[at] = hi;
-    o[at + BK / 2] = lo;
+  __nv_bfloat16* __restrict__ o = J.job[j].ws + (size_t)row * steps * (PARTS * BK);
+#pragma unroll 4
+  for (int k = 4 * lane; k < steps * BK; k += 128) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (vec) {
+      if (k < p) v = __ldg(reinterpret_cast<const float4*>(r + k));
+    } else {
+      if (k < p) v.x = r[k];
+      if (k + 1 < p) v.y = r[k + 1];
+      if (k + 2 < p) v.z = r[k + 2];
+      if (k + 3 < p) v.w = r[k + 3];
+    }
+    uint2 hi, mid, lo;
+    split_triple(v.x, v.y, hi.x, mid.x, lo.x);
+    split_triple(v.z, v.w, hi.y, mid.y, lo.y);
+    __nv_bfloat16* d = o + (k / BK) * (PARTS * BK) + k % BK;
+    *reinterpret_cast<uint2*>(d) = hi;
+    *reinterpret_cast<uint2*>(d + BK) = mid;
+    *reinterpret_cast<uint2*>(d + 2 * BK) = lo;
   }
-  if (lane == 0) winv[row] = m >= HUGE_ROW ? __int_as_float(0x7fffffff) : split_inverse(ex);   // NaN: the column is summed again
 }
 
 // D[tmem] (+)= A[tmem] * B[smem desc]
@@ -132,7 +137,7 @@ __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.
 // the sum as the float32 kernels have it: one chain of fused multiply-adds in ascending k
 __device__ __noinline__ float chain(const float* x, const float* w, int p) {
   float s = 0.f;
-  for (int k = 0; k < p; ++k) s = fmaf(__ldg(x + k), __ldg(w + k), s);
+  for (int k = 0; k < p && s == s; ++k) s = fmaf(__ldg(x + k), __ldg(w + k), s);   // a NaN stays one
   return s;
 }
 
@@ -140,23 +145,20 @@ template <int BN, bool GLU>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const Params P) {
   using G = Geo<BN>;
-  constexpr int NX = G::NX, NW = G::NW, NACC = G::NACC, CPW = BN / 2;          // accumulator columns of a flush warp
+  constexpr int NX = G::NX, NW = G::NW, NACC = G::NACC, NA = G::NA, CPW = BN / 2;          // accumulator columns of a flush warp
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  float* scales = reinterpret_cast<float*>(smem + G::OFF_SCALE);
   float* cvals = reinterpret_cast<float*>(smem + G::OFF_COLS);
-  int* huge = reinterpret_cast<int*>(smem + G::OFF_HUGE);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + G::OFF_BAR);
   uint64_t* xfull = bars;                  // [NX] x has landed
   uint64_t* xempty = xfull + NX;           // [NX] and has been read by the converters
   uint64_t* wfull = xempty + NX;           // [NW] w has landed
   uint64_t* wempty = wfull + NW;           // [NW] and has been read by the MMAs
-  uint64_t* sfull = wempty + NW;           // [SLOTS] scales of a K block are written
-  uint64_t* afull = sfull + SLOTS;         // [NA] hi and lo of x are in tensor memory
+  uint64_t* afull = wempty + NW;           // [NA] the parts of x are in tensor memory
   uint64_t* aempty = afull + NA;           // [NA] and have been read
   uint64_t* tfull = aempty + NA;           // [NACC] the K block's sums are complete
   uint64_t* tempty = tfull + NACC;         // [NACC] the sums have been read
-  uint64_t* cfull = tempty + NACC;         // [2] a tile's column values are there
+  uint64_t* cfull = tempty + NACC;         // [2] a tile's biases are there
   uint64_t* cempty = cfull + 2;            // [2] and have been used
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + G::NBARS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -164,7 +166,6 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
   if (threadIdx.x == 0) {
     for (int s = 0; s < NX; ++s) { tc::mbar_init(xfull + s, 1); tc::mbar_init(xempty + s, CONV_WARPS); }
     for (int s = 0; s < NW; ++s) { tc::mbar_init(wfull + s, 1); tc::mbar_init(wempty + s, 1); }
-    for (int s = 0; s < SLOTS; ++s) tc::mbar_init(sfull + s, CONV_WARPS);
     for (int b = 0; b < NA; ++b) { tc::mbar_init(afull + b, CONV_WARPS); tc::mbar_init(aempty + b, 1); }
     for (int b = 0; b < 2; ++b) { tc::mbar_init(cfull + b, 32); tc::mbar_init(cempty + b, FLUSH_WARPS); }
     for (int b = 0; b < NACC; ++b) { tc::mbar_init(tfull + b, 1); tc::mbar_init(tempty + b, FLUSH_WARPS); }
@@ -180,7 +181,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
   tc::tc_fence_before();
   __syncthreads();
   tc::tc_fence_after();
-  const uint32_t tmem = *tmem_slot, tmem_a = tmem + NACC * BN;       // buffer b: hi at 64 b, lo at 64 b + 32
+  const uint32_t tmem = *tmem_slot, tmem_a = tmem + NACC * BN;       // buffer b from A_COLS b on
   pdl_wait();
 
   const int blocks = GLU ? 2 * P.steps : P.steps;    // K blocks of a tile; those of the GLU's factor follow those of its gate
@@ -213,8 +214,9 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
           if (!ok) break;
           unsigned char* sw = smem + G::OFF_W + ws * G::W_BYTES;
           tc::mbar_expect_tx(wfull + ws, G::W_BYTES);
-          tc::tma_load_2d(sw, &tmW, wfull + ws, s * 2 * BK, b * P.q + nt * BN);
-          tc::tma_load_2d(sw + BN * 128, &tmW, wfull + ws, s * 2 * BK + BK, b * P.q + nt * BN);
+#pragma unroll
+          for (int i = 0; i < PARTS; ++i)
+            tc::tma_load_2d(sw + i * BN * 128, &tmW, wfull + ws, (s * PARTS + i) * BK, b * P.q + nt * BN);
           if (++ws == NW) { ws = 0; wphase ^= 1; }
         }
       }
@@ -224,8 +226,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
   } else if (warp == 1) {
     // ---- MMA issue ----
     if (tc::elect_one()) {
-      constexpr uint32_t idesc = tc::make_idesc(BM, BN, 0);
-      const uint64_t b_hi = tc::smem_desc_k_sw128(tc::smem_u32(smem + G::OFF_W)), b_lo = tc::desc_advance(b_hi, BN * 128 >> 4);
+      constexpr uint32_t idesc = tc::make_idesc(BM, BN, 1);
+      const uint64_t w0 = tc::smem_desc_k_sw128(tc::smem_u32(smem + G::OFF_W));
       int stage = 0; uint32_t phase = 0, it = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < P.total && ok; tile += gridDim.x) {
@@ -236,13 +238,13 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
                tc::mbar_wait(afull + ab, (it / NA) & 1, abort_flag, tc::ST_TIMEOUT_MMA);
           if (!ok) break;
           tc::tc_fence_after();
-          const uint32_t acc = tmem + buf * BN, a = tmem_a + ab * 64, off = (uint32_t)(stage * (G::W_BYTES >> 4));
+          const uint32_t acc = tmem + buf * BN, a = tmem_a + ab * A_COLS, off = (uint32_t)(stage * (G::W_BYTES >> 4));
+          constexpr int PART_X[6] = {2, 0, 1, 1, 0, 0}, PART_W[6] = {0, 2, 1, 0, 1, 0};      // small terms first
 #pragma unroll
-          for (int kk = 0; kk < BK / 16; ++kk) mma_ts(acc, a + 32 + 8 * kk, tc::desc_advance(b_hi, off + 2 * kk), idesc, kk ? 1u : 0u);
+          for (int i = 0; i < 6; ++i)
 #pragma unroll
-          for (int kk = 0; kk < BK / 16; ++kk) mma_ts(acc, a + 8 * kk, tc::desc_advance(b_lo, off + 2 * kk), idesc, 1u);
-#pragma unroll
-          for (int kk = 0; kk < BK / 16; ++kk) mma_ts(acc, a + 8 * kk, tc::desc_advance(b_hi, off + 2 * kk), idesc, 1u);
+            for (int kk = 0; kk < BK / 16; ++kk)
+              mma_ts(acc, a + 32 * PART_X[i] + 8 * kk, tc::desc_advance(w0, off + PART_W[i] * (BN * 128 >> 4) + 2 * kk), idesc, i || kk ? 1u : 0u);
           tc::mma_commit(wempty + stage);
           tc::mma_commit(aempty + ab);
           tc::mma_commit(tfull + buf);
@@ -250,8 +252,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         }
       }
     }
-  } else if (warp == 2) {
-    // ---- column values of the tiles ----
+  } else if (warp == 2 && !GLU) {
+    // ---- biases of the tiles ----
     uint32_t n = 0;
     for (int tile = blockIdx.x; tile < P.total; tile += gridDim.x, ++n) {
       int mt, nt, kb;
@@ -259,13 +261,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
       bool ok = tc::mbar_wait(cempty + (n & 1), ((n >> 1) & 1) ^ 1, abort_flag, tc::ST_TIMEOUT_EMPTY);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
-      float* dst = cvals + (n & 1) * 2 * BN;
-      for (int j = lane; j < BN; j += 32) {
-        const bool in = nt * BN + j < P.q;
-        const long long c = (long long)kb * P.q + nt * BN + j;
-        dst[j] = in ? __ldg(P.winv + c) : 0.f;
-        dst[BN + j] = !in ? 0.f : GLU ? __ldg(P.winv + c + (long long)P.partner * P.q) : P.bias ? __ldg(P.bias + c) : 0.f;
-      }
+      float* dst = cvals + (n & 1) * BN;
+      for (int j = lane; j < BN; j += 32) dst[j] = P.bias && nt * BN + j < P.q ? __ldg(P.bias + (long long)kb * P.q + nt * BN + j) : 0.f;
       tc::mbar_arrive(cfull + (n & 1));
     }
   } else if (warp >= CONV0) {
@@ -281,50 +278,39 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         ok = tc::mbar_wait(xfull + stage, (it / NX) & 1, abort_flag, tc::ST_TIMEOUT_TMA);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
-        const int slot = it & (SLOTS - 1);
         const unsigned char* p0 = smem + stage * X_BYTES + r * 128;
-        float4 v[16];
-        float m = 0.f;
+        uint4 v[16];
+        uint32_t bits = 0;
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
-          v[j] = *reinterpret_cast<const float4*>(p0 + (j < 8 ? 0 : BM * 128) + (((j & 7) * 16) ^ sw));
-          m = fmaxf(m, fmaxf(fmaxf(fabsf(v[j].x), fabsf(v[j].y)), fmaxf(fabsf(v[j].z), fabsf(v[j].w))));
+          v[j] = *reinterpret_cast<const uint4*>(p0 + (j < 8 ? 0 : BM * 128) + (((j & 7) * 16) ^ sw));
+          bits |= v[j].x | v[j].y | v[j].z | v[j].w;
         }
-        // The vote needs every lane's values, the store the vote: the arrival behind it finds all loads complete.  (Right behind the
-        // loads it overtook them, and the next rows landed under those that were still waiting for shared memory.)
-        const bool any = __any_sync(0xffffffffu, m >= HUGE_ROW);
-        if (lane == 0) {
-          huge[slot * CONV_WARPS + cw] = any;
-          tc::mbar_arrive(xempty + stage);
-        }
-        const uint32_t ex = split_exponent(m);
-        const f32x2 s = f2_splat(split_scale(ex));
-        scales[slot * BM + r] = split_inverse(ex);
-        const uint32_t ab = it % NA, ta = tq + ab * 64;
+        // The vote needs every lane's values, and its result decides who arrives (either may): the arrival finds all loads complete.
+        // (Right behind the loads it overtook them, and the next rows landed under those that were still waiting for shared memory.)
+        if (lane == __any_sync(0xffffffffu, bits == 1u)) tc::mbar_arrive(xempty + stage);
+        const uint32_t ab = it % NA, ta = tq + ab * A_COLS;
         ok = tc::mbar_wait(aempty + ab, ((it / NA) & 1) ^ 1, abort_flag, tc::ST_TIMEOUT_MMA);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc::tc_fence_after();
 #pragma unroll
         for (int j = 0; j < 4; ++j) {                  // 16 columns: eight tensor-memory columns of pairs
-          uint32_t hi[8], lo[8];
+          uint32_t hi[8], mid[8], lo[8];
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const float4& q = v[4 * j + (i >> 1)];
-            float y0, y1;
-            f2_unpack(f2_mul((i & 1) ? f2_pack(q.z, q.w) : f2_pack(q.x, q.y), s), y0, y1);
-            split_pair(y0, y1, hi[i], lo[i]);
+          for (int i = 0; i < 8; i += 2) {
+            const uint4& q = v[4 * j + (i >> 1)];
+            split_triple(__uint_as_float(q.x), __uint_as_float(q.y), hi[i], mid[i], lo[i]);
+            split_triple(__uint_as_float(q.z), __uint_as_float(q.w), hi[i + 1], mid[i + 1], lo[i + 1]);
           }
           tmem_st8(ta + 8 * j, hi);
-          tmem_st8(ta + 32 + 8 * j, lo);
+          tmem_st8(ta + 32 + 8 * j, mid);
+          tmem_st8(ta + 64 + 8 * j, lo);
         }
         tmem_st_wait();
         tc::tc_fence_before();
         __syncwarp();
-        if (lane == 0) {
-          tc::mbar_arrive(afull + ab);
-          tc::mbar_arrive(sfull + slot);
-        }
+        if (lane == 0) tc::mbar_arrive(afull + ab);
       }
     }
   } else if (warp >= FLUSH0) {
@@ -337,21 +323,16 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
       int mt, nt, kb;
       decode(tile, mt, nt, kb);
       f32x2 acc[GLU ? 2 : 1][CPW / 2];
-      int big = 0;
 #pragma unroll
       for (int g = 0; g < (GLU ? 2 : 1); ++g) {
 #pragma unroll
         for (int j = 0; j < CPW / 2; ++j) acc[g][j] = 0;
         for (int c = 0; c < P.steps; ++c, ++it) {
-          const int buf = it % NACC, slot = it & (SLOTS - 1);
-          ok = ok && tc::mbar_wait(sfull + slot, (it / SLOTS) & 1, abort_flag, tc::ST_TIMEOUT_EPI) &&
-               tc::mbar_wait(tfull + buf, (it / NACC) & 1, abort_flag, tc::ST_TIMEOUT_EPI);
+          const int buf = it % NACC;
+          ok = tc::mbar_wait(tfull + buf, (it / NACC) & 1, abort_flag, tc::ST_TIMEOUT_EPI);
           ok = __all_sync(0xffffffffu, ok);
           if (!ok) break;
           tc::tc_fence_after();
-          const f32x2 rs = f2_splat(scales[slot * BM + quarter * 32 + lane]);
-          const int4 h = *reinterpret_cast<const int4*>(huge + slot * CONV_WARPS);
-          big |= h.x | h.y | h.z | h.w;
 #pragma unroll
           for (int c0 = 0; c0 < CPW; c0 += 16) {
             uint32_t t[16];
@@ -359,7 +340,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
             tc::tmem_ld_wait();
 #pragma unroll
             for (int j = 0; j < 8; ++j)
-              acc[g][c0 / 2 + j] = f2_fma(f2_pack(__uint_as_float(t[2 * j]), __uint_as_float(t[2 * j + 1])), rs, acc[g][c0 / 2 + j]);
+              acc[g][c0 / 2 + j] = f2_add(f2_pack(__uint_as_float(t[2 * j]), __uint_as_float(t[2 * j + 1])), acc[g][c0 / 2 + j]);
           }
           tc::tc_fence_before();
           __syncwarp();
@@ -367,35 +348,35 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         }
       }
       if (!ok) break;
-      ok = tc::mbar_wait(cfull + (n & 1), (n >> 1) & 1, abort_flag, tc::ST_TIMEOUT_EPI);
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
+      if (!GLU) {
+        ok = tc::mbar_wait(cfull + (n & 1), (n >> 1) & 1, abort_flag, tc::ST_TIMEOUT_EPI);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+      }
       const int t = mt * BM + quarter * 32 + lane, c0 = nt * BN + half * CPW;
       const long long base = (long long)(t / P.L) * P.osb + (long long)(t % P.L) * P.ost;
-      const float* cv = cvals + (n & 1) * 2 * BN + half * CPW;
+      const float* cv = cvals + (n & 1) * BN + half * CPW;
       float* orow = P.out + base + ((long long)kb * P.q + c0) * P.osc;
-      bool again = big != 0;
+      float bad = 0.f;                       // a NaN where a result is not finite
 #pragma unroll
       for (int j8 = 0; j8 < CPW; j8 += 8) {
         uint32_t v[8];
 #pragma unroll
         for (int j = 0; j < 8; j += 4) {
-          const float4 w = *reinterpret_cast<const float4*>(cv + j8 + j), b = *reinterpret_cast<const float4*>(cv + BN + j8 + j);
-          again |= !(w.x + w.y + w.z + w.w < 3e38f);
           float a0, a1, a2, a3;
           if (GLU) {
-            again |= !(b.x + b.y + b.z + b.w < 3e38f);
             float n0, n1, n2, n3;
-            f2_unpack(f2_mul(acc[0][(j8 + j) / 2], f2_pack(w.x, w.y)), a0, a1);
-            f2_unpack(f2_mul(acc[0][(j8 + j) / 2 + 1], f2_pack(w.z, w.w)), a2, a3);
-            f2_unpack(f2_mul(acc[GLU ? 1 : 0][(j8 + j) / 2], f2_pack(b.x, b.y)), n0, n1);
-            f2_unpack(f2_mul(acc[GLU ? 1 : 0][(j8 + j) / 2 + 1], f2_pack(b.z, b.w)), n2, n3);
+            f2_unpack(acc[0][(j8 + j) / 2], a0, a1);
+            f2_unpack(acc[0][(j8 + j) / 2 + 1], a2, a3);
+            f2_unpack(acc[GLU ? 1 : 0][(j8 + j) / 2], n0, n1);
+            f2_unpack(acc[GLU ? 1 : 0][(j8 + j) / 2 + 1], n2, n3);
             a0 = gelu_erf(a0) * n0; a1 = gelu_erf(a1) * n1; a2 = gelu_erf(a2) * n2; a3 = gelu_erf(a3) * n3;
           } else {
-            // the scale is a power of two: one rounding, as in a sum followed by the bias
-            f2_unpack(f2_fma(acc[0][(j8 + j) / 2], f2_pack(w.x, w.y), f2_pack(b.x, b.y)), a0, a1);
-            f2_unpack(f2_fma(acc[0][(j8 + j) / 2 + 1], f2_pack(w.z, w.w), f2_pack(b.z, b.w)), a2, a3);
+            const float4 b = *reinterpret_cast<const float4*>(cv + j8 + j);
+            f2_unpack(f2_add(acc[0][(j8 + j) / 2], f2_pack(b.x, b.y)), a0, a1);
+            f2_unpack(f2_add(acc[0][(j8 + j) / 2 + 1], f2_pack(b.z, b.w)), a2, a3);
           }
+          bad = fmaf(0.f, a0, fmaf(0.f, a1, fmaf(0.f, a2, fmaf(0.f, a3, bad))));
           v[j] = __float_as_uint(a0); v[j + 1] = __float_as_uint(a1); v[j + 2] = __float_as_uint(a2); v[j + 3] = __float_as_uint(a3);
         }
         if (t >= P.tokens) continue;
@@ -408,8 +389,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
         }
       }
       __syncwarp();
-      if (lane == 0) tc::mbar_arrive(cempty + (n & 1));
-      if (again && t < P.tokens) {
+      if (!GLU && lane == 0) tc::mbar_arrive(cempty + (n & 1));
+      if (bad != bad && t < P.tokens) {
         const float* xr = P.x + (long long)t * P.ldx + (long long)kb * P.p;
         for (int j = 0; j < CPW && c0 + j < P.q; ++j) {
           const long long c = (long long)kb * P.q + c0 + j;
@@ -451,9 +432,8 @@ template <int BN, bool GLU>
 static int launch(Params& P, int nblocks, cudaStream_t st) {
   CUtensorMap tmX, tmW;
   int rc;
-  const uint64_t rows = (uint64_t)nblocks * P.q, pitch = (uint64_t)P.steps * 2 * BK;
+  const uint64_t rows = (uint64_t)nblocks * P.q, pitch = (uint64_t)P.steps * PARTS * BK;
   if ((rc = make_tmap_rows(&tmX, P.x, P.p, nblocks, P.tokens, P.ldx))) return rc;
-  // 16-bit elements are moved as they are: the bf16 map serves fp16
   if ((rc = m2_make_tmap_bf16_2d(&tmW, P.ws, rows, pitch, pitch, BN))) return rc;
   P.n_tiles = (P.q + BN - 1) / BN;
   P.m_tiles = (P.tokens + BM - 1) / BM;
@@ -465,29 +445,28 @@ static int launch(Params& P, int nblocks, cudaStream_t st) {
   return m2_launch("gemm_split_kernel", (long long)P.tokens * P.p * nblocks, kern, P.total < sms ? P.total : sms, THREADS, SMEM, st, tmX, tmW, P);
 }
 
-// Columns of a tile: a K block of 64 costs some 1150 clocks at 128 columns, 750 at 64, 600 at 32.
+// Columns of a tile: a K block of 64 takes some 2300 clocks at 128 columns, 1490 at 64, 1130 at 32 (768 -> 2304, 8192 rows: 138, 169, 245 us
+// with each width alone).  Over 25 shapes from 1 to 8192 rows the width picked so is the fastest of the three or within 2 % of it.
 static int pick_bn(const Params& P, int blocks) {
   const int sms = m2_sm_count();
   auto cost = [&](int bn, double per) {
     const long long tiles = (long long)((P.tokens + BM - 1) / BM) * ((P.q + bn - 1) / bn) * blocks;
     return (double)((tiles + sms - 1) / sms) * P.steps * per;
   };
-  const double c128 = cost(128, 1150), c64 = cost(64, 750), c32 = cost(32, 600);
+  const double c128 = cost(128, 2300), c64 = cost(64, 1490), c32 = cost(32, 1130);
   return c128 <= c64 && c128 <= c32 ? 128 : (c64 <= c32 ? 64 : 32);
 }
 
-// Below 128 products a chain is about as exact (68 columns: 1.3e-7 of the result both) and as fast (36 columns, 100 rows: 10.3 us
-// both).
+// Below 128 products a chain is about as exact (68 columns: 1.3e-7 of the result) and as fast (36 columns, 100 rows: 10.3 us both).
 static bool columns_ok(int p) { return p >= 2 * BK && p % 4 == 0; }
 // What the TMA loads need: rows that start on 16-byte boundaries; `ws` as m2_split_weights writes it.
 static bool rows_ok(const void* x, long long ld, const void* ws, int p) {
   return ws && columns_ok(p) && ld % 4 == 0 && m2_aligned(x, 16) && m2_aligned(ws, 16);
 }
-static size_t split_halves(long long rows, int p) { return (size_t)rows * ((p + BK - 1) / BK) * 2 * BK; }
-static void set_weights(Params& P, const void* w, const void* ws, long long rows) {
+static size_t split_halves(long long rows, int p) { return (size_t)rows * ((p + BK - 1) / BK) * PARTS * BK; }
+static void set_weights(Params& P, const void* w, const void* ws) {
   P.w = (const float*)w;
-  P.ws = (const __half*)ws;
-  P.winv = reinterpret_cast<const float*>(P.ws + split_halves(rows, P.p));
+  P.ws = (const __nv_bfloat16*)ws;
   P.steps = (P.p + BK - 1) / BK;
 }
 
@@ -511,7 +490,7 @@ int linear_split_launch(const m2_linear_args* a, cudaStream_t st) {
   P.bias = a->bias;
   P.out = (float*)a->out; P.osb = a->out_sb; P.ost = a->out_st; P.osc = a->out_sc;
   P.tokens = a->batch * a->seq_len; P.L = a->seq_len; P.p = a->in_features; P.q = a->out_features;
-  f32s::set_weights(P, a->w, a->w_split, P.q);
+  f32s::set_weights(P, a->w, a->w_split);
   P.vec = a->out_sc == 1 && m2_aligned(a->out, 32) && a->out_st % 8 == 0 && (a->batch == 1 || a->out_sb % 8 == 0);
   return f32s::run(P, 1, st);
 }
@@ -527,7 +506,7 @@ int blockdiag_split_launch(const m2_blockdiag_args* a, cudaStream_t st) {
   P.bias = a->bias;
   P.out = (float*)a->out; P.ost = a->ldo; P.osc = 1;
   P.tokens = P.L = a->m; P.p = a->p; P.q = a->q;
-  f32s::set_weights(P, a->w, a->w_split, (long long)a->nblocks * a->q);
+  f32s::set_weights(P, a->w, a->w_split);
   P.vec = m2_aligned(a->out, 32) && a->ldo % 8 == 0 && a->q % 8 == 0;
   return f32s::run(P, a->nblocks, st);
 }
@@ -542,7 +521,7 @@ int glu_split_launch(const m2_glu_args* a, cudaStream_t st) {
   P.out = (float*)a->h; P.ost = a->ldh; P.osc = 1;
   P.tokens = P.L = a->m; P.p = a->d_model / a->nblocks; P.q = 2 * a->inter / a->nblocks;
   P.partner = a->nblocks / 2;
-  f32s::set_weights(P, a->wg, a->wg_split, (long long)a->nblocks * P.q);
+  f32s::set_weights(P, a->wg, a->wg_split);
   P.vec = m2_aligned(a->h, 32) && a->ldh % 8 == 0 && P.q % 8 == 0;
   return f32s::launch<64, true>(P, a->nblocks, st);
 }
@@ -558,9 +537,8 @@ static int split_weights_launch(const WeightRows* rows, int n, long long element
     M2_REQUIRE(r.rows > 0 && r.rows < (1LL << 31) - 8 && r.p > 0, M2_ERR_ARG, "m2_split_weights: bad sizes rows=%lld p=%d", r.rows, r.p);
     M2_REQUIRE(r.w && r.out, M2_ERR_ARG, "m2_split_weights: NULL pointer");
     M2_REQUIRE(m2_aligned(r.out, 16), M2_ERR_ALIGN, "m2_split_weights: out must be 16-byte aligned");
-    __half* ws = static_cast<__half*>(r.out);
-    J.job[i] = {static_cast<const float*>(r.w), ws, reinterpret_cast<float*>(ws + split_halves(r.rows, r.p)), (int)r.rows, r.p,
-                (r.p + BK - 1) / BK, (int)blocks};
+    J.job[i] = {static_cast<const float*>(r.w), static_cast<__nv_bfloat16*>(r.out), (int)r.rows, r.p, (r.p + BK - 1) / BK, (int)blocks,
+                r.p % 4 == 0 && m2_aligned(r.w, 16)};
     blocks += (r.rows + 7) / 8;
   }
   M2_REQUIRE(blocks < (1LL << 31), M2_ERR_UNSUPPORTED, "m2_split_weights: too many rows");
@@ -572,7 +550,7 @@ static int split_weights_launch(const WeightRows* rows, int n, long long element
 
 extern "C" size_t m2_split_weights_bytes(long long rows, int p) {
   if (rows <= 0 || p <= 0) return 0;
-  return m2::f32s::split_halves(rows, p) * 2 + (size_t)rows * 4;
+  return m2::f32s::split_halves(rows, p) * 2;
 }
 
 extern "C" int m2_split_weights_used(int p) { return m2::f32s::columns_ok(p); }

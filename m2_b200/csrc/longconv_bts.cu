@@ -103,9 +103,20 @@ taps_f32_kernel(const float* __restrict__ kfilt, float* __restrict__ taps, int D
 
 template <int ID, int N> __device__ __forceinline__ void group_sync() { asm volatile("barrier.cta.sync %0, %1;" ::"n"(ID), "n"(N) : "memory"); }
 
+// the largest magnitude's biased exponent -> scale that brings it to [2^14, 2^15), and its inverse
+__device__ __forceinline__ float split_scale(uint32_t ex) { return __uint_as_float((268u - ex) << 23); }
+__device__ __forceinline__ float split_inverse(uint32_t ex) { return __uint_as_float((ex - 14u) << 23); }
+__device__ __forceinline__ uint32_t split_exponent(float m) { return max(27u, __float_as_uint(m) >> 23); }
+__device__ __forceinline__ void split_pair(float y0, float y1, uint32_t& hi, uint32_t& lo) {
+  const __half2 h = __floats2half2_rn(y0, y1);
+  const float2 hf = __half22float2(h);
+  const __half2 l = __floats2half2_rn(y0 - hf.x, y1 - hf.y);
+  hi = *reinterpret_cast<const uint32_t*>(&h);
+  lo = *reinterpret_cast<const uint32_t*>(&l);
+}
 // scale of a row whose largest magnitude is m: NaN (and with it the whole row) where m is not finite
-__device__ __forceinline__ float row_scale(float m) { return m <= 3.402823466e38f ? f32s::split_scale(f32s::split_exponent(m)) : __int_as_float(0x7fffffff); }
-__device__ __forceinline__ float row_inverse(float m) { return m <= 3.402823466e38f ? f32s::split_inverse(f32s::split_exponent(m)) : __int_as_float(0x7fffffff); }
+__device__ __forceinline__ float row_scale(float m) { return m <= 3.402823466e38f ? split_scale(split_exponent(m)) : __int_as_float(0x7fffffff); }
+__device__ __forceinline__ float row_inverse(float m) { return m <= 3.402823466e38f ? split_inverse(split_exponent(m)) : __int_as_float(0x7fffffff); }
 
 __global__ void __launch_bounds__(THREADS, 1)
 longconv_bts_kernel(const Params P) {
@@ -255,7 +266,7 @@ longconv_bts_kernel(const Params P) {
         for (uint32_t i = 2 * bt; i < TB / 2; i += 2 * 32 * BUILD_WARPS) {
           uint32_t t0, t1, hi, lo;
           asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(t0), "=r"(t1) : "r"(T + 4 * i));
-          f32s::split_pair((i == 128u * NB ? h0 : __uint_as_float(t0)) * sc, __uint_as_float(t1) * sc, hi, lo);   // 128 NB is even
+          split_pair((i == 128u * NB ? h0 : __uint_as_float(t0)) * sc, __uint_as_float(t1) * sc, hi, lo);   // 128 NB is even
           asm volatile("st.shared.b32 [%0], %1;" ::"r"(tb + 2 * i), "r"(hi) : "memory");
           asm volatile("st.shared.b32 [%0], %1;" ::"r"(tb + TB + 2 * i), "r"(lo) : "memory");
         }
@@ -462,7 +473,7 @@ longconv_bts_kernel(const Params P) {
           const uint32_t w[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
           uint32_t hi[4], lo[4];
 #pragma unroll
-          for (int j = 0; j < 4; ++j) f32s::split_pair(__uint_as_float(w[2 * j]) * sc, __uint_as_float(w[2 * j + 1]) * sc, hi[j], lo[j]);
+          for (int j = 0; j < 4; ++j) split_pair(__uint_as_float(w[2 * j]) * sc, __uint_as_float(w[2 * j + 1]) * sc, hi[j], lo[j]);
           sts128(op + it * 128, hi[0], hi[1], hi[2], hi[3]);
           sts128(op + it * 128 + REG, lo[0], lo[1], lo[2], lo[3]);
         }

@@ -120,3 +120,51 @@ def test_many_tiles_a_block(m, nb, p, q):
     for f in (lambda: ops.blockdiag_fwd(x, w, None, nb * p, nb * q, w_split=ws), lambda: ops.blockdiag_glu_fwd(x, w, nb * q // 2, w_split=ws)):
         y = [f() for _ in range(30)]
         assert all(torch.equal(t, y[0]) for t in y)
+
+
+@pytest.mark.parametrize("T,K,N", [(1, 128, 8), (130, 132, 65), (300, 768, 2304), (2048, 1536, 768)])
+def test_values_beside_one_another_of_any_size(T, K, N):
+    """Columns of x times a power of two and the same columns of w by its inverse: every product is the same, and so is every bit."""
+    x, w = rand(1, T, K), rand(N, K, seed=2)
+    y = ops.linear_fwd(x, w, None, w_split=ops.split_weights(w))
+    for spread in (12, 24, 40):
+        e = torch.randint(-spread, spread + 1, (K,), generator=torch.Generator().manual_seed(spread)).to(DEV)
+        xs, ws = torch.ldexp(x, e), torch.ldexp(w, -e)
+        assert torch.equal(ops.linear_fwd(xs, ws, None, w_split=ops.split_weights(ws)), y)
+    g, h = rand(T, 4 * K), rand(4, 2 * K, K, seed=2, scale=K ** -0.5)
+    e = torch.randint(-40, 41, (4, K), generator=torch.Generator().manual_seed(5)).to(DEV)
+    gs, hs = torch.ldexp(g.view(T, 4, K), e).view(T, 4 * K), torch.ldexp(h, -e[:, None])
+    assert torch.equal(ops.blockdiag_glu_fwd(gs, hs, 4 * K, w_split=ops.split_weights(hs)),
+                       ops.blockdiag_glu_fwd(g, h, 4 * K, w_split=ops.split_weights(h)))
+
+
+# Operands of one sign: every truncation goes the same way, 2^-23 of a quarter, a half, three quarters and all of the sum of 64
+# products, what the small terms and the additions in float32 add is below 1.5 * 2^-23 together.
+@pytest.mark.parametrize("K", [128, 768, 1536])
+def test_one_sign(K):
+    x, w = rand(1, 256, K).abs(), rand(256, K, seed=2).abs()
+    ref = F.linear(x.double(), w.double())
+    assert error(ops.linear_fwd(x, w, None, w_split=ops.split_weights(w)), ref) < 2 ** -21
+
+
+def test_the_largest_values():
+    """Finite values that bf16 rounds to infinity, sums that overflow on the way: the float32 chain's result."""
+    x, w = rand(1, 200, 256), rand(136, 256, seed=2)
+    x[0, 3, 5], x[0, 150, 70], w[7, 9], w[130, 200] = 3.4028234e38, -3.4e38, 3.4028e38, -3.401e38
+    x[0, 9], w[9] = x[0, 9] * 1e19, w[9] * 1e19
+    for wz in (w, torch.zeros_like(w)):
+        y, ref = ops.linear_fwd(x, wz, None, w_split=ops.split_weights(wz)), ops.linear_fwd(x, wz, None)
+        assert torch.equal(torch.isnan(y), torch.isnan(ref)) and torch.equal(torch.isinf(y), torch.isinf(ref))
+        for rows in ((3,), (150,)):
+            assert torch.equal(y[0, rows], ref[0, rows])
+        assert torch.equal(y[..., (7, 130)], ref[..., (7, 130)])
+
+
+def test_calls_in_one_launch_are_planned():
+    """What test_modules compares as one native call did run as one."""
+    from m2_b200 import BertGatedLinearUnitMLP
+    mlp = BertGatedLinearUnitMLP(Cfg(hidden_size=256, intermediate_size=512, monarch_mlp_nblocks=4, layer_norm_eps=1e-12, hidden_dropout_prob=0.0)).eval().to(DEV)
+    mixer, _ = build_mixer(dict(C.CASES["mixer_small"], L=40, l_max=40, D=256, B=2, order=32, residual=True, seed=7), DEV)
+    with torch.no_grad():
+        mlp(rand(2, 40, 256)), mixer(rand(2, 40, 256))
+    assert mlp._plans.plans and mixer._plans.plans
