@@ -13,7 +13,8 @@
 // same bits as without), and operands of one sign in 128 columns 2.1e-7.
 //
 // A result that is not finite is summed again as the ascending float32 chain of gemm_f32.cu: products of infinities with the parts of
-// a value, and values that round up to an infinite hi, end here.
+// a value, and values that round up to an infinite hi, end here.  So is one below 2^-100 that is not zero, as rows of such values have
+// lost parts; beyond that a part below 2^-133 is missed only where its partner in the product is beyond 2^100 or so.
 //
 // Roles: warp 0 brings float32 rows of x and split rows of w to shared memory by TMA, warps 12-19 convert (a thread owns a row
 // of x; four warps take the even K blocks, four the odd ones) and leave the three parts in tensor memory, from where the MMAs take
@@ -37,6 +38,7 @@ namespace f32s {
 constexpr int BM = 128, BK = 64;
 constexpr int FLUSH0 = 4, FLUSH_WARPS = 8, CONV0 = 12, CONV_WARPS = 4, THREADS = 32 * (CONV0 + 2 * CONV_WARPS);
 constexpr int PARTS = 3, A_COLS = PARTS * BK / 2;       // tensor-memory columns of a K block of x: hi, mid, lo, 32 each
+constexpr uint32_t TINY = 27u << 23;       // 2^-100
 constexpr int X_BYTES = BM * 256;          // two boxes of 32 float32 columns
 
 template <int BN> struct Geo {
@@ -358,6 +360,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
       const float* cv = cvals + (n & 1) * BN + half * CPW;
       float* orow = P.out + base + ((long long)kb * P.q + c0) * P.osc;
       float bad = 0.f;                       // a NaN where a result is not finite
+      uint32_t least = ~0u;                  // twice the smallest result's bits but its sign, less one: zeros are the largest
 #pragma unroll
       for (int j8 = 0; j8 < CPW; j8 += 8) {
         uint32_t v[8];
@@ -377,6 +380,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
             f2_unpack(f2_add(acc[0][(j8 + j) / 2 + 1], f2_pack(b.z, b.w)), a2, a3);
           }
           bad = fmaf(0.f, a0, fmaf(0.f, a1, fmaf(0.f, a2, fmaf(0.f, a3, bad))));
+          least = min(min(least, 2 * __float_as_uint(a0) - 1), min(2 * __float_as_uint(a1) - 1, min(2 * __float_as_uint(a2) - 1, 2 * __float_as_uint(a3) - 1)));
           v[j] = __float_as_uint(a0); v[j + 1] = __float_as_uint(a1); v[j + 2] = __float_as_uint(a2); v[j + 3] = __float_as_uint(a3);
         }
         if (t >= P.tokens) continue;
@@ -390,12 +394,13 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant
       }
       __syncwarp();
       if (!GLU && lane == 0) tc::mbar_arrive(cempty + (n & 1));
-      if (bad != bad && t < P.tokens) {
+      if ((bad != bad || least < 2 * TINY - 1) && t < P.tokens) {
         const float* xr = P.x + (long long)t * P.ldx + (long long)kb * P.p;
         for (int j = 0; j < CPW && c0 + j < P.q; ++j) {
           const long long c = (long long)kb * P.q + c0 + j;
           float* po = P.out + base + c * P.osc;
-          if (fabsf(*po) <= 3.402823466e38f) continue;
+          const float size = fabsf(*po);
+          if (size == 0.f || (size >= __uint_as_float(TINY) && size <= 3.402823466e38f)) continue;
           float v = chain(xr, P.w + c * P.p, P.p);
           if (GLU) v = gelu_erf(v) * chain(xr + (long long)P.partner * P.p, P.w + (c + (long long)P.partner * P.q) * P.p, P.p);
           else if (P.bias) v += __ldg(P.bias + c);

@@ -168,3 +168,18 @@ def test_calls_in_one_launch_are_planned():
     with torch.no_grad():
         mlp(rand(2, 40, 256)), mixer(rand(2, 40, 256))
     assert mlp._plans.plans and mixer._plans.plans
+
+
+@pytest.mark.parametrize("exponent", [-99, -108, -118, -124])
+def test_the_smallest_values(exponent):
+    """Parts below the range of bf16: results below 2^-100 are the float32 chain's, those above keep its accuracy; zeros stay zeros."""
+    x, w, g = rand(1, 200, 256), rand(136, 256, seed=2), rand(4, 128, 256, seed=3)
+    x[0, 40] = 0.0
+    xs = x * 2.0 ** exponent
+    y, ref = ops.linear_fwd(xs, w, None, w_split=ops.split_weights(w)), ops.linear_fwd(xs, w, None)
+    small = y.abs() < 2.0 ** -100
+    assert torch.equal(y[small], ref[small]) and small[0, 40].all() and (small.all() or exponent > -108)
+    assert error(y * 2.0 ** 90, F.linear(xs.double() * 2.0 ** 90, w.double())) < 2 ** -24 * (256 / 3) ** 0.5     # a chain of 256 products
+    if exponent < -110:                              # every result is that small: sums of 256 products below 2^-110
+        h = rand(200, 1024, seed=4) * 2.0 ** exponent
+        assert torch.equal(ops.blockdiag_fwd(h, g, None, 1024, 512, w_split=ops.split_weights(g)), ops.blockdiag_fwd(h, g, None, 1024, 512))
